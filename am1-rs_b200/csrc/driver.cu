@@ -811,7 +811,7 @@ int build_batch(const am1gpu_molecule* in, const am1gpu_options& o, std::vector<
             dq_bytes += p.nch * (2LL * kOzPlanes * p.nao * oz_ldq(p.nao) + 256);
         }
     }
-    const int sp2_nblk = std::max(1, std::min(32, (maxn + 7) / 8));
+    const int sp2_nblk = sp2_init_blocks(maxn), dens_nblk = dens_blocks(maxn);
     // ---- staged (host -> device) region layout
     size_t st = 0;
     auto take = [](size_t& cur, size_t bytes) {
@@ -861,7 +861,7 @@ int build_batch(const am1gpu_molecule* in, const am1gpu_options& o, std::vector<
         const long long tn = (p.nao + 63) / 64;
         const long long sp2part = 2 * std::max<long long>(sp2_nblk, tn * (tn + 1) / 2);
         const long long cpart = CP_N * tn * (tn + 1) / 2;
-        misc += p.nch * (5LL * p.nao + p.npad + (long long)nblk * (RED_N + 1) + sp2part + cpart + 4 + 128);
+        misc += p.nch * (5LL * p.nao + p.npad + (long long)nblk * RED_N + dens_nblk + sp2part + cpart + 4 + 128);
     }
     const size_t o_misc = take(dv, sizeof(double) * misc);
     const size_t o_colid = take(dv, sizeof(int) * (size_t)(nch_total * (b.maxn + 64)));
@@ -1058,7 +1058,7 @@ int build_batch(const am1gpu_molecule* in, const am1gpu_options& o, std::vector<
             cj.red = d_misc + mi_off;
             mi_off += (long long)nblk * RED_N;
             cj.red2 = d_misc + mi_off;
-            mi_off += nblk;
+            mi_off += dens_nblk;
             cj.ntiles = (int)(tn_ * (tn_ + 1) / 2);
             cj.cpart = d_misc + mi_off;
             mi_off += (long long)CP_N * cj.ntiles;
@@ -1334,7 +1334,7 @@ int launch_core(Batch& b, Mem* ws, const DevElem* dp, Run* run) {
         ++k;
     }
     if (b.natoms > 0) {
-        k_core_diag<<<cdiv(b.natoms, 128), 128, 0, s>>>(b.d_mols, b.d_atom_mol, b.natoms, dp, b.d_atom_z, b.d_wstore, b.d_arena);
+        k_core_diag<<<cdiv((long long)b.natoms * CORE_DIAG_LANES, 128), 128, 0, s>>>(b.d_mols, b.d_atom_mol, b.natoms, dp, b.d_atom_z, b.d_wstore, b.d_arena);
         ++k;
     }
     k_core_energy<<<b.nmol, 256, 0, s>>>(b.d_mols, b.d_ecc, b.d_st);
@@ -1537,7 +1537,7 @@ int enq_head(IterEnq& e, bool lowp_left) {
     k_post_fock<<<dim3(e.nblk, e.njobs), 256, 0, s>>>(b.d_jobs, b.d_mols, b.d_st, e.nblk, 0, 0);
     run.launched(AM1GPU_PHASE_COMMUTATOR, 2);
     if ((rc = run.end(AM1GPU_PHASE_COMMUTATOR, e.ph)) || (rc = run.begin(&e.ph))) return rc;
-    k_diis_solve<<<cdiv(b.nmol, 64), 64, 0, s>>>(b.d_mols, b.d_jobs, b.d_job0, b.nmol, b.d_st, b.d_status, e.nblk, e.prm);
+    k_diis_solve<<<cdiv(b.nmol, SCF_MOL_WARPS), 32 * SCF_MOL_WARPS, 0, s>>>(b.d_mols, b.d_jobs, b.d_job0, b.nmol, b.d_st, b.d_status, e.nblk, e.prm);
     k_combine<<<dim3(e.rowblk, e.njobs), 256, 0, s>>>(b.d_jobs, b.d_st, 0);
     run.launched(AM1GPU_PHASE_ACCEL, 2);
     if ((rc = run.end(AM1GPU_PHASE_ACCEL, e.ph)) || (rc = run.begin(&e.ph))) return rc;
@@ -1546,7 +1546,7 @@ int enq_head(IterEnq& e, bool lowp_left) {
         k_sp2_bounds<<<e.njobs, 512, 3 * sizeof(double) * b.maxn, s>>>(b.d_sp2, b.d_st);
         if ((rc = launch_big_bounds(b, s))) return rc;
         k_sp2_init<<<dim3(b.sp2_nblk, e.njobs), 256, 0, s>>>(b.d_sp2, b.d_sp2_state, b.d_st, b.sp2_nblk);
-        k_sp2_start<<<cdiv(e.njobs, 128), 128, 0, s>>>(b.d_sp2, b.d_sp2_state, b.d_st, e.njobs, b.sp2_nblk);
+        k_sp2_start<<<cdiv(e.njobs, SP2_UPDATE_WARPS), 32 * SP2_UPDATE_WARPS, 0, s>>>(b.d_sp2, b.d_sp2_state, b.d_st, e.njobs, b.sp2_nblk);
         CK(cudaMemsetAsync(b.d_need_eigen, 0, sizeof(int) * b.nmol, s));
         run.launched(AM1GPU_PHASE_EIGEN,
                      3 + big_launches(big_split((int)b.sp2_big.size(), [&](int i) { return b.jobs[b.sp2_big[i]].n; }),
@@ -1560,7 +1560,7 @@ int enq_head(IterEnq& e, bool lowp_left) {
 // while any molecule may be in its TF32 phase), then the trace bookkeeping.  zero_count: clear the
 // count of channels still purifying first (the captured loop's condition kernel clears it instead).
 // cond (captured solve only): the update also takes the loop's decision on that handle
-// (k_sp2_update_cond, batches of at most SP2_UPDATE_ONE channels), so no k_sp2_cond follows.
+// (k_sp2_update_cond).
 int enq_step(IterEnq& e, int sp2_max, bool lowp_left, bool zero_count, const cudaGraphConditionalHandle* cond = nullptr) {
     Batch& b = e.b;
     const cudaStream_t s = e.s;
@@ -1600,10 +1600,12 @@ int enq_step(IterEnq& e, int sp2_max, bool lowp_left, bool zero_count, const cud
     run.launched(AM1GPU_PHASE_DENSITY_CORE, nl);
     if ((rc = run.end(AM1GPU_PHASE_DENSITY_CORE, pc))) return rc;
     if (cond) {
-        k_sp2_update_cond<<<1, SP2_UPDATE_ONE, 0, s>>>(b.d_sp2, b.d_sp2_state, e.njobs, sp2_max, b.d_work, *cond, b.d_loop);
+        k_sp2_update_cond<<<cdiv(e.njobs, SP2_UPDATE_WARPS), 32 * SP2_UPDATE_WARPS, 0, s>>>(b.d_sp2, b.d_sp2_state, e.njobs, sp2_max,
+                                                                                           b.d_work, *cond, b.d_loop);
     } else {
         if (zero_count) CK(cudaMemsetAsync(b.d_sp2_active, 0, sizeof(int), s));
-        k_sp2_update<<<cdiv(e.njobs, 128), 128, 0, s>>>(b.d_sp2, b.d_sp2_state, e.njobs, sp2_max, b.d_sp2_active, b.d_work);
+        k_sp2_update<<<cdiv(e.njobs, SP2_UPDATE_WARPS), 32 * SP2_UPDATE_WARPS, 0, s>>>(b.d_sp2, b.d_sp2_state, e.njobs, sp2_max,
+                                                                                      b.d_sp2_active, b.d_work);
     }
     run.launched(AM1GPU_PHASE_EIGEN);
     CK(cudaGetLastError());
@@ -1669,8 +1671,8 @@ int enq_tail_rest(IterEnq& e) {
     Run& run = *e.run;
     int rc;
     if (density_mode() == 0 && ((rc = run.end(AM1GPU_PHASE_EIGEN, e.ph)) || (rc = run.begin(&e.ph)))) return rc;
-    k_density_post<<<dim3(e.nblk, e.njobs), 256, 0, s>>>(b.d_jobs, b.d_st, e.nblk);
-    k_converge<<<cdiv(b.nmol, 128), 128, 0, s>>>(b.d_mols, b.d_jobs, b.d_job0, b.nmol, b.d_st, b.d_status, e.nblk, e.prm,
+    k_density_post<<<dim3(dens_blocks(b.maxn), e.njobs), 256, 0, s>>>(b.d_jobs, b.d_st, e.nblk);
+    k_converge<<<cdiv(b.nmol, SCF_MOL_WARPS), 32 * SCF_MOL_WARPS, 0, s>>>(b.d_mols, b.d_jobs, b.d_job0, b.nmol, b.d_st, b.d_status, e.nblk, e.prm,
                                                  b.d_active);
     run.launched(AM1GPU_PHASE_DENSITY, 2);
     if ((rc = run.end(AM1GPU_PHASE_DENSITY, e.ph))) return rc;
@@ -1745,10 +1747,9 @@ int add_if(cudaGraph_t g, cudaGraphNode_t dep, cudaGraphConditionalHandle h, cud
 }
 
 // The SCF loop of run_device as one graph launch:
-//   k_scf_arm -> WHILE(scf) { head -> k_sp2_arm -> WHILE(sp2) { step -> k_sp2_cond } -> tail -> k_scf_cond }
-// (for batches of at most SP2_UPDATE_ONE channels the step's update kernel sets the purification
-// loop's condition itself, k_sp2_update_cond, in place of k_sp2_update + k_sp2_cond) and, in a graph
-// kept for a resident batch's later runs, the tail split as
+//   k_scf_arm -> WHILE(scf) { head -> k_sp2_arm -> WHILE(sp2) { step } -> tail -> k_scf_cond }
+// (the step's update kernel sets the purification loop's condition itself, k_sp2_update_cond) and, in a
+// graph kept for a resident batch's later runs, the tail split as
 //   finish -> k_stall_arm -> IF(stall) { stalled-purification eigensolver } -> rest -> k_scf_cond.
 // The kernels are the eager loop's, in the same order; only the loop decisions moved to the device
 // (k_graph.cu), and the eigensolver kernels for stalled purifications, which change nothing in an
@@ -1798,22 +1799,18 @@ int scf_loop_graph(IterEnq& e, const am1gpu_options& o, bool* launched) {
     if ((rc = capture_into(cs, body, nullptr, 0, &head, [&]() -> int {
              int r = enq_head(ce, false);
              if (r) return r;
-             k_sp2_arm<<<1, 32, 0, cs>>>(h_sp2, b.d_loop, b.d_sp2_active);
+             k_sp2_arm<<<1, 32, 0, cs>>>(h_sp2, b.d_loop);
              return AM1GPU_OK;
          })))
         return rc;
     const int64_t per_head = cnt.kernel_launches - head0 + 1;
     if ((rc = add_while(body, head, h_sp2, &w_sp2, &body2))) return rc;
     const int64_t step0 = cnt.kernel_launches;
-    const bool fused = e.njobs <= SP2_UPDATE_ONE;  // the update takes the loop's decision itself
     if ((rc = capture_into(cs, body2, nullptr, 0, &step, [&]() -> int {
-             int r = enq_step(ce, sp2_max, false, false, fused ? &h_sp2 : nullptr);
-             if (r) return r;
-             if (!fused) k_sp2_cond<<<1, 32, 0, cs>>>(h_sp2, b.d_loop, b.d_sp2_active, sp2_max);
-             return AM1GPU_OK;
+             return enq_step(ce, sp2_max, false, false, &h_sp2);  // its update takes the loop's decision
          })))
         return rc;
-    const int64_t per_step = cnt.kernel_launches - step0 + (fused ? 0 : 1);
+    const int64_t per_step = cnt.kernel_launches - step0;
     const int64_t tail0 = cnt.kernel_launches;
     int64_t per_stall = 0, per_tail = 0;
     if (b.graph_cacheable) {
@@ -1899,7 +1896,7 @@ int run_device(Batch& b, Mem& mem, const DevElem* dp, const am1gpu_options& o, a
     CK(cudaGetLastError());
     if ((rc = run.end(AM1GPU_PHASE_CORE, ph))) return rc;
     ScfParams prm{o.max_scf, o.use_diis, o.accelerator, o.e_tol, o.p_tol, o.adiis_switch, lowp_switch(), lowp_max_iter()};
-    IterEnq e{b, ws, s, dp, prm, b.nblk, std::max(1, std::min(64, (b.maxn + 7) / 8)), njobs, &run, 0};
+    IterEnq e{b, ws, s, dp, prm, b.nblk, std::max(1, std::min(512, (b.maxn + 7) / 8)), njobs, &run, 0};
     int done = 0;
     bool graph = graph_ok(b, o, run.timed);
     if (graph) {
@@ -1942,13 +1939,13 @@ int run_device(Batch& b, Mem& mem, const DevElem* dp, const am1gpu_options& o, a
     if ((rc = run.begin(&ph))) return rc;
     k_fock<<<cdiv(b.natoms, 8), 256, 0, s>>>(b.d_mols, b.d_atom_mol, b.natoms, dp, b.d_atom_z, b.d_wstore, b.d_arena, b.d_st, 1);
     k_post_fock<<<dim3(nblk, njobs), 256, 0, s>>>(b.d_jobs, b.d_mols, b.d_st, nblk, 1, 1);
-    k_final_energy<<<cdiv(b.nmol, 128), 128, 0, s>>>(b.d_mols, b.d_jobs, b.d_job0, b.nmol, b.d_st, nblk);
+    k_final_energy<<<cdiv(b.nmol, SCF_MOL_WARPS), 32 * SCF_MOL_WARPS, 0, s>>>(b.d_mols, b.d_jobs, b.d_job0, b.nmol, b.d_st, nblk);
     // eigenvalues of the last F* (mo_energies, HOMO/LUMO): tridiagonalisation + bisection
     if ((rc = launch_tridiag(b, ws))) return rc;
     int64_t big_tri_launches = 0;
     if ((rc = launch_big_tridiag(b, s, &big_tri_launches))) return rc;
     bisect_launch(b.d_tri, njobs, b.maxn, s, true);
-    k_results<<<cdiv(b.nmol, 128), 128, 0, s>>>(b.d_mols, b.d_jobs, b.d_job0, b.nmol, b.d_st, b.d_status, dp, b.d_atom_z,
+    k_results<<<b.nmol, RESULT_THREADS, 0, s>>>(b.d_mols, b.d_jobs, b.d_job0, b.nmol, b.d_st, b.d_status, dp, b.d_atom_z,
                                                  b.d_atom_xyz, b.d_res, b.d_charges);
     run.launched(AM1GPU_PHASE_FINAL, 5 + (int)b.tri_buckets.size() + (int)big_tri_launches);
     CK(cudaGetLastError());
@@ -2746,7 +2743,7 @@ int density_purify_one(int n, const double* F, double nocc, double weight, int p
     int* dact = (int*)(D + o_act);
     k_sp2_bounds<<<1, 512, 3 * sizeof(double) * n, s>>>(dj, dms);
     k_sp2_init<<<dim3(nblk, 1), 256, 0, s>>>(dj, dsst, dms, nblk);
-    k_sp2_start<<<1, 128, 0, s>>>(dj, dsst, dms, 1, nblk);
+    k_sp2_start<<<1, 32 * SP2_UPDATE_WARPS, 0, s>>>(dj, dsst, dms, 1, nblk);
     CK(cudaGetLastError());
     const bool pairs = n % 2 == 0;  // every slot here starts on 256 bytes
     int* hact = (int*)(H + staged);
@@ -2768,7 +2765,7 @@ int density_purify_one(int n, const double* F, double nocc, double weight, int p
             k_sp2_step_tc<<<nt128, 128, tc_smem_bytes(), s>>>(dj, d128, nt128, dsst, dact + 2);
         }
         CK(cudaMemsetAsync(dact, 0, sizeof(int), s));
-        k_sp2_update<<<1, 128, 0, s>>>(dj, dsst, 1, kSp2MaxSteps, dact, (double*)(D + o_work));
+        k_sp2_update<<<1, 32 * SP2_UPDATE_WARPS, 0, s>>>(dj, dsst, 1, kSp2MaxSteps, dact, (double*)(D + o_work));
         CK(cudaGetLastError());
         if (step >= 12 && (step % 6) == 5) {
             CK(cudaMemcpyAsync(hact, dact, 16, cudaMemcpyDeviceToHost, s));

@@ -423,18 +423,30 @@ __global__ void k_bisect(const TriJob* __restrict__ jobs, const int* __restrict_
     extern __shared__ double sh[];
     double* d = sh;
     double* e2 = sh + n;
-    __shared__ double bounds[2];
+    __shared__ double bounds[2], wlo[32], whi[32];
+    double lo_t = 1e300, hi_t = -1e300;  // Gershgorin bounds of T (every thread's share, then the CTA's)
     for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        d[i] = jb.d[i];
-        e2[i] = i + 1 < n ? jb.e[i] * jb.e[i] : 0.0;
+        const double di = jb.d[i], er = i + 1 < n ? jb.e[i] : 0.0;
+        d[i] = di;
+        e2[i] = er * er;
+        const double r = (i > 0 ? fabs(jb.e[i - 1]) : 0.0) + fabs(er);
+        lo_t = fmin(lo_t, di - r);
+        hi_t = fmax(hi_t, di + r);
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+        lo_t = fmin(lo_t, __shfl_xor_sync(0xffffffffu, lo_t, o));
+        hi_t = fmax(hi_t, __shfl_xor_sync(0xffffffffu, hi_t, o));
+    }
+    if ((threadIdx.x & 31) == 0) {
+        wlo[threadIdx.x >> 5] = lo_t;
+        whi[threadIdx.x >> 5] = hi_t;
     }
     __syncthreads();
     if (threadIdx.x == 0) {
         double lo = 1e300, hi = -1e300;
-        for (int i = 0; i < n; ++i) {
-            const double r = (i > 0 ? fabs(jb.e[i - 1]) : 0.0) + (i + 1 < n ? fabs(jb.e[i]) : 0.0);
-            lo = fmin(lo, d[i] - r);
-            hi = fmax(hi, d[i] + r);
+        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) {
+            lo = fmin(lo, wlo[w]);
+            hi = fmax(hi, whi[w]);
         }
         const double pad = 1e-12 * fmax(fabs(lo), fabs(hi)) + 1e-300;
         bounds[0] = lo - pad;

@@ -23,24 +23,14 @@ __global__ void k_scf_arm(cudaGraphConditionalHandle h, GraphLoop* loop, int max
     cudaGraphSetConditional(h, max_scf > 0 ? 1u : 0u);
 }
 
-// Before each purification loop: its step counter and active count to 0, the loop armed.
-__global__ void k_sp2_arm(cudaGraphConditionalHandle h, GraphLoop* loop, int* active_count) {
+// Before each purification loop: its step counter and the counters of the step's update
+// (k_sp2_update_cond, which decides the loop) to 0, the loop armed.
+__global__ void k_sp2_arm(cudaGraphConditionalHandle h, GraphLoop* loop) {
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
     loop->sp2_step = 0;
-    *active_count = 0;
+    loop->sp2_active = 0;
+    loop->ticket = 0;
     cudaGraphSetConditional(h, 1u);
-}
-
-// After each purification step (k_sp2_update has counted the channels still purifying): go round
-// again while any is and fewer than max_steps steps were taken; the count restarts at 0.
-__global__ void k_sp2_cond(cudaGraphConditionalHandle h, GraphLoop* loop, int* active_count, int max_steps) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    const int step = loop->sp2_step + 1;
-    loop->sp2_step = step;
-    loop->sp2_total += 1;
-    const int more = *active_count > 0 && step < max_steps;
-    *active_count = 0;
-    cudaGraphSetConditional(h, more ? 1u : 0u);
 }
 
 // After the purified densities of an iteration: the stalled-purification eigensolver runs only if

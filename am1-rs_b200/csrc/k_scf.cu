@@ -279,8 +279,26 @@ __global__ void __launch_bounds__(DG_THREADS, 4) k_commutator_tma(const ChanJob*
     commutator_body<2>(jobs, tiles, ntiles, st, maps, err);
 }
 
-// Gaussian elimination with partial pivoting; false when a pivot is below 1e-12.
-__device__ bool solve_small(int n, double* m, double* rhs, double* x) {
+// ---- the extrapolation, a warp per molecule.  The kernel is a handful of tiny dense problems behind
+// one long list of partial sums, so it is bound by latency: one thread per molecule walked the list (a
+// memory round trip every few entries) and worked on arrays in local memory.  Here lane k sums quantity k,
+// the list's loads batched ahead of the adds, and the small problems run over the lanes in shared memory
+// and registers.  Every sum keeps its order and every element its expression, so the bits are those of
+// the one-thread form.  Measured: 676 -> 74 us on a 3072-orbital molecule, 38 -> 10 us on 32 waters, 18 ->
+// 10 us on methane.
+constexpr int DIIS_DIM = MAX_DIIS + 1;
+
+struct DiisWarp {  // one warp's shared memory
+    double tot[RED_N];
+    double bm[MAX_DIIS * MAX_DIIS], gm[MAX_DIIS * MAX_DIIS];  // the Gram matrices, logical order
+    double B[DIIS_DIM * DIIS_DIM], rhs[DIIS_DIM], x[DIIS_DIM];
+};
+
+// Gaussian elimination with partial pivoting on w.B (n x n, n <= DIIS_DIM) and w.rhs, a lane per row;
+// false when a pivot is below 1e-12.  The solution is in w.x.
+__device__ __forceinline__ bool solve_small(int n, DiisWarp& w, int lane) {
+    double* m = w.B;
+    double* rhs = w.rhs;
     for (int col = 0; col < n; ++col) {
         int piv = col;
         double best = fabs(m[col * n + col]);
@@ -292,180 +310,277 @@ __device__ bool solve_small(int n, double* m, double* rhs, double* x) {
             }
         }
         if (best < 1.0e-12) return false;
+        __syncwarp();
         if (piv != col) {
-            for (int j = 0; j < n; ++j) {
-                const double t = m[col * n + j];
-                m[col * n + j] = m[piv * n + j];
-                m[piv * n + j] = t;
+            if (lane < n) {
+                const double t = m[col * n + lane];
+                m[col * n + lane] = m[piv * n + lane];
+                m[piv * n + lane] = t;
+            } else if (lane == 31) {
+                const double t = rhs[col];
+                rhs[col] = rhs[piv];
+                rhs[piv] = t;
             }
-            const double t = rhs[col];
-            rhs[col] = rhs[piv];
-            rhs[piv] = t;
+            __syncwarp();
         }
-        for (int row = col + 1; row < n; ++row) {
+        const int row = col + 1 + lane;
+        if (row < n) {
             const double factor = m[row * n + col] / m[col * n + col];
-            if (factor == 0.0) continue;
-            for (int j = col; j < n; ++j) m[row * n + j] -= factor * m[col * n + j];
-            rhs[row] -= factor * rhs[col];
+            if (factor != 0.0) {
+                for (int j = col; j < n; ++j) m[row * n + j] -= factor * m[col * n + j];
+                rhs[row] -= factor * rhs[col];
+            }
         }
+        __syncwarp();
     }
-    for (int col = n - 1; col >= 0; --col) {
-        double sum = rhs[col];
-        for (int j = col + 1; j < n; ++j) sum -= m[col * n + j] * x[j];
-        x[col] = sum / m[col * n + col];
-    }
+    if (lane == 0)
+        for (int col = n - 1; col >= 0; --col) {
+            double sum = rhs[col];
+            for (int j = col + 1; j < n; ++j) sum -= m[col * n + j] * w.x[j];
+            w.x[col] = sum / m[col * n + col];
+        }
+    __syncwarp();
     return true;
 }
 
-// Euclidean projection onto the probability simplex (sort descending, running threshold).
-__device__ void simplex_project(int n, const double* v, double* out) {
-    double u[MAX_DIIS];
-    for (int i = 0; i < n; ++i) u[i] = v[i];
-    for (int i = 1; i < n; ++i) {  // insertion sort, descending
-        const double x = u[i];
-        int j = i - 1;
-        while (j >= 0 && u[j] < x) {
-            u[j + 1] = u[j];
-            --j;
-        }
-        u[j + 1] = x;
-    }
-    double css = 0.0, theta = 0.0;
-    for (int j = 0; j < n; ++j) {
-        css += u[j];
-        const double t = (css - 1.0) / ((double)j + 1.0);
-        if (u[j] - t > 0.0) theta = t;
-    }
-    for (int i = 0; i < n; ++i) out[i] = fmax(v[i] - theta, 0.0);
-}
-
-__device__ void adiis_simplex(int m, const double* d, const double* S, double* c) {
+// A-DIIS: projected gradient on the probability simplex (the Euclidean projection: sort descending,
+// running threshold) for f(c) = 2 d.c + c.S c from c = e_m.  Lane k holds row k of S + S^T; every lane
+// holds all of c.  The sort is a network on registers (entries past m are -inf and stay last) and the
+// threshold's divisions run a lane per rank.
+__device__ __forceinline__ void adiis_simplex(int m, double dk, const double (&Sk)[MAX_DIIS], double (&c)[MAX_DIIS], int lane) {
+    constexpr unsigned ALL = 0xffffffffu;
     double L = 1.0e-12;
-    for (int i = 0; i < m; ++i) {
+    {
         double row = 0.0;
-        for (int j = 0; j < m; ++j) row += fabs(S[i * MAX_DIIS + j] + S[j * MAX_DIIS + i]);
-        L = fmax(L, row);
+#pragma unroll
+        for (int j = 0; j < MAX_DIIS; ++j)
+            if (j < m) row += fabs(Sk[j]);
+#pragma unroll
+        for (int i = 0; i < MAX_DIIS; ++i) {
+            const double r = __shfl_sync(ALL, row, i);
+            if (i < m) L = fmax(L, r);
+        }
     }
     const double lr = 1.0 / L;
-    for (int i = 0; i < m; ++i) c[i] = 0.0;
-    c[m - 1] = 1.0;
+    const double ninf = __longlong_as_double(0xfff0000000000000LL);
+    double ck = lane == m - 1 ? 1.0 : 0.0;  // this lane's own entry of c
+#pragma unroll
+    for (int i = 0; i < MAX_DIIS; ++i) c[i] = i == m - 1 ? 1.0 : 0.0;
     for (int it = 0; it < 400; ++it) {
-        double trial[MAX_DIIS], proj[MAX_DIIS];
-        for (int k = 0; k < m; ++k) {
-            double acc = 2.0 * d[k];
-            for (int j = 0; j < m; ++j) acc += (S[k * MAX_DIIS + j] + S[j * MAX_DIIS + k]) * c[j];
-            trial[k] = c[k] - lr * acc;
+        double acc = 2.0 * dk;
+#pragma unroll
+        for (int j = 0; j < MAX_DIIS; ++j)
+            if (j < m) acc += Sk[j] * c[j];
+        const double trial = ck - lr * acc;
+        double v[MAX_DIIS], u[MAX_DIIS];
+#pragma unroll
+        for (int i = 0; i < MAX_DIIS; ++i) {
+            v[i] = __shfl_sync(ALL, trial, i);
+            u[i] = i < m ? v[i] : ninf;
         }
-        simplex_project(m, trial, proj);
+        // Batcher's odd-even merge sort of eight, descending
+        auto cx = [&](int a, int b) {
+            const bool sw = u[a] < u[b];
+            const double hi = sw ? u[b] : u[a], lo = sw ? u[a] : u[b];
+            u[a] = hi;
+            u[b] = lo;
+        };
+        cx(0, 1); cx(2, 3); cx(4, 5); cx(6, 7);
+        cx(0, 2); cx(1, 3); cx(4, 6); cx(5, 7);
+        cx(1, 2); cx(5, 6);
+        cx(0, 4); cx(1, 5); cx(2, 6); cx(3, 7);
+        cx(2, 4); cx(3, 5);
+        cx(1, 2); cx(3, 4); cx(5, 6);
+        double css = 0.0, mine = 0.0, uj = 0.0;
+#pragma unroll
+        for (int j = 0; j < MAX_DIIS; ++j) {
+            if (j < m) css += u[j];
+            if (j == lane) {
+                mine = css;
+                uj = u[j];
+            }
+        }
+        const double t = (mine - 1.0) / ((double)lane + 1.0);
+        const unsigned on = __ballot_sync(ALL, lane < m && uj - t > 0.0);
+        const double theta = on ? __shfl_sync(ALL, t, 31 - __clz(on)) : 0.0;
         double delta = 0.0;
-        for (int i = 0; i < m; ++i) {
-            delta += fabs(proj[i] - c[i]);
-            c[i] = proj[i];
-        }
-        if (delta < 1.0e-12) break;
+#pragma unroll
+        for (int i = 0; i < MAX_DIIS; ++i)
+            if (i < m) {
+                const double p = fmax(v[i] - theta, 0.0);
+                delta += fabs(p - c[i]);
+                c[i] = p;
+            }
+        ck = fmax(trial - theta, 0.0);
+        if (delta < 1.0e-12) break;  // the same in every lane
     }
 }
 
-__global__ void k_diis_solve(const MolDesc* __restrict__ mols, const ChanJob* __restrict__ jobs, const int* __restrict__ mol_job0,
-                             int nmol, MolState* __restrict__ st, int* __restrict__ mol_status, int nblk, ScfParams prm) {
-    const int mi = blockIdx.x * blockDim.x + threadIdx.x;
+// Adds `count` values of a list to t in order: p[k * stride], SUM_BATCH loads ahead of their adds.
+constexpr int SUM_BATCH = 16;
+__device__ __forceinline__ double ordered_sum(double t, const double* __restrict__ p, int stride, int count) {
+    for (int k0 = 0; k0 < count; k0 += SUM_BATCH) {
+        double v[SUM_BATCH];
+#pragma unroll
+        for (int u = 0; u < SUM_BATCH; ++u) v[u] = k0 + u < count ? __ldcg(p + (long long)(k0 + u) * stride) : 0.0;
+#pragma unroll
+        for (int u = 0; u < SUM_BATCH; ++u)
+            if (k0 + u < count) t += v[u];
+    }
+    return t;
+}
+
+__global__ void __launch_bounds__(32 * SCF_MOL_WARPS) k_diis_solve(const MolDesc* __restrict__ mols, const ChanJob* __restrict__ jobs,
+                                                                   const int* __restrict__ mol_job0, int nmol, MolState* __restrict__ st,
+                                                                   int* __restrict__ mol_status, int nblk, ScfParams prm) {
+    __shared__ DiisWarp sh[SCF_MOL_WARPS];
+    const int lane = threadIdx.x & 31, mi = blockIdx.x * SCF_MOL_WARPS + (threadIdx.x >> 5);
     if (mi >= nmol) return;
     MolState& s = st[mi];
     if (!s.active) return;
-    const MolDesc md = mols[mi];
-    double tot[RED_N];
-    for (int k = 0; k < RED_N; ++k) tot[k] = 0.0;
-    for (int c = 0; c < md.nch; ++c) {
-        const ChanJob& jb = jobs[mol_job0[mi] + c];
-        for (int b = 0; b < red_blocks(jb.n); ++b)
-            for (int k = 0; k < RED_N; ++k) tot[k] += jb.red[(long long)b * RED_N + k];
-        for (int t = 0; t < jb.ntiles; ++t) {  // the commutator pass, in tile order
-            tot[RED_ERR2] += jb.cpart[(long long)t * CP_N + CP_ERR2];
-            for (int k = 0; k < MAX_DIIS; ++k) tot[RED_B + k] += jb.cpart[(long long)t * CP_N + CP_B + k];
+    DiisWarp& w = sh[threadIdx.x >> 5];
+    const int nch = mols[mi].nch, job0 = mol_job0[mi];
+    {
+        double t = 0.0;
+        for (int c = 0; c < nch; ++c) {
+            const ChanJob& jb = jobs[job0 + c];
+            if (lane < RED_N) t = ordered_sum(t, jb.red + lane, RED_N, red_blocks(jb.n));
+            // the commutator pass, in tile order: CP_ERR2 into RED_ERR2, CP_B + k into RED_B + k
+            static_assert(RED_B == RED_ERR2 + 1 && CP_B == CP_ERR2 + 1, "one lane per commutator sum");
+            if (lane >= RED_ERR2 && lane < RED_ERR2 + CP_N) t = ordered_sum(t, jb.cpart + (lane - RED_ERR2), CP_N, jb.ntiles);
         }
+        if (lane < RED_N) w.tot[lane] = t;
     }
-    const double e_elec = 0.5 * (tot[RED_E_H] + tot[RED_E_F]);
-    const double err = sqrt(tot[RED_ERR2]);
+    for (int i = lane; i < MAX_DIIS * MAX_DIIS; i += 32) {
+        w.bm[i] = s.bmat[i];
+        w.gm[i] = s.gmat[i];
+    }
     // history bookkeeping: physical slot of logical index i is (head + i) % 8
     const int cnt = s.hist_count;
-    int newslot;
+    int newslot, head = s.hist_head;
     unsigned live;
     live_slots(s, newslot, live);
+    __syncwarp();
+    const double* tot = w.tot;
+    const double e_elec = 0.5 * (tot[RED_E_H] + tot[RED_E_F]);
+    const double err = sqrt(tot[RED_ERR2]);
     if (cnt == MAX_DIIS) {  // drop the oldest: shift the Gram matrices up-left
-        for (int i = 0; i < MAX_DIIS - 1; ++i)
-            for (int j = 0; j < MAX_DIIS - 1; ++j) {
-                s.bmat[i * MAX_DIIS + j] = s.bmat[(i + 1) * MAX_DIIS + j + 1];
-                s.gmat[i * MAX_DIIS + j] = s.gmat[(i + 1) * MAX_DIIS + j + 1];
-            }
-        s.hist_head = (s.hist_head + 1) % MAX_DIIS;
-        s.hist_count = MAX_DIIS;
-    } else {
-        s.hist_count = cnt + 1;
+        double b2[2], g2[2];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            const int e = lane + 32 * u, i = e / MAX_DIIS, j = e % MAX_DIIS;
+            const bool in = i < MAX_DIIS - 1 && j < MAX_DIIS - 1;
+            b2[u] = w.bm[in ? e + MAX_DIIS + 1 : e];
+            g2[u] = w.gm[in ? e + MAX_DIIS + 1 : e];
+        }
+        __syncwarp();
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            w.bm[lane + 32 * u] = b2[u];
+            w.gm[lane + 32 * u] = g2[u];
+        }
+        head = (head + 1) % MAX_DIIS;
+        __syncwarp();
     }
-    const int m = s.hist_count, last = m - 1;
-    for (int i = 0; i < m; ++i) {
-        const int phys = (s.hist_head + i) % MAX_DIIS;
+    const int m = cnt == MAX_DIIS ? MAX_DIIS : cnt + 1, last = m - 1;
+    if (lane < m) {
+        const int phys = (head + lane) % MAX_DIIS;
         const double b = 2.0 * tot[RED_B + phys];
-        s.bmat[last * MAX_DIIS + i] = b;
-        s.bmat[i * MAX_DIIS + last] = b;
-        s.gmat[last * MAX_DIIS + i] = tot[RED_GROW + phys];  // <D_last, F_i>
-        s.gmat[i * MAX_DIIS + last] = tot[RED_GCOL + phys];  // <D_i, F_last>
+        w.bm[last * MAX_DIIS + lane] = b;
+        w.bm[lane * MAX_DIIS + last] = b;
+        if (lane != last) {
+            w.gm[last * MAX_DIIS + lane] = tot[RED_GROW + phys];  // <D_last, F_i>
+            w.gm[lane * MAX_DIIS + last] = tot[RED_GCOL + phys];  // <D_i, F_last>
+        } else {
+            w.gm[last * MAX_DIIS + last] = tot[RED_GROW + newslot];
+        }
     }
-    s.gmat[last * MAX_DIIS + last] = tot[RED_GROW + newslot];
-    s.e_elec = e_elec;
-    s.err_norm = err;
-    s.mode = 0;
-    s.accel_used = 0;
-    if (!isfinite(e_elec) || !isfinite(err)) {
-        s.status = 4;  // AM1GPU_SCF_DIVERGED
-        mol_status[mi] = 4;
-        s.active = 0;
-        s.iter += 1;
-        return;
+    __syncwarp();
+    for (int i = lane; i < MAX_DIIS * MAX_DIIS; i += 32) {
+        s.bmat[i] = w.bm[i];
+        s.gmat[i] = w.gm[i];
     }
+    const bool diverged = !isfinite(e_elec) || !isfinite(err);
+    if (lane == 0) {
+        s.hist_head = head;
+        s.hist_count = m;
+        s.e_elec = e_elec;
+        s.err_norm = err;
+        s.mode = 0;
+        s.accel_used = 0;
+        if (diverged) {
+            s.status = 4;  // AM1GPU_SCF_DIVERGED
+            mol_status[mi] = 4;
+            s.active = 0;
+            s.iter += 1;
+        }
+    }
+    if (diverged) return;
     int accel = prm.use_diis ? prm.accelerator : 0;
-    if (md.nch == 2) accel = prm.use_diis ? 1 : 0;  // UHF: CDIIS only (scf.rs:770-803)
+    if (nch == 2) accel = prm.use_diis ? 1 : 0;  // UHF: CDIIS only (scf.rs:770-803)
     bool use_adiis = accel == 2 && err > prm.adiis_switch;
     if (accel == 1 || (accel == 2 && !use_adiis)) {
         if (m >= 2) {
             const int dim = m + 1;
-            double B[(MAX_DIIS + 1) * (MAX_DIIS + 1)], rhs[MAX_DIIS + 1], x[MAX_DIIS + 1];
-            for (int i = 0; i < dim * dim; ++i) B[i] = 0.0;
-            for (int i = 0; i < m; ++i) {
-                for (int j = 0; j < m; ++j) B[i * dim + j] = s.bmat[i * MAX_DIIS + j];
-                B[i * dim + m] = -1.0;
-                B[m * dim + i] = -1.0;
+            for (int e = lane; e < dim * dim; e += 32) {
+                const int i = e / dim, j = e % dim;
+                w.B[e] = i < m && j < m ? w.bm[i * MAX_DIIS + j] : i == j ? 0.0 : -1.0;
             }
-            for (int i = 0; i < dim; ++i) rhs[i] = 0.0;
-            rhs[m] = -1.0;
-            if (solve_small(dim, B, rhs, x)) {
+            if (lane < dim) w.rhs[lane] = lane == m ? -1.0 : 0.0;
+            __syncwarp();
+            if (solve_small(dim, w, lane)) {
                 double wsum = 0.0;
                 bool fin = true;
                 for (int i = 0; i < m; ++i) {
-                    wsum += fabs(x[i]);
-                    fin = fin && isfinite(x[i]);
+                    wsum += fabs(w.x[i]);
+                    fin = fin && isfinite(w.x[i]);
                 }
                 if (isfinite(wsum) && fin) {
-                    for (int i = 0; i < m; ++i) s.coeff[i] = x[i];
-                    s.mode = 1;
-                    s.accel_used = 1;
+                    if (lane < m) s.coeff[lane] = w.x[lane];
+                    if (lane == 0) {
+                        s.mode = 1;
+                        s.accel_used = 1;
+                    }
                 }
             }
         }
     } else if (use_adiis && m >= 2) {
-        double d[MAX_DIIS], S[MAX_DIIS * MAX_DIIS], c[MAX_DIIS];
-        const double gll = s.gmat[last * MAX_DIIS + last];
-        for (int i = 0; i < m; ++i) d[i] = s.gmat[i * MAX_DIIS + last] - gll;
-        for (int i = 0; i < m; ++i)
-            for (int j = 0; j < m; ++j)
-                S[i * MAX_DIIS + j] = s.gmat[i * MAX_DIIS + j] - s.gmat[i * MAX_DIIS + last] - s.gmat[last * MAX_DIIS + j] + gll;
-        adiis_simplex(m, d, S, c);
+        const double gll = w.gm[last * MAX_DIIS + last];
+        double Sk[MAX_DIIS], c[MAX_DIIS], dk = 0.0;
         bool fin = true;
-        for (int i = 0; i < m; ++i) fin = fin && isfinite(c[i]);
-        if (fin) {
-            for (int i = 0; i < m; ++i) s.coeff[i] = c[i];
-            s.mode = 1;
-            s.accel_used = 2;
+#pragma unroll
+        for (int j = 0; j < MAX_DIIS; ++j) Sk[j] = 0.0;
+        if (lane < m) {
+            const int k = lane;
+            dk = w.gm[k * MAX_DIIS + last] - gll;
+            fin = isfinite(dk);
+#pragma unroll
+            for (int j = 0; j < MAX_DIIS; ++j)
+                if (j < m) {
+                    const double skj = w.gm[k * MAX_DIIS + j] - w.gm[k * MAX_DIIS + last] - w.gm[last * MAX_DIIS + j] + gll;
+                    const double sjk = w.gm[j * MAX_DIIS + k] - w.gm[j * MAX_DIIS + last] - w.gm[last * MAX_DIIS + k] + gll;
+                    Sk[j] = skj + sjk;
+                    fin = fin && isfinite(Sk[j]);
+                }
+        }
+        // a Gram matrix that is not finite has no simplex minimum: plain F (energy and error are finite
+        // here, so this takes an overflow in the products of two histories)
+        if (__all_sync(0xffffffffu, fin)) {
+            adiis_simplex(m, dk, Sk, c, lane);
+#pragma unroll
+            for (int i = 0; i < MAX_DIIS; ++i)
+                if (i < m) {
+                    fin = fin && isfinite(c[i]);
+                }
+            if (fin) {  // c is the same in every lane
+#pragma unroll
+                for (int i = 0; i < MAX_DIIS; ++i)
+                    if (i < m && lane == i) s.coeff[i] = c[i];
+                if (lane == 0) {
+                    s.mode = 1;
+                    s.accel_used = 2;
+                }
+            }
         }
     }
 }
@@ -550,7 +665,7 @@ __global__ void k_combine(const ChanJob* __restrict__ jobs, const MolState* __re
 __global__ void k_density_post(const ChanJob* __restrict__ jobs, const MolState* __restrict__ st, int nblk) {
     const ChanJob jb = jobs[blockIdx.y];
     if (!st[jb.mol].active) return;
-    const int nb = red_blocks(jb.n);
+    const int nb = dens_blocks(jb.n);
     if ((int)blockIdx.x >= nb) return;
     const long long nn = (long long)jb.n * jb.n;
     double acc = 0.0;
@@ -585,27 +700,38 @@ __global__ void k_density_post(const ChanJob* __restrict__ jobs, const MolState*
     }
 }
 
-__global__ void k_converge(const MolDesc* __restrict__ mols, const ChanJob* __restrict__ jobs, const int* __restrict__ mol_job0,
-                           int nmol, MolState* __restrict__ st, int* __restrict__ mol_status, int nblk, ScfParams prm,
-                           int* __restrict__ active_count) {
-    const int mi = blockIdx.x * blockDim.x + threadIdx.x;
+// A warp per molecule: its lanes fetch the partial sums, 32 blocks of a channel at a time, every lane
+// adds them in block order, and lane 0 takes the decision.
+__global__ void __launch_bounds__(32 * SCF_MOL_WARPS) k_converge(const MolDesc* __restrict__ mols, const ChanJob* __restrict__ jobs,
+                                                                 const int* __restrict__ mol_job0, int nmol, MolState* __restrict__ st,
+                                                                 int* __restrict__ mol_status, int nblk, ScfParams prm,
+                                                                 int* __restrict__ active_count) {
+    const int lane = threadIdx.x & 31, mi = blockIdx.x * SCF_MOL_WARPS + (threadIdx.x >> 5);
     if (mi >= nmol) return;
     MolState& s = st[mi];
     if (!s.active) return;
     if (mol_status[mi] != 0) {  // the eigensolver refused its input
-        s.active = 0;
-        s.status = mol_status[mi];
-        s.iter += 1;
+        __syncwarp();
+        if (lane == 0) {
+            s.active = 0;
+            s.status = mol_status[mi];
+            s.iter += 1;
+        }
         return;
     }
-    const MolDesc md = mols[mi];
+    const int nch = mols[mi].nch, job0 = mol_job0[mi];
     double dp = 0.0;
-    for (int c = 0; c < md.nch; ++c) {
-        const ChanJob& jb = jobs[mol_job0[mi] + c];
+    for (int c = 0; c < nch; ++c) {
+        const ChanJob& jb = jobs[job0 + c];
+        const int nb = dens_blocks(jb.n);
         double ss = 0.0;
-        for (int b = 0; b < red_blocks(jb.n); ++b) ss += jb.red2[b];
+        for (int b0 = 0; b0 < nb; b0 += 32) {
+            const double v = b0 + lane < nb ? __ldcg(jb.red2 + b0 + lane) : 0.0;
+            for (int b = 0; b < min(32, nb - b0); ++b) ss += __shfl_sync(0xffffffffu, v, b);
+        }
         dp += sqrt(ss / fmax((double)jb.n * jb.n, 1.0));
     }
+    if (lane != 0) return;
     const double de = fabs(s.e_elec - s.e_old);
     s.dp = dp;
     s.e_old = s.e_elec;
@@ -641,42 +767,45 @@ __global__ void k_converge(const MolDesc* __restrict__ mols, const ChanJob* __re
     }
 }
 
-__global__ void k_final_energy(const MolDesc* __restrict__ mols, const ChanJob* __restrict__ jobs, const int* __restrict__ mol_job0,
-                               int nmol, MolState* __restrict__ st, int nblk) {
-    const int mi = blockIdx.x * blockDim.x + threadIdx.x;
+// A warp per molecule: lanes 0 and 1 add the two energy traces, in block order.
+__global__ void __launch_bounds__(32 * SCF_MOL_WARPS) k_final_energy(const MolDesc* __restrict__ mols, const ChanJob* __restrict__ jobs,
+                                                                     const int* __restrict__ mol_job0, int nmol,
+                                                                     MolState* __restrict__ st, int nblk) {
+    const int lane = threadIdx.x & 31, mi = blockIdx.x * SCF_MOL_WARPS + (threadIdx.x >> 5);
     if (mi >= nmol) return;
-    const MolDesc md = mols[mi];
-    double eh = 0.0, ef = 0.0;
-    for (int c = 0; c < md.nch; ++c) {
-        const ChanJob& jb = jobs[mol_job0[mi] + c];
-        for (int b = 0; b < red_blocks(jb.n); ++b) {
-            eh += jb.red[(long long)b * RED_N + RED_E_H];
-            ef += jb.red[(long long)b * RED_N + RED_E_F];
-        }
+    const int nch = mols[mi].nch, job0 = mol_job0[mi];
+    double t = 0.0;
+    for (int c = 0; c < nch; ++c) {
+        const ChanJob& jb = jobs[job0 + c];
+        if (lane < 2) t = ordered_sum(t, jb.red + (lane == 0 ? RED_E_H : RED_E_F), RED_N, red_blocks(jb.n));
     }
-    st[mi].e_final = 0.5 * (eh + ef);
+    const double ef = __shfl_sync(0xffffffffu, t, 1);
+    if (lane == 0) st[mi].e_final = 0.5 * (t + ef);
 }
 
 // Result record of one molecule (src/scf.rs:370-438): energies, heat of formation, Mulliken
-// charges, dipole (point charges + s-p hybrid term), frontier orbitals.
-__global__ void k_results(const MolDesc* __restrict__ mols, const ChanJob* __restrict__ jobs, const int* __restrict__ mol_job0,
-                          int nmol, const MolState* __restrict__ st, const int* __restrict__ mol_status,
-                          const DevElem* __restrict__ params, const int* __restrict__ atom_z, const double* __restrict__ atom_xyz,
-                          double* __restrict__ res, double* __restrict__ charges) {
-    const int mi = blockIdx.x * blockDim.x + threadIdx.x;
+// charges, dipole (point charges + s-p hybrid term), frontier orbitals.  A CTA per molecule, a thread
+// per atom (the sums over atoms: thread-strided, then a fixed tree, so they depend on the molecule alone).
+// One thread per molecule cost a chain of memory round trips per atom: 1956 us for 1536 atoms, now 37 us.
+__global__ void __launch_bounds__(RESULT_THREADS) k_results(const MolDesc* __restrict__ mols, const ChanJob* __restrict__ jobs,
+                                                            const int* __restrict__ mol_job0, int nmol, const MolState* __restrict__ st,
+                                                            const int* __restrict__ mol_status, const DevElem* __restrict__ params,
+                                                            const int* __restrict__ atom_z, const double* __restrict__ atom_xyz,
+                                                            double* __restrict__ res, double* __restrict__ charges) {
+    __shared__ double part[5][RESULT_THREADS / 32];
+    const int mi = blockIdx.x;
     if (mi >= nmol) return;
     const MolDesc md = mols[mi];
     const MolState& s = st[mi];
-    const int n = md.nao, h = md.nheavy;
-    const long long nn = (long long)n * n;
+    const int n = md.nao, h = md.nheavy, tid = threadIdx.x;
     const double* P0 = jobs[mol_job0[mi]].P;
     const double* P1 = md.nch == 2 ? jobs[mol_job0[mi] + 1].P : nullptr;
-    double e_isol = 0.0, eheat = 0.0, dip[3] = {0.0, 0.0, 0.0};
-    for (int A = 0; A < md.natoms; ++A) {
+    double sum[5] = {0.0, 0.0, 0.0, 0.0, 0.0};  // e_isol, eheat, dipole
+    for (int A = tid; A < md.natoms; A += RESULT_THREADS) {
         const int a = md.atom_base + A;
         const DevElem& e = params[md.method * (MAX_Z + 1) + atom_z[a]];
-        e_isol += e.e_isol;
-        eheat += e.eheat_ev;
+        sum[0] += e.e_isol;
+        sum[1] += e.eheat_ev;
         const int o = A < h ? 4 * A : 4 * h + (A - h), no = A < h ? 4 : 1;
         double pop = 0.0;
         for (int k = 0; k < no; ++k) {
@@ -685,16 +814,30 @@ __global__ void k_results(const MolDesc* __restrict__ mols, const ChanJob* __res
         }
         const double q = e.core_charge - pop;
         charges[a] = q;
-        for (int k = 0; k < 3; ++k) dip[k] += atom_xyz[3 * a + k] * q;
+        for (int k = 0; k < 3; ++k) sum[2 + k] += atom_xyz[3 * a + k] * q;
         if (e.norb == 4) {
             const double hyb = -2.0 * e.dd;
             for (int k = 0; k < 3; ++k) {
                 const long long idx = (long long)o * n + o + 1 + k;
-                dip[k] += hyb * (P1 ? P0[idx] + P1[idx] : P0[idx]);
+                sum[2 + k] += hyb * (P1 ? P0[idx] + P1[idx] : P0[idx]);
             }
         }
     }
-    (void)nn;
+#pragma unroll
+    for (int k = 0; k < 5; ++k) {
+        double v = sum[k];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        if ((tid & 31) == 0) part[k][tid >> 5] = v;
+    }
+    __syncthreads();
+    if (tid != 0) return;
+    for (int k = 0; k < 5; ++k) {
+        sum[k] = part[k][0];
+        for (int w = 1; w < RESULT_THREADS / 32; ++w) sum[k] += part[k][w];
+    }
+    const double e_isol = sum[0], eheat = sum[1];
+    const double* dip = sum + 2;
     double* r = res + (long long)mi * RES_N;
     const double total = s.e_final + s.core_ev;
     r[RES_ELEC] = s.e_final;

@@ -520,23 +520,58 @@ __global__ void k_sp2_init(const Sp2Job* __restrict__ jobs, Sp2State* __restrict
     }
 }
 
-// Reduce the init partials: state of step 0.
-__global__ void k_sp2_start(const Sp2Job* __restrict__ jobs, Sp2State* __restrict__ sst, const MolState* __restrict__ st, int njobs,
-                            int nblk) {
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
+// Sum of `count` (trace, Frobenius) partial pairs in order, by one warp: the lanes fetch 64 pairs at a
+// time into the warp's shared buffer (the next 64 in flight meanwhile), then lane 0 adds the traces and
+// lane 1 the Frobenius shares, one after the other.  The order, and so every bit, is that of one thread
+// walking the list; that walk cost a memory round trip per few pairs (137 us for the 1176 tiles of a
+// 3072-orbital matrix, 15 us with the fetches batched; 35 -> 7 us for a batch with 1200 orbitals).  Lane 0
+// gets both sums.
+constexpr int SP2_SUM_CHUNK = 64;
+__device__ __forceinline__ void sp2_sum_parts(const double* __restrict__ part, int count, double* __restrict__ buf, double& tr, double& fr) {
+    const int lane = threadIdx.x & 31;
+    constexpr int PER = 2 * SP2_SUM_CHUNK / 32;
+    double v[PER], t = 0.0;
+#pragma unroll
+    for (int u = 0; u < PER; ++u) v[u] = lane + 32 * u < 2 * count ? __ldcg(part + lane + 32 * u) : 0.0;
+    for (int k0 = 0; k0 < count; k0 += SP2_SUM_CHUNK) {
+#pragma unroll
+        for (int u = 0; u < PER; ++u) buf[lane + 32 * u] = v[u];
+        __syncwarp();
+        const int at = 2 * (k0 + SP2_SUM_CHUNK) + lane;
+#pragma unroll
+        for (int u = 0; u < PER; ++u) v[u] = at + 32 * u < 2 * count ? __ldcg(part + at + 32 * u) : 0.0;
+        if (lane < 2) {
+            const int m = min(SP2_SUM_CHUNK, count - k0);
+            if (m == SP2_SUM_CHUNK) {
+#pragma unroll 16
+                for (int k = 0; k < SP2_SUM_CHUNK; ++k) t += buf[2 * k + lane];
+            } else {
+                for (int k = 0; k < m; ++k) t += buf[2 * k + lane];
+            }
+        }
+        __syncwarp();
+    }
+    tr = t;
+    fr = __shfl_sync(0xffffffffu, t, 1);
+}
+
+// Reduce the init partials: state of step 0.  A warp per channel.
+__global__ void __launch_bounds__(32 * SP2_UPDATE_WARPS) k_sp2_start(const Sp2Job* __restrict__ jobs, Sp2State* __restrict__ sst,
+                                                                     const MolState* __restrict__ st, int njobs, int nblk) {
+    __shared__ double buf[SP2_UPDATE_WARPS][2 * SP2_SUM_CHUNK];
+    const int warp = threadIdx.x >> 5, j = blockIdx.x * SP2_UPDATE_WARPS + warp;
     if (j >= njobs) return;
-    const Sp2Job jb = jobs[j];
+    const Sp2Job& jb = jobs[j];
+    const MolState& ms = st[jb.mol];
+    double tr, fr;
+    sp2_sum_parts(jb.part, sp2_init_blocks(jb.n), buf[warp], tr, fr);
+    if ((threadIdx.x & 31) != 0) return;
     Sp2State& s = sst[j];
-    s.active = st[jb.mol].active;
-    s.lowp = st[jb.mol].lowp;
+    s.active = ms.active;
+    s.lowp = ms.lowp;
     s.steps = 0;
     s.cur = 0;
     s.converged = 0;
-    double tr = 0.0, fr = 0.0;
-    for (int b = 0; b < sp2_init_blocks(jb.n); ++b) {
-        tr += jb.part[2 * b];
-        fr += jb.part[2 * b + 1];
-    }
     s.trX = tr;
     s.trX2 = fr;
     s.idem[0] = s.idem[1] = 1e300;
@@ -645,28 +680,31 @@ __global__ void __launch_bounds__(DG_THREADS, 4) k_sp2_step_tma(const Sp2Job* __
 }
 
 // After a step: reduce the tile partials (in tile order), test idempotency, choose the next branch.
-// The update of channel j after its product; true while it still purifies.
+// The update of channel j after its product, by one warp (buf: its 2 SP2_SUM_CHUNK doubles of shared
+// memory); lane 0 returns true while the channel still purifies.
 __device__ __forceinline__ bool sp2_update_job(const Sp2Job* __restrict__ jobs, Sp2State* __restrict__ sst, int j, int max_steps,
-                                               double* __restrict__ work) {
+                                               double* __restrict__ work, double* __restrict__ buf) {
     Sp2State& s = sst[j];
-    if (!s.active) return false;
-    const Sp2Job jb = jobs[j];
+    if (!s.active) return false;  // uniform over the warp
+    const Sp2Job& jb = jobs[j];
+    // the partial sums come from the tiles of the kernel that took the product
+    const bool lowp = s.lowp != 0;
+    const int nparts = lowp ? (jb.lowp_tc ? jb.tc_ntiles : jb.ntiles) : (jb.oz ? jb.oz_ntiles : jb.ntiles);
+    double tr, fr;
+    sp2_sum_parts(jb.part, nparts, buf, tr, fr);
+    __syncwarp();
+    if ((threadIdx.x & 31) != 0) return false;
     // algorithmic work of the product just taken: a symmetric X.X, n^3 flops
-    if (s.lowp) {
+    const double nd = (double)jb.n;
+    if (lowp) {
         atomicAdd(&work[4], 1.0);
-        atomicAdd(&work[5], (double)jb.n * jb.n * jb.n);
+        atomicAdd(&work[5], nd * nd * nd);
     } else {
         atomicAdd(&work[0], 1.0);
-        atomicAdd(&work[1], (double)jb.n * jb.n * jb.n);
-        atomicAdd(&work[3], 16.0 * jb.n * jb.n);  // read X, write X^2 (both triangles), FP64
+        atomicAdd(&work[1], nd * nd * nd);
+        atomicAdd(&work[3], 16.0 * nd * nd);  // read X, write X^2 (both triangles), FP64
     }
-    double tr = 0.0, fr = 0.0;
-    // the partial sums come from the tiles of the kernel that took the product
-    const int nparts = s.lowp ? (jb.lowp_tc ? jb.tc_ntiles : jb.ntiles) : (jb.oz ? jb.oz_ntiles : jb.ntiles);
-    for (int t = 0; t < nparts; ++t) {
-        tr += jb.part[2 * t];
-        fr += jb.part[2 * t + 1];
-    }
+    const double nocc = jb.nocc;
     s.cur ^= 1;
     s.steps += 1;
     s.trX = tr;
@@ -676,10 +714,10 @@ __device__ __forceinline__ bool sp2_update_job(const Sp2Job* __restrict__ jobs, 
     const bool floor_reached = idem < 1.0e-6 && idem >= s.idem[0];  // stagnation at the rounding floor
     // TF32 runs stop at their own rounding level (about 1e-6 relative per eigenvalue), and their
     // result is always taken: it only starts the FP64 iterations
-    const bool low_done = s.lowp && ((idem < 1.0e-2 * jb.n && idem >= s.idem[0]) || idem < 1.0e-5 * jb.n);
+    const bool low_done = lowp && ((idem < 1.0e-2 * jb.n && idem >= s.idem[0]) || idem < 1.0e-5 * jb.n);
     s.idem[0] = s.idem[1];
     s.idem[1] = idem;
-    if (low_done || floor_reached || idem < 1.0e-15 * fmax(1.0, (double)jb.n)) {
+    if (low_done || floor_reached || idem < 1.0e-15 * fmax(1.0, nd)) {
         s.active = 0;
         s.converged = 1;
         return false;
@@ -689,32 +727,44 @@ __device__ __forceinline__ bool sp2_update_job(const Sp2Job* __restrict__ jobs, 
         s.converged = s.lowp;
         return false;
     }
-    s.square = fabs(fr - jb.nocc) < fabs(2.0 * tr - fr - jb.nocc) ? 1 : 0;
+    s.square = fabs(fr - nocc) < fabs(2.0 * tr - fr - nocc) ? 1 : 0;
     return true;
 }
 
-__global__ void k_sp2_update(const Sp2Job* __restrict__ jobs, Sp2State* __restrict__ sst, int njobs, int max_steps,
-                             int* __restrict__ active_count, double* __restrict__ work) {
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(32 * SP2_UPDATE_WARPS) k_sp2_update(const Sp2Job* __restrict__ jobs, Sp2State* __restrict__ sst,
+                                                                      int njobs, int max_steps, int* __restrict__ active_count,
+                                                                      double* __restrict__ work) {
+    __shared__ double buf[SP2_UPDATE_WARPS][2 * SP2_SUM_CHUNK];
+    const int warp = threadIdx.x >> 5, j = blockIdx.x * SP2_UPDATE_WARPS + warp;
     if (j >= njobs) return;
-    if (sp2_update_job(jobs, sst, j, max_steps, work)) atomicAdd(active_count, 1);
+    if (sp2_update_job(jobs, sst, j, max_steps, work, buf[warp])) atomicAdd(active_count, 1);
 }
 
-// The update of every channel and the purification loop's decision in one CTA (the captured solve
-// of a batch of at most SP2_UPDATE_ONE channels): the same per-channel update, the channels still
-// purifying counted by the CTA, then k_sp2_cond's step counters and condition.
-__global__ void __launch_bounds__(SP2_UPDATE_ONE) k_sp2_update_cond(const Sp2Job* __restrict__ jobs, Sp2State* __restrict__ sst, int njobs,
-                                                                    int max_steps, double* __restrict__ work,
-                                                                    cudaGraphConditionalHandle h, GraphLoop* __restrict__ loop) {
-    const int j = threadIdx.x;
-    const bool more_j = j < njobs && sp2_update_job(jobs, sst, j, max_steps, work);
-    const int active = __syncthreads_count(more_j);
-    if (threadIdx.x == 0) {
-        const int step = loop->sp2_step + 1;
-        loop->sp2_step = step;
-        loop->sp2_total += 1;
-        cudaGraphSetConditional(h, (active > 0 && step < max_steps) ? 1u : 0u);
+// The update of every channel and the purification loop's decision in one launch (the captured
+// solve): the same per-channel update; the last CTA to finish (a ticket in *loop) has the count of
+// the channels still purifying and sets the loop's condition.  The tickets and the count start at
+// zero (k_sp2_arm) and are put back to zero by that CTA.
+__global__ void __launch_bounds__(32 * SP2_UPDATE_WARPS) k_sp2_update_cond(const Sp2Job* __restrict__ jobs, Sp2State* __restrict__ sst,
+                                                                           int njobs, int max_steps, double* __restrict__ work,
+                                                                           cudaGraphConditionalHandle h, GraphLoop* __restrict__ loop) {
+    __shared__ double buf[SP2_UPDATE_WARPS][2 * SP2_SUM_CHUNK];
+    const int warp = threadIdx.x >> 5, j = blockIdx.x * SP2_UPDATE_WARPS + warp;
+    const bool more_j = j < njobs && sp2_update_job(jobs, sst, j, max_steps, work, buf[warp]);
+    const int more = __syncthreads_count(more_j);
+    if (threadIdx.x != 0) return;
+    int active = more;
+    if (gridDim.x > 1) {
+        if (more) atomicAdd(&loop->sp2_active, more);
+        __threadfence();
+        if (atomicAdd(&loop->ticket, 1) != (int)gridDim.x - 1) return;
+        __threadfence();
+        active = atomicExch(&loop->sp2_active, 0);
+        loop->ticket = 0;
     }
+    const int step = loop->sp2_step + 1;
+    loop->sp2_step = step;
+    loop->sp2_total += 1;
+    cudaGraphSetConditional(h, (active > 0 && step < max_steps) ? 1u : 0u);
 }
 
 // P_new = w X (the converged X); molecules whose purification stalled are flagged for the

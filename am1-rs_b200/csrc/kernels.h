@@ -134,10 +134,11 @@ struct GraphLoop {
     int sp2_step;   // purification steps of the current iteration
     int sp2_total;  // purification steps of this launch
     int eig_runs;   // iterations of this launch in which the stalled-purification eigensolver ran
+    int sp2_active; // channels still purifying, counted by the CTAs of the step's update
+    int ticket;     // CTAs of the step's update that are done
 };
 __global__ void k_scf_arm(cudaGraphConditionalHandle h, GraphLoop* loop, int max_scf);
-__global__ void k_sp2_arm(cudaGraphConditionalHandle h, GraphLoop* loop, int* active_count);
-__global__ void k_sp2_cond(cudaGraphConditionalHandle h, GraphLoop* loop, int* active_count, int max_steps);
+__global__ void k_sp2_arm(cudaGraphConditionalHandle h, GraphLoop* loop);
 __global__ void k_stall_arm(cudaGraphConditionalHandle h, GraphLoop* loop, const int* need_eigen, int nmol);
 __global__ void k_scf_cond(cudaGraphConditionalHandle h, GraphLoop* loop, const int* active, int max_scf);
 
@@ -153,6 +154,7 @@ struct ScfParams {
 __global__ void k_pair_integrals(const MolDesc* mols, int nmol, const long long* pair_prefix, long long npairs,
                                  const DevElem* params, const int* atom_z, const double* atom_xyz, double* wstore,
                                  double* hmat, double* ecc, int* mol_status);
+constexpr int CORE_DIAG_LANES = 16;  // lanes per atom of k_core_diag
 __global__ void k_core_diag(const MolDesc* mols, const int* atom_mol, int natoms_total, const DevElem* params,
                             const int* atom_z, const double* wstore, double* hmat);
 __global__ void k_core_energy(const MolDesc* mols, const double* ecc, MolState* st);
@@ -179,8 +181,16 @@ __global__ void k_sp2_bounds_cl(const Sp2Job* jobs, const int* big, const MolSta
 // sums are the same whatever else is in its batch; a launch's x extent is the batch's largest
 // count, and the blocks past a channel's own count leave at once.
 __host__ __device__ __forceinline__ int red_blocks(int n) { return n >= 497 ? 32 : (n + 15) / 16 < 1 ? 1 : (n + 15) / 16; }
-__host__ __device__ __forceinline__ int sp2_init_blocks(int n) { return n >= 249 ? 32 : (n + 7) / 8 < 1 ? 1 : (n + 7) / 8; }
+__host__ __device__ __forceinline__ int sp2_init_blocks(int n) {
+    return n >= 512 ? (n < 4096 ? n / 16 : 256) : n >= 249 ? 32 : (n + 7) / 8 < 1 ? 1 : (n + 7) / 8;
+}
+// The density change is only compared with thresholds, so its blocks may grow with n past the 32 that fill
+// the GPU for a batch: one 3072-orbital molecule's pass 268 -> 56 us with 192 blocks, its purification start
+// 190 -> 41 us.
+__host__ __device__ __forceinline__ int dens_blocks(int n) { return n >= 512 ? (n < 4096 ? n / 16 : 256) : red_blocks(n); }
 __global__ void k_sp2_init(const Sp2Job* jobs, Sp2State* sst, const MolState* st, int nblk);
+// the purification's per-channel bookkeeping: a warp per channel, SP2_UPDATE_WARPS channels per CTA
+constexpr int SP2_UPDATE_WARPS = 8;
 __global__ void k_sp2_start(const Sp2Job* jobs, Sp2State* sst, const MolState* st, int njobs, int nblk);
 // *16: every matrix of the tile list has even n and 16-byte aligned rows (16-byte copies);
 // *8: any matrix (8-byte copies)
@@ -205,7 +215,6 @@ __global__ void k_commutator_tma(const ChanJob* jobs, const GemmTile* tiles, int
                                  int* err);
 size_t dgemm_smem_bytes();
 __global__ void k_sp2_update(const Sp2Job* jobs, Sp2State* sst, int njobs, int max_steps, int* active_count, double* work);
-constexpr int SP2_UPDATE_ONE = 1024;  // channels k_sp2_update_cond takes in its one CTA
 __global__ void k_sp2_update_cond(const Sp2Job* jobs, Sp2State* sst, int njobs, int max_steps, double* work, cudaGraphConditionalHandle h,
                                   GraphLoop* loop);
 size_t tc_smem_bytes();
@@ -343,6 +352,9 @@ constexpr int kLowpMaxOpenShellAo = 448;
 __global__ void k_state_init(MolState* st, const MolDesc* mols, int nmol, int lowp);
 __global__ void k_post_fock(const ChanJob* jobs, const MolDesc* mols, const MolState* st, int nblk, int energy_only,
                             int force);
+// per-molecule bookkeeping: a warp per molecule, SCF_MOL_WARPS per CTA (k_results: a CTA per molecule)
+constexpr int SCF_MOL_WARPS = 4;
+constexpr int RESULT_THREADS = 128;
 __global__ void k_diis_solve(const MolDesc* mols, const ChanJob* jobs, const int* mol_job0, int nmol, MolState* st,
                              int* mol_status, int nblk, ScfParams prm);
 __global__ void k_combine(const ChanJob* jobs, const MolState* st, int force);
