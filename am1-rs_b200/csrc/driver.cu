@@ -239,6 +239,15 @@ int device_ctx(DeviceCtx** out) {
                               (const void*)k_commutator8})
             if ((err = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dgemm_smem_bytes())) != cudaSuccess)
                 return bad("tile kernel smem attribute", err);
+        for (const void* f : {(const void*)k_sp2_res, (const void*)k_sp2_clu}) {
+            cudaFuncAttributes fb{};
+            if ((err = cudaFuncGetAttributes(&fb, f)) != cudaSuccess) return bad("one-launch purification attributes", err);
+            if ((err = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - (int)fb.sharedSizeBytes)) !=
+                cudaSuccess)
+                return bad("one-launch purification smem attribute", err);
+        }
+        if ((err = cudaFuncSetAttribute(k_sp2_clu, cudaFuncAttributeNonPortableClusterSizeAllowed, 1)) != cudaSuccess)
+            return bad("one-launch purification cluster attribute", err);
         for (const void* f : {(const void*)k_sp2_step_tma, (const void*)k_commutator_tma})
             if ((err = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dgemm_tma_smem_bytes())) != cudaSuccess)
                 return bad("tensor-map tile kernel smem attribute", err);
@@ -286,7 +295,8 @@ struct Mem {
     char* hpin = nullptr;
     size_t hcap = 0;
     std::vector<cudaEvent_t> events;  // timing events, reused across calls
-    cudaStream_t cap_stream = nullptr;  // stream the SCF graph is captured on
+    cudaStream_t cap_stream = nullptr;  // stream the SCF graph is captured on, and the one-launch purifications' own in the host-driven loop
+    cudaEvent_t fork = nullptr, join = nullptr;  // order the two streams in the host-driven loop
 };
 
 // Stream priority asked for by the calling host thread (am1gpu_set_stream_priority).
@@ -324,7 +334,17 @@ void mem_release(Mem& w) {
     for (auto e : w.events) cudaEventDestroy(e);
     if (w.stream) cudaStreamDestroy(w.stream);
     if (w.cap_stream) cudaStreamDestroy(w.cap_stream);
+    if (w.fork) cudaEventDestroy(w.fork);
+    if (w.join) cudaEventDestroy(w.join);
     w = Mem();
+}
+
+// The second stream (of the first's priority) and its events, created on first use.
+int mem_side_stream(Mem& w) {
+    if (!w.cap_stream) CK(cudaStreamCreateWithPriority(&w.cap_stream, cudaStreamNonBlocking, w.priority));
+    if (!w.fork) CK(cudaEventCreateWithFlags(&w.fork, cudaEventDisableTiming));
+    if (!w.join) CK(cudaEventCreateWithFlags(&w.join, cudaEventDisableTiming));
+    return AM1GPU_OK;
 }
 
 thread_local Mem tl_mem;
@@ -595,10 +615,24 @@ struct MolPlan {
 // mixed path's two FP32 iterates of n rows of (n rounded up to 4) floats plus 16-byte alignment.
 long long vs_rows(const MolPlan& p) { return std::max<long long>(p.npad, ((p.nao + 3) & ~3) + 2); }
 
+// Which channels purify in one launch (k_sp2_fused.cu).  Up to FU_RES_MAX orbitals (what two iterates in one
+// CTA's shared memory allow) always: alone the launch-per-step form of so small a matrix is all latency (methane 2.54
+// against 1.14 ms a solve; 192 gradients 45.2 against 44.5).  Only with kResPerSm channels per SM and more (a batch
+// of thousands) do the tiles fill the GPU as well (4096 molecules: 526.5-529.1 ms with tiles, 528.9-529.4 with one
+// launch), and the batch takes the tiles throughout.  Above FU_RES_MAX (to 448) while the whole batch's clusters are resident at once
+// (sp2_cluster_for); past that the tiles of the launch-per-step kernels fill the GPU, while a cluster's rate does not
+// grow with the batch (n = 384: 32 us a product on 16 SMs against 30 on 21 tiles' SMs plus 11 of update and launches).
+constexpr int kResPerSm = 4;
+constexpr int kResSmall = 72;  // two CTAs of k_sp2_res per SM up to here
+int sp2_fused_kind(const MolPlan& p) {
+    if (density_mode() != 0 || p.cluster <= 0 || fp64_oz_for(p.nao) || p.nao < 1) return FU_NONE;
+    return p.nao <= FU_RES_MAX ? FU_RES : FU_CLU;
+}
+int sp2_cluster_for(int channels) { return channels < 1 ? 0 : channels <= 8 ? 16 : channels <= 16 ? 8 : 0; }
+
 // Largest molecule (orbitals) the purification path takes: the Lanczos bounds and the bisection hold
 // 3 n and 2 n doubles in one CTA's shared memory.
 constexpr int kMaxAo = 8192;
-int density_mode();
 
 int choose_cluster(int n, int* npad_out, int* c_out) {
     static const int cs[5] = {1, 2, 4, 8, 16};
@@ -737,6 +771,18 @@ struct Batch {
     Sp2State* d_sp2_state;
     TriJob* d_tri;
     int* d_need_eigen;
+    // channels whose FP64 purifications run in one launch each: groups of d_fused (k_sp2_res with C = 1, or
+    // clusters of C CTAs of k_sp2_clu), and how many channels take the launch-per-step kernels instead
+    struct FusedGroup {
+        int off, count, C;
+        size_t smem;
+    };
+    std::vector<FusedGroup> fused_groups;
+    int* d_fused = nullptr;
+    int unfused = 0;
+    // their tiles: the leading ones of the two tile lists (largest matrix first, and only the smallest
+    // matrices purify in one launch while others do not)
+    int nt_step_pairs = 0, nt_step_other = 0;
     int* d_sp2_active;
     double* d_work;  // [0] purification steps, [1] their flops, [2] eigensolver fallbacks, [3] their bytes,
                      // [4] TF32 purification steps, [5] their flops
@@ -811,6 +857,19 @@ int build_batch(const am1gpu_molecule* in, const am1gpu_options& o, std::vector<
             dq_bytes += p.nch * (2LL * kOzPlanes * p.nao * oz_ldq(p.nao) + 256);
         }
     }
+    // clusters of the one-launch purification: only while every such channel's cluster is resident at once
+    int clu_jobs = 0, res_jobs = 0;
+    long long clu_doubles = 0;
+    for (auto& p : b.plans) {
+        const int kind = sp2_fused_kind(p);
+        clu_jobs += kind == FU_CLU ? p.nch : 0;
+        res_jobs += kind == FU_RES ? p.nch : 0;
+    }
+    const bool one_launch = res_jobs <= kResPerSm * g_sms;
+    const int clu_size = one_launch ? sp2_cluster_for(clu_jobs) : 0;
+    if (clu_size)
+        for (auto& p : b.plans)
+            if (sp2_fused_kind(p) == FU_CLU) clu_doubles += p.nch * sp2_clu_doubles(p.nao);
     const int sp2_nblk = sp2_init_blocks(maxn), dens_nblk = dens_blocks(maxn);
     // ---- staged (host -> device) region layout
     size_t st = 0;
@@ -840,6 +899,7 @@ int build_batch(const am1gpu_molecule* in, const am1gpu_options& o, std::vector<
     const size_t o_ozt = take(st, sizeof(GemmTile) * std::max(tiles_oz, 1));
     const size_t o_tri = take(st, sizeof(TriJob) * 5 * nch_total);  // the jobs, then up to 4 continuations each
     const size_t o_sp2big = take(st, sizeof(int) * nch_total);
+    const size_t o_fused = take(st, sizeof(int) * nch_total);
     const size_t o_st = take(st, sizeof(MolState) * b.nmol);
     const size_t par_bytes = host_tab ? sizeof(DevElem) * 2 * (MAX_Z + 1) : 0;
     const size_t o_par = take(st, par_bytes);
@@ -874,6 +934,7 @@ int build_batch(const am1gpu_molecule* in, const am1gpu_options& o, std::vector<
     const size_t o_bstall = take(dv, sizeof(int) * std::max<long long>(nch_total, 1));
     const size_t o_loop = take(dv, sizeof(GraphLoop));
     const size_t o_dq = take(dv, (size_t)std::max<long long>(dq_bytes, 16));
+    const size_t o_xc = take(dv, sizeof(double) * (size_t)std::max<long long>(clu_doubles, 2));
     const size_t dtotal = align256(dv);
     // pinned staging also receives the outputs
     size_t hs = staged;
@@ -918,6 +979,10 @@ int build_batch(const am1gpu_molecule* in, const am1gpu_options& o, std::vector<
     long long dq_off = 0;
     b.d_tri = (TriJob*)dptr(o_tri);
     b.d_sp2_big = (int*)dptr(o_sp2big);
+    b.d_fused = (int*)dptr(o_fused);
+    std::vector<int> fused_jobs[2];  // k_sp2_res, k_sp2_clu
+    long long xc_off = 0;
+    b.unfused = 0;
     b.d_need_eigen = (int*)dptr(o_need);
     b.d_sp2_active = (int*)dptr(o_sp2a);
     b.d_work = (double*)dptr(o_work);
@@ -1117,6 +1182,17 @@ int build_batch(const am1gpu_molecule* in, const am1gpu_options& o, std::vector<
             }
             sj.oz_ntiles = noz - sj.oz_tile0;
             if (!sj.fallback) b.sp2_big.push_back(job);
+            sj.fused = one_launch ? sp2_fused_kind(p) : FU_NONE;
+            if (sj.fused == FU_CLU) {
+                if (clu_size) {
+                    sj.Xc = (double*)dptr(o_xc) + xc_off;
+                    xc_off += sp2_clu_doubles((int)n);
+                } else {
+                    sj.fused = FU_NONE;
+                }
+            }
+            if (sj.fused == FU_NONE) ++b.unfused;
+            else fused_jobs[sj.fused == FU_CLU].push_back(job);
             sj.tile0 = (int)tl.size();  // tile index inside its own launch
             for (int x = 0; x < (int)tn_; ++x)
                 for (int y = x; y < (int)tn_; ++y) tl.push_back(GemmTile{job, x, y});
@@ -1193,6 +1269,13 @@ int build_batch(const am1gpu_molecule* in, const am1gpu_options& o, std::vector<
     for (size_t i = 0; i < tiles_pairs.size(); ++i) hsp2t[i] = tiles_pairs[i];
     for (size_t i = 0; i < tiles_other.size(); ++i) hsp2t[tiles_pairs.size() + i] = tiles_other[i];
     b.nt_sp2_pairs = (int)tiles_pairs.size();
+    auto stepped = [&](const std::vector<GemmTile>& v) {
+        int k = (int)v.size();
+        while (k > 0 && hsp2[v[k - 1].job].fused != FU_NONE) --k;
+        return k;
+    };
+    b.nt_step_pairs = stepped(tiles_pairs);
+    b.nt_step_other = stepped(tiles_other);
     b.nt_tc = ntc;
     b.nt_oz = noz;
     b.nt_sp2 = (int)(tiles_pairs.size() + tiles_other.size());
@@ -1282,6 +1365,23 @@ int build_batch(const am1gpu_molecule* in, const am1gpu_options& o, std::vector<
     }
     std::stable_sort(b.sp2_big.begin(), b.sp2_big.end(), [&](int x, int y) { return hsp2[x].n > hsp2[y].n; });
     std::copy(b.sp2_big.begin(), b.sp2_big.end(), (int*)(Hs + o_sp2big));
+    // one-launch purifications, largest first; the on-chip ones in two launches, so that the smaller
+    // half's CTAs are sized (and packed on the SMs) by their own largest matrix
+    b.fused_groups.clear();
+    int* hfused = (int*)(Hs + o_fused);
+    int nf = 0;
+    for (int kind = 0; kind < 2; ++kind) {
+        std::vector<int>& v = fused_jobs[kind];
+        std::stable_sort(v.begin(), v.end(), [&](int x, int y) { return hsp2[x].n > hsp2[y].n; });
+        for (int j : v) {
+            const int jn = hsp2[j].n, C = kind == 1 ? clu_size : 1;
+            const bool small = kind == 0 && jn <= kResSmall;
+            if (b.fused_groups.empty() || b.fused_groups.back().C != C || (small && hsp2[hfused[nf - 1]].n > kResSmall))
+                b.fused_groups.push_back({nf, 0, C, sp2_fused_smem_bytes(jn, kind == 0)});
+            b.fused_groups.back().count++;
+            hfused[nf++] = j;
+        }
+    }
     b.mols.assign(hm, hm + b.nmol);
     b.jobs.assign(hj, hj + job);
     b.job0.assign(hj0, hj0 + b.nmol);
@@ -1319,10 +1419,12 @@ int big_fallback(Batch& b, Mem* ws);
 namespace {
 
 // The upper-triangle tile kernels run as up to two launches: the 16-byte-copy tiles, then the rest.
+// step: only the tiles of the channels that purify in a launch per step.
 template <class F>
-void launch_tiles(const Batch& b, cudaStream_t, F&& launch) {
-    if (b.nt_sp2_pairs > 0) launch(b.d_sp2_tiles, b.nt_sp2_pairs, true);
-    if (b.nt_sp2 > b.nt_sp2_pairs) launch(b.d_sp2_tiles + b.nt_sp2_pairs, b.nt_sp2 - b.nt_sp2_pairs, false);
+void launch_tiles(const Batch& b, bool step, F&& launch) {
+    const int np = step ? b.nt_step_pairs : b.nt_sp2_pairs, no = step ? b.nt_step_other : b.nt_sp2 - b.nt_sp2_pairs;
+    if (np > 0) launch(b.d_sp2_tiles, np, true);
+    if (no > 0) launch(b.d_sp2_tiles + b.nt_sp2_pairs, no, false);
 }
 
 int launch_core(Batch& b, Mem* ws, const DevElem* dp, Run* run) {
@@ -1501,6 +1603,23 @@ int launch_jacobi(Batch& b, Mem* ws, int force, const int* mask = nullptr, cudaS
     return AM1GPU_OK;
 }
 
+// The one-launch purifications of the iteration: group k of the batch.
+int launch_fused(Batch& b, size_t k, cudaStream_t s, int max_steps, Run* run) {
+    const Batch::FusedGroup& gr = b.fused_groups[k];
+    const Sp2Job* jobs = b.d_sp2;
+    const int* list = b.d_fused + gr.off;
+    const MolState* stp = b.d_st;
+    if (gr.C == 1) {
+        k_sp2_res<<<gr.count, 256, gr.smem, s>>>(jobs, list, b.d_sp2_state, stp, b.d_need_eigen, b.d_work, max_steps);
+        CK(cudaGetLastError());
+    } else {
+        void* args[] = {&jobs, &list, &b.d_sp2_state, &stp, &b.d_need_eigen, &b.d_work, &max_steps};
+        CK(launch_clusters((const void*)k_sp2_clu, gr.C, gr.count, 256, gr.smem, s, args));
+    }
+    run->launched(AM1GPU_PHASE_EIGEN);
+    return AM1GPU_OK;
+}
+
 // One SCF iteration's launches, shared by the host-driven loop and the captured graph.
 struct IterEnq {
     Batch& b;
@@ -1513,10 +1632,9 @@ struct IterEnq {
     size_t ph;  // start event of the phase being timed
 };
 
-// Fock build, commutator and history, extrapolation, and (purification path) the spectral bounds
-// and the start of the purification.
-int enq_head(IterEnq& e, bool lowp_left) {
-    (void)lowp_left;
+// Fock build, commutator and history, extrapolation; with enq_sp2_start it is the first half of an
+// iteration.
+int enq_head(IterEnq& e) {
     Batch& b = e.b;
     const cudaStream_t s = e.s;
     Run& run = *e.run;
@@ -1526,7 +1644,7 @@ int enq_head(IterEnq& e, bool lowp_left) {
     k_fock<<<cdiv(b.natoms, 8), 256, 0, s>>>(b.d_mols, b.d_atom_mol, b.natoms, e.dp, b.d_atom_z, b.d_wstore, b.d_arena, b.d_st, 0);
     run.launched(AM1GPU_PHASE_FOCK);
     if ((rc = run.end(AM1GPU_PHASE_FOCK, e.ph)) || (rc = run.begin(&e.ph))) return rc;
-    launch_tiles(b, s, [&](const GemmTile* t, int nt, bool pairs) {
+    launch_tiles(b, false, [&](const GemmTile* t, int nt, bool pairs) {
         if (pairs && b.sp2_tma)
             k_commutator_tma<<<nt, 128, dgemm_tma_smem_bytes(), s>>>(b.d_jobs, t, nt, b.d_st, b.d_sp2_maps, b.d_sp2_active + 2);
         else if (pairs)
@@ -1541,13 +1659,23 @@ int enq_head(IterEnq& e, bool lowp_left) {
     k_combine<<<dim3(e.rowblk, e.njobs), 256, 0, s>>>(b.d_jobs, b.d_st, 0);
     run.launched(AM1GPU_PHASE_ACCEL, 2);
     if ((rc = run.end(AM1GPU_PHASE_ACCEL, e.ph)) || (rc = run.begin(&e.ph))) return rc;
+    if (density_mode() == 0) CK(cudaMemsetAsync(b.d_need_eigen, 0, sizeof(int) * b.nmol, s));
+    CK(cudaGetLastError());
+    return AM1GPU_OK;
+}
+
+// The spectral bounds and the start of the launch-per-step purifications (every channel that does not
+// purify in one launch).
+int enq_sp2_start(IterEnq& e) {
+    Batch& b = e.b;
+    const cudaStream_t s = e.s;
+    Run& run = *e.run;
+    int rc;
     if (density_mode() == 0) {
-        // purification: P from F* by SP2, eigensolver only for molecules whose purification stalls
         k_sp2_bounds<<<e.njobs, 512, 3 * sizeof(double) * b.maxn, s>>>(b.d_sp2, b.d_st);
         if ((rc = launch_big_bounds(b, s))) return rc;
         k_sp2_init<<<dim3(b.sp2_nblk, e.njobs), 256, 0, s>>>(b.d_sp2, b.d_sp2_state, b.d_st, b.sp2_nblk);
         k_sp2_start<<<cdiv(e.njobs, SP2_UPDATE_WARPS), 32 * SP2_UPDATE_WARPS, 0, s>>>(b.d_sp2, b.d_sp2_state, b.d_st, e.njobs, b.sp2_nblk);
-        CK(cudaMemsetAsync(b.d_need_eigen, 0, sizeof(int) * b.nmol, s));
         run.launched(AM1GPU_PHASE_EIGEN,
                      3 + big_launches(big_split((int)b.sp2_big.size(), [&](int i) { return b.jobs[b.sp2_big[i]].n; }),
                                       (int)b.sp2_big.size()));
@@ -1569,7 +1697,7 @@ int enq_step(IterEnq& e, int sp2_max, bool lowp_left, bool zero_count, const cud
     size_t pc;
     if ((rc = run.begin(&pc))) return rc;
     int nl = 0;
-    launch_tiles(b, s, [&](const GemmTile* t, int nt, bool pairs) {
+    launch_tiles(b, true, [&](const GemmTile* t, int nt, bool pairs) {
         if (pairs && b.sp2_tma)
             k_sp2_step_tma<<<nt, 128, dgemm_tma_smem_bytes(), s>>>(b.d_sp2, t, nt, b.d_sp2_state, b.d_sp2_maps, b.d_sp2_active + 2);
         else if (pairs)
@@ -1583,7 +1711,7 @@ int enq_step(IterEnq& e, int sp2_max, bool lowp_left, bool zero_count, const cud
         ++nl;
     }
     if (lowp_left) {
-        launch_tiles(b, s, [&](const GemmTile* t, int nt, bool) {
+        launch_tiles(b, false, [&](const GemmTile* t, int nt, bool) {
             k_sp2_step_tf32<<<nt, 128, tf32_smem_bytes(), s>>>(b.d_sp2, t, nt, b.d_sp2_state);
             ++nl;
         });
@@ -1618,16 +1746,18 @@ int enq_step(IterEnq& e, int sp2_max, bool lowp_left, bool zero_count, const cud
 // its kernels skip every other molecule, and the captured solve runs it only in iterations where
 // some purification stalled), and the rest (enq_tail_rest).  The Jacobi density path (density_mode
 // != 0) is all in enq_tail_finish.
-int enq_tail_finish(IterEnq& e) {
+int enq_tail_finish(IterEnq& e, bool lowp_left) {
     Batch& b = e.b;
     const cudaStream_t s = e.s;
     Run& run = *e.run;
     int rc;
     if (density_mode() == 0) {
-        const unsigned fin_blocks = std::max(8u, std::min(256u, cdiv((long long)b.maxn * b.maxn, 65536)));
-        k_sp2_finish<<<dim3(fin_blocks, e.njobs), 256, 0, s>>>(b.d_sp2, b.d_sp2_state, b.d_st, b.d_need_eigen, b.d_work,
-                                                               b.d_big_stall, b.d_active + 3);
-        run.launched(AM1GPU_PHASE_EIGEN);
+        if (b.unfused > 0 || lowp_left) {
+            const unsigned fin_blocks = std::max(8u, std::min(256u, cdiv((long long)b.maxn * b.maxn, 65536)));
+            k_sp2_finish<<<dim3(fin_blocks, e.njobs), 256, 0, s>>>(b.d_sp2, b.d_sp2_state, b.d_st, b.d_need_eigen, b.d_work,
+                                                                   b.d_big_stall, b.d_active + 3);
+            run.launched(AM1GPU_PHASE_EIGEN);
+        }
         if (!b.sp2_big.empty() && (rc = big_fallback(b, e.ws))) return rc;
     } else {
         k_gemm_nn<<<b.nt_gt, 256, 0, s>>>(b.d_gj_gt, b.d_gt_gt, b.nt_gt, b.d_st, 0, nullptr);
@@ -1680,9 +1810,9 @@ int enq_tail_rest(IterEnq& e) {
     return AM1GPU_OK;
 }
 
-int enq_tail(IterEnq& e) {
+int enq_tail(IterEnq& e, bool lowp_left) {
     int rc;
-    if ((rc = enq_tail_finish(e)) || (rc = enq_tail_stall(e)) || (rc = enq_tail_rest(e))) return rc;
+    if ((rc = enq_tail_finish(e, lowp_left)) || (rc = enq_tail_stall(e)) || (rc = enq_tail_rest(e))) return rc;
     return AM1GPU_OK;
 }
 
@@ -1747,7 +1877,8 @@ int add_if(cudaGraph_t g, cudaGraphNode_t dep, cudaGraphConditionalHandle h, cud
 }
 
 // The SCF loop of run_device as one graph launch:
-//   k_scf_arm -> WHILE(scf) { head -> k_sp2_arm -> WHILE(sp2) { step } -> tail -> k_scf_cond }
+//   k_scf_arm -> WHILE(scf) { head -> [one-launch purifications | start -> k_sp2_arm -> WHILE(sp2) { step }]
+//                             -> tail -> k_scf_cond }
 // (the step's update kernel sets the purification loop's condition itself, k_sp2_update_cond) and, in a
 // graph kept for a resident batch's later runs, the tail split as
 //   finish -> k_stall_arm -> IF(stall) { stalled-purification eigensolver } -> rest -> k_scf_cond.
@@ -1762,7 +1893,7 @@ int scf_loop_graph(IterEnq& e, const am1gpu_options& o, bool* launched) {
     Batch& b = e.b;
     Mem& m = *e.ws;
     const int sp2_max = sp2_max_steps();
-    if (!m.cap_stream) CK(cudaStreamCreateWithFlags(&m.cap_stream, cudaStreamNonBlocking));
+    if (int rc0 = mem_side_stream(m)) return rc0;
     const cudaStream_t cs = m.cap_stream;
     if (b.graph_cacheable && b.graph_exec) {  // a resident batch's graph, captured on its first run
         *launched = true;
@@ -1794,22 +1925,33 @@ int scf_loop_graph(IterEnq& e, const am1gpu_options& o, bool* launched) {
         return rc;
     cudaGraph_t body = nullptr, body2 = nullptr;
     if ((rc = add_while(g, arm, h_scf, &w_scf, &body))) return rc;
-    CK(cudaGraphConditionalHandleCreate(&h_sp2, body, 0, 0));
+    if (b.unfused > 0) CK(cudaGraphConditionalHandleCreate(&h_sp2, body, 0, 0));
     const int64_t head0 = cnt.kernel_launches;
-    if ((rc = capture_into(cs, body, nullptr, 0, &head, [&]() -> int {
-             int r = enq_head(ce, false);
-             if (r) return r;
-             k_sp2_arm<<<1, 32, 0, cs>>>(h_sp2, b.d_loop);
-             return AM1GPU_OK;
-         })))
+    if ((rc = capture_into(cs, body, nullptr, 0, &head, [&]() -> int { return enq_head(ce); }))) return rc;
+    // the purifications, side by side: a branch per group of one-launch ones, and the launch-per-step loop
+    std::vector<cudaGraphNode_t> purified;
+    for (size_t k = 0; k < b.fused_groups.size(); ++k) {
+        cudaGraphNode_t node;
+        if ((rc = capture_into(cs, body, &head, 1, &node, [&]() -> int { return launch_fused(b, k, cs, sp2_max, &crun); }))) return rc;
+        purified.push_back(node);
+    }
+    if (b.unfused > 0 && (rc = capture_into(cs, body, &head, 1, &head, [&]() -> int {
+                              int r = enq_sp2_start(ce);
+                              if (r) return r;
+                              k_sp2_arm<<<1, 32, 0, cs>>>(h_sp2, b.d_loop);
+                              return AM1GPU_OK;
+                          })))
         return rc;
-    const int64_t per_head = cnt.kernel_launches - head0 + 1;
-    if ((rc = add_while(body, head, h_sp2, &w_sp2, &body2))) return rc;
+    const int64_t per_head = cnt.kernel_launches - head0 + (b.unfused > 0 ? 1 : 0);
     const int64_t step0 = cnt.kernel_launches;
-    if ((rc = capture_into(cs, body2, nullptr, 0, &step, [&]() -> int {
-             return enq_step(ce, sp2_max, false, false, &h_sp2);  // its update takes the loop's decision
-         })))
-        return rc;
+    if (b.unfused > 0) {
+        if ((rc = add_while(body, head, h_sp2, &w_sp2, &body2))) return rc;
+        if ((rc = capture_into(cs, body2, nullptr, 0, &step, [&]() -> int {
+                 return enq_step(ce, sp2_max, false, false, &h_sp2);  // its update takes the loop's decision
+             })))
+            return rc;
+        purified.push_back(w_sp2);
+    }
     const int64_t per_step = cnt.kernel_launches - step0;
     const int64_t tail0 = cnt.kernel_launches;
     int64_t per_stall = 0, per_tail = 0;
@@ -1819,8 +1961,8 @@ int scf_loop_graph(IterEnq& e, const am1gpu_options& o, bool* launched) {
         cudaGraphConditionalHandle h_stall;
         CK(cudaGraphConditionalHandleCreate(&h_stall, body, 0, 0));
         cudaGraphNode_t fin, w_stall, stall_last;
-        if ((rc = capture_into(cs, body, &w_sp2, 1, &fin, [&]() -> int {
-                 int r = enq_tail_finish(ce);
+        if ((rc = capture_into(cs, body, purified.data(), purified.size(), &fin, [&]() -> int {
+                 int r = enq_tail_finish(ce, false);
                  if (r) return r;
                  k_stall_arm<<<1, 256, 0, cs>>>(h_stall, b.d_loop, b.d_need_eigen, b.nmol);
                  return AM1GPU_OK;
@@ -1840,8 +1982,8 @@ int scf_loop_graph(IterEnq& e, const am1gpu_options& o, bool* launched) {
             return rc;
         per_tail = cnt.kernel_launches - tail0 + 2 - per_stall;
     } else {
-        if ((rc = capture_into(cs, body, &w_sp2, 1, &tail, [&]() -> int {
-                 int r = enq_tail(ce);
+        if ((rc = capture_into(cs, body, purified.data(), purified.size(), &tail, [&]() -> int {
+                 int r = enq_tail(ce, false);
                  if (r) return r;
                  k_scf_cond<<<1, 32, 0, cs>>>(h_scf, b.d_loop, b.d_active, o.max_scf);
                  return AM1GPU_OK;
@@ -1912,9 +2054,21 @@ int run_device(Batch& b, Mem& mem, const DevElem* dp, const am1gpu_options& o, a
         const int check = b.nmol > 64 ? 4 : 1;
         while (done < o.max_scf) {
             for (int k = 0; k < check && done < o.max_scf; ++k, ++done) {
-                if ((rc = enq_head(e, lowp_left))) return rc;
-                if (density_mode() == 0) {
-                    const int sp2_max = sp2_max_steps();
+                if ((rc = enq_head(e))) return rc;
+                // one-launch purifications beside the launch-per-step ones, where the batch has both
+                const int sp2_max = sp2_max_steps();
+                const bool stepped = density_mode() == 0 && (b.unfused > 0 || lowp_left);
+                const bool forked = stepped && !b.fused_groups.empty();
+                if (forked) {
+                    if ((rc = mem_side_stream(mem))) return rc;
+                    CK(cudaEventRecord(mem.fork, s));
+                    CK(cudaStreamWaitEvent(mem.cap_stream, mem.fork, 0));
+                }
+                for (size_t g = 0; g < b.fused_groups.size(); ++g)
+                    if ((rc = launch_fused(b, g, forked ? mem.cap_stream : s, sp2_max, &run))) return rc;
+                if (forked) CK(cudaEventRecord(mem.join, mem.cap_stream));
+                if (stepped) {
+                    if ((rc = enq_sp2_start(e))) return rc;
                     for (int step = 0; step < sp2_max; ++step) {
                         if ((rc = enq_step(e, sp2_max, lowp_left, true))) return rc;
                         if (step >= 12 && (step % 6) == 5) {
@@ -1924,7 +2078,8 @@ int run_device(Batch& b, Mem& mem, const DevElem* dp, const am1gpu_options& o, a
                         }
                     }
                 }
-                if ((rc = enq_tail(e))) return rc;
+                if (forked) CK(cudaStreamWaitEvent(s, mem.join, 0));
+                if ((rc = enq_tail(e, lowp_left))) return rc;
             }
             CK(cudaMemcpyAsync(b.h_active, b.d_active, sizeof(int), cudaMemcpyDeviceToHost, s));
             if (lowp_left) CK(cudaMemcpyAsync(b.h_active + 2, b.d_active + 1, sizeof(int), cudaMemcpyDeviceToHost, s));
@@ -2618,7 +2773,7 @@ int big_fallback(Batch& b, Mem* ws) {
 // Density of one symmetric matrix F by purification, P = w * (projector onto its nocc lowest
 // eigenvectors): the step an SCF iteration takes after the extrapolation (the reference's
 // symmetric_eigen + density_from_coeff, src/scf.rs:654-661, 503-524), alone, at the precision of
-// the batched path's products: 0 FP64 tensor cores (k_sp2_step_tma/16/8), 1 FP32-accurate products on
+// the batched path's products: 0 FP64 tensor cores (in one launch, k_sp2_res / k_sp2_clu), 1 FP32-accurate products on
 // tcgen05 (k_sp2_step_tc, 3xTF32), 2 TF32 mma.sync (k_sp2_step_tf32), 3 FP64 from digit planes
 // (k_sp2_step_oz), 4 TF32 on tcgen05 in one pass (k_sp2_step_tc1).  The reduced-precision runs
 // stop at their own rounding floor and are rescaled to the exact trace, as in the mixed SCF.
@@ -2646,7 +2801,7 @@ int density_purify_one(int n, const double* F, double nocc, double weight, int p
         off += bytes;
         return o;
     };
-    const size_t o_job = take(sizeof(Sp2Job)), o_maps = take(4 * sizeof(TmaDesc)), o_xfmaps = take(2 * sizeof(TmaDesc)),
+    const size_t o_job = take(sizeof(Sp2Job)), o_xfmaps = take(2 * sizeof(TmaDesc)),
                  o_t64 = take(sizeof(GemmTile) * nt64),
                  o_t128 = take(sizeof(GemmTile) * nt128),
                  o_toz = take(sizeof(GemmTile) * ntoz),
@@ -2656,6 +2811,7 @@ int density_purify_one(int n, const double* F, double nocc, double weight, int p
                  o_part = take(16 * (size_t)std::max(32, nt64)), o_xf = take(8 * (size_t)n * ldf + 64), o_need = take(16),
                  o_work = take(8 * kWorkN), o_act = take(16), o_stall = take(16),
                  o_dq = take(2 * (size_t)kOzPlanes * n * ldq);
+    const size_t o_xc = take(precision == 0 && n > FU_RES_MAX ? 8 * (size_t)sp2_clu_doubles(n) : 16), o_list = take(sizeof(int));
     Workspace* ws;
     if (mem_override) {
         if ((rc = mem_ensure(*mem_override, align256(off), staged + align256(sizeof(Sp2State)) + 256))) return rc;
@@ -2685,6 +2841,8 @@ int density_purify_one(int n, const double* F, double nocc, double weight, int p
     jb.ldf = ldf;
     jb.Xf0 = (float*)(((uintptr_t)(D + o_xf) + 15) & ~(uintptr_t)15);
     jb.Xf1 = jb.Xf0 + (size_t)n * ldf;
+    jb.fused = precision != 0 ? FU_NONE : n <= FU_RES_MAX ? FU_RES : FU_CLU;
+    jb.Xc = (double*)(D + o_xc);
     jb.lowp_tc = precision == 1 ? 1 : precision == 4 ? 2 : 0;
     jb.tc_tile0 = 0;
     jb.tc_ntiles = (precision == 1 || precision == 4) ? nt128 : 0;
@@ -2695,8 +2853,6 @@ int density_purify_one(int n, const double* F, double nocc, double weight, int p
     jb.Dq0 = (int8_t*)(D + o_dq);
     jb.Dq1 = jb.Dq0 + (size_t)kOzPlanes * n * ldq;
     std::memcpy(H + o_job, &jb, sizeof jb);
-    TmaDesc* hmaps = (TmaDesc*)(H + o_maps);
-    const bool tma = encode_square_map(&hmaps[0], jb.X0, n) && encode_square_map(&hmaps[1], jb.X1, n);
     TmaDesc* hxfmaps = (TmaDesc*)(H + o_xfmaps);
     if (precision == 4 && !(encode_rows_map_f32(&hxfmaps[0], jb.Xf0, ldf, n) && encode_rows_map_f32(&hxfmaps[1], jb.Xf1, ldf, n)))
         return fail(AM1GPU_UNSUPPORTED, "no tensor-map encoder on this device: the single-pass tcgen05 products are not available");
@@ -2741,42 +2897,50 @@ int density_purify_one(int n, const double* F, double nocc, double weight, int p
     const GemmTile* d64 = (const GemmTile*)(D + o_t64);
     const GemmTile* d128 = (const GemmTile*)(D + o_t128);
     int* dact = (int*)(D + o_act);
-    k_sp2_bounds<<<1, 512, 3 * sizeof(double) * n, s>>>(dj, dms);
-    k_sp2_init<<<dim3(nblk, 1), 256, 0, s>>>(dj, dsst, dms, nblk);
-    k_sp2_start<<<1, 32 * SP2_UPDATE_WARPS, 0, s>>>(dj, dsst, dms, 1, nblk);
-    CK(cudaGetLastError());
-    const bool pairs = n % 2 == 0;  // every slot here starts on 256 bytes
     int* hact = (int*)(H + staged);
-    for (int step = 0; step < kSp2MaxSteps; ++step) {
-        if (precision == 0) {
-            if (tma)
-                k_sp2_step_tma<<<nt64, 128, dgemm_tma_smem_bytes(), s>>>(dj, d64, nt64, dsst, (const TmaDesc*)(D + o_maps), dact + 2);
-            else if (pairs)
-                k_sp2_step16<<<nt64, 128, dgemm_smem_bytes(), s>>>(dj, d64, nt64, dsst);
-            else
-                k_sp2_step8<<<nt64, 128, dgemm_smem_bytes(), s>>>(dj, d64, nt64, dsst);
-        } else if (precision == 3) {
-            k_sp2_step_oz<<<ntoz, 128, oz_smem_bytes(), s>>>(dj, (const GemmTile*)(D + o_toz), ntoz, dsst, dact + 2);
-        } else if (precision == 2) {
-            k_sp2_step_tf32<<<nt64, 128, tf32_smem_bytes(), s>>>(dj, d64, nt64, dsst);
-        } else if (precision == 4) {
-            k_sp2_step_tc1<<<nt128, 128, tc1_smem_bytes(), s>>>(dj, d128, nt128, dsst, (const TmaDesc*)(D + o_xfmaps), dact + 2);
+    if (precision == 0) {  // the whole purification in one launch (the list is the one job, 0)
+        CK(cudaMemsetAsync(D + o_list, 0, sizeof(int), s));
+        const int* list = (const int*)(D + o_list);
+        int* need = (int*)(D + o_need);
+        double* work = (double*)(D + o_work);
+        int max_steps = kSp2MaxSteps;
+        const size_t smem = sp2_fused_smem_bytes(n, jb.fused == FU_RES);
+        if (jb.fused == FU_RES) {
+            k_sp2_res<<<1, 256, smem, s>>>(dj, list, dsst, dms, need, work, max_steps);
+            CK(cudaGetLastError());
         } else {
-            k_sp2_step_tc<<<nt128, 128, tc_smem_bytes(), s>>>(dj, d128, nt128, dsst, dact + 2);
+            void* args[] = {&dj, &list, &dsst, &dms, &need, &work, &max_steps};
+            CK(launch_clusters((const void*)k_sp2_clu, sp2_cluster_for(1), 1, 256, smem, s, args));
         }
-        CK(cudaMemsetAsync(dact, 0, sizeof(int), s));
-        k_sp2_update<<<1, 32 * SP2_UPDATE_WARPS, 0, s>>>(dj, dsst, 1, kSp2MaxSteps, dact, (double*)(D + o_work));
+    } else {
+        k_sp2_bounds<<<1, 512, 3 * sizeof(double) * n, s>>>(dj, dms);
+        k_sp2_init<<<dim3(nblk, 1), 256, 0, s>>>(dj, dsst, dms, nblk);
+        k_sp2_start<<<1, 32 * SP2_UPDATE_WARPS, 0, s>>>(dj, dsst, dms, 1, nblk);
         CK(cudaGetLastError());
-        if (step >= 12 && (step % 6) == 5) {
-            CK(cudaMemcpyAsync(hact, dact, 16, cudaMemcpyDeviceToHost, s));
-            CK(cudaStreamSynchronize(s));
-            if (hact[0] == 0) break;
+        for (int step = 0; step < kSp2MaxSteps; ++step) {
+            if (precision == 3) {
+                k_sp2_step_oz<<<ntoz, 128, oz_smem_bytes(), s>>>(dj, (const GemmTile*)(D + o_toz), ntoz, dsst, dact + 2);
+            } else if (precision == 2) {
+                k_sp2_step_tf32<<<nt64, 128, tf32_smem_bytes(), s>>>(dj, d64, nt64, dsst);
+            } else if (precision == 4) {
+                k_sp2_step_tc1<<<nt128, 128, tc1_smem_bytes(), s>>>(dj, d128, nt128, dsst, (const TmaDesc*)(D + o_xfmaps), dact + 2);
+            } else {
+                k_sp2_step_tc<<<nt128, 128, tc_smem_bytes(), s>>>(dj, d128, nt128, dsst, dact + 2);
+            }
+            CK(cudaMemsetAsync(dact, 0, sizeof(int), s));
+            k_sp2_update<<<1, 32 * SP2_UPDATE_WARPS, 0, s>>>(dj, dsst, 1, kSp2MaxSteps, dact, (double*)(D + o_work));
+            CK(cudaGetLastError());
+            if (step >= 12 && (step % 6) == 5) {
+                CK(cudaMemcpyAsync(hact, dact, 16, cudaMemcpyDeviceToHost, s));
+                CK(cudaStreamSynchronize(s));
+                if (hact[0] == 0) break;
+            }
         }
+        k_sp2_finish<<<dim3(std::max(8u, std::min(256u, cdiv(nn, 65536))), 1), 256, 0, s>>>(dj, dsst, dms, (int*)(D + o_need),
+                                                                                           (double*)(D + o_work), (int*)(D + o_stall),
+                                                                                           dact + 3);
+        CK(cudaGetLastError());
     }
-    k_sp2_finish<<<dim3(std::max(8u, std::min(256u, cdiv(nn, 65536))), 1), 256, 0, s>>>(dj, dsst, dms, (int*)(D + o_need),
-                                                                                       (double*)(D + o_work), (int*)(D + o_stall),
-                                                                                       dact + 3);
-    CK(cudaGetLastError());
     Sp2State* hs = (Sp2State*)(H + staged + 256);
     CK(cudaMemcpyAsync(hs, dsst, sizeof(Sp2State), cudaMemcpyDeviceToHost, s));
     CK(cudaMemcpyAsync(hact, dact, 16, cudaMemcpyDeviceToHost, s));
@@ -3356,6 +3520,11 @@ int am1gpu_set_stream_priority(int32_t priority) {
         w.stream = nullptr;
         CK(cudaStreamCreateWithPriority(&w.stream, cudaStreamNonBlocking, p));
         w.priority = p;
+        if (w.cap_stream) {
+            CK(cudaStreamSynchronize(w.cap_stream));
+            CK(cudaStreamDestroy(w.cap_stream));
+            w.cap_stream = nullptr;
+        }
     }
     return AM1GPU_OK;
 }

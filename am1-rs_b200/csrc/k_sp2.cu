@@ -17,6 +17,7 @@
 #include "am1gpu_internal.h"
 #include "dmma_gemm.cuh"
 #include "kernels.h"
+#include "sp2_lanczos.cuh"
 
 namespace am1 {
 
@@ -34,11 +35,6 @@ namespace cg = cooperative_groups;
 // Lanczos tridiagonal T) and w = theta_max - theta_min.  An eigenvalue left slightly outside
 // the interval maps just outside [0, 1], where the trace-correcting steps pull it back; a run
 // that still fails to converge falls back to the eigensolver.  One CTA per channel.
-constexpr int SP2_LANCZOS = 12;
-// largest widening of a reused spectral interval, as a fraction of the width of the last Lanczos run's
-constexpr double SP2_REUSE_FRAC = 0.01;
-constexpr int SP2_BOUND_THREADS = 512;
-
 __device__ double bounds_block_sum(double v, double* red) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -50,79 +46,9 @@ __device__ double bounds_block_sum(double v, double* red) {
     return t;
 }
 
-// Eigenvalues of T (m x m, diagonal a, off-diagonal b) below x.
-__device__ int lz_count(const double* a, const double* b, int m, double x) {
-    int c = 0;
-    double q = a[0] - x;
-    if (q < 0.0) ++c;
-    for (int i = 1; i < m; ++i) {
-        q = a[i] - x - b[i - 1] * b[i - 1] / (q == 0.0 ? 1e-300 : q);
-        if (q < 0.0) ++c;
-    }
-    return c;
-}
-
-// k-th smallest eigenvalue of T by bisection inside [lo, hi].
-__device__ double lz_eig(const double* a, const double* b, int m, int k, double lo, double hi) {
-    for (int it = 0; it < 200; ++it) {
-        const double mid = 0.5 * (lo + hi);
-        if (!(mid > lo && mid < hi)) break;
-        if (lz_count(a, b, m, mid) <= k) lo = mid;
-        else hi = mid;
-    }
-    return 0.5 * (lo + hi);
-}
-
-// The same eigenvalue by one warp: 32-way multisection, each round 31 Sturm counts at interior
-// points of [lo, hi] on the lanes and the interval narrowed to the gap where the count passes k (a
-// factor 32 per round; 11 rounds reach the rounding level of the bisection).  Every lane of the warp
-// calls it and gets the same value.
-__device__ double lz_eig_warp(const double* a, const double* b, int m, int k, double lo, double hi) {
-    const int lane = threadIdx.x & 31;
-    for (int round = 0; round < 11; ++round) {
-        const double h = (hi - lo) * (1.0 / 32.0);
-        if (!(h > 0.0)) break;
-        const double x = lo + h * (lane + 1);
-        const bool below = lane < 31 && lz_count(a, b, m, x) <= k;  // x <= the k-th eigenvalue
-        const unsigned ball = __ballot_sync(0xffffffffu, below);
-        const int j = ball ? 31 - __clz(ball) : -1;  // the last interior point still below it
-        const double nlo = j >= 0 ? lo + h * (j + 1) : lo;
-        const double nhi = j + 2 <= 31 ? lo + h * (j + 2) : hi;
-        lo = nlo;
-        hi = nhi;
-    }
-    return 0.5 * (lo + hi);
-}
-
-// |last component| of the unit eigenvector of T for an exterior eigenvalue: inverse iteration
-// with the shift sigma just outside the spectrum, so T - sigma I is definite and the
-// tridiagonal solve needs no pivoting.
-__device__ double lz_last_component(const double* a, const double* b, int m, double sigma) {
-    double x[SP2_LANCZOS], cp[SP2_LANCZOS], rp[SP2_LANCZOS];
-    for (int i = 0; i < m; ++i) x[i] = 1.0;
-    for (int it = 0; it < 3; ++it) {
-        double den = a[0] - sigma;
-        cp[0] = m > 1 ? b[0] / den : 0.0;
-        rp[0] = x[0] / den;
-        for (int i = 1; i < m; ++i) {
-            den = a[i] - sigma - b[i - 1] * cp[i - 1];
-            cp[i] = i + 1 < m ? b[i] / den : 0.0;
-            rp[i] = (x[i] - b[i - 1] * rp[i - 1]) / den;
-        }
-        x[m - 1] = rp[m - 1];
-        for (int i = m - 2; i >= 0; --i) x[i] = rp[i] - cp[i] * x[i + 1];
-        double nrm = 0.0;
-        for (int i = 0; i < m; ++i) nrm += x[i] * x[i];
-        nrm = sqrt(nrm);
-        if (!(nrm > 0.0) || !isfinite(nrm)) return 1.0;
-        for (int i = 0; i < m; ++i) x[i] /= nrm;
-    }
-    return fabs(x[m - 1]);
-}
-
-__global__ void __launch_bounds__(SP2_BOUND_THREADS) k_sp2_bounds(const Sp2Job* __restrict__ jobs, const MolState* __restrict__ st) {
+__global__ void __launch_bounds__(SP2_BOUND_THREADS, 2) k_sp2_bounds(const Sp2Job* __restrict__ jobs, const MolState* __restrict__ st) {
     const Sp2Job jb = jobs[blockIdx.x];
-    if (!st[jb.mol].active || !jb.fallback) return;  // large matrices: k_sp2_bounds_big
+    if (!st[jb.mol].active || !jb.fallback || sp2_fused_now(jb, st[jb.mol].lowp)) return;  // large matrices: k_sp2_bounds_big
     const int n = jb.n;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     constexpr int NW = SP2_BOUND_THREADS / 32;
@@ -422,7 +348,7 @@ __device__ void sp2_bounds_group(const Sp2Job& jb, int G, int gi, Sync sync) {
     if (gi == 0 && tid == 0) lz_interval(alpha, beta, m, glo, ghi, jb.bounds);
 }
 
-__global__ void __launch_bounds__(SP2_BOUND_THREADS) k_sp2_bounds_big(const Sp2Job* __restrict__ jobs, int job,
+__global__ void __launch_bounds__(SP2_BOUND_THREADS, 2) k_sp2_bounds_big(const Sp2Job* __restrict__ jobs, int job,
                                                                        const MolState* __restrict__ st) {
     cg::grid_group grid = cg::this_grid();
     const Sp2Job jb = jobs[job];
@@ -432,7 +358,7 @@ __global__ void __launch_bounds__(SP2_BOUND_THREADS) k_sp2_bounds_big(const Sp2J
 
 // One cluster (gridDim.x CTAs) per large matrix; blockIdx.y indexes big[], the purification jobs
 // without the eigensolver fallback.
-__global__ void __launch_bounds__(SP2_BOUND_THREADS) k_sp2_bounds_cl(const Sp2Job* __restrict__ jobs, const int* __restrict__ big,
+__global__ void __launch_bounds__(SP2_BOUND_THREADS, 2) k_sp2_bounds_cl(const Sp2Job* __restrict__ jobs, const int* __restrict__ big,
                                                                       const MolState* __restrict__ st) {
     cg::cluster_group cl = cg::this_cluster();
     const Sp2Job jb = jobs[big[blockIdx.y]];
@@ -443,7 +369,7 @@ __global__ void __launch_bounds__(SP2_BOUND_THREADS) k_sp2_bounds_cl(const Sp2Jo
 // X0 = (e_max I - F*) / (e_max - e_min); per-block partial sums of tr X0 and ||X0||_F^2.
 __global__ void k_sp2_init(const Sp2Job* __restrict__ jobs, Sp2State* __restrict__ sst, const MolState* __restrict__ st, int nblk) {
     const Sp2Job jb = jobs[blockIdx.y];
-    if (!st[jb.mol].active) return;
+    if (!st[jb.mol].active || sp2_fused_now(jb, st[jb.mol].lowp)) return;
     const int n = jb.n;
     const int nb = sp2_init_blocks(n);
     if ((int)blockIdx.x >= nb) return;
@@ -563,6 +489,10 @@ __global__ void __launch_bounds__(32 * SP2_UPDATE_WARPS) k_sp2_start(const Sp2Jo
     if (j >= njobs) return;
     const Sp2Job& jb = jobs[j];
     const MolState& ms = st[jb.mol];
+    if (sp2_fused_now(jb, ms.lowp)) {
+        if ((threadIdx.x & 31) == 0) sst[j].active = 0;
+        return;
+    }
     double tr, fr;
     sp2_sum_parts(jb.part, sp2_init_blocks(jb.n), buf[warp], tr, fr);
     if ((threadIdx.x & 31) != 0) return;
@@ -774,7 +704,7 @@ __global__ void k_sp2_finish(const Sp2Job* __restrict__ jobs, const Sp2State* __
                              int* __restrict__ need_eigen, double* __restrict__ work, int* __restrict__ big_stall,
                              int* __restrict__ big_count) {
     const Sp2Job jb = jobs[blockIdx.y];
-    if (!st[jb.mol].active) return;
+    if (!st[jb.mol].active || sp2_fused_now(jb, st[jb.mol].lowp)) return;
     const Sp2State& s = sst[blockIdx.y];
     if (!s.converged) {
         if (blockIdx.x == 0 && threadIdx.x == 0) {

@@ -101,7 +101,15 @@ struct Sp2Job {
     int oz, oz_tile0, oz_ntiles, ldq;
     int8_t* Dq0;
     int8_t* Dq1;
+    // the FP64 purifications of the channel run whole, in one launch (k_sp2_fused.cu): FU_RES one CTA with
+    // the iterates on chip, FU_CLU a cluster with the iterates in Xc (sp2_clu_doubles(n),
+    // 16-byte aligned); FU_NONE the launch-per-step kernels
+    int fused;
+    double* Xc;
 };
+enum { FU_NONE = 0, FU_RES = 1, FU_CLU = 2 };
+// this channel's purification of the iteration runs in k_sp2_res / k_sp2_clu (FP64 only)
+__host__ __device__ __forceinline__ bool sp2_fused_now(const Sp2Job& jb, int lowp) { return jb.fused != FU_NONE && !lowp; }
 constexpr int kOzPlanes = 8;  // 7-bit digits of an iterate: 2^-5 .. 2^-54
 constexpr int kOzGroups = 9;  // digit-plane products kept: i + j <= 8
 
@@ -217,6 +225,13 @@ size_t dgemm_smem_bytes();
 __global__ void k_sp2_update(const Sp2Job* jobs, Sp2State* sst, int njobs, int max_steps, int* active_count, double* work);
 __global__ void k_sp2_update_cond(const Sp2Job* jobs, Sp2State* sst, int njobs, int max_steps, double* work, cudaGraphConditionalHandle h,
                                   GraphLoop* loop);
+// one whole FP64 purification per channel job of list[] (k_sp2_res: grid count; k_sp2_clu: grid (C, count) in
+// clusters of C CTAs), sp2_fused_smem_bytes(largest n, res) of dynamic shared memory, 256 threads
+constexpr int FU_RES_MAX = 112;
+__global__ void k_sp2_res(const Sp2Job* jobs, const int* list, Sp2State* sst, const MolState* st, int* need_eigen, double* work, int max_steps);
+__global__ void k_sp2_clu(const Sp2Job* jobs, const int* list, Sp2State* sst, const MolState* st, int* need_eigen, double* work, int max_steps);
+size_t sp2_fused_smem_bytes(int n, bool res);
+long long sp2_clu_doubles(int n);
 size_t tc_smem_bytes();
 size_t tc1_smem_bytes();
 size_t oz_smem_bytes();
