@@ -297,6 +297,7 @@ struct Mem {
     std::vector<cudaEvent_t> events;  // timing events, reused across calls
     cudaStream_t cap_stream = nullptr;  // stream the SCF graph is captured on, and the one-launch purifications' own in the host-driven loop
     cudaEvent_t fork = nullptr, join = nullptr;  // order the two streams in the host-driven loop
+    std::vector<cudaStream_t> pipes;  // streams of the transfer pipelines (g_matrix_batch)
 };
 
 // Stream priority asked for by the calling host thread (am1gpu_set_stream_priority).
@@ -334,6 +335,7 @@ void mem_release(Mem& w) {
     for (auto e : w.events) cudaEventDestroy(e);
     if (w.stream) cudaStreamDestroy(w.stream);
     if (w.cap_stream) cudaStreamDestroy(w.cap_stream);
+    for (auto q : w.pipes) cudaStreamDestroy(q);
     if (w.fork) cudaEventDestroy(w.fork);
     if (w.join) cudaEventDestroy(w.join);
     w = Mem();
@@ -808,6 +810,7 @@ struct Batch {
     int* d_big_stall = nullptr;  // per channel job: 1 when a large molecule's purification stalled this iteration
     GraphLoop* d_loop = nullptr;  // loop counters of the captured solve
     GraphLoop* h_loop = nullptr;  // their pinned host copy
+    char *d_extra = nullptr, *h_extra = nullptr;  // the caller's own regions (build_batch's extra_dev, extra_host)
     // kernels per captured head (+ arm), step (+ condition), tail (+ its two control kernels), and
     // stalled-purification eigensolver (run in GraphLoop::eig_runs iterations)
     int64_t graph_counts[4] = {0, 0, 0, 0};
@@ -817,7 +820,8 @@ struct Batch {
 
 // Lays out the batch in one device pool and one pinned staging area, copies inputs.
 int build_batch(const am1gpu_molecule* in, const am1gpu_options& o, std::vector<MolPlan>&& plans, Batch& b, Mem& mem,
-                am1gpu_call_stats* stats, double spin_scale_override = -1.0, const DevElem* host_tab = nullptr) {
+                am1gpu_call_stats* stats, double spin_scale_override = -1.0, const DevElem* host_tab = nullptr,
+                size_t extra_dev = 0, size_t extra_host = 0) {
     b.plans = std::move(plans);
     b.nmol = (int)b.plans.size();
     const int method = o.method == AM1GPU_METHOD_RM1 ? 1 : 0;
@@ -935,6 +939,7 @@ int build_batch(const am1gpu_molecule* in, const am1gpu_options& o, std::vector<
     const size_t o_loop = take(dv, sizeof(GraphLoop));
     const size_t o_dq = take(dv, (size_t)std::max<long long>(dq_bytes, 16));
     const size_t o_xc = take(dv, sizeof(double) * (size_t)std::max<long long>(clu_doubles, 2));
+    const size_t o_extra = take(dv, extra_dev);
     const size_t dtotal = align256(dv);
     // pinned staging also receives the outputs
     size_t hs = staged;
@@ -945,6 +950,7 @@ int build_batch(const am1gpu_molecule* in, const am1gpu_options& o, std::vector<
     const size_t h_o_eps = take(hs, sizeof(double) * std::max<long long>(eps_total, 1));
     const size_t h_o_grad = take(hs, sizeof(double) * 3 * std::max<long long>(natoms, 1));
     const size_t h_o_loop = take(hs, sizeof(GraphLoop));
+    const size_t h_o_extra = take(hs, extra_host);
     int rc = mem_ensure(mem, dtotal, align256(hs));
     if (rc) return rc;
     Mem* ws = &mem;
@@ -1004,6 +1010,8 @@ int build_batch(const am1gpu_molecule* in, const am1gpu_options& o, std::vector<
     b.d_big_stall = (int*)dptr(o_bstall);
     b.d_loop = (GraphLoop*)dptr(o_loop);
     b.h_loop = (GraphLoop*)(Hs + h_o_loop);
+    b.d_extra = D + o_extra;
+    b.h_extra = Hs + h_o_extra;
     b.eps_total = eps_total;
     b.h_active = (int*)(Hs + h_o_active);
     b.h_work = (double*)(Hs + h_o_work);
@@ -2517,11 +2525,20 @@ int build_fock_one(const am1gpu_molecule* mol, int method, const double* p_tot, 
 }
 
 // G(P_r) = J(P_r) - K(P_r / 2) for nrhs densities of one molecule (build_g_matrix,
-// src/fock.rs:556-575, FockBase::Zero).  The right-hand sides become copies of the molecule in one
-// batch, in chunks of at most kGChunk, each with its own closed-shell channel: the pair integrals
-// are formed once per copy (cheap next to the Fock build), H_core is zeroed, and one k_fock launch
-// builds every copy's matrix, so F = 0 + J(P_r) - 1/2 K(P_r) exactly.
-constexpr int kGChunk = 64;
+// src/fock.rs:556-575, FockBase::Zero).  The pair integrals are formed once; the right-hand sides are
+// copies of the molecule that share them and a zero H_core, each with its own closed-shell channel, so
+// k_fock builds F = 0 + J(P_r) - 1/2 K(P_r) exactly.
+//
+// The arithmetic is 1% of the call: it is bound by moving the matrices between the caller's pageable
+// memory and the device (2 x 85 MB for 288 matrices of 192 orbitals).  They go in chunks of about
+// kGChunkBytes through up to kGPipes pipelines, a host thread, a stream and a pinned slot each: one
+// pipeline's copies to and from its slot overlap the others' transfers and kernels, and the reordering to and from
+// the internal AO order runs on the device.  One matrix at a time, reordered on the host with a pageable
+// copy and a synchronisation each, took 60 ms for those 288; now 15, most of it the first touch of the result's
+// pages (4 to 16 pipelines, chunks of 1 to 4 MB: 14.9 to 16.7 ms).
+constexpr size_t kGChunkBytes = 2u << 20;
+constexpr int kGPipes = 8;
+constexpr size_t kGPinnedMax = 64u << 20;  // pinned memory of all slots; larger matrices go straight from and to the caller's
 
 int g_matrix_batch(const am1gpu_molecule* mol, int method, int nrhs, const double* dens, double* g) {
     g_err.clear();
@@ -2543,43 +2560,117 @@ int g_matrix_batch(const am1gpu_molecule* mol, int method, int nrhs, const doubl
     MolPlan p;
     rc = plan_molecule(m, o, 0, p);
     if (rc) return rc;
-    const int n = p.nao;
-    const size_t nn = (size_t)n * n;
+    const int n = p.nao, natoms = p.natoms;
+    const size_t nn = (size_t)n * n, bytes = sizeof(double) * nn;
+    // matrices per chunk, and pipelines
+    const int R = (int)std::max<size_t>(1, std::min<size_t>({(size_t)nrhs, kGChunkBytes / bytes, (size_t)64}));
+    const int chunks = (nrhs + R - 1) / R;
+    const bool pinned = bytes * R <= kGPinnedMax;
+    const int pipes = !pinned ? 1
+                              : (int)std::min<size_t>({(size_t)chunks, (size_t)kGPipes, kGPinnedMax / (bytes * R),
+                                                       (size_t)std::max(1u, std::thread::hardware_concurrency())});
+    // device: the copies' records, then per pipeline [zero H | R x (F, FX, P) | R matrices in the caller's order]
+    const size_t arena_doubles = nn * (1 + 3 * (size_t)R), pipe_doubles = arena_doubles + nn * R;
+    size_t off = 0;
+    auto take = [&off](size_t sz) {
+        off = align256(off);
+        const size_t o2 = off;
+        off += sz;
+        return o2;
+    };
+    const size_t o_mols = take(sizeof(MolDesc) * R), o_am = take(sizeof(int) * (size_t)R * natoms), o_z = take(sizeof(int) * (size_t)R * natoms),
+                 o_map = take(sizeof(int) * 2 * (size_t)n), records = align256(off), o_pipe = take(sizeof(double) * pipe_doubles * pipes);
     Workspace* ws;
     tl_stats = am1gpu_call_stats{};
     rc = workspace(&ws, 0, 0);
     if (rc) return rc;
-    std::vector<double> t(nn);
-    for (int r0 = 0; r0 < nrhs; r0 += kGChunk) {
-        const int cnt = std::min(kGChunk, nrhs - r0);
-        std::vector<am1gpu_molecule> copies(cnt, m);
-        std::vector<MolPlan> plans(cnt, p);
-        for (int c = 0; c < cnt; ++c) plans[c].user = c;
-        Batch b;
-        rc = build_batch(copies.data(), o, std::move(plans), b, *ws, &tl_stats);
-        if (!rc) rc = launch_core(b, ws, ctx->d_params, nullptr);
-        if (rc) return rc;
-        const auto& map = b.plans[0].ao_map;
-        for (int c = 0; c < cnt; ++c) {
-            const double* pr = dens + (size_t)(r0 + c) * nn;
-            for (int i = 0; i < n; ++i)
-                for (int j = 0; j < n; ++j) t[(size_t)i * n + j] = pr[(size_t)map[i] * n + map[j]];
-            CK(cudaMemcpyAsync(b.jobs[c].P, t.data(), sizeof(double) * nn, cudaMemcpyHostToDevice, ws->stream));
-            CK(cudaMemsetAsync(const_cast<double*>(b.jobs[c].H), 0, sizeof(double) * nn, ws->stream));  // the copy's own H_core
-            CK(cudaStreamSynchronize(ws->stream));  // t is reused for the next copy
+    std::vector<MolPlan> plans{p};
+    Batch b;
+    rc = build_batch(&m, o, std::move(plans), b, *ws, &tl_stats, -1.0, nullptr, align256(off), records + (pinned ? bytes * R * pipes : 0));
+    if (rc) return rc;
+    while ((int)ws->pipes.size() < pipes) {
+        cudaStream_t q;
+        CK(cudaStreamCreateWithPriority(&q, cudaStreamNonBlocking, ws->priority));
+        ws->pipes.push_back(q);
+    }
+    if ((rc = mem_side_stream(*ws))) return rc;
+    {
+        MolDesc* hm = (MolDesc*)(b.h_extra + o_mols);
+        int *ham = (int*)(b.h_extra + o_am), *hz = (int*)(b.h_extra + o_z), *hmap = (int*)(b.h_extra + o_map);
+        for (int c = 0; c < R; ++c) {
+            hm[c] = b.mols[0];
+            hm[c].atom_base = c * natoms;
+            hm[c].h_base = 0;
+            hm[c].ch_base[0] = (long long)(nn * (1 + 3 * (size_t)c));  // slots F, FX (not used) and P
+            for (int a = 0; a < natoms; ++a) {
+                ham[c * natoms + a] = c;
+                hz[c * natoms + a] = m.z[p.order[a]];
+            }
         }
-        k_fock<<<cdiv(b.natoms, 8), 256, 0, ws->stream>>>(b.d_mols, b.d_atom_mol, b.natoms, ctx->d_params, b.d_atom_z, b.d_wstore,
-                                                          b.d_arena, b.d_st, 1);
-        CK(cudaGetLastError());
-        tl_stats.kernel_launches += 1;
-        for (int c = 0; c < cnt; ++c) {
-            rc = fetch_matrix(ws, b.jobs[c].F, n, t, &tl_stats);
-            if (rc) return rc;
-            double* gr = g + (size_t)(r0 + c) * nn;
-            for (int i = 0; i < n; ++i)
-                for (int j = 0; j < n; ++j) gr[(size_t)map[i] * n + map[j]] = t[(size_t)i * n + j];
+        for (int i = 0; i < n; ++i) {  // internal AO -> caller's, and back
+            hmap[i] = p.ao_map[i];
+            hmap[n + p.ao_map[i]] = i;
+        }
+        CK(cudaMemcpyAsync(b.d_extra, b.h_extra, records, cudaMemcpyHostToDevice, ws->stream));
+        tl_stats.h2d_bytes += (int64_t)records;
+    }
+    if ((rc = launch_core(b, ws, ctx->d_params, nullptr))) return rc;
+    CK(cudaEventRecord(ws->fork, ws->stream));
+    const MolDesc* dm = (const MolDesc*)(b.d_extra + o_mols);
+    const int *dam = (const int*)(b.d_extra + o_am), *dz = (const int*)(b.d_extra + o_z), *dmap = (const int*)(b.d_extra + o_map);
+    int dev = 0;
+    CK(cudaGetDevice(&dev));
+    std::atomic<int> next{0}, failed{0};
+    std::mutex mu;
+    std::string msg;
+    // one pipeline: takes chunks until none is left
+    auto pipeline = [&](int k) -> int {
+        CK(cudaSetDevice(dev));
+        const cudaStream_t s = ws->pipes[k];
+        CK(cudaStreamWaitEvent(s, ws->fork, 0));
+        double* arena = (double*)(b.d_extra + o_pipe) + pipe_doubles * k;
+        double* raw = arena + arena_doubles;
+        double* slot = (double*)(b.h_extra + records) + nn * R * k;
+        CK(cudaMemsetAsync(arena, 0, bytes, s));
+        for (int c; !failed.load() && (c = next.fetch_add(1)) < chunks;) {
+            const int r0 = c * R, cnt = std::min(R, nrhs - r0);
+            const double* src = dens + (size_t)r0 * nn;
+            double* dst = g + (size_t)r0 * nn;
+            if (pinned) std::memcpy(slot, src, bytes * cnt);
+            CK(cudaMemcpyAsync(raw, pinned ? slot : src, bytes * cnt, cudaMemcpyHostToDevice, s));
+            k_permute_square<<<dim3(n, cnt), 128, 0, s>>>(raw, (long long)nn, arena + nn * (1 + SLOT_P), (long long)(3 * nn), dmap, n);
+            k_fock<<<cdiv((long long)cnt * natoms, 8), 256, 0, s>>>(dm, dam, cnt * natoms, ctx->d_params, dz, b.d_wstore, arena, b.d_st, 1);
+            k_permute_square<<<dim3(n, cnt), 128, 0, s>>>(arena + nn * (1 + SLOT_F), (long long)(3 * nn), raw, (long long)nn, dmap + n, n);
+            CK(cudaGetLastError());
+            CK(cudaMemcpyAsync(pinned ? slot : dst, raw, bytes * cnt, cudaMemcpyDeviceToHost, s));
+            CK(cudaStreamSynchronize(s));
+            if (pinned) std::memcpy(dst, slot, bytes * cnt);
+        }
+        return AM1GPU_OK;
+    };
+    auto guarded = [&](int k) {
+        const int r = pipeline(k);
+        if (r) {
+            std::lock_guard<std::mutex> lock(mu);
+            if (!failed.exchange(r)) msg = g_err;
+        }
+        cudaStreamSynchronize(ws->pipes[k]);
+    };
+    std::vector<std::thread> pool;
+    for (int k = 1; k < pipes; ++k) {
+        try {
+            pool.emplace_back(guarded, k);
+        } catch (...) {  // no thread to be had: the pipelines there are take every chunk
+            break;
         }
     }
+    guarded(0);
+    for (auto& th : pool) th.join();
+    if (failed.load()) return fail(failed.load(), msg);
+    CK(cudaStreamSynchronize(ws->stream));
+    tl_stats.kernel_launches += 3LL * chunks;
+    tl_stats.h2d_bytes += (int64_t)(bytes * nrhs);
+    tl_stats.d2h_bytes += (int64_t)(bytes * nrhs);
     return AM1GPU_OK;
 }
 

@@ -274,4 +274,15 @@ __global__ void __launch_bounds__(32 * FOCK_WARPS, 2) k_fock(const MolDesc* __re
     }
 }
 
+// Rows and columns of a stack of square matrices into another AO order.  The maps keep each atom's AOs
+// together, so a row's reads are runs of a heavy atom's four words and single words of hydrogens, within one
+// row that L1 holds; the writes are contiguous.  Bound by its two passes over memory.
+__global__ void __launch_bounds__(128) k_permute_square(const double* __restrict__ in, long long si, double* __restrict__ out,
+                                                        long long so, const int* __restrict__ map, int n) {
+    const int i = blockIdx.x;
+    const double* row = in + blockIdx.y * si + (long long)map[i] * n;
+    double* dst = out + blockIdx.y * so + (long long)i * n;
+    for (int j = threadIdx.x; j < n; j += 128) dst[j] = row[map[j]];
+}
+
 }  // namespace am1

@@ -172,6 +172,9 @@ __global__ void k_gradient(const MolDesc* mols, const int* atom_mol, int natoms_
                            const double* atom_xyz, const ChanJob* jobs, const int* mol_job0, double* gradient, int* mol_status);
 __global__ void k_fock(const MolDesc* mols, const int* atom_mol, int natoms_total, const DevElem* params,
                        const int* atom_z, const double* wstore, double* arena, const MolState* st, int force);
+// out_r[i][j] = in_r[map[i]][map[j]] for matrices r = blockIdx.y, n x n, at strides so and si (doubles);
+// grid (n, count), 128 threads: a CTA per row
+__global__ void k_permute_square(const double* in, long long si, double* out, long long so, const int* map, int n);
 // C = alpha A B (A row-major M x K) and C = alpha A^T B (A stored K x M)
 // mask (optional): only molecules with mask[mol] != 0 take part
 __global__ void k_gemm_nn(const GemmJob* jobs, const GemmTile* tiles, int ntiles, const MolState* st, int force, const int* mask);
