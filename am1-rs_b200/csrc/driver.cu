@@ -753,7 +753,17 @@ struct Batch {
     int nt_gt = 0, nt_dn = 0;
     EigJob* d_eig;
     int neig = 0;
-    struct Bucket { int off, count, C; size_t smem; };
+    struct Bucket {
+        int off, count, C;
+        size_t smem;
+        int threads = 0;  // eigensolver jobs
+        void add(int n, int npad) {  // one more eigensolver job
+            ++count;
+            const size_t two = jacobi_smem_bytes2(n, npad, C);
+            smem = std::max(smem, C > 1 && two <= (size_t)g_jacobi_budget ? two : jacobi_smem_bytes(n, npad, C));
+            threads = std::max(threads, jacobi_threads(npad, C));
+        }
+    };
     std::vector<Bucket> buckets;      // eigensolver jobs by cluster size
     std::vector<Bucket> tri_buckets;  // tridiagonalisation jobs by cluster size
     std::vector<TriJob> tri_big;      // matrices too large for a cluster's shared memory (d_tri[0 .. count))
@@ -1298,10 +1308,8 @@ int build_batch(const am1gpu_molecule* in, const am1gpu_options& o, std::vector<
     for (size_t i = 0; i < idx.size(); ++i) {
         heig[i] = eig_all[idx[i]];
         const int C = eig_cluster[idx[i]];
-        const size_t sm = jacobi_smem_bytes(eig_all[idx[i]].n, eig_all[idx[i]].npad, C);
         if (b.buckets.empty() || b.buckets.back().C != C) b.buckets.push_back({(int)i, 0, C, 0});
-        b.buckets.back().count++;
-        b.buckets.back().smem = std::max(b.buckets.back().smem, sm);
+        b.buckets.back().add(eig_all[idx[i]].n, eig_all[idx[i]].npad);
     }
     b.neig = (int)idx.size();
     // tridiagonalisation jobs grouped by cluster size, largest first
@@ -1591,23 +1599,27 @@ int launch_big_tridiag(Batch& b, cudaStream_t s, int64_t* launches) {
 }
 
 // stream: where to launch (NULL: the workspace's own stream)
+int launch_jacobi_bucket(const Batch::Bucket& bk, const EigJob* jobs, const MolState* st, int* status, int force, const int* mask,
+                         cudaStream_t s) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(bk.count * bk.C, 1, 1);
+    cfg.blockDim = dim3(bk.threads, 1, 1);
+    cfg.dynamicSmemBytes = bk.smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = bk.C;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    CK(cudaLaunchKernelEx(&cfg, k_jacobi, jobs + bk.off, st, status, force, mask));
+    return AM1GPU_OK;
+}
+
 int launch_jacobi(Batch& b, Mem* ws, int force, const int* mask = nullptr, cudaStream_t stream = nullptr) {
-    for (auto& bk : b.buckets) {
-        cudaLaunchConfig_t cfg{};
-        cfg.gridDim = dim3(bk.count * bk.C, 1, 1);
-        cfg.blockDim = dim3(256, 1, 1);
-        cfg.dynamicSmemBytes = bk.smem;
-        cfg.stream = stream ? stream : ws->stream;
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = bk.C;
-        attr[0].val.clusterDim.y = 1;
-        attr[0].val.clusterDim.z = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
-        CK(cudaLaunchKernelEx(&cfg, k_jacobi, (const EigJob*)(b.d_eig + bk.off), (const MolState*)b.d_st, b.d_status, force,
-                              mask));
-    }
+    for (auto& bk : b.buckets)
+        if (int rc = launch_jacobi_bucket(bk, b.d_eig, b.d_st, b.d_status, force, mask, stream ? stream : ws->stream)) return rc;
     return AM1GPU_OK;
 }
 
@@ -3044,6 +3056,138 @@ int density_purify_one(int n, const double* F, double nocc, double weight, int p
     return AM1GPU_OK;
 }
 
+// Eigenproblems of the cluster Jacobi's sizes (n <= 448): the caller's matrices and outputs, and the result code.
+struct SmallEig {
+    int i, n, npad, C;
+    const double* a;
+    double *w, *v;
+    int code = AM1GPU_OK;  // LINALG when the matrix is not finite (then bad) or Jacobi did not converge
+    bool bad = false;
+};
+
+// All of them in one call.  They go by cluster size, each group on a stream of its own: its matrices are
+// staged and copied, prepared (mirrored, bounds, identity) on the device, solved, sorted and turned into columns
+// there, and fetched, so one group's copies and host staging run under the others' solves and the groups share the
+// SMs.  One group after the other on one stream, prepared and transposed on the host, took 94 ms for 96
+// matrices of 24 to 320 rows; now 30.
+int jacobi_eigen_small(std::vector<SmallEig>& items, Mem& mem) {
+    if (items.empty()) return AM1GPU_OK;
+    std::stable_sort(items.begin(), items.end(), [](const SmallEig& x, const SmallEig& y) { return x.C != y.C ? x.C > y.C : x.n > y.n; });
+    const int m = (int)items.size();
+    struct Group {
+        Batch::Bucket bk;
+        int nmax = 0;
+        size_t in0, in1, out0, out1;
+    };
+    std::vector<Group> groups;
+    size_t off = 0;
+    auto take = [&off](size_t bytes) {
+        off = align256(off);
+        const size_t o2 = off;
+        off += bytes;
+        return o2;
+    };
+    // staged: records, then the matrices; fetched: two codes per matrix, then w and v; device only: the rest
+    const size_t o_job = take(sizeof(EigJob) * m), o_prep = take(sizeof(EigPrep) * m), o_st = take(sizeof(MolState) * m),
+                 records = align256(off);
+    std::vector<size_t> o_a(m), o_out(m), o_dev(m);
+    for (int k = 0; k < m; ++k) o_a[k] = take(sizeof(double) * items[k].n * items[k].n);
+    const size_t o_code = take(sizeof(int) * 2 * m);
+    for (int k = 0; k < m; ++k) o_out[k] = take(sizeof(double) * ((size_t)items[k].n * items[k].n + items[k].n));
+    const size_t host_bytes = align256(off);
+    for (int k = 0; k < m; ++k) {
+        const size_t n = items[k].n, np = items[k].npad;
+        o_dev[k] = take(sizeof(double) * (2 * n * n + np * n + 2 * np + n));  // Gt, Ct, Vs, lam, column ids, rowmin
+    }
+    int rc = mem_ensure(mem, align256(off), host_bytes);
+    if (rc) return rc;
+    if ((rc = mem_side_stream(mem))) return rc;
+    char *D = mem.dpool, *H = mem.hpin;
+    EigJob* hj = (EigJob*)(H + o_job);
+    EigPrep* hp = (EigPrep*)(H + o_prep);
+    MolState* hs = (MolState*)(H + o_st);
+    for (int k = 0; k < m; ++k) {
+        const SmallEig& it = items[k];
+        const size_t n = it.n, np = it.npad;
+        double* gt = (double*)(D + o_dev[k]);
+        double *ct = gt + n * n, *vs = ct + n * n, *lam = vs + np * n, *ids = lam + np, *rmin = ids + np;
+        double* out = (double*)(D + o_out[k]);
+        hp[k] = EigPrep{(const double*)(D + o_a[k]), gt, ct, rmin, out + n, it.n};
+        hj[k] = EigJob{};
+        hj[k].Gt = gt;
+        hj[k].Ct = ct;
+        hj[k].Vs = vs;
+        hj[k].lam = lam;
+        hj[k].colid_out = (int*)ids;
+        hj[k].eps = out;
+        hj[k].Ct_out = ct;
+        hj[k].rowmin = rmin;
+        hj[k].n = it.n;
+        hj[k].npad = it.npad;
+        hj[k].mol = k;
+        hs[k] = MolState{};
+        hs[k].active = 1;
+        if (groups.empty() || groups.back().bk.C != it.C) groups.push_back(Group{{k, 0, it.C, 0}, 0, o_a[k], 0, o_out[k], 0});
+        Group& gr = groups.back();
+        gr.bk.add(it.n, it.npad);
+        gr.nmax = std::max(gr.nmax, it.n);
+        gr.in1 = o_a[k] + sizeof(double) * n * n;
+        gr.out1 = o_out[k] + sizeof(double) * (n * n + n);
+    }
+    while (mem.pipes.size() < groups.size()) {
+        cudaStream_t q;
+        CK(cudaStreamCreateWithPriority(&q, cudaStreamNonBlocking, mem.priority));
+        mem.pipes.push_back(q);
+    }
+    const EigJob* dj = (const EigJob*)(D + o_job);
+    const EigPrep* dp = (const EigPrep*)(D + o_prep);
+    int *bad = (int*)(D + o_code), *status = bad + m;
+    CK(cudaMemcpyAsync(D, H, records, cudaMemcpyHostToDevice, mem.stream));
+    CK(cudaMemsetAsync(bad, 0, sizeof(int) * 2 * m, mem.stream));
+    CK(cudaEventRecord(mem.fork, mem.stream));
+    auto enqueue = [&](size_t gi) -> int {
+        const Group& gr = groups[gi];
+        const cudaStream_t s = mem.pipes[gi];
+        const int k0 = gr.bk.off, cnt = gr.bk.count;
+        CK(cudaStreamWaitEvent(s, mem.fork, 0));
+        for (int k = k0; k < k0 + cnt; ++k) std::memcpy(H + o_a[k], items[k].a, sizeof(double) * items[k].n * items[k].n);
+        CK(cudaMemcpyAsync(D + gr.in0, H + gr.in0, gr.in1 - gr.in0, cudaMemcpyHostToDevice, s));
+        const unsigned tiles = cdiv(gr.nmax, 32);
+        k_eig_mirror<<<dim3(tiles, tiles, cnt), dim3(32, 8), 0, s>>>(dp + k0, bad + k0);
+        k_eig_rowmin<<<dim3(cdiv(gr.nmax, 128), cnt), 128, 0, s>>>(dp + k0);
+        CK(cudaGetLastError());
+        if (int r = launch_jacobi_bucket(gr.bk, dj, (const MolState*)(D + o_st), status, 1, nullptr, s)) return r;
+        k_eig_sort<<<cnt, 512, 0, s>>>(dj + k0, (const MolState*)(D + o_st), 1, nullptr);
+        k_eig_columns<<<dim3(tiles, tiles, cnt), dim3(32, 8), 0, s>>>(dp + k0);
+        CK(cudaGetLastError());
+        CK(cudaMemcpyAsync(H + gr.out0, D + gr.out0, gr.out1 - gr.out0, cudaMemcpyDeviceToHost, s));
+        CK(cudaMemcpyAsync(H + o_code + sizeof(int) * k0, bad + k0, sizeof(int) * cnt, cudaMemcpyDeviceToHost, s));
+        CK(cudaMemcpyAsync(H + o_code + sizeof(int) * (m + k0), status + k0, sizeof(int) * cnt, cudaMemcpyDeviceToHost, s));
+        return AM1GPU_OK;
+    };
+    for (size_t gi = 0; gi < groups.size() && !rc; ++gi) rc = enqueue(gi);
+    // the smallest cluster's matrices are done first
+    for (size_t gi = groups.size(); gi-- > 0;) {
+        const cudaError_t e = cudaStreamSynchronize(mem.pipes[gi]);
+        if (rc) continue;
+        CK(e);
+        const Group& gr = groups[gi];
+        for (int k = gr.bk.off; k < gr.bk.off + gr.bk.count; ++k) {
+            SmallEig& it = items[k];
+            const int* code = (const int*)(H + o_code);
+            it.bad = code[k] != 0;
+            if (it.bad || code[m + k]) {
+                it.code = AM1GPU_LINALG;
+                continue;
+            }
+            const double* out = (const double*)(H + o_out[k]);
+            std::memcpy(it.w, out, sizeof(double) * it.n);
+            std::memcpy(it.v, out + it.n, sizeof(double) * it.n * it.n);
+        }
+    }
+    return rc;
+}
+
 int symmetric_eigen_one(int n, const double* a, double* w, double* v, Mem* mem_override = nullptr) {
     g_err.clear();
     if (n < 0 || (n > 0 && (!a || !w || !v))) return fail(AM1GPU_INVALID_INPUT, "null argument");
@@ -3062,78 +3206,11 @@ int symmetric_eigen_one(int n, const double* a, double* w, double* v, Mem* mem_o
         if (n > kMaxAo) return fail(AM1GPU_UNSUPPORTED, "matrix with " + std::to_string(n) + " rows exceeds " + std::to_string(kMaxAo));
         return symmetric_eigen_large(n, a, w, v, mem_override);
     }
-    // layout: Gt (n*n, the lower triangle mirrored), Ct (n*n identity), Vs (npad*n), lam, colid, eps, rowmin, state
-    const size_t nn = (size_t)n * n;
-    size_t off = 0;
-    auto take = [&off](size_t bytes) {
-        off = align256(off);
-        const size_t o2 = off;
-        off += bytes;
-        return o2;
-    };
-    const size_t o_g = take(nn * 8), o_c = take(nn * 8), o_v = take((size_t)npad * n * 8), o_l = take(npad * 8),
-                 o_id = take(npad * 4), o_e = take(n * 8), o_r = take(n * 8), o_st = take(sizeof(MolState)),
-                 o_status = take(16), o_job = take(sizeof(EigJob));
-    Workspace* ws;
-    if (mem_override) {
-        rc = mem_ensure(*mem_override, align256(off), align256(off));
-        ws = mem_override;
-    } else {
-        rc = workspace(&ws, align256(off), align256(off));
-    }
-    if (rc) return rc;
-    char* D = ws->dpool;
-    char* Hh = ws->hpin;
-    double* g = (double*)(Hh + o_g);
-    double* c = (double*)(Hh + o_c);
-    double* rmin = (double*)(Hh + o_r);
-    for (int i = 0; i < n; ++i) {
-        double bound = 0.0;
-        for (int j = 0; j < n; ++j) {
-            const double x = i >= j ? a[(size_t)i * n + j] : a[(size_t)j * n + i];  // lower triangle
-            g[(size_t)i * n + j] = x;
-            c[(size_t)i * n + j] = i == j ? 1.0 : 0.0;
-            if (i != j) bound += std::fabs(x);
-        }
-        rmin[i] = g[(size_t)i * n + i] - bound;
-    }
-    MolState* hs = (MolState*)(Hh + o_st);
-    *hs = MolState{};
-    hs->active = 1;
-    EigJob* ej = (EigJob*)(Hh + o_job);
-    *ej = EigJob{};
-    ej->Gt = (double*)(D + o_g);
-    ej->Ct = (double*)(D + o_c);
-    ej->Vs = (double*)(D + o_v);
-    ej->lam = (double*)(D + o_l);
-    ej->colid_out = (int*)(D + o_id);
-    ej->eps = (double*)(D + o_e);
-    ej->Ct_out = (double*)(D + o_c);
-    ej->rowmin = (double*)(D + o_r);
-    ej->n = n;
-    ej->npad = npad;
-    ej->mol = 0;
-    std::memset(Hh + o_status, 0, 16);
-    CK(cudaMemcpyAsync(D, Hh, align256(off), cudaMemcpyHostToDevice, ws->stream));
-    Batch b;
-    b.d_eig = (EigJob*)(D + o_job);
-    b.d_st = (MolState*)(D + o_st);
-    b.d_status = (int*)(D + o_status);
-    b.buckets = {{0, 1, C, jacobi_smem_bytes(n, npad, C)}};
-    b.neig = 1;
-    rc = launch_jacobi(b, ws, 1);
-    if (rc) return rc;
-    k_eig_sort<<<1, 512, 0, ws->stream>>>(b.d_eig, b.d_st, 1, nullptr);
-    CK(cudaGetLastError());
-    std::vector<double> ct(nn);
-    int st = 0;
-    CK(cudaMemcpyAsync(w, D + o_e, n * 8, cudaMemcpyDeviceToHost, ws->stream));
-    CK(cudaMemcpyAsync(ct.data(), D + o_c, nn * 8, cudaMemcpyDeviceToHost, ws->stream));
-    CK(cudaMemcpyAsync(&st, D + o_status, 4, cudaMemcpyDeviceToHost, ws->stream));
-    CK(cudaStreamSynchronize(ws->stream));
-    if (st) return fail(AM1GPU_LINALG, "Jacobi eigensolver did not converge");
-    for (int k = 0; k < n; ++k)
-        for (int i = 0; i < n; ++i) v[(size_t)i * n + k] = ct[(size_t)k * n + i];
+    Workspace* ws = mem_override;
+    if (!ws && (rc = workspace(&ws, 0, 0))) return rc;
+    std::vector<SmallEig> one{{0, n, npad, C, a, w, v}};
+    if ((rc = jacobi_eigen_small(one, *ws))) return rc;
+    if (one[0].code) return fail(AM1GPU_LINALG, "Jacobi eigensolver did not converge");
     return AM1GPU_OK;
 }
 
@@ -3203,8 +3280,7 @@ int symmetric_eigenvalues_one(int n, const double* a, double* w) {
 // Many independent symmetric eigenproblems in one set of launches: the subsystem blocks of the
 // divide-and-conquer SCF (solve_subsystems, src/divide_conquer.rs:587-617), each of which the
 // reference diagonalises with its own symmetric_eigen call.  Every matrix gets the cluster Jacobi
-// job symmetric_eigen_one would give it (same cluster size, same arithmetic), the jobs are
-// grouped by cluster size and launched together, then sorted.  status[i] receives matrix i's
+// job symmetric_eigen_one gives it (jacobi_eigen_small serves both).  status[i] receives matrix i's
 // code; the return value is the first nonzero one.
 int symmetric_eigen_batch(int count, const int32_t* ns, const double* const* a, double* const* w, double* const* v, int32_t* status) {
     g_err.clear();
@@ -3218,134 +3294,45 @@ int symmetric_eigen_batch(int count, const int32_t* ns, const double* const* a, 
             first_msg = msg;
         }
     };
-    struct Item {
-        int i, n, npad, C;
-        size_t o_g, o_c, o_v, o_l, o_id, o_e, o_r;
-    };
-    std::vector<Item> items;
+    DeviceCtx* ctx = nullptr;
+    std::vector<SmallEig> items;
     std::vector<int> large;
-    size_t off = 0;
-    auto take = [&off](size_t bytes) {
-        off = align256(off);
-        const size_t o2 = off;
-        off += bytes;
-        return o2;
-    };
+    std::vector<std::pair<int, std::string>> refused(std::max(count, 0), {AM1GPU_OK, std::string()});
     for (int i = 0; i < count; ++i) {
         const int n = ns[i];
-        set(i, AM1GPU_OK, "");
         if (n < 0 || (n > 0 && (!a[i] || !w[i] || !v[i]))) {
-            set(i, AM1GPU_INVALID_INPUT, "matrix " + std::to_string(i) + ": null argument or negative size");
+            refused[i] = {AM1GPU_INVALID_INPUT, ": null argument or negative size"};
             continue;
         }
         if (n == 0) continue;
+        if (!ctx)
+            if (const int rc = device_ctx(&ctx)) return rc;
+        SmallEig it{i, n, 0, 0, a[i], w[i], v[i]};
+        if (choose_cluster(n, &it.npad, &it.C)) {
+            items.push_back(it);
+            continue;
+        }
         bool finite = true;
         for (long long k = 0; k < (long long)n * n && finite; ++k) finite = std::isfinite(a[i][k]);
-        if (!finite) {
-            set(i, AM1GPU_LINALG, "matrix " + std::to_string(i) + " handed to the eigensolver is not finite");
-            continue;
-        }
-        Item it{i, n, 0, 0};
-        if (!choose_cluster(n, &it.npad, &it.C)) {
-            if (n > kMaxAo)
-                set(i, AM1GPU_UNSUPPORTED, "matrix " + std::to_string(i) + " has more than " + std::to_string(kMaxAo) + " rows");
-            else
-                large.push_back(i);  // past the cluster Jacobi: the large-matrix path, one at a time, after the batch
-            continue;
-        }
-        const size_t nn = (size_t)n * n;
-        it.o_g = take(nn * 8);
-        it.o_c = take(nn * 8);
-        it.o_v = take((size_t)it.npad * n * 8);
-        it.o_l = take((size_t)it.npad * 8);
-        it.o_id = take((size_t)it.npad * 4);
-        it.o_e = take((size_t)n * 8);
-        it.o_r = take((size_t)n * 8);
-        items.push_back(it);
+        if (!finite)
+            refused[i] = {AM1GPU_LINALG, " handed to the eigensolver is not finite"};
+        else if (n > kMaxAo)
+            refused[i] = {AM1GPU_UNSUPPORTED, " has more than " + std::to_string(kMaxAo) + " rows"};
+        else
+            large.push_back(i);  // past the cluster Jacobi: the large-matrix path, one at a time, after the batch
     }
     if (!items.empty()) {
-        // cluster-size groups, largest clusters (and matrices) first, as the batched SCF orders them
-        std::stable_sort(items.begin(), items.end(), [](const Item& x, const Item& y) { return x.C != y.C ? x.C > y.C : x.n > y.n; });
-        const int m = (int)items.size();
-        const size_t o_st = take(sizeof(MolState) * m), o_status = take(sizeof(int) * m), o_job = take(sizeof(EigJob) * m);
-        DeviceCtx* ctx;
-        int rc = device_ctx(&ctx);
-        if (rc) return rc;
         Workspace* ws;
-        rc = workspace(&ws, align256(off), align256(off));
+        int rc = workspace(&ws, 0, 0);
+        if (!rc) rc = jacobi_eigen_small(items, *ws);
         if (rc) return rc;
-        char* D = ws->dpool;
-        char* Hh = ws->hpin;
-        Batch b;
-        b.buckets.clear();
-        for (int k = 0; k < m; ++k) {
-            const Item& it = items[k];
-            const int n = it.n;
-            const double* ak = a[it.i];
-            double* g = (double*)(Hh + it.o_g);
-            double* c = (double*)(Hh + it.o_c);
-            double* rmin = (double*)(Hh + it.o_r);
-            for (int r = 0; r < n; ++r) {
-                double bound = 0.0;
-                for (int q = 0; q < n; ++q) {
-                    const double x = r >= q ? ak[(size_t)r * n + q] : ak[(size_t)q * n + r];  // lower triangle
-                    g[(size_t)r * n + q] = x;
-                    c[(size_t)r * n + q] = r == q ? 1.0 : 0.0;
-                    if (r != q) bound += std::fabs(x);
-                }
-                rmin[r] = g[(size_t)r * n + r] - bound;
-            }
-            MolState* hs = (MolState*)(Hh + o_st) + k;
-            *hs = MolState{};
-            hs->active = 1;
-            EigJob* ej = (EigJob*)(Hh + o_job) + k;
-            *ej = EigJob{};
-            ej->Gt = (double*)(D + it.o_g);
-            ej->Ct = (double*)(D + it.o_c);
-            ej->Vs = (double*)(D + it.o_v);
-            ej->lam = (double*)(D + it.o_l);
-            ej->colid_out = (int*)(D + it.o_id);
-            ej->eps = (double*)(D + it.o_e);
-            ej->Ct_out = (double*)(D + it.o_c);
-            ej->rowmin = (double*)(D + it.o_r);
-            ej->n = n;
-            ej->npad = it.npad;
-            ej->mol = k;
-            const size_t sm = jacobi_smem_bytes(n, it.npad, it.C);
-            if (b.buckets.empty() || b.buckets.back().C != it.C) b.buckets.push_back({k, 0, it.C, 0});
-            b.buckets.back().count++;
-            b.buckets.back().smem = std::max(b.buckets.back().smem, sm);
-        }
-        std::memset(Hh + o_status, 0, sizeof(int) * m);
-        CK(cudaMemcpyAsync(D, Hh, align256(off), cudaMemcpyHostToDevice, ws->stream));
-        b.d_eig = (EigJob*)(D + o_job);
-        b.d_st = (MolState*)(D + o_st);
-        b.d_status = (int*)(D + o_status);
-        b.neig = m;
-        rc = launch_jacobi(b, ws, 1);
-        if (rc) return rc;
-        k_eig_sort<<<m, 512, 0, ws->stream>>>(b.d_eig, b.d_st, 1, nullptr);
-        CK(cudaGetLastError());
-        CK(cudaMemcpyAsync(Hh, D, align256(off), cudaMemcpyDeviceToHost, ws->stream));
-        CK(cudaStreamSynchronize(ws->stream));
-        for (int k = 0; k < m; ++k) {
-            const Item& it = items[k];
-            const int n = it.n;
-            if (((int*)(Hh + o_status))[k]) {
-                set(it.i, AM1GPU_LINALG, "matrix " + std::to_string(it.i) + ": Jacobi eigensolver did not converge");
-                continue;
-            }
-            std::memcpy(w[it.i], Hh + it.o_e, sizeof(double) * n);
-            const double* ct = (const double*)(Hh + it.o_c);
-            for (int q = 0; q < n; ++q)
-                for (int r = 0; r < n; ++r) v[it.i][(size_t)r * n + q] = ct[(size_t)q * n + r];
-        }
+        for (const SmallEig& it : items)
+            if (it.bad) refused[it.i] = {AM1GPU_LINALG, " handed to the eigensolver is not finite"};
     }
-    if (!large.empty()) {
-        DeviceCtx* ctx;
-        const int rc = device_ctx(&ctx);
-        if (rc) return rc;
-    }
+    for (int i = 0; i < count; ++i)
+        set(i, refused[i].first, refused[i].first ? "matrix " + std::to_string(i) + refused[i].second : std::string());
+    for (const SmallEig& it : items)
+        if (it.code && !it.bad) set(it.i, it.code, "matrix " + std::to_string(it.i) + ": Jacobi eigensolver did not converge");
     for (int i : large) {
         const int rc = symmetric_eigen_large(ns[i], a[i], w[i], v[i], nullptr);
         if (rc == AM1GPU_DEVICE_ERROR) return rc;

@@ -125,10 +125,12 @@ __device__ __forceinline__ int rotate_pair(double* __restrict__ gp, double* __re
     al = warp_sum(al);
     be = warp_sum(be);
     ga = warp_sum(ga);
-    if (!(fabs(ga) > tol * sqrt(al * be)) || al == 0.0 || be == 0.0) return 0;
+    // the angle beside the test, not behind it: both are chains of square roots and divisions
+    const double thr = tol * sqrt(al * be);
     const double zeta = (be - al) / (2.0 * ga);
     const double tt = copysign(1.0, zeta) / (fabs(zeta) + sqrt(1.0 + zeta * zeta));
     const double c = 1.0 / sqrt(1.0 + tt * tt), s = c * tt;
+    if (!(fabs(ga) > thr) || al == 0.0 || be == 0.0) return 0;
     for (int i = lane; i < n; i += 32) {
         const double x = gp[i], y = gq[i];
         gp[i] = c * x - s * y;
@@ -140,11 +142,17 @@ __device__ __forceinline__ int rotate_pair(double* __restrict__ gp, double* __re
     return 1;
 }
 
-constexpr int JAC_THREADS = 256;
+constexpr int JAC_RED = 8;  // warps that form the Gershgorin minimum
 constexpr int JAC_MAX_SWEEPS = 60;
 
-// Shared memory: nbuf = 2q + 2 buffers of 2n doubles ([g | v]), then int metadata.
-__global__ void __launch_bounds__(JAC_THREADS) k_jacobi(const EigJob* __restrict__ jobs, const MolState* __restrict__ st,
+// Bound by latency: a round is one rotation per pair (two columns from shared memory, three butterflies, a chain
+// of square roots and divisions: about 2000 cycles) and, in a cluster, the exchange of two columns.  So a warp per
+// pair of the CTA (up to 32: blockDim.x is the launch's, jacobi_threads), where eight warps took the 20 pairs of
+// a CTA at 320 rows in three turns, and two landing zones used in turn where shared memory has room
+// for them: a column may then be sent while the neighbour still copies the last one out, which leaves one cluster
+// barrier per round.  96 matrices of 24 to 320 rows: 62 -> 33 ms of kernels one after the other.
+// Shared memory: nbuf = 2q + 2 (or + 4) buffers of 2n doubles ([g | v]), then int metadata.
+__global__ void __launch_bounds__(1024) k_jacobi(const EigJob* __restrict__ jobs, const MolState* __restrict__ st,
                                                         int* __restrict__ mol_status, int force, const int* __restrict__ mask) {
     extern __shared__ double smem[];
     cg::cluster_group cluster = cg::this_cluster();
@@ -154,26 +162,31 @@ __global__ void __launch_bounds__(JAC_THREADS) k_jacobi(const EigJob* __restrict
     if (!force && !st[jb.mol].active) return;  // uniform over the cluster
     if (mask && !mask[jb.mol]) return;
     const int n = jb.n, npad = jb.npad, m = npad / 2, q = m / C;
-    const int nbuf = 2 * q + 2;
-    const int LAND_TOP = 2 * q, LAND_BOT = 2 * q + 1;
+    unsigned dyn;
+    asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(dyn));
+    const bool two_zones = C > 1 && jacobi_smem_bytes2(n, npad, C) <= dyn;  // uniform over the cluster
+    const int nbuf = 2 * q + (two_zones ? 4 : 2);
     double* buf = smem;
     int* colid = (int*)(smem + (long long)nbuf * 2 * n);
     int* Tring = colid + nbuf;  // top ring (buffer ids)
     int* Bring = Tring + q;     // bottom ring
     int* ctl = Bring + q;       // [0] ht, [1] hb, [2] rot counter, [3] bad input, [4] total
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = JAC_THREADS / 32;
+    const int nthr = blockDim.x;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = nthr >> 5;
     const double tol = fmax(1.0e-14, 2.0 * n * 2.220446049250313e-16);
 
     // shift sigma from the Gershgorin lower bound of F (rowmin) so F + sigma I > 0
     double mn = 1e300;
-    for (int i = tid; i < n; i += JAC_THREADS) mn = fmin(mn, jb.rowmin[i]);
-    __shared__ double red[JAC_THREADS / 32];
-    for (int o = 16; o > 0; o >>= 1) mn = fmin(mn, __shfl_xor_sync(0xffffffffu, mn, o));
-    if (lane == 0) red[warp] = mn;
+    __shared__ double red[JAC_RED];  // the launch has at least JAC_RED warps
+    if (warp < JAC_RED) {
+        for (int i = tid; i < n; i += 32 * JAC_RED) mn = fmin(mn, jb.rowmin[i]);
+        for (int o = 16; o > 0; o >>= 1) mn = fmin(mn, __shfl_xor_sync(0xffffffffu, mn, o));
+        if (lane == 0) red[warp] = mn;
+    }
     __syncthreads();
     if (tid == 0) {
         double v = red[0];
-        for (int w = 1; w < nwarps; ++w) v = fmin(v, red[w]);
+        for (int w = 1; w < JAC_RED; ++w) v = fmin(v, red[w]);
         red[0] = v;
     }
     __syncthreads();
@@ -187,13 +200,13 @@ __global__ void __launch_bounds__(JAC_THREADS) k_jacobi(const EigJob* __restrict
         ctl[3] = 0;
         ctl[4] = 0;
     }
-    for (int b = tid; b < 2 * q; b += JAC_THREADS) {
+    for (int b = tid; b < 2 * q; b += nthr) {
         colid[b] = b < q ? crank * q + b : m + crank * q + (b - q);
         if (b < q) Tring[b] = b;
         else Bring[b - q] = b;
     }
     __syncthreads();
-    for (long long e = tid; e < (long long)2 * q * n; e += JAC_THREADS) {
+    for (long long e = tid; e < (long long)2 * q * n; e += nthr) {
         const int b = (int)(e / n), i = (int)(e % n);
         const int col = colid[b];
         double g = 0.0, v = 0.0;
@@ -265,20 +278,22 @@ __global__ void __launch_bounds__(JAC_THREADS) k_jacobi(const EigJob* __restrict
                 __syncthreads();
                 continue;
             }
+            const int zone = two_zones ? s & 1 : 0;
+            const int LAND_TOP = 2 * q + 2 * zone, LAND_BOT = LAND_TOP + 1;
             __syncthreads();
-            cluster.sync();
+            if (!two_zones) cluster.sync();
             // send top[q-1] right and bot[0] left (full [g|v] buffers and their column ids)
             const int LT = top_buf(q - 1, s), LB = bot_buf(0, s);
             if (crank < C - 1) {
                 double* dst = cluster.map_shared_rank(buf + (long long)LAND_TOP * 2 * n, crank + 1);
                 const double* src = buf + (long long)LT * 2 * n;
-                for (int i = tid; i < 2 * n; i += JAC_THREADS) dst[i] = src[i];
+                for (int i = tid; i < 2 * n; i += nthr) dst[i] = src[i];
                 if (tid == 0) *cluster.map_shared_rank(&colid[LAND_TOP], crank + 1) = colid[LT];
             }
             if (crank > 0) {
                 double* dst = cluster.map_shared_rank(buf + (long long)LAND_BOT * 2 * n, crank - 1);
                 const double* src = buf + (long long)LB * 2 * n;
-                for (int i = tid; i < 2 * n; i += JAC_THREADS) dst[i] = src[i];
+                for (int i = tid; i < 2 * n; i += nthr) dst[i] = src[i];
                 if (tid == 0) *cluster.map_shared_rank(&colid[LAND_BOT], crank - 1) = colid[LB];
             }
             cluster.sync();
@@ -309,13 +324,13 @@ __global__ void __launch_bounds__(JAC_THREADS) k_jacobi(const EigJob* __restrict
             if (copy_top_to >= 0) {
                 double* d = buf + (long long)copy_top_to * 2 * n;
                 const double* sgl = buf + (long long)LAND_TOP * 2 * n;
-                for (int i = tid; i < 2 * n; i += JAC_THREADS) d[i] = sgl[i];
+                for (int i = tid; i < 2 * n; i += nthr) d[i] = sgl[i];
                 if (tid == 0) colid[copy_top_to] = colid[LAND_TOP];
             }
             if (copy_bot_to >= 0) {
                 double* d = buf + (long long)copy_bot_to * 2 * n;
                 const double* sgl = buf + (long long)LAND_BOT * 2 * n;
-                for (int i = tid; i < 2 * n; i += JAC_THREADS) d[i] = sgl[i];
+                for (int i = tid; i < 2 * n; i += nthr) d[i] = sgl[i];
                 if (tid == 0) colid[copy_bot_to] = colid[LAND_BOT];
             }
             __syncthreads();
@@ -420,10 +435,80 @@ __global__ void __launch_bounds__(512) k_eig_sort(const EigJob* __restrict__ job
     }
 }
 
+// ---------------------------------------------------------------------------------------
+// Caller's matrices to the eigensolver's inputs, and its vectors back to columns
+// ---------------------------------------------------------------------------------------
+// 32 x 32 tiles through shared memory, each element read and written in runs of 32: bound by memory.
+__global__ void __launch_bounds__(256) k_eig_mirror(const EigPrep* __restrict__ prep, int* __restrict__ bad) {
+    __shared__ double t[32][33];
+    const EigPrep p = prep[blockIdx.z];
+    const int n = p.n, bx = blockIdx.x, by = blockIdx.y;
+    if (32 * by >= n || bx > by) return;  // tiles of the lower triangle
+    const int x = threadIdx.x;
+    bool fin = true;
+    for (int y = threadIdx.y; y < 32; y += 8) {
+        const int r = 32 * by + y, c = 32 * bx + x, ru = 32 * bx + y, cu = 32 * by + x;
+        double v = 0.0;
+        if (r < n && c < n) v = p.a[(size_t)r * n + c];
+        fin = fin && isfinite(v);
+        if (bx < by && ru < n && cu < n) fin = fin && isfinite(p.a[(size_t)ru * n + cu]);  // the unread triangle too
+        t[y][x] = v;
+    }
+    __syncthreads();
+    for (int y = threadIdx.y; y < 32; y += 8) {
+        const int r = 32 * by + y, c = 32 * bx + x;
+        if (r < n && c < n) {
+            const double v = c <= r ? t[y][x] : t[x][y];  // above the diagonal only in a diagonal tile
+            p.gt[(size_t)r * n + c] = v;
+            p.ct[(size_t)r * n + c] = r == c ? 1.0 : 0.0;
+        }
+        const int rt = 32 * bx + y, ct = 32 * by + x;  // the mirrored tile
+        if (bx < by && rt < n && ct < n) {
+            p.gt[(size_t)rt * n + ct] = t[x][y];
+            p.ct[(size_t)rt * n + ct] = 0.0;
+        }
+    }
+    if (__syncthreads_or(!fin) && threadIdx.x == 0 && threadIdx.y == 0) bad[blockIdx.z] = 1;
+}
+
+// A thread per row; column by column of the symmetric matrix, so a warp reads 32 consecutive words.
+__global__ void __launch_bounds__(128) k_eig_rowmin(const EigPrep* __restrict__ prep) {
+    const EigPrep p = prep[blockIdx.y];
+    const int n = p.n, r = blockIdx.x * 128 + threadIdx.x;
+    if (r >= n) return;
+    double bound = 0.0;
+    for (int c0 = 0; c0 < n; c0 += 16) {
+        double x[16];
+#pragma unroll
+        for (int u = 0; u < 16; ++u) x[u] = c0 + u < n ? p.gt[(size_t)(c0 + u) * n + r] : 0.0;
+#pragma unroll
+        for (int u = 0; u < 16; ++u)
+            if (c0 + u < n && c0 + u != r) bound += fabs(x[u]);
+    }
+    p.rowmin[r] = p.gt[(size_t)r * n + r] - bound;
+}
+
+__global__ void __launch_bounds__(256) k_eig_columns(const EigPrep* __restrict__ prep) {
+    __shared__ double t[32][33];
+    const EigPrep p = prep[blockIdx.z];
+    const int n = p.n, r0 = 32 * blockIdx.y, c0 = 32 * blockIdx.x, x = threadIdx.x;
+    if (r0 >= n || c0 >= n) return;
+    for (int y = threadIdx.y; y < 32; y += 8)
+        if (r0 + y < n && c0 + x < n) t[y][x] = p.ct[(size_t)(r0 + y) * n + c0 + x];
+    __syncthreads();
+    for (int y = threadIdx.y; y < 32; y += 8)
+        if (c0 + y < n && r0 + x < n) p.v[(size_t)(c0 + y) * n + r0 + x] = t[x][y];
+}
+
 size_t jacobi_smem_bytes(int n, int npad, int C) {
     const int q = npad / 2 / C;
     const int nbuf = 2 * q + 2;
     return (size_t)nbuf * 2 * n * sizeof(double) + (size_t)(nbuf + 2 * q + 8) * sizeof(int);
+}
+
+int jacobi_threads(int npad, int C) {
+    const int q = npad / 2 / C;
+    return 32 * (q <= 8 ? 8 : q >= 32 ? 32 : (q + 3) / 4 * 4);
 }
 
 }  // namespace am1

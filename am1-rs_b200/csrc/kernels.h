@@ -180,6 +180,19 @@ __global__ void k_permute_square(const double* in, long long si, double* out, lo
 __global__ void k_gemm_nn(const GemmJob* jobs, const GemmTile* tiles, int ntiles, const MolState* st, int force, const int* mask);
 __global__ void k_gemm_tn(const GemmJob* jobs, const GemmTile* tiles, int ntiles, const MolState* st, int force, const int* mask);
 __global__ void k_jacobi(const EigJob* jobs, const MolState* st, int* mol_status, int force, const int* mask);
+// The inputs of k_jacobi from count matrices in the caller's order (one EigPrep each): Gt the matrix with its
+// lower triangle mirrored, Ct the identity, rowmin the Gershgorin row minima (each row's sum over ascending
+// columns); bad[i] is set when matrix i has an element that is not finite.  k_eig_mirror: grid (ceil(nmax / 32),
+// ceil(nmax / 32), count), block (32, 8); then k_eig_rowmin: grid (ceil(nmax / 128), count), 128 threads.
+// k_eig_columns: v = Ct_out transposed, the eigenvectors as columns (grid and block of k_eig_mirror).
+struct EigPrep {
+    const double* a;  // n x n as the caller holds it (its lower triangle is read)
+    double *gt, *ct, *rowmin, *v;
+    int n;
+};
+__global__ void k_eig_mirror(const EigPrep* prep, int* bad);
+__global__ void k_eig_rowmin(const EigPrep* prep);
+__global__ void k_eig_columns(const EigPrep* prep);
 __global__ void k_eig_sort(const EigJob* jobs, const MolState* st, int force, const int* mask);
 // one CTA of 512 threads per job, 3 n doubles of dynamic shared memory; jobs without an eigensolver
 // fallback (large matrices) are left to k_sp2_bounds_big (one cooperative launch per matrix) or
@@ -292,7 +305,15 @@ __global__ void k_tridiag_panel(TriJob job, int k, int bw);
 __global__ void k_tridiag_syr2k16(TriJob job, int t0);
 __global__ void k_tridiag_syr2k8(TriJob job, int t0);
 size_t tridiag_panel_smem_bytes(int n);
+// k_jacobi: the shared memory a matrix needs (what its cluster size is chosen by), the same with a second
+// landing zone for the columns neighbours send (taken when the launch has that much), and the threads of
+// a launch whose largest share is npad / 2 / C pairs per CTA
 size_t jacobi_smem_bytes(int n, int npad, int C);
+__host__ __device__ inline size_t jacobi_smem_bytes2(int n, int npad, int C) {
+    const int q = npad / 2 / C, nbuf = 2 * q + 4;
+    return (size_t)nbuf * 2 * n * sizeof(double) + (size_t)(nbuf + 2 * q + 8) * sizeof(int);
+}
+int jacobi_threads(int npad, int C);
 
 // Eigenvectors of one large matrix (k_stein.cu): after the global-memory reduction (reflector s
 // in row s of W, columns > s) and k_bisect.  Inverse iteration on T: k_stein_prep (one block of

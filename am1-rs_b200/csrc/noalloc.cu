@@ -191,7 +191,7 @@ extern "C" int am1gpu_symmetric_eigen_noalloc(int32_t n, const double* a, double
     k_noalloc_prepare<<<1, 256, 0, s>>>(a, n, npad);
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(C, 1, 1);
-    cfg.blockDim = dim3(256, 1, 1);
+    cfg.blockDim = dim3(jacobi_threads(npad, C), 1, 1);
     cfg.dynamicSmemBytes = jacobi_smem_bytes(n, npad, C);
     cfg.stream = s;
     cudaLaunchAttribute attr[1];
