@@ -490,15 +490,16 @@ bool encode_rows_map_f32(TmaDesc* out, const float* base, int ldf, int n) {
 }
 
 // k_bisect for njobs matrices of at most maxn rows: a warp per eigenvalue while the whole launch stays
-// within about two waves of resident threads (one molecule, small batches), a thread per eigenvalue
-// otherwise (the warp form does about seven times the work, so it only pays when the GPU is idle).
-// warp_ok = false keeps the thread-per-eigenvalue bisection: the eigenvalues that seed inverse
-// iteration (whose cluster treatment was tuned on them).
-void bisect_launch(const TriJob* jobs, int njobs, int maxn, cudaStream_t s, bool warp_ok) {
-    constexpr long long kTwoWaves = 2LL * 148 * 2048;  // resident threads of two waves on a B200
-    const int lanes = warp_ok && (long long)njobs * maxn * 32 <= kTwoWaves ? 32 : 1;
-    const int per_block = 512 / lanes;
-    k_bisect<<<dim3(njobs, (maxn + per_block - 1) / per_block), 512, 2 * sizeof(double) * maxn, s>>>(jobs, nullptr, lanes);
+// within about four waves of resident threads (one molecule, one large matrix, small batches), a thread per
+// eigenvalue otherwise (the warp form does about seven times the work, so it only pays when the GPU is
+// idle).  The eigenvalues are the same.
+void bisect_launch(const TriJob* jobs, int njobs, int maxn, cudaStream_t s) {
+    constexpr long long kFourWaves = 4LL * 148 * 2048;  // resident threads of four waves on a B200
+    const int lanes = (long long)njobs * maxn * 32 <= kFourWaves ? 32 : 1;
+    // few warps: small blocks, so that they spread over the SMs
+    const long long warps = (long long)njobs * maxn;
+    const int threads = lanes == 1 || warps > 148 * 16 ? 512 : warps > 148 * 4 ? 128 : 64, per_block = threads / lanes;
+    k_bisect<<<dim3(njobs, (maxn + per_block - 1) / per_block), threads, 2 * sizeof(double) * maxn, s>>>(jobs, nullptr, lanes);
 }
 
 inline int oz_ldq(int n) { return (n + 15) & ~15; }
@@ -537,18 +538,23 @@ int density_mode() {
 
 // Matrices too large for a cluster's shared memory (tridiagonalisation, Lanczos bounds): one of
 // at least kBigGridN orbitals takes the whole GPU (a cooperative launch each); all the others of
-// the batch get a cluster of big_cluster(count) CTAs each, in one launch.
+// the batch get a cluster of big_cluster(count) CTAs each, in one launch (the tridiagonalisation of few
+// matrices takes the whole GPU earlier: tri_split).
 // AM1GPU_BIG=grid / cluster forces one form (for measurements).
 constexpr int kBigGridN = 2048;
 
-bool big_on_grid(int n) {
+int big_forced() {  // 0 no, 1 grid, 2 cluster
     static const int force = [] {
         const char* e = std::getenv("AM1GPU_BIG");
         if (e && std::strcmp(e, "grid") == 0) return 1;
         if (e && std::strcmp(e, "cluster") == 0) return 2;
         return 0;
     }();
-    if (force) return force == 1;
+    return force;
+}
+
+bool big_on_grid(int n) {
+    if (big_forced()) return big_forced() == 1;
     return n >= kBigGridN;
 }
 
@@ -1568,10 +1574,34 @@ int blocked_tridiag(TriJob tj, cudaStream_t s, int64_t* launches) {
     return AM1GPU_OK;
 }
 
+// How many of the leading matrices (sizes descending) the reduction takes one by one on the whole GPU; the
+// rest go in one launch of a cluster each.  All of at least kBigGridN rows, and below that as many as make
+// the sum of the two least.  Milliseconds fitted to measurements on a B200 (the reductions alone): whole GPU 8.6 at
+// 1024 rows, 16 at 1501, 26 at 2000; cluster 4.8 at 600, 12.6 at 1024, 30 at 1501, 61 at 2000, a launch of
+// several about as long as its largest.  So a lone matrix leaves the cluster at about 650 rows, and the tens
+// of matrices of a serving batch stay there.
+int tri_split(int count, const TriJob* jobs) {
+    int least = 0;
+    while (least < count && big_on_grid(jobs[least].n)) ++least;
+    auto grid_ms = [](double n) { return 8.0e-3 * n + 1.3e-9 * n * n * n; };
+    auto cluster_ms = [](double n) { return 5.5e-3 * n + 6.5e-9 * n * n * n; };
+    double sum = 0.0, best = 0.0;
+    int at = least;
+    for (int k = least; k <= count; ++k) {
+        const double t = sum + (k < count ? cluster_ms(jobs[k].n) : 0.0);
+        if (k == least || t < best) {
+            best = t;
+            at = k;
+        }
+        if (k < count) sum += grid_ms(jobs[k].n);
+    }
+    return big_forced() ? least : at;
+}
+
 int launch_big_tridiag(Batch& b, cudaStream_t s, int64_t* launches) {
     const int count = (int)b.tri_big.size();
     if (count == 0) return AM1GPU_OK;
-    const int k = big_split(count, [&](int i) { return b.tri_big[i].n; });
+    const int k = tri_split(count, b.tri_big.data());
     for (int i = 0; i < k; ++i) {  // the whole GPU per matrix
         if (tridiag_blocked()) {
             int rc = blocked_tridiag(b.tri_big[i], s, launches);
@@ -2119,7 +2149,7 @@ int run_device(Batch& b, Mem& mem, const DevElem* dp, const am1gpu_options& o, a
     if ((rc = launch_tridiag(b, ws))) return rc;
     int64_t big_tri_launches = 0;
     if ((rc = launch_big_tridiag(b, s, &big_tri_launches))) return rc;
-    bisect_launch(b.d_tri, njobs, b.maxn, s, true);
+    bisect_launch(b.d_tri, njobs, b.maxn, s);
     k_results<<<b.nmol, RESULT_THREADS, 0, s>>>(b.d_mols, b.d_jobs, b.d_job0, b.nmol, b.d_st, b.d_status, dp, b.d_atom_z,
                                                  b.d_atom_xyz, b.d_res, b.d_charges);
     run.launched(AM1GPU_PHASE_FINAL, 5 + (int)b.tri_buckets.size() + (int)big_tri_launches);
@@ -2779,7 +2809,7 @@ int eigen_large_run(int n, const double* a_host, const double* a_dev, Mem& m, cu
     b.tri_big = {tj};
     int64_t launches = 0;
     if ((rc = launch_big_tridiag(b, s, &launches))) return rc;
-    bisect_launch(b.d_tri, 1, n, s, false);
+    bisect_launch(b.d_tri, 1, n, s);
     CK(cudaGetLastError());
     SteinJob sj{};
     sj.d = tj.d;
@@ -3270,7 +3300,7 @@ int symmetric_eigenvalues_one(int n, const double* a, double* w) {
         rc = launch_big_tridiag(b, ws->stream, &launches);
     }
     if (rc) return rc;
-    bisect_launch(b.d_tri, 1, n, ws->stream, true);
+    bisect_launch(b.d_tri, 1, n, ws->stream);
     CK(cudaGetLastError());
     CK(cudaMemcpyAsync(w, D + o_eps, (size_t)n * 8, cudaMemcpyDeviceToHost, ws->stream));
     CK(cudaStreamSynchronize(ws->stream));

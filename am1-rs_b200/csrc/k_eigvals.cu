@@ -384,52 +384,78 @@ __global__ void __launch_bounds__(TRIB_THREADS) k_tridiag_cl(const TriJob* __res
 // critical path (one FMA per step).  The pair (p_{i-1}, p_{i-2}) is rescaled by a power of two
 // every 8 steps (exact), which keeps it far from overflow and underflow; a zero p_i is replaced by a
 // tiny multiple of p_{i-1} (a zero pivot counts as non-negative, as in the division form).
-__device__ __forceinline__ int sturm_count(const double* d, const double* e2, int n, double x) {
-    int c = 0;
+// Eight steps go without a test on the critical path (one FMA a step; signs and zeros are read off the high
+// words beside it); a block that met a zero is taken again with the replacement.
+__device__ __forceinline__ int sturm_count(const double2* de, int n, double x) {
     double p2 = 1.0;
-    double p1 = d[0] - x;
+    double p1 = de[0].x - x;
     if (p1 == 0.0) p1 = 0x1p-200;
-    bool neg = p1 < 0.0;
-    if (neg) ++c;
-    for (int i = 1; i < n; ++i) {
-        double p = fma(d[i] - x, p1, -e2[i - 1] * p2);
-        if (p == 0.0) p = 0x1p-200 * p1;
-        const bool ng = p < 0.0;
-        c += ng != neg;
-        neg = ng;
-        p2 = p1;
-        p1 = p;
-        if ((i & 7) == 0) {
-            const double m = fmax(fabs(p1), fabs(p2));
-            const int ex = (int)((__double_as_longlong(m) >> 52) & 0x7ff) - 1023;
-            if (ex > 400 || ex < -400) {
-                const double sc = __longlong_as_double((long long)(1023 - ex) << 52);  // 2^-ex
-                p1 *= sc;
-                p2 *= sc;
+    int sign = __double2hiint(p1);  // of p1, in the top bit
+    int c = (unsigned)sign >> 31;
+    for (int i = 1; i < n; i += 8) {
+        const int m = min(8, n - i);
+        bool zero = m < 8;
+        if (!zero) {
+            double q2 = p2, q1 = p1;
+            int s = sign, cc = 0;
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                const double2 r = de[i + u];
+                const double p = fma(r.x - x, q1, -r.y * q2);
+                const int h = __double2hiint(p);
+                zero |= ((h << 1) | __double2loint(p)) == 0;
+                cc += (unsigned)(h ^ s) >> 31;
+                s = h;
+                q2 = q1;
+                q1 = p;
             }
+            if (!zero) {
+                p2 = q2;
+                p1 = q1;
+                sign = s;
+                c += cc;
+            }
+        }
+        if (zero) {
+            for (int u = 0; u < m; ++u) {
+                const double2 r = de[i + u];
+                double p = fma(r.x - x, p1, -r.y * p2);
+                if (p == 0.0) p = 0x1p-200 * p1;
+                const int h = __double2hiint(p);
+                c += (unsigned)(h ^ sign) >> 31;
+                sign = h;
+                p2 = p1;
+                p1 = p;
+            }
+        }
+        const int ex = max(__double2hiint(p1) & 0x7fffffff, __double2hiint(p2) & 0x7fffffff) >> 20;  // biased, of the larger
+        if (ex > 1423 || ex < 623) {
+            const double sc = __longlong_as_double((long long)(2046 - ex) << 52);  // 2^-(ex - 1023)
+            p1 *= sc;
+            p2 *= sc;
         }
     }
     return c;
 }
 
-// lanes = 1: a thread per eigenvalue, bisection; lanes = 32: a warp per eigenvalue, 32-way
-// multisection (31 Sturm counts per round on the lanes, the interval narrowed to the gap where the
-// count passes k: a factor 32 per round, to the bisection's stopping width), for launches with few
-// eigenvalues, where the latency of one thread's ~50 dependent counts is the cost.
+// Eigenvalue k of T by bisection to the width 4 eps max(|lo|, |hi|).  lanes = 1: a thread per eigenvalue;
+// lanes = 32: a warp per eigenvalue, five levels of the bisection per round, the 31 midpoints that five steps can
+// reach counted on the lanes and the steps then walked; for launches with few eigenvalues, where the latency
+// of one thread's ~50 dependent counts is the cost.  The midpoints, the counts and so
+// the eigenvalues are the same either way.  n = 1501: 5.0 -> 0.7 ms, 192 orbitals alone 107 -> 83 us (32-way multisection
+// before, whose eigenvalues differed from the thread form's in the last bits), a batch of 192 molecules 1.07 -> 0.83 ms.
 __global__ void k_bisect(const TriJob* __restrict__ jobs, const int* __restrict__ mask, int lanes) {
     const TriJob jb = jobs[blockIdx.x];
     if (mask && !mask[jb.mol]) return;
     const int n = jb.n;
-    extern __shared__ double sh[];
-    double* d = sh;
-    double* e2 = sh + n;
+    extern __shared__ __align__(16) double sh[];
+    double2* de = reinterpret_cast<double2*>(sh);  // d_i, e_{i-1}^2
     __shared__ double bounds[2], wlo[32], whi[32];
     double lo_t = 1e300, hi_t = -1e300;  // Gershgorin bounds of T (every thread's share, then the CTA's)
     for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        const double di = jb.d[i], er = i + 1 < n ? jb.e[i] : 0.0;
-        d[i] = di;
-        e2[i] = er * er;
-        const double r = (i > 0 ? fabs(jb.e[i - 1]) : 0.0) + fabs(er);
+        const double di = jb.d[i], er = i + 1 < n ? jb.e[i] : 0.0, el = i > 0 ? jb.e[i - 1] : 0.0;
+        de[i] = make_double2(di, el * el);
+        const double r = fabs(el) + fabs(er);
         lo_t = fmin(lo_t, di - r);
         hi_t = fmax(hi_t, di + r);
     }
@@ -457,17 +483,30 @@ __global__ void k_bisect(const TriJob* __restrict__ jobs, const int* __restrict_
         const int k = (blockIdx.y * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
         if (k >= n) return;  // whole warps: blockDim is a multiple of 32
         double lo = bounds[0], hi = bounds[1];
-        for (int round = 0; round < 16; ++round) {
-            const double h = (hi - lo) * (1.0 / 32.0);
-            if (!(h > 0.0) || hi - lo <= 4.0 * 2.220446049250313e-16 * fmax(fabs(lo), fabs(hi))) break;
-            const double x = lo + h * (lane + 1);
-            const bool below = lane < 31 && sturm_count(d, e2, n, x) <= k;
-            const unsigned ball = __ballot_sync(0xffffffffu, below);
-            const int j = ball ? 31 - __clz(ball) : -1;
-            const double nlo = j >= 0 ? lo + h * (j + 1) : lo;
-            const double nhi = j + 2 <= 31 ? lo + h * (j + 2) : hi;
-            lo = nlo;
-            hi = nhi;
+        bool done = false;
+        for (int round = 0; round < 40 && !done; ++round) {
+            // lane's node of the tree, in heap order (node 0 the root, children 2 i + 1 below and 2 i + 2
+            // above its midpoint): the interval that its parents' answers would leave
+            double l = lo, h = hi, mid = 0.5 * (lo + hi);
+            const int node = lane + 1;  // 1-based; lane 31 idles
+            for (int bit = 30 - __clz(node); bit >= 0; --bit) {
+                if (node >> bit & 1) l = mid;
+                else h = mid;
+                mid = 0.5 * (l + h);
+            }
+            const bool up = lane < 31 && mid > l && mid < h && sturm_count(de, n, mid) <= k;
+            const unsigned ball = __ballot_sync(0xffffffffu, up);
+            for (int step = 0, at = 1; step < 5; ++step) {
+                mid = 0.5 * (lo + hi);
+                if (!(mid > lo && mid < hi) || hi - lo <= 4.0 * 2.220446049250313e-16 * fmax(fabs(lo), fabs(hi))) {
+                    done = true;
+                    break;
+                }
+                const bool above = ball >> (at - 1) & 1;
+                if (above) lo = mid;
+                else hi = mid;
+                at = 2 * at + (above ? 1 : 0);
+            }
         }
         if (lane == 0) jb.eps[k] = 0.5 * (lo + hi);
         return;
@@ -480,7 +519,7 @@ __global__ void k_bisect(const TriJob* __restrict__ jobs, const int* __restrict_
             const double mid = 0.5 * (lo + hi);
             if (!(mid > lo && mid < hi)) break;
             if (hi - lo <= 4.0 * 2.220446049250313e-16 * fmax(fabs(lo), fabs(hi))) break;
-            if (sturm_count(d, e2, n, mid) <= k) lo = mid;
+            if (sturm_count(de, n, mid) <= k) lo = mid;
             else hi = mid;
         }
         jb.eps[k] = 0.5 * (lo + hi);
@@ -507,75 +546,91 @@ namespace am1 {
 //   p    = beta (A v - V (W^T v) - W (V^T v))                      over rows and columns > c
 //   w    = p - (beta/2)(p . v) v,  V_.j = v,  W_.j = w
 // W^T v and V^T v come from W^T x and V^T x (summed with |x|^2 in the first grid barrier) and
-// row c+1 of W and V.  Two grid barriers per column: row c+1's newest entries of V and W, which
-// its owner writes after the second barrier, every CTA forms itself (v_{c+1} and p_{c+1} are
-// known to all by then) for the next column's first phase.  Rows are cyclic over the CTAs (r % G).
+// row c+1 of W and V; they are needed only after the second barrier, which sums v . A v, since
+// p . v = beta (v . A v - 2 (V^T v) . (W^T v)).  Two grid barriers per column: row c+1's newest
+// entries of V and W, which its owner writes after the second barrier, every CTA forms itself for
+// the next column's first phase.  Rows are cyclic over the CTAs (r % G).
 // Scratch (job.work, 16-byte aligned): VW[n][2B] = [V | W] | WVt[2B][n] = [W | V]^T | x[n] |
-// p[n] | share[G][2B + 2]; dynamic shared memory: v (n doubles) and W^T v, V^T v.  As in
+// u[n] | share[2B + 2][G] | sums[2B]; dynamic shared memory: v (n doubles) and W^T v, V^T v.  As in
 // tridiag_group, row c of job.W ends holding reflector v_c in columns c+1..n-1.
 // ---------------------------------------------------------------------------------------------
 
 size_t tridiag_panel_smem_bytes(int n) { return sizeof(double) * ((size_t)n + 2 * TRP_B); }
 
+// Sum over the CTAs of one slot's shares (consecutive words) by a warp: lane-strided in ascending order, then
+// a butterfly, as group_share_sum; up to 160 shares' loads are in flight at once.
+__device__ __forceinline__ double panel_share_sum(const double* __restrict__ share, int G) {
+    constexpr int U = 5;
+    const int lane = threadIdx.x & 31;
+    double t = 0.0;
+    for (int q0 = 0; q0 < G; q0 += 32 * U) {
+        double v[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) v[u] = q0 + 32 * u + lane < G ? __ldcg(share + q0 + 32 * u + lane) : 0.0;
+#pragma unroll
+        for (int u = 0; u < U; ++u) t += v[u];
+    }
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    return t;
+}
+
+// Bound by the chain of a column: two grid barriers (2.5k cycles each), the L2 round trips between them, and
+// from about 1500 rows on the pass over the trailing matrix.  In its first form every CTA summed every slot's
+// shares itself, from records a CTA apart: 60 MB of L2 sectors per column (clock stamps at n = 1501, cycles per
+// column: 4.1k for the column, 15.7k for the reflector, 6.7k for A v, 8.7k for w).  Now a slot is summed by one CTA,
+// from consecutive words, while the others multiply, and A v's rows are reduced behind one barrier: 2.5k, 3.2k, 8.2k and
+// 2.3k; eigenvalues alone, with copies and bisection, 1501 rows 34.8 -> 17.5 ms, 3072 rows 92 -> 53 ms.
 __global__ void __launch_bounds__(TRIB_THREADS) k_tridiag_panel(TriJob jb, int k, int bw) {
     cg::grid_group grid = cg::this_grid();
     const int G = (int)gridDim.x, gi = (int)blockIdx.x;
     const int n = jb.n;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     constexpr int NW = TRIB_THREADS / 32;
-    constexpr int B = TRP_B, SW = 2 * TRP_B + 2;
+    constexpr int B = TRP_B;
     double* A = jb.W;
     double* VW = jb.work;
     double* WVt = VW + (size_t)2 * B * n;
     double* xb = WVt + (size_t)2 * B * n;
-    double* pb = xb + n;
-    double* share = pb + n;
+    double* ub = xb + n;
+    double* share = ub + n;                        // [2B + 2][G]: |x|^2, W^T x, V^T x (as the column has them), v.u
+    double* sums = share + (size_t)(2 * B + 2) * G;  // [2B]: W^T v, V^T v
     extern __shared__ double psh[];
     double* sv = psh;      // v, rows c+1..n-1
     double* st = psh + n;  // [0, B): W^T v;  [B, 2B): V^T v
     __shared__ double xr[64];  // this CTA's x_i of the current column (its rows > c, at most 64 of them)
-    __shared__ int xi_row[64];
     __shared__ double red[NW];
     // the panel's V and W on this CTA's own rows (row gi + q G in slot q), kept here as they are
     // formed: the per-column corrections read them from shared memory, not global
     __shared__ double svw[64][2 * TRP_B];
-    __shared__ double rowc[2];  // V and W of row c in the previous column (formed locally)
-    __shared__ double red4[4][NW];
+    __shared__ double srow[2 * TRP_B];  // V and W of row c (formed locally in the previous column, or read)
+    __shared__ double redr[64][NW];     // A v of the own rows, each warp's share of the columns
     for (int j = 0; j < bw; ++j) {
         const int c = k + j;
-        __syncthreads();  // own rows' V, W of the previous column, and rowc, are written
+        __syncthreads();  // own rows' V, W of the previous column, and srow, are written
         // ---- phase 1: column c for own rows i >= c, and this CTA's shares of |x|^2, W^T x, V^T x
         const int first = c + ((gi - c % G) % G + G) % G;  // first own row >= c
-        int nr = 0;
-        for (int i = first; i < n; i += G) ++nr;  // own rows >= c (<= 64: n <= 8192 and G >= 128)
+        const int nr = first < n ? (n - 1 - first) / G + 1 : 0;  // own rows >= c (<= 64: n <= 8192 and G >= 128)
         const int q0 = (first - gi) / G;  // slot of the first own row >= c
+        const int qa = first > c ? 0 : 1;  // first own row > c
         if (tid < nr) {
             const int i = first + tid * G;
             const double* Vi = svw[q0 + tid];
-            const double* Vc = VW + (size_t)c * 2 * B;
             double x = __ldcg(A + (size_t)i * n + c);
-            for (int l = 0; l < j; ++l) {
-                // row c's entries of the previous column are not yet visible from its owner
-                const double vc = l + 1 == j ? rowc[0] : __ldcg(Vc + l), wc = l + 1 == j ? rowc[1] : __ldcg(Vc + B + l);
-                x -= Vi[l] * wc + Vi[B + l] * vc;
-            }
+            for (int l = 0; l < j; ++l) x -= Vi[l] * srow[B + l] + Vi[B + l] * srow[l];
             xr[tid] = x;
-            xi_row[tid] = i;
             xb[i] = x;
             if (i == c) jb.d[c] = x;
         }
         __syncthreads();
         if (tid < 2 * j + 1) {  // share slot 0: |x_{>c}|^2; 1..j: W^T x; j+1..2j: V^T x
             double s = 0.0;
-            for (int q = 0; q < nr; ++q) {
-                const int i = xi_row[q];
-                if (i <= c) continue;
-                const double x = xr[q];
-                if (tid == 0) s += x * x;
-                else if (tid <= j) s += svw[q0 + q][B + (tid - 1)] * x;
-                else s += svw[q0 + q][tid - 1 - j] * x;
+            for (int q = qa; q < nr; ++q) {
+                const double xq = xr[q];
+                if (tid == 0) s += xq * xq;
+                else if (tid <= j) s += svw[q0 + q][B + (tid - 1)] * xq;
+                else s += svw[q0 + q][tid - 1 - j] * xq;
             }
-            share[(size_t)gi * SW + tid] = s;
+            share[(size_t)tid * G + gi] = s;
         }
         grid.sync();
         // ---- the reflector (every CTA forms the same values: fixed-order sums of the shares)
@@ -591,40 +646,38 @@ __global__ void __launch_bounds__(TRIB_THREADS) k_tridiag_panel(TriJob jb, int k
             }
             break;
         }
-        double nrm2 = 0.0;
-        for (int q = lane; q < G; q += 32) nrm2 += __ldcg(share + (size_t)q * SW);
-        for (int o = 16; o > 0; o >>= 1) nrm2 += __shfl_xor_sync(0xffffffffu, nrm2, o);
-        const double alpha = sqrt(nrm2);
+        for (int i0 = c + 1 + tid; i0 < n; i0 += 4 * TRIB_THREADS) {
+            double v[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) v[u] = i0 + u * TRIB_THREADS < n ? __ldcg(xb + i0 + u * TRIB_THREADS) : 0.0;
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (i0 + u * TRIB_THREADS < n) sv[i0 + u * TRIB_THREADS] = v[u];
+        }
+        // |x|^2 in warp 0; slot gi (W^T x or V^T x) of the shares in warp 1, summed for all CTAs
+        const double* V1 = VW + (size_t)(c + 1) * 2 * B;
+        const double sum = warp == 0 ? panel_share_sum(share, G)
+                           : warp == 1 && gi < 2 * j ? panel_share_sum(share + (size_t)(1 + gi) * G, G) : 0.0;
+        const double v1 = warp == 1 && gi < 2 * j ? __ldcg(V1 + (gi < j ? B + gi : gi - j)) : 0.0;
+        if (warp == 0 && lane == 0) red[0] = sum;
+        __syncthreads();
+        const double alpha = sqrt(red[0]);
         const double sg = x1 >= 0.0 ? 1.0 : -1.0;
         const double beta = alpha == 0.0 ? 0.0 : 1.0 / (alpha * (alpha + fabs(x1)));
-        const double* V1 = VW + (size_t)(c + 1) * 2 * B;
-        // W^T v and V^T v: slot s < 2j summed over the CTAs by one warp, lane-strided in a fixed
-        // order (as group_share_sum), plus the e_{c+1} part of v = x + sg alpha e_{c+1}
-        for (int sl = warp; sl < 2 * j; sl += NW) {
-            double t = 0.0;
-            for (int q = lane; q < G; q += 32) t += __ldcg(share + (size_t)q * SW + 1 + sl);
-            for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-            if (lane == 0) {
-                const int l = sl < j ? sl : sl - j;
-                t += sg * alpha * (sl < j ? __ldcg(V1 + B + l) : __ldcg(V1 + l));
-                st[sl < j ? l : B + l] = t;
-            }
-        }
-        for (int i = c + 1 + tid; i < n; i += TRIB_THREADS) sv[i] = __ldcg(xb + i);
-        __syncthreads();
+        if (warp == 1 && lane == 0 && gi < 2 * j)  // plus the e_{c+1} part of v = x + sg alpha e_{c+1}
+            sums[gi < j ? gi : B + gi - j] = sum + sg * alpha * v1;
         if (tid == 0) sv[c + 1] = x1 + sg * alpha;
         __syncthreads();
-        // ---- phase 2a: p_i for own rows i > c, this CTA's share of p . v.  Rows go in groups of
+        // ---- phase 2a: u = A v on own rows i > c, this CTA's share of v . u.  Rows go in groups of
         // four; every thread takes a stride of the columns for all four (many loads in flight),
         // and the partial sums are reduced over the CTA in a fixed order.
-        double part = 0.0;
-        for (int g0 = first > c ? 0 : 1; g0 < nr; g0 += 4) {
+        for (int g0 = qa; g0 < nr; g0 += 4) {
             const int gr = min(4, nr - g0);
             const double* Ar[4];
 #pragma unroll
             for (int u = 0; u < 4; ++u) Ar[u] = A + (size_t)(first + (g0 + (u < gr ? u : 0)) * G) * n;
             double acc[4] = {0.0, 0.0, 0.0, 0.0};
-#pragma unroll 4
+#pragma unroll 2
             for (int m = c + 1 + tid; m < n; m += TRIB_THREADS) {
                 const double vm = sv[m];
 #pragma unroll
@@ -635,52 +688,66 @@ __global__ void __launch_bounds__(TRIB_THREADS) k_tridiag_panel(TriJob jb, int k
                 for (int o = 16; o > 0; o >>= 1) acc[u] += __shfl_xor_sync(0xffffffffu, acc[u], o);
             if (lane == 0)
 #pragma unroll
-                for (int u = 0; u < 4; ++u) red4[u][warp] = acc[u];
-            __syncthreads();
-            if (tid < gr) {
-                const int q = g0 + tid, i = first + q * G;
-                double t = 0.0;
-                for (int w = 0; w < NW; ++w) t += red4[tid][w];
-                const double* Vi = svw[q0 + q];
-                for (int l = 0; l < j; ++l) t -= Vi[l] * st[l] + Vi[B + l] * st[B + l];
-                const double pi = beta * t;
-                pb[i] = pi;
-                part += pi * sv[i];
-            }
-            __syncthreads();
+                for (int u = 0; u < 4; ++u)
+                    if (u < gr) redr[g0 + u][warp] = acc[u];
         }
-        for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
-        if (lane == 0) red[warp] = part;
         __syncthreads();
-        if (tid == 0) {
-            double t = 0.0;
-            for (int q = 0; q < NW; ++q) t += red[q];
-            share[(size_t)gi * SW + SW - 1] = t;
-        }
-        grid.sync();
-        // ---- phase 2b: w = p - kk v for own rows i > c; column j of V and W in both layouts
-        double pv = 0.0;
-        for (int q = lane; q < G; q += 32) pv += __ldcg(share + (size_t)q * SW + SW - 1);
-        for (int o = 16; o > 0; o >>= 1) pv += __shfl_xor_sync(0xffffffffu, pv, o);
-        const double kk = 0.5 * beta * pv;
-        if (tid < nr) {
-            const int i = first + tid * G;
-            if (i > c) {
-                const double v = sv[i], w = __ldcg(pb + i) - kk * v;
-                svw[q0 + tid][j] = v;
-                svw[q0 + tid][B + j] = w;
-                VW[(size_t)i * 2 * B + j] = v;
-                VW[(size_t)i * 2 * B + B + j] = w;
-                WVt[(size_t)j * n + i] = w;
-                WVt[(size_t)(B + j) * n + i] = v;
-                A[(size_t)c * n + i] = v;  // reflector c into row c (columns > c), which nothing reads again
+        double ui = 0.0;  // u of this thread's own row, kept for phase 2b
+        if (warp < 2) {   // at most 64 own rows
+            double part = 0.0;
+            if (tid >= qa && tid < nr) {
+                const int i = first + tid * G;
+                for (int w = 0; w < NW; ++w) ui += redr[tid][w];
+                if (i == c + 1) ub[i] = ui;
+                part = ui * sv[i];
             }
+            for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
+            if (lane == 0) red[1 + warp] = part;
+        }
+        __syncthreads();
+        if (tid == 0) share[(size_t)(2 * B + 1) * G + gi] = red[1] + red[2];
+        grid.sync();
+        // ---- phase 2b: p = beta (u - V (W^T v) - W (V^T v)), w = p - kk v for own rows i > c with
+        // kk = (beta / 2) p . v, p . v = beta (v . u - 2 (V^T v) . (W^T v)); column j of V and W in both
+        // layouts; and row c + 1 of V and W (its p formed by every CTA) for the next column's phase 1
+        if (warp == 0) {
+            const double vu = panel_share_sum(share + (size_t)(2 * B + 1) * G, G);
+            if (lane == 0) red[0] = vu;
+        } else if (warp < 1 + 2 * B / 32) {
+            const int e = tid - 32, l = e < B ? e : e - B;
+            if (l < j) st[e] = __ldcg(sums + e);
+        } else if (warp < 1 + 4 * B / 32) {
+            const int e = tid - 32 - 2 * B, l = e < B ? e : e - B;
+            if (l < j) srow[e] = __ldcg(V1 + e);  // [V | W], as VW's rows
+        }
+        const double u1 = tid == TRIB_THREADS - 1 ? __ldcg(ub + c + 1) : 0.0;
+        __syncthreads();
+        const bool next_row = tid == TRIB_THREADS - 1, own = tid >= qa && tid < nr;
+        const double* Vi = next_row ? srow : svw[own ? q0 + tid : 0];
+        double t = next_row ? u1 : ui, vv = 0.0;
+        if (own || next_row) {
+            for (int l = 0; l < j; ++l) {
+                t -= Vi[l] * st[l] + Vi[B + l] * st[B + l];
+                vv += st[l] * st[B + l];
+            }
+        }
+        const double p = beta * t, kk = 0.5 * beta * (beta * (red[0] - 2.0 * vv));
+        if (own) {
+            const int i = first + tid * G;
+            const double v = sv[i], w = p - kk * v;
+            svw[q0 + tid][j] = v;
+            svw[q0 + tid][B + j] = w;
+            VW[(size_t)i * 2 * B + j] = v;
+            VW[(size_t)i * 2 * B + B + j] = w;
+            WVt[(size_t)j * n + i] = w;
+            WVt[(size_t)(B + j) * n + i] = v;
+            A[(size_t)c * n + i] = v;  // reflector c into row c (columns > c), which nothing reads again
+        }
+        if (next_row) {
+            srow[j] = sv[c + 1];
+            srow[B + j] = p - kk * sv[c + 1];
         }
         if (gi == c % G && tid == 0) jb.e[c] = alpha == 0.0 ? 0.0 : -sg * alpha;
-        if (tid == 0) {  // row c+1's entries of this column, for the next column's phase 1
-            rowc[0] = sv[c + 1];
-            rowc[1] = __ldcg(pb + c + 1) - kk * sv[c + 1];
-        }
     }
 }
 

@@ -299,7 +299,7 @@ size_t tridiag_big_smem_bytes(int n);
 // k_tridiag_panel (tridiag_panel_smem_bytes(n); grid <= co-resident CTAs and >= n / 64), then,
 // unless it was the last panel, the trailing update over the upper tiles of [k + TRP_B, n)
 // (k_tridiag_syr2k16 when n is even, else ...8; dgemm_smem_bytes()).  job.work: 16-byte aligned,
-// 4 TRP_B n + 2 n + grid (2 TRP_B + 2) doubles.
+// 4 TRP_B n + 2 n + grid (2 TRP_B + 2) + 2 TRP_B doubles.
 constexpr int TRP_B = 32;
 __global__ void k_tridiag_panel(TriJob job, int k, int bw);
 __global__ void k_tridiag_syr2k16(TriJob job, int t0);
