@@ -744,7 +744,7 @@ int plan_molecule(const am1gpu_molecule& m, const am1gpu_options& o, int user, M
 }
 
 struct Batch {
-    int nmol = 0, natoms = 0, nblk = 1, maxn = 0;
+    int nmol = 0, natoms = 0, nblk = 1, maxn = 0, maxheavy = 0;
     long long npairs = 0;
     std::vector<MolPlan> plans;
     // device pointers (into the pool)
@@ -837,7 +837,7 @@ struct Batch {
 // Lays out the batch in one device pool and one pinned staging area, copies inputs.
 int build_batch(const am1gpu_molecule* in, const am1gpu_options& o, std::vector<MolPlan>&& plans, Batch& b, Mem& mem,
                 am1gpu_call_stats* stats, double spin_scale_override = -1.0, const DevElem* host_tab = nullptr,
-                size_t extra_dev = 0, size_t extra_host = 0) {
+                size_t extra_dev = 0, size_t extra_host = 0, bool zero_arena = true) {
     b.plans = std::move(plans);
     b.nmol = (int)b.plans.size();
     const int method = o.method == AM1GPU_METHOD_RM1 ? 1 : 0;
@@ -856,6 +856,7 @@ int build_batch(const am1gpu_molecule* in, const am1gpu_options& o, std::vector<
         hist += p.nch * MAX_DIIS * (ls + la + ((adiis && p.nch == 1) ? ls : 0)) + 64;
         nch_total += p.nch;
         maxn = std::max(maxn, p.nao);
+        b.maxheavy = std::max(b.maxheavy, p.nheavy);
     }
     b.natoms = (int)natoms;
     b.npairs = npairs;
@@ -1411,7 +1412,7 @@ int build_batch(const am1gpu_molecule* in, const am1gpu_options& o, std::vector<
     CK(cudaMemcpyAsync(D, Hs, staged, cudaMemcpyHostToDevice, ws->stream));
     if (stats) stats->h2d_bytes += (int64_t)staged;
     CK(cudaMemsetAsync(b.d_status, 0, sizeof(int) * b.nmol, ws->stream));
-    CK(cudaMemsetAsync(b.d_arena, 0, sizeof(double) * arena, ws->stream));
+    if (zero_arena) CK(cudaMemsetAsync(b.d_arena, 0, sizeof(double) * arena, ws->stream));
     CK(cudaMemsetAsync(b.d_big_stall, 0, sizeof(int) * std::max<long long>(nch_total, 1), ws->stream));
     return AM1GPU_OK;
 }
@@ -1691,7 +1692,7 @@ int enq_head(IterEnq& e) {
     int rc;
     CK(cudaMemsetAsync(b.d_active, 0, 4 * sizeof(int), s));
     if ((rc = run.begin(&e.ph))) return rc;
-    k_fock<<<cdiv(b.natoms, 8), 256, 0, s>>>(b.d_mols, b.d_atom_mol, b.natoms, e.dp, b.d_atom_z, b.d_wstore, b.d_arena, b.d_st, 0);
+    k_fock<<<fock_grid(b.natoms, b.maxheavy), 32 * FOCK_WARPS, 0, s>>>(b.d_mols, b.d_atom_mol, b.natoms, e.dp, b.d_atom_z, b.d_wstore, b.d_arena, b.d_st, 0);
     run.launched(AM1GPU_PHASE_FOCK);
     if ((rc = run.end(AM1GPU_PHASE_FOCK, e.ph)) || (rc = run.begin(&e.ph))) return rc;
     launch_tiles(b, false, [&](const GemmTile* t, int nt, bool pairs) {
@@ -2070,7 +2071,8 @@ int run_device(Batch& b, Mem& mem, const DevElem* dp, const am1gpu_options& o, a
     CK(cudaMemsetAsync(b.d_status, 0, sizeof(int) * b.nmol, s));
     CK(cudaMemsetAsync(b.d_work, 0, sizeof(double) * kWorkN, s));
     CK(cudaMemsetAsync(b.d_sp2_active, 0, 4 * sizeof(int), s));  // [2]: error word of the tensor-core steps
-    CK(cudaMemsetAsync(b.d_arena, 0, sizeof(double) * b.arena_doubles, s));
+    // P (zero) and the eigensolver's warm start (the identity); every other slot is written before it is read
+    k_slots_init<<<dim3(std::max(1u, cdiv(2LL * b.maxn * b.maxn, 16384)), (unsigned)b.jobs.size()), 256, 0, s>>>(b.d_jobs);
     // mixed precision: every molecule starts with TF32 purification (k_converge ends that phase)
     const bool mixed = o.precision == AM1GPU_PRECISION_MIXED && density_mode() == 0;
     bool lowp_left = mixed;  // some molecule may still be in its TF32 phase
@@ -2083,8 +2085,7 @@ int run_device(Batch& b, Mem& mem, const DevElem* dp, const am1gpu_options& o, a
         k_sad_init<<<cdiv(b.natoms, 128), 128, 0, s>>>(b.d_mols, b.d_atom_mol, b.natoms, dp, b.d_atom_z, b.d_arena);
         run.launched(AM1GPU_PHASE_CORE);
     }
-    k_identity<<<dim3(cdiv(b.maxn, 256), njobs), 256, 0, s>>>(b.d_jobs);
-    run.launched(AM1GPU_PHASE_CORE);
+    run.launched(AM1GPU_PHASE_CORE);  // k_slots_init
     CK(cudaGetLastError());
     if ((rc = run.end(AM1GPU_PHASE_CORE, ph))) return rc;
     ScfParams prm{o.max_scf, o.use_diis, o.accelerator, o.e_tol, o.p_tol, o.adiis_switch, lowp_switch(), lowp_max_iter()};
@@ -2142,7 +2143,7 @@ int run_device(Batch& b, Mem& mem, const DevElem* dp, const am1gpu_options& o, a
     const int nblk = b.nblk;
     // final energy at the final density (src/scf.rs:698-701, 835-839) and the result records
     if ((rc = run.begin(&ph))) return rc;
-    k_fock<<<cdiv(b.natoms, 8), 256, 0, s>>>(b.d_mols, b.d_atom_mol, b.natoms, dp, b.d_atom_z, b.d_wstore, b.d_arena, b.d_st, 1);
+    k_fock<<<fock_grid(b.natoms, b.maxheavy), 32 * FOCK_WARPS, 0, s>>>(b.d_mols, b.d_atom_mol, b.natoms, dp, b.d_atom_z, b.d_wstore, b.d_arena, b.d_st, 1);
     k_post_fock<<<dim3(nblk, njobs), 256, 0, s>>>(b.d_jobs, b.d_mols, b.d_st, nblk, 1, 1);
     k_final_energy<<<cdiv(b.nmol, SCF_MOL_WARPS), 32 * SCF_MOL_WARPS, 0, s>>>(b.d_mols, b.d_jobs, b.d_job0, b.nmol, b.d_st, nblk);
     // eigenvalues of the last F* (mo_energies, HOMO/LUMO): tridiagonalisation + bisection
@@ -2441,7 +2442,7 @@ int scf_batch(int nmol, const am1gpu_molecule* mols, const am1gpu_options* opts_
         Workspace* ws;
         rc = workspace(&ws, 0, 0);
         if (!rc && opts->precision == AM1GPU_PRECISION_MIXED) rc = tune_lowp_kernels(plans);
-        if (!rc) rc = build_batch(mols, *opts, std::move(plans), b, *ws, &tl_stats, -1.0, tab_all);
+        if (!rc) rc = build_batch(mols, *opts, std::move(plans), b, *ws, &tl_stats, -1.0, tab_all, 0, 0, false);
         const DevElem* dp = b.d_params ? b.d_params : ctx->d_params;
         if (!rc) rc = run_device(b, *ws, dp, *opts, &tl_stats);
         if (!rc && grads) rc = run_gradient(b, *ws, dp, &tl_stats);
@@ -2555,7 +2556,7 @@ int build_fock_one(const am1gpu_molecule* mol, int method, const double* p_tot, 
         }
     CK(cudaMemcpyAsync(b.jobs[0].P, p0.data(), sizeof(double) * n * n, cudaMemcpyHostToDevice, ws->stream));
     CK(cudaMemcpyAsync(b.jobs[1].P, p1.data(), sizeof(double) * n * n, cudaMemcpyHostToDevice, ws->stream));
-    k_fock<<<cdiv(b.natoms, 8), 256, 0, ws->stream>>>(b.d_mols, b.d_atom_mol, b.natoms, ctx->d_params, b.d_atom_z, b.d_wstore,
+    k_fock<<<fock_grid(b.natoms, b.maxheavy), 32 * FOCK_WARPS, 0, ws->stream>>>(b.d_mols, b.d_atom_mol, b.natoms, ctx->d_params, b.d_atom_z, b.d_wstore,
                                                       b.d_arena, b.d_st, 1);
     CK(cudaGetLastError());
     std::vector<double> t;
@@ -2681,7 +2682,7 @@ int g_matrix_batch(const am1gpu_molecule* mol, int method, int nrhs, const doubl
             if (pinned) std::memcpy(slot, src, bytes * cnt);
             CK(cudaMemcpyAsync(raw, pinned ? slot : src, bytes * cnt, cudaMemcpyHostToDevice, s));
             k_permute_square<<<dim3(n, cnt), 128, 0, s>>>(raw, (long long)nn, arena + nn * (1 + SLOT_P), (long long)(3 * nn), dmap, n);
-            k_fock<<<cdiv((long long)cnt * natoms, 8), 256, 0, s>>>(dm, dam, cnt * natoms, ctx->d_params, dz, b.d_wstore, arena, b.d_st, 1);
+            k_fock<<<fock_grid((long long)cnt * natoms, b.maxheavy), 32 * FOCK_WARPS, 0, s>>>(dm, dam, cnt * natoms, ctx->d_params, dz, b.d_wstore, arena, b.d_st, 1);
             k_permute_square<<<dim3(n, cnt), 128, 0, s>>>(arena + nn * (1 + SLOT_F), (long long)(3 * nn), raw, (long long)nn, dmap + n, n);
             CK(cudaGetLastError());
             CK(cudaMemcpyAsync(pinned ? slot : dst, raw, bytes * cnt, cudaMemcpyDeviceToHost, s));

@@ -1,7 +1,11 @@
 // Fock G(P) build: F^s = H_core + J(P_tot) - K(spin_scale * P^s), am1-rs src/fock.rs:249-511.
 //
-// One warp per atom A; every off-diagonal block has exactly one writer and every sum is a
-// gather in a fixed order, so the result is deterministic and needs no atomics.
+// A warp per atom A.  Its heavy-heavy exchange blocks go to further warps, FOCK_XX_CHUNK partners each, unless
+// the batch has FOCK_SPLIT_ATOMS atoms and more: one warp walking all of them makes an atom's time grow with
+// the molecule (42 us for 32 waters, 16 split; 512 waters 750 and 288 us; 192 molecules 148 and 115), while a batch that
+// fills the GPU with its atoms only pays for the idle warps (4096 molecules: 528.8 ms whole, 533.1 split);
+// every off-diagonal block has exactly one writer and every sum is a gather in a fixed order, so the result is
+// deterministic and needs no atomics.
 //   * the Coulomb term J_A = sum_B (A A | B B) . P_BB (src/fock.rs:427-448) is gathered
 //     lane-parallel, a partner per lane, 32 at a time, in registers, and reduced over the warp once
 //     per atom;
@@ -23,27 +27,22 @@ namespace am1 {
 // register arrays with it at compile time
 __host__ __device__ constexpr int pack2(int a, int b) { return a > b ? a * (a + 1) / 2 + b : b * (b + 1) / 2 + a; }
 
-// One-centre integral (a b | c d) of one atom (src/fock.rs:27-65).
-__device__ __forceinline__ double oc_integral(int a, int b, int c, int d, const DevElem& e) {
-    if (a == b && c == d) {
-        if (a == 0 && c == 0) return e.g_ss;
-        if ((a == 0) != (c == 0)) return e.g_sp;
-        return a == c ? e.g_pp : e.g_p2;
-    }
-    const int ba = min(a, b), bb = max(a, b), kc = min(c, d), kd = max(c, d);
-    if (ba == 0 && bb != 0 && kc == 0 && kd != 0 && bb == kd) return e.h_sp;
-    if (ba != 0 && bb != 0 && ba != bb && ba == kc && bb == kd) return 0.5 * (e.g_pp - e.g_p2);
-    return 0.0;
+// The one-centre integrals of one atom that do not vanish (src/fock.rs:27-65): (mm|ll) and (ml|ml).
+__device__ __forceinline__ double oc_coulomb(int m, int l, const DevElem& e) {
+    return m == l ? (m == 0 ? e.g_ss : e.g_pp) : (m == 0) != (l == 0) ? e.g_sp : e.g_p2;
+}
+__device__ __forceinline__ double oc_exchange(int m, int l, const DevElem& e) {
+    return m == l ? (m == 0 ? e.g_ss : e.g_pp) : (m == 0) != (l == 0) ? e.h_sp : 0.5 * (e.g_pp - e.g_p2);
 }
 
-constexpr int FOCK_WARPS = 8;
 constexpr int FOCK_XX_ROUND = 4;  // heavy-heavy exchange blocks per round of a warp
+static_assert(FOCK_XX_CHUNK % FOCK_XX_ROUND == 0, "whole rounds");
 
 // the AO pair of packed index q (inverse of pack2)
 __host__ __device__ constexpr int pair_hi(int q) { return q < 1 ? 0 : q < 3 ? 1 : q < 6 ? 2 : 3; }
 __host__ __device__ constexpr int pair_lo(int q) { return q - pair_hi(q) * (pair_hi(q) + 1) / 2; }
 
-__global__ void __launch_bounds__(32 * FOCK_WARPS, 2) k_fock(const MolDesc* __restrict__ mols, const int* __restrict__ atom_mol,
+__global__ void __launch_bounds__(32 * FOCK_WARPS, 4) k_fock(const MolDesc* __restrict__ mols, const int* __restrict__ atom_mol,
                                                          int natoms_total, const DevElem* __restrict__ params,
                                                          const int* __restrict__ atom_z, const double* __restrict__ wstore,
                                                          double* __restrict__ arena, const MolState* __restrict__ st, int force) {
@@ -74,6 +73,68 @@ __global__ void __launch_bounds__(32 * FOCK_WARPS, 2) k_fock(const MolDesc* __re
     double* wb = s_w[warp];
     auto ptot = [&](long long idx) { return P1 ? P0[idx] + P1[idx] : P0[idx]; };
 
+    // exchange blocks with heavy partners Bs .. Be - 1 > A (A is the pair's first atom), four at a time:
+    // lanes 8p..8p+7 take B0 + p, a lane per two output elements of the 4 x 4 block (each element the same
+    // sum, in the same order, as one partner at a time)
+    auto exchange = [&](int Bs, int Be) {
+        const int slot = lane >> 3, l8 = lane & 7;
+        for (int B0 = Bs; B0 < Be; B0 += FOCK_XX_ROUND) {
+            const int nb = min(FOCK_XX_ROUND, Be - B0);  // partners in this round
+            const double* blk0 = w + 100LL * ((long long)A * h - (long long)A * (A + 1) / 2 + (B0 - A - 1));
+            for (int l = lane; l < 100 * nb; l += 32) wb[l] = blk0[l];  // the blocks of (A, B0 ..) are adjacent
+            const int B = B0 + slot;
+            const bool mine = slot < nb;
+            const int oB = 4 * B;
+            double hab[2] = {0.0, 0.0};
+            if (mine) {
+#pragma unroll
+                for (int u = 0; u < 2; ++u) {
+                    const int e = 2 * l8 + u;
+                    const long long idx = (long long)(oA + (e >> 2)) * n + oB + (e & 3);
+                    hab[u] = H0[idx];
+                    s_pab[warp][slot][0][e] = P0[idx];
+                    if (P1) s_pab[warp][slot][1][e] = P1[idx];
+                }
+            }
+            __syncwarp();
+            if (mine) {
+                const double* wbh = wb + 100 * slot;
+#pragma unroll
+                for (int u = 0; u < 2; ++u) {
+                    const int e = 2 * l8 + u;
+                    const int mu = e >> 2, la = e & 3;
+                    const long long ab = (long long)(oA + mu) * n + oB + la;
+                    const long long ba = (long long)(oB + la) * n + oA + mu;
+                    for (int c = 0; c < md.nch; ++c) {
+                        double acc = 0.0;
+#pragma unroll
+                        for (int nu = 0; nu < 4; ++nu) {
+                            const double* row = wbh + pack2(mu, nu) * 10;
+#pragma unroll
+                            for (int sg = 0; sg < 4; ++sg) acc += s_pab[warp][slot][c][nu * 4 + sg] * row[pack2(la, sg)];
+                        }
+                        const double v = hab[u] - acc * sc;
+                        double* F = c == 0 ? F0 : F1;
+                        F[ab] = v;
+                        F[ba] = v;
+                    }
+                }
+            }
+            __syncwarp();
+        }
+    };
+    if (blockIdx.y > 0) {  // a chunk of the exchange blocks
+        const int Bs = A + 1 + ((int)blockIdx.y - 1) * FOCK_XX_CHUNK;
+        if (aheavy && Bs < h) exchange(Bs, min(h, Bs + FOCK_XX_CHUNK));
+        return;
+    }
+    if (aheavy && gridDim.y == 1) exchange(A + 1, h);  // a batch that fills the GPU with its atoms: all of them
+    // this lane's element of the atom's own density block, for the one-centre terms
+    const int mu = (lane >> 2) & 3, nu = lane & 3;
+    const bool centre = lane < 16 && mu < naA && nu < naA;
+    const long long dd = (long long)(oA + mu) * n + oA + nu;
+    const double pc[2] = {centre ? P0[dd] : 0.0, centre && P1 ? P1[dd] : 0.0};
+    const double pt = P1 ? pc[0] + pc[1] : pc[0], hdd = centre ? H0[dd] : 0.0;
     // Coulomb gather J_A (per lane over its partners, reduced over the warp once at the end)
     double jl[10];
 #pragma unroll
@@ -109,53 +170,6 @@ __global__ void __launch_bounds__(32 * FOCK_WARPS, 2) k_fock(const MolDesc* __re
                     jl[k] += acc;
                 }
             }
-        }
-        // exchange blocks with the heavier-indexed heavy partners (A is the pair's first atom), four
-        // partners at a time: lanes 8p..8p+7 take B0 + p, a lane per two output elements of the 4 x 4
-        // block (each element the same sum, in the same order, as one partner at a time)
-        const int slot = lane >> 3, l8 = lane & 7;
-        for (int B0 = A + 1; B0 < h; B0 += FOCK_XX_ROUND) {
-            const int nb = min(FOCK_XX_ROUND, h - B0);  // partners in this round
-            const double* blk0 = w + 100LL * ((long long)A * h - (long long)A * (A + 1) / 2 + (B0 - A - 1));
-            for (int l = lane; l < 100 * nb; l += 32) wb[l] = blk0[l];  // the blocks of (A, B0 ..) are adjacent
-            const int B = B0 + slot;
-            const bool mine = slot < nb;
-            const int oB = 4 * B;
-            if (mine) {
-#pragma unroll
-                for (int u = 0; u < 2; ++u) {
-                    const int e = 2 * l8 + u;
-                    const long long idx = (long long)(oA + (e >> 2)) * n + oB + (e & 3);
-                    s_pab[warp][slot][0][e] = P0[idx];
-                    if (P1) s_pab[warp][slot][1][e] = P1[idx];
-                }
-            }
-            __syncwarp();
-            if (mine) {
-                const double* wbh = wb + 100 * slot;
-#pragma unroll
-                for (int u = 0; u < 2; ++u) {
-                    const int e = 2 * l8 + u;
-                    const int mu = e >> 2, la = e & 3;
-                    const long long ab = (long long)(oA + mu) * n + oB + la;
-                    const long long ba = (long long)(oB + la) * n + oA + mu;
-                    const double hab = H0[ab];
-                    for (int c = 0; c < md.nch; ++c) {
-                        double acc = 0.0;
-#pragma unroll
-                        for (int nu = 0; nu < 4; ++nu) {
-                            const double* row = wbh + pack2(mu, nu) * 10;
-#pragma unroll
-                            for (int sg = 0; sg < 4; ++sg) acc += s_pab[warp][slot][c][nu * 4 + sg] * row[pack2(la, sg)];
-                        }
-                        const double v = hab - acc * sc;
-                        double* F = c == 0 ? F0 : F1;
-                        F[ab] = v;
-                        F[ba] = v;
-                    }
-                }
-            }
-            __syncwarp();
         }
     }
     // every other partner, lane-parallel
@@ -252,25 +266,38 @@ __global__ void __launch_bounds__(32 * FOCK_WARPS, 2) k_fock(const MolDesc* __re
     __syncwarp();
     if (lane < npA) s_j[warp][lane] = s_q[warp][lane];
     __syncwarp();
-    // one-centre terms and the diagonal block
-    if (lane < 16) {
-        const int mu = lane >> 2, nu = lane & 3;
-        if (mu < naA && nu < naA) {
-            const DevElem& e = params[md.method * (MAX_Z + 1) + atom_z[a]];
-            for (int c = 0; c < md.nch; ++c) {
-                const double* Pc = c == 0 ? P0 : P1;
-                double acc = 0.0;
-                for (int la = 0; la < naA; ++la)
-                    for (int sg = 0; sg < naA; ++sg) {
-                        const long long idx = (long long)(oA + la) * n + oA + sg;
-                        acc += ptot(idx) * oc_integral(mu, nu, la, sg, e);
-                        acc -= sc * Pc[idx] * oc_integral(mu, la, nu, sg, e);
-                    }
-                const long long d = (long long)(oA + mu) * n + oA + nu;
-                double* F = c == 0 ? F0 : F1;
-                F[d] = H0[d] + acc + s_j[warp][pack2(mu, nu)];
+    // one-centre terms and the diagonal block: of the sums over (la, sg) only the terms with a non-zero
+    // integral, in the order of the full loops: la = sg in a diagonal element, (mu, nu) and (nu, mu) in another
+    const DevElem& e = params[md.method * (MAX_Z + 1) + atom_z[a]];
+    const double ptt = __shfl_sync(0xffffffffu, pt, nu * 4 + mu);
+    double ptd[4];
+#pragma unroll
+    for (int l = 0; l < 4; ++l) ptd[l] = __shfl_sync(0xffffffffu, pt, 5 * l);
+    for (int c = 0; c < md.nch; ++c) {
+        const double p = c == 0 ? pc[0] : pc[1], pT = __shfl_sync(0xffffffffu, p, nu * 4 + mu);
+        double pd[4];
+#pragma unroll
+        for (int l = 0; l < 4; ++l) pd[l] = __shfl_sync(0xffffffffu, p, 5 * l);
+        if (!centre) continue;
+        double acc = 0.0;
+        if (mu == nu) {
+#pragma unroll
+            for (int l = 0; l < 4; ++l)
+                if (l < naA) {
+                    acc += ptd[l] * oc_coulomb(mu, l, e);
+                    acc -= sc * pd[l] * oc_exchange(mu, l, e);
+                }
+        } else {
+            const double x = oc_exchange(mu, nu, e), g = oc_coulomb(mu, nu, e);
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const bool own = (mu < nu) == (u == 0);  // (la, sg) = (mu, nu), else (nu, mu)
+                acc += (own ? pt : ptt) * x;
+                acc -= sc * (own ? p : pT) * (own ? g : x);
             }
         }
+        double* F = c == 0 ? F0 : F1;
+        F[dd] = hdd + acc + s_j[warp][pack2(mu, nu)];
     }
 }
 

@@ -67,11 +67,17 @@ __global__ void k_state_init(MolState* __restrict__ st, const MolDesc* __restric
     st[i] = s;
 }
 
-// Identity warm start for the eigensolver (C^T = I; the slot is zero-filled beforehand).
-__global__ void k_identity(const ChanJob* __restrict__ jobs) {
-    const ChanJob jb = jobs[blockIdx.y];
-    double* Ct = jb.Ct;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < jb.n; i += gridDim.x * blockDim.x) Ct[(long long)i * jb.n + i] = 1.0;
+// P = 0 (k_sad_init then sets its diagonal) and the eigensolver's warm start C^T = I, the two slots a run reads
+// before it writes them.  Bound by the writes; the whole arena, six slots and more a channel, was zeroed for these
+// two, and twice in a batched call (25 GB each time for 4096 molecules, 7 ms a call).
+__global__ void __launch_bounds__(256) k_slots_init(const ChanJob* __restrict__ jobs) {
+    static_assert(SLOT_CT == SLOT_P + 1, "P and Ct adjacent");
+    const ChanJob& jb = jobs[blockIdx.y];
+    const int n = jb.n;
+    double* P = jb.P;
+    const long long nn = (long long)n * n;
+    for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < 2 * nn; i += (long long)gridDim.x * 256)
+        P[i] = i >= nn && (i - nn) % (n + 1) == 0 ? 1.0 : 0.0;
 }
 
 __device__ __forceinline__ void live_slots(const MolState& s, int& newslot, unsigned& live_mask) {

@@ -170,6 +170,12 @@ __global__ void k_core_energy(const MolDesc* mols, const double* ecc, MolState* 
 // 3 doubles per atom, internal atom order
 __global__ void k_gradient(const MolDesc* mols, const int* atom_mol, int natoms_total, const DevElem* params, const int* atom_z,
                            const double* atom_xyz, const ChanJob* jobs, const int* mol_job0, double* gradient, int* mol_status);
+// grid fock_grid(...), 32 FOCK_WARPS threads
+constexpr int FOCK_WARPS = 4, FOCK_XX_CHUNK = 16, FOCK_SPLIT_ATOMS = 32768;
+inline dim3 fock_grid(long long natoms, int most_heavy) {  // atoms of the launch, most heavy atoms of a molecule
+    const unsigned chunks = natoms >= FOCK_SPLIT_ATOMS || most_heavy < 2 ? 0u : (unsigned)((most_heavy - 1 + FOCK_XX_CHUNK - 1) / FOCK_XX_CHUNK);
+    return dim3((unsigned)((natoms + FOCK_WARPS - 1) / FOCK_WARPS), 1 + chunks);
+}
 __global__ void k_fock(const MolDesc* mols, const int* atom_mol, int natoms_total, const DevElem* params,
                        const int* atom_z, const double* wstore, double* arena, const MolState* st, int force);
 // out_r[i][j] = in_r[map[i]][map[j]] for matrices r = blockIdx.y, n x n, at strides so and si (doubles);
@@ -385,7 +391,8 @@ __device__ __forceinline__ double group_share_sum(const double* share, int G) {
 
 __global__ void k_sad_init(const MolDesc* mols, const int* atom_mol, int natoms_total, const DevElem* params,
                            const int* atom_z, double* arena);
-__global__ void k_identity(const ChanJob* jobs);
+// P = 0, Ct = I of every channel (adjacent slots); grid (any, channels)
+__global__ void k_slots_init(const ChanJob* jobs);
 // largest open-shell molecule (orbitals) that takes the mixed path's TF32 phase
 constexpr int kLowpMaxOpenShellAo = 448;
 __global__ void k_state_init(MolState* st, const MolDesc* mols, int nmol, int lowp);
