@@ -744,6 +744,12 @@ int plan_molecule(const am1gpu_molecule& m, const am1gpu_options& o, int user, M
 }
 
 struct Batch {
+    Batch() = default;
+    Batch(const Batch&) = delete;
+    Batch& operator=(const Batch&) = delete;
+    ~Batch() {
+        if (graph_exec) cudaGraphExecDestroy(graph_exec);  // one still running is freed once it completes
+    }
     int nmol = 0, natoms = 0, nblk = 1, maxn = 0, maxheavy = 0;
     long long npairs = 0;
     std::vector<MolPlan> plans;
@@ -788,7 +794,7 @@ struct Batch {
     int nt_oz = 0;
     Sp2State* d_sp2_state;
     TriJob* d_tri;
-    int* d_need_eigen;
+    int* d_need_eigen;  // per molecule: its purification stalled; [-1]: some molecule's did
     // channels whose FP64 purifications run in one launch each: groups of d_fused (k_sp2_res with C = 1, or
     // clusters of C CTAs of k_sp2_clu), and how many channels take the launch-per-step kernels instead
     struct FusedGroup {
@@ -827,11 +833,9 @@ struct Batch {
     GraphLoop* d_loop = nullptr;  // loop counters of the captured solve
     GraphLoop* h_loop = nullptr;  // their pinned host copy
     char *d_extra = nullptr, *h_extra = nullptr;  // the caller's own regions (build_batch's extra_dev, extra_host)
-    // kernels per captured head (+ arm), step (+ condition), tail (+ its two control kernels), and
-    // stalled-purification eigensolver (run in GraphLoop::eig_runs iterations)
-    int64_t graph_counts[4] = {0, 0, 0, 0};
-    bool graph_cacheable = false;  // a resident batch keeps its instantiated graph across runs
-    cudaGraphExec_t graph_exec = nullptr;
+    // kernels per captured head (+ arm), step and tail (+ condition)
+    int64_t graph_counts[3] = {0, 0, 0};
+    cudaGraphExec_t graph_exec = nullptr;  // the captured loop; a resident batch keeps it across runs
 };
 
 // Lays out the batch in one device pool and one pinned staging area, copies inputs.
@@ -928,7 +932,7 @@ int build_batch(const am1gpu_molecule* in, const am1gpu_options& o, std::vector<
     // ---- device-only region
     size_t dv = staged;
     const size_t o_status = take(dv, sizeof(int) * b.nmol);
-    const size_t o_need = take(dv, sizeof(int) * b.nmol);
+    const size_t o_need = take(dv, sizeof(int) * (b.nmol + 1));
     const size_t o_sp2a = take(dv, sizeof(int) * 4);
     const size_t o_work = take(dv, sizeof(double) * kWorkN);
     const size_t o_sp2s = take(dv, sizeof(Sp2State) * nch_total);
@@ -1006,7 +1010,7 @@ int build_batch(const am1gpu_molecule* in, const am1gpu_options& o, std::vector<
     std::vector<int> fused_jobs[2];  // k_sp2_res, k_sp2_clu
     long long xc_off = 0;
     b.unfused = 0;
-    b.d_need_eigen = (int*)dptr(o_need);
+    b.d_need_eigen = (int*)dptr(o_need) + 1;
     b.d_sp2_active = (int*)dptr(o_sp2a);
     b.d_work = (double*)dptr(o_work);
     b.d_sp2_state = (Sp2State*)dptr(o_sp2s);
@@ -1681,6 +1685,9 @@ struct IterEnq {
     int nblk, rowblk, njobs;
     Run* run;
     size_t ph;  // start event of the phase being timed
+    // the second half of the iteration for the molecules with (mask[mol] != 0) == want only (NULL: all)
+    const int* mask = nullptr;
+    int want = 0;
 };
 
 // Fock build, commutator and history, extrapolation; with enq_sp2_start it is the first half of an
@@ -1710,7 +1717,7 @@ int enq_head(IterEnq& e) {
     k_combine<<<dim3(e.rowblk, e.njobs), 256, 0, s>>>(b.d_jobs, b.d_st, 0);
     run.launched(AM1GPU_PHASE_ACCEL, 2);
     if ((rc = run.end(AM1GPU_PHASE_ACCEL, e.ph)) || (rc = run.begin(&e.ph))) return rc;
-    if (density_mode() == 0) CK(cudaMemsetAsync(b.d_need_eigen, 0, sizeof(int) * b.nmol, s));
+    if (density_mode() == 0) CK(cudaMemsetAsync(b.d_need_eigen - 1, 0, sizeof(int) * (b.nmol + 1), s));
     CK(cudaGetLastError());
     return AM1GPU_OK;
 }
@@ -1836,11 +1843,13 @@ int enq_tail_stall(IterEnq& e) {
     Run& run = *e.run;
     int rc;
     if (density_mode() != 0) return AM1GPU_OK;
-    k_gemm_nn<<<b.nt_gt, 256, 0, s>>>(b.d_gj_gt, b.d_gt_gt, b.nt_gt, b.d_st, 0, b.d_need_eigen);
+    // few CTAs: there is rarely anything to do (a CTA per tile cost 0.6 ms an iteration for 4096 molecules)
+    const int ctas_nn = std::min(b.nt_gt, 4 * g_sms), ctas_tn = std::min(b.nt_dn, 4 * g_sms);
+    k_gemm_nn<<<ctas_nn, 256, 0, s>>>(b.d_gj_gt, b.d_gt_gt, b.nt_gt, b.d_st, 0, b.d_need_eigen);
     if ((rc = launch_jacobi(b, e.ws, 0, b.d_need_eigen, e.s))) return rc;
     run.launched(AM1GPU_PHASE_EIGEN, (int)b.buckets.size());
     if (b.neig > 0) k_eig_sort<<<b.neig, 512, 0, s>>>(b.d_eig, b.d_st, 0, b.d_need_eigen);
-    k_gemm_tn<<<b.nt_dn, 256, 0, s>>>(b.d_gj_dn, b.d_gt_dn, b.nt_dn, b.d_st, 0, b.d_need_eigen);
+    k_gemm_tn<<<ctas_tn, 256, 0, s>>>(b.d_gj_dn, b.d_gt_dn, b.nt_dn, b.d_st, 0, b.d_need_eigen);
     run.launched(AM1GPU_PHASE_EIGEN, 3);
     CK(cudaGetLastError());
     return AM1GPU_OK;
@@ -1852,9 +1861,9 @@ int enq_tail_rest(IterEnq& e) {
     Run& run = *e.run;
     int rc;
     if (density_mode() == 0 && ((rc = run.end(AM1GPU_PHASE_EIGEN, e.ph)) || (rc = run.begin(&e.ph)))) return rc;
-    k_density_post<<<dim3(dens_blocks(b.maxn), e.njobs), 256, 0, s>>>(b.d_jobs, b.d_st, e.nblk);
-    k_converge<<<cdiv(b.nmol, SCF_MOL_WARPS), 32 * SCF_MOL_WARPS, 0, s>>>(b.d_mols, b.d_jobs, b.d_job0, b.nmol, b.d_st, b.d_status, e.nblk, e.prm,
-                                                 b.d_active);
+    k_density_post<<<dim3(dens_blocks(b.maxn), e.njobs), 256, 0, s>>>(b.d_jobs, b.d_st, e.nblk, e.mask, e.want);
+    k_converge<<<cdiv(b.nmol, SCF_MOL_WARPS), 32 * SCF_MOL_WARPS, 0, s>>>(b.d_mols, b.d_jobs, b.d_job0, b.nmol, b.d_st, b.d_status, e.nblk,
+                                                                                 e.prm, b.d_active, e.mask, e.want);
     run.launched(AM1GPU_PHASE_DENSITY, 2);
     if ((rc = run.end(AM1GPU_PHASE_DENSITY, e.ph))) return rc;
     CK(cudaGetLastError());
@@ -1915,30 +1924,18 @@ int add_while(cudaGraph_t g, cudaGraphNode_t dep, cudaGraphConditionalHandle h, 
     return AM1GPU_OK;
 }
 
-// An IF node after `dep` in g, with handle h; its body graph in *body.
-int add_if(cudaGraph_t g, cudaGraphNode_t dep, cudaGraphConditionalHandle h, cudaGraphNode_t* node, cudaGraph_t* body) {
-    cudaGraphNodeParams np{};
-    np.type = cudaGraphNodeTypeConditional;
-    np.conditional.handle = h;
-    np.conditional.type = cudaGraphCondTypeIf;
-    np.conditional.size = 1;
-    CK(cudaGraphAddNode(node, g, &dep, 1, &np));
-    *body = np.conditional.phGraph_out[0];
-    return AM1GPU_OK;
-}
-
 // The SCF loop of run_device as one graph launch:
 //   k_scf_arm -> WHILE(scf) { head -> [one-launch purifications | start -> k_sp2_arm -> WHILE(sp2) { step }]
 //                             -> tail -> k_scf_cond }
-// (the step's update kernel sets the purification loop's condition itself, k_sp2_update_cond) and, in a
-// graph kept for a resident batch's later runs, the tail split as
-//   finish -> k_stall_arm -> IF(stall) { stalled-purification eigensolver } -> rest -> k_scf_cond.
-// The kernels are the eager loop's, in the same order; only the loop decisions moved to the device
-// (k_graph.cu), and the eigensolver kernels for stalled purifications, which change nothing in an
-// iteration where no purification stalled, run only in iterations where one did.  So the results
-// are the same bit for bit.  The purification loop stops as soon as no
-// channel purifies (the eager loop looks every six steps from the twelfth on); the extra eager
-// steps change nothing, because finished channels skip their products.
+// (the step's update kernel sets the purification loop's condition itself, k_sp2_update_cond).
+// The kernels are the host-driven loop's, in the same order; only the loop decisions moved to the device
+// (k_graph.cu).  The eigensolver for stalled purifications is not in the graph (four launches and more in every
+// iteration, of which next to none has work: 0.1 of methane's 1.1 ms): an iteration in which a purification
+// stalled completes every other molecule and ends the loop, the host runs the eigensolver and the rest of that
+// iteration for the stalled ones (run_device) and launches the graph again.  So the results are the same bit for
+// bit.  The purification loop stops as soon as no channel purifies (the host-driven loop looks every six
+// steps from the twelfth on); the extra steps there change nothing, because finished channels skip their
+// products.
 // *launched: the graph was launched (an error before that leaves the stream untouched).
 int scf_loop_graph(IterEnq& e, const am1gpu_options& o, bool* launched) {
     Batch& b = e.b;
@@ -1946,7 +1943,7 @@ int scf_loop_graph(IterEnq& e, const am1gpu_options& o, bool* launched) {
     const int sp2_max = sp2_max_steps();
     if (int rc0 = mem_side_stream(m)) return rc0;
     const cudaStream_t cs = m.cap_stream;
-    if (b.graph_cacheable && b.graph_exec) {  // a resident batch's graph, captured on its first run
+    if (b.graph_exec) {  // captured on the batch's first run
         *launched = true;
         CK(cudaGraphLaunch(b.graph_exec, e.s));
         CK(cudaMemcpyAsync(b.h_loop, b.d_loop, sizeof(GraphLoop), cudaMemcpyDeviceToHost, e.s));
@@ -2005,55 +2002,25 @@ int scf_loop_graph(IterEnq& e, const am1gpu_options& o, bool* launched) {
     }
     const int64_t per_step = cnt.kernel_launches - step0;
     const int64_t tail0 = cnt.kernel_launches;
-    int64_t per_stall = 0, per_tail = 0;
-    if (b.graph_cacheable) {
-        // a graph kept for the batch's later runs: the stalled-purification eigensolver behind an IF
-        // node (its extra capture and instantiation cost more than they save in a one-off graph)
-        cudaGraphConditionalHandle h_stall;
-        CK(cudaGraphConditionalHandleCreate(&h_stall, body, 0, 0));
-        cudaGraphNode_t fin, w_stall, stall_last;
-        if ((rc = capture_into(cs, body, purified.data(), purified.size(), &fin, [&]() -> int {
-                 int r = enq_tail_finish(ce, false);
-                 if (r) return r;
-                 k_stall_arm<<<1, 256, 0, cs>>>(h_stall, b.d_loop, b.d_need_eigen, b.nmol);
-                 return AM1GPU_OK;
-             })))
-            return rc;
-        const int64_t stall0 = cnt.kernel_launches;
-        cudaGraph_t body3 = nullptr;
-        if ((rc = add_if(body, fin, h_stall, &w_stall, &body3))) return rc;
-        if ((rc = capture_into(cs, body3, nullptr, 0, &stall_last, [&]() -> int { return enq_tail_stall(ce); }))) return rc;
-        per_stall = cnt.kernel_launches - stall0;
-        if ((rc = capture_into(cs, body, &w_stall, 1, &tail, [&]() -> int {
-                 int r = enq_tail_rest(ce);
-                 if (r) return r;
-                 k_scf_cond<<<1, 32, 0, cs>>>(h_scf, b.d_loop, b.d_active, o.max_scf);
-                 return AM1GPU_OK;
-             })))
-            return rc;
-        per_tail = cnt.kernel_launches - tail0 + 2 - per_stall;
-    } else {
-        if ((rc = capture_into(cs, body, purified.data(), purified.size(), &tail, [&]() -> int {
-                 int r = enq_tail(ce, false);
-                 if (r) return r;
-                 k_scf_cond<<<1, 32, 0, cs>>>(h_scf, b.d_loop, b.d_active, o.max_scf);
-                 return AM1GPU_OK;
-             })))
-            return rc;
-        per_tail = cnt.kernel_launches - tail0 + 1;
-    }
+    ce.mask = b.d_need_eigen;  // molecules whose purification stalled wait for the host
+    if ((rc = capture_into(cs, body, purified.data(), purified.size(), &tail, [&]() -> int {
+             int r = enq_tail_finish(ce, false);
+             if (!r) r = enq_tail_rest(ce);
+             if (r) return r;
+             k_scf_cond<<<1, 32, 0, cs>>>(h_scf, b.d_loop, b.d_active, b.d_need_eigen, o.max_scf);
+             return AM1GPU_OK;
+         })))
+        return rc;
+    const int64_t per_tail = cnt.kernel_launches - tail0 + 1;
     cudaGraphExec_t ge = nullptr;
     CK(cudaGraphInstantiate(&ge, g, 0));
+    b.graph_exec = ge;
     *launched = true;
-    const cudaError_t le = cudaGraphLaunch(ge, e.s);
-    if (b.graph_cacheable && le == cudaSuccess) b.graph_exec = ge;
-    else cudaGraphExecDestroy(ge);  // an executable graph still running is freed once it completes
-    CK(le);
+    CK(cudaGraphLaunch(ge, e.s));
     CK(cudaMemcpyAsync(b.h_loop, b.d_loop, sizeof(GraphLoop), cudaMemcpyDeviceToHost, e.s));
     b.graph_counts[0] = per_head;
     b.graph_counts[1] = per_step;
     b.graph_counts[2] = per_tail;
-    b.graph_counts[3] = per_stall;
     return AM1GPU_OK;
 }
 
@@ -2099,6 +2066,8 @@ int run_device(Batch& b, Mem& mem, const DevElem* dp, const am1gpu_options& o, a
         if (rc) {  // the graph could not be built here: the host-driven loop runs the same kernels
             graph = false;
             cudaGetLastError();
+        } else {
+            stats->graph_launches += 1;
         }
     }
     if (!graph) {
@@ -2139,43 +2108,57 @@ int run_device(Batch& b, Mem& mem, const DevElem* dp, const am1gpu_options& o, a
             if (lowp_left && b.h_active[2] == 0) lowp_left = false;  // no molecule returns to TF32
         }
     }
-    stats->scf_cycles = done;
     const int nblk = b.nblk;
-    // final energy at the final density (src/scf.rs:698-701, 835-839) and the result records
-    if ((rc = run.begin(&ph))) return rc;
-    k_fock<<<fock_grid(b.natoms, b.maxheavy), 32 * FOCK_WARPS, 0, s>>>(b.d_mols, b.d_atom_mol, b.natoms, dp, b.d_atom_z, b.d_wstore, b.d_arena, b.d_st, 1);
-    k_post_fock<<<dim3(nblk, njobs), 256, 0, s>>>(b.d_jobs, b.d_mols, b.d_st, nblk, 1, 1);
-    k_final_energy<<<cdiv(b.nmol, SCF_MOL_WARPS), 32 * SCF_MOL_WARPS, 0, s>>>(b.d_mols, b.d_jobs, b.d_job0, b.nmol, b.d_st, nblk);
-    // eigenvalues of the last F* (mo_energies, HOMO/LUMO): tridiagonalisation + bisection
-    if ((rc = launch_tridiag(b, ws))) return rc;
-    int64_t big_tri_launches = 0;
-    if ((rc = launch_big_tridiag(b, s, &big_tri_launches))) return rc;
-    bisect_launch(b.d_tri, njobs, b.maxn, s);
-    k_results<<<b.nmol, RESULT_THREADS, 0, s>>>(b.d_mols, b.d_jobs, b.d_job0, b.nmol, b.d_st, b.d_status, dp, b.d_atom_z,
-                                                 b.d_atom_xyz, b.d_res, b.d_charges);
-    run.launched(AM1GPU_PHASE_FINAL, 5 + (int)b.tri_buckets.size() + (int)big_tri_launches);
-    CK(cudaGetLastError());
-    if ((rc = run.end(AM1GPU_PHASE_FINAL, ph))) return rc;
     size_t t1;
-    if ((rc = run.event(&t1))) return rc;
-    CK(cudaMemcpyAsync(b.h_work, b.d_work, sizeof(double) * kWorkN, cudaMemcpyDeviceToHost, s));
-    CK(cudaMemcpyAsync(b.h_active + 2, b.d_sp2_active + 2, sizeof(int), cudaMemcpyDeviceToHost, s));
-    CK(cudaStreamSynchronize(s));
-    if (b.h_active[2] & (1 << 10)) return fail(AM1GPU_LINALG, "a purification iterate left the range of its digit planes (|x| >= 2)");
-    if (b.h_active[2]) return fail(AM1GPU_DEVICE_ERROR, "a tensor-core step gave up waiting for its MMAs or operand copies");
+    for (bool again = true; again;) {
+        again = false;
+        // final energy at the final density (src/scf.rs:698-701, 835-839) and the result records
+        if ((rc = run.begin(&ph))) return rc;
+        k_fock<<<fock_grid(b.natoms, b.maxheavy), 32 * FOCK_WARPS, 0, s>>>(b.d_mols, b.d_atom_mol, b.natoms, dp, b.d_atom_z, b.d_wstore,
+                                                                           b.d_arena, b.d_st, 1);
+        k_post_fock<<<dim3(nblk, njobs), 256, 0, s>>>(b.d_jobs, b.d_mols, b.d_st, nblk, 1, 1);
+        k_final_energy<<<cdiv(b.nmol, SCF_MOL_WARPS), 32 * SCF_MOL_WARPS, 0, s>>>(b.d_mols, b.d_jobs, b.d_job0, b.nmol, b.d_st, nblk);
+        // eigenvalues of the last F* (mo_energies, HOMO/LUMO): tridiagonalisation + bisection
+        if ((rc = launch_tridiag(b, ws))) return rc;
+        int64_t big_tri_launches = 0;
+        if ((rc = launch_big_tridiag(b, s, &big_tri_launches))) return rc;
+        bisect_launch(b.d_tri, njobs, b.maxn, s);
+        k_results<<<b.nmol, RESULT_THREADS, 0, s>>>(b.d_mols, b.d_jobs, b.d_job0, b.nmol, b.d_st, b.d_status, dp, b.d_atom_z,
+                                                     b.d_atom_xyz, b.d_res, b.d_charges);
+        run.launched(AM1GPU_PHASE_FINAL, 5 + (int)b.tri_buckets.size() + (int)big_tri_launches);
+        CK(cudaGetLastError());
+        if ((rc = run.end(AM1GPU_PHASE_FINAL, ph))) return rc;
+        if ((rc = run.event(&t1))) return rc;
+        CK(cudaMemcpyAsync(b.h_work, b.d_work, sizeof(double) * kWorkN, cudaMemcpyDeviceToHost, s));
+        CK(cudaMemcpyAsync(b.h_active + 2, b.d_sp2_active + 2, sizeof(int), cudaMemcpyDeviceToHost, s));
+        CK(cudaStreamSynchronize(s));
+        if (b.h_active[2] & (1 << 10)) return fail(AM1GPU_LINALG, "a purification iterate left the range of its digit planes (|x| >= 2)");
+        if (b.h_active[2]) return fail(AM1GPU_DEVICE_ERROR, "a tensor-core step gave up waiting for its MMAs or operand copies");
+        if (!graph) break;
+        // what the captured loops launched, and whether they ended on a stalled purification (the results
+        // just formed are then of an unfinished solve, and are formed again)
+        const GraphLoop lp = *b.h_loop;
+        b.h_loop->stalled = b.h_loop->scf_iter = b.h_loop->sp2_total = 0;
+        done += lp.scf_iter;
+        stats->kernel_launches += 1 + (int64_t)lp.scf_iter * (b.graph_counts[0] + b.graph_counts[2]) + (int64_t)lp.sp2_total * b.graph_counts[1];
+        if (lp.stalled) {
+            again = true;
+            e.mask = b.d_need_eigen;
+            e.want = 1;
+            if ((rc = run.begin(&e.ph)) || (rc = enq_tail_stall(e)) || (rc = enq_tail_rest(e))) return rc;
+            CK(cudaMemcpyAsync(b.h_active, b.d_active, sizeof(int), cudaMemcpyDeviceToHost, s));
+            CK(cudaStreamSynchronize(s));
+            bool launched = false;
+            if (b.h_active[0] > 0 && (rc = scf_loop_graph(e, o, &launched))) return rc;
+        }
+    }
+    stats->scf_cycles = done;
     stats->purification_steps += b.h_work[0];
     stats->purification_flops += b.h_work[1];
     stats->purification_bytes += b.h_work[3];
     stats->eigen_fallbacks += (int32_t)b.h_work[2];
     stats->lowp_purification_steps += b.h_work[4];
     stats->lowp_purification_flops += b.h_work[5];
-    if (graph) {  // what the captured loops launched
-        const GraphLoop lp = *b.h_loop;
-        stats->scf_cycles = lp.scf_iter;
-        stats->kernel_launches += 1 + (int64_t)lp.scf_iter * (b.graph_counts[0] + b.graph_counts[2]) +
-                                  (int64_t)lp.sp2_total * b.graph_counts[1] + (int64_t)lp.eig_runs * b.graph_counts[3];
-        stats->graph_launches += 1;
-    }
     float ms = 0.f;
     CK(cudaEventElapsedTime(&ms, mem.events[t0], mem.events[t1]));
     stats->device_ms += ms;
@@ -3035,7 +3018,7 @@ int density_purify_one(int n, const double* F, double nocc, double weight, int p
     if (precision == 0) {  // the whole purification in one launch (the list is the one job, 0)
         CK(cudaMemsetAsync(D + o_list, 0, sizeof(int), s));
         const int* list = (const int*)(D + o_list);
-        int* need = (int*)(D + o_need);
+        int* need = (int*)(D + o_need) + 1;
         double* work = (double*)(D + o_work);
         int max_steps = kSp2MaxSteps;
         const size_t smem = sp2_fused_smem_bytes(n, jb.fused == FU_RES);
@@ -3070,7 +3053,7 @@ int density_purify_one(int n, const double* F, double nocc, double weight, int p
                 if (hact[0] == 0) break;
             }
         }
-        k_sp2_finish<<<dim3(std::max(8u, std::min(256u, cdiv(nn, 65536))), 1), 256, 0, s>>>(dj, dsst, dms, (int*)(D + o_need),
+        k_sp2_finish<<<dim3(std::max(8u, std::min(256u, cdiv(nn, 65536))), 1), 256, 0, s>>>(dj, dsst, dms, (int*)(D + o_need) + 1,
                                                                                            (double*)(D + o_work), (int*)(D + o_stall),
                                                                                            dact + 3);
         CK(cudaGetLastError());
@@ -3557,7 +3540,6 @@ int am1gpu_batch_create(int32_t nmol, const am1gpu_molecule* mols, const am1gpu_
     if (!plans.empty()) {
         if (opts->precision == AM1GPU_PRECISION_MIXED) rc = tune_lowp_kernels(plans);
         if (!rc) rc = build_batch(mols, *opts, std::move(plans), h->b, h->mem, &h->stats);
-        h->b.graph_cacheable = true;
         if (!rc && cudaStreamSynchronize(h->mem.stream) != cudaSuccess) rc = fail(AM1GPU_DEVICE_ERROR, "upload failed");
         if (rc) {
             mem_release(h->mem);
@@ -3609,6 +3591,7 @@ void am1gpu_batch_destroy(am1gpu_batch* h) {
     if (h->b.graph_exec) {
         cudaStreamSynchronize(h->mem.stream);
         cudaGraphExecDestroy(h->b.graph_exec);
+        h->b.graph_exec = nullptr;
     }
     am1::mem_release(h->mem);
     delete h;

@@ -19,7 +19,7 @@ __global__ void k_scf_arm(cudaGraphConditionalHandle h, GraphLoop* loop, int max
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
     loop->scf_iter = 0;
     loop->sp2_total = 0;
-    loop->eig_runs = 0;
+    loop->stalled = 0;
     cudaGraphSetConditional(h, max_scf > 0 ? 1u : 0u);
 }
 
@@ -33,25 +33,15 @@ __global__ void k_sp2_arm(cudaGraphConditionalHandle h, GraphLoop* loop) {
     cudaGraphSetConditional(h, 1u);
 }
 
-// After the purified densities of an iteration: the stalled-purification eigensolver runs only if
-// some molecule's purification stalled (need_eigen set by k_sp2_finish).  One CTA.
-__global__ void k_stall_arm(cudaGraphConditionalHandle h, GraphLoop* loop, const int* need_eigen, int nmol) {
-    int any = 0;
-    for (int i = threadIdx.x; i < nmol; i += blockDim.x) any |= need_eigen[i] != 0;
-    any = __syncthreads_or(any);
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
-        if (any) loop->eig_runs += 1;
-        cudaGraphSetConditional(h, any ? 1u : 0u);
-    }
-}
-
-// After each SCF iteration (k_converge has counted the molecules still iterating in active[0]):
-// go round again while any is and fewer than max_scf iterations were done.
-__global__ void k_scf_cond(cudaGraphConditionalHandle h, GraphLoop* loop, const int* active, int max_scf) {
+// After each SCF iteration (k_converge has counted the molecules still iterating in active[0]): go round
+// again while any is and fewer than max_scf iterations were done, unless some purification stalled
+// (need_eigen[-1]): those molecules wait for the host, which runs their eigensolver.
+__global__ void k_scf_cond(cudaGraphConditionalHandle h, GraphLoop* loop, const int* active, const int* need_eigen, int max_scf) {
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    const int it = loop->scf_iter + 1;
+    const int it = loop->scf_iter + 1, stalled = need_eigen[-1] != 0;
     loop->scf_iter = it;
-    cudaGraphSetConditional(h, (active[0] > 0 && it < max_scf) ? 1u : 0u);
+    loop->stalled = stalled;
+    cudaGraphSetConditional(h, (active[0] > 0 && it < max_scf && !stalled) ? 1u : 0u);
 }
 
 }  // namespace am1

@@ -35,59 +35,60 @@ __device__ __forceinline__ void gemm_tile(const GemmJob* __restrict__ jobs, cons
                                           const MolState* __restrict__ st, int force, const int* __restrict__ mask) {
     __shared__ double As[GB_K][GB_M + 1];
     __shared__ double Bs[GB_K][GB_N + 1];
-    const int t = blockIdx.x;
-    if (t >= ntiles) return;
-    const GemmTile tl = tiles[t];
-    const GemmJob jb = jobs[tl.job];
-    if (!force && !st[jb.mol].active) return;
-    if (mask && !mask[jb.mol]) return;
-    const int m0 = tl.tm * GB_M, n0 = tl.tn * GB_N;
-    const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
-    double acc[4][4];
+    if (mask && !mask[-1]) return;
+    for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
+        const GemmTile tl = tiles[t];
+        const GemmJob jb = jobs[tl.job];
+        if (!force && !st[jb.mol].active) continue;
+        if (mask && !mask[jb.mol]) continue;
+        const int m0 = tl.tm * GB_M, n0 = tl.tn * GB_N;
+        const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
+        double acc[4][4];
 #pragma unroll
-    for (int r = 0; r < 4; ++r)
+        for (int r = 0; r < 4; ++r)
 #pragma unroll
-        for (int c = 0; c < 4; ++c) acc[r][c] = 0.0;
-    for (int k0 = 0; k0 < jb.K; k0 += GB_K) {
+            for (int c = 0; c < 4; ++c) acc[r][c] = 0.0;
+        for (int k0 = 0; k0 < jb.K; k0 += GB_K) {
 #pragma unroll
-        for (int l = 0; l < 4; ++l) {
-            const int idx = tid + l * 256;
-            if (TA) {  // A is K x M: element (k, i)
-                const int i = idx & 63, k = idx >> 6;
-                const int gi = m0 + i, gk = k0 + k;
-                As[k][i] = (gi < jb.M && gk < jb.K) ? jb.A[(long long)gk * jb.lda + gi] : 0.0;
-            } else {  // A is M x K: element (i, k)
-                const int k = idx & 15, i = idx >> 4;
-                const int gi = m0 + i, gk = k0 + k;
-                As[k][i] = (gi < jb.M && gk < jb.K) ? jb.A[(long long)gi * jb.lda + gk] : 0.0;
+            for (int l = 0; l < 4; ++l) {
+                const int idx = tid + l * 256;
+                if (TA) {  // A is K x M: element (k, i)
+                    const int i = idx & 63, k = idx >> 6;
+                    const int gi = m0 + i, gk = k0 + k;
+                    As[k][i] = (gi < jb.M && gk < jb.K) ? jb.A[(long long)gk * jb.lda + gi] : 0.0;
+                } else {  // A is M x K: element (i, k)
+                    const int k = idx & 15, i = idx >> 4;
+                    const int gi = m0 + i, gk = k0 + k;
+                    As[k][i] = (gi < jb.M && gk < jb.K) ? jb.A[(long long)gi * jb.lda + gk] : 0.0;
+                }
+                const int j = idx & 63, kb = idx >> 6;
+                const int gj = n0 + j, gkb = k0 + kb;
+                Bs[kb][j] = (gj < jb.N && gkb < jb.K) ? jb.B[(long long)gkb * jb.ldb + gj] : 0.0;
             }
-            const int j = idx & 63, kb = idx >> 6;
-            const int gj = n0 + j, gkb = k0 + kb;
-            Bs[kb][j] = (gj < jb.N && gkb < jb.K) ? jb.B[(long long)gkb * jb.ldb + gj] : 0.0;
+            __syncthreads();
+#pragma unroll
+            for (int k = 0; k < GB_K; ++k) {
+                double a[4], b[4];
+#pragma unroll
+                for (int r = 0; r < 4; ++r) a[r] = As[k][ty + 16 * r];
+#pragma unroll
+                for (int c = 0; c < 4; ++c) b[c] = Bs[k][tx + 16 * c];
+#pragma unroll
+                for (int r = 0; r < 4; ++r)
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) acc[r][c] = fma(a[r], b[c], acc[r][c]);
+            }
+            __syncthreads();
         }
-        __syncthreads();
 #pragma unroll
-        for (int k = 0; k < GB_K; ++k) {
-            double a[4], b[4];
+        for (int r = 0; r < 4; ++r) {
+            const int gi = m0 + ty + 16 * r;
+            if (gi >= jb.M) continue;
 #pragma unroll
-            for (int r = 0; r < 4; ++r) a[r] = As[k][ty + 16 * r];
-#pragma unroll
-            for (int c = 0; c < 4; ++c) b[c] = Bs[k][tx + 16 * c];
-#pragma unroll
-            for (int r = 0; r < 4; ++r)
-#pragma unroll
-                for (int c = 0; c < 4; ++c) acc[r][c] = fma(a[r], b[c], acc[r][c]);
-        }
-        __syncthreads();
-    }
-#pragma unroll
-    for (int r = 0; r < 4; ++r) {
-        const int gi = m0 + ty + 16 * r;
-        if (gi >= jb.M) continue;
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-            const int gj = n0 + tx + 16 * c;
-            if (gj < jb.N) jb.C[(long long)gi * jb.ldc + gj] = jb.alpha * acc[r][c];
+            for (int c = 0; c < 4; ++c) {
+                const int gj = n0 + tx + 16 * c;
+                if (gj < jb.N) jb.C[(long long)gi * jb.ldc + gj] = jb.alpha * acc[r][c];
+            }
         }
     }
 }

@@ -668,9 +668,10 @@ __global__ void k_combine(const ChanJob* __restrict__ jobs, const MolState* __re
     }
 }
 
-__global__ void k_density_post(const ChanJob* __restrict__ jobs, const MolState* __restrict__ st, int nblk) {
+__global__ void k_density_post(const ChanJob* __restrict__ jobs, const MolState* __restrict__ st, int nblk, const int* __restrict__ mask,
+                               int want) {
     const ChanJob jb = jobs[blockIdx.y];
-    if (!st[jb.mol].active) return;
+    if (!st[jb.mol].active || (mask && (mask[jb.mol] != 0) != (want != 0))) return;
     const int nb = dens_blocks(jb.n);
     if ((int)blockIdx.x >= nb) return;
     const long long nn = (long long)jb.n * jb.n;
@@ -711,11 +712,11 @@ __global__ void k_density_post(const ChanJob* __restrict__ jobs, const MolState*
 __global__ void __launch_bounds__(32 * SCF_MOL_WARPS) k_converge(const MolDesc* __restrict__ mols, const ChanJob* __restrict__ jobs,
                                                                  const int* __restrict__ mol_job0, int nmol, MolState* __restrict__ st,
                                                                  int* __restrict__ mol_status, int nblk, ScfParams prm,
-                                                                 int* __restrict__ active_count) {
+                                                                 int* __restrict__ active_count, const int* __restrict__ mask, int want) {
     const int lane = threadIdx.x & 31, mi = blockIdx.x * SCF_MOL_WARPS + (threadIdx.x >> 5);
     if (mi >= nmol) return;
     MolState& s = st[mi];
-    if (!s.active) return;
+    if (!s.active || (mask && (mask[mi] != 0) != (want != 0))) return;
     if (mol_status[mi] != 0) {  // the eigensolver refused its input
         __syncwarp();
         if (lane == 0) {

@@ -710,7 +710,7 @@ __global__ void k_sp2_finish(const Sp2Job* __restrict__ jobs, const Sp2State* __
         if (blockIdx.x == 0 && threadIdx.x == 0) {
             atomicAdd(&work[2], 1.0);
             if (jb.fallback) {
-                need_eigen[jb.mol] = 1;
+                need_eigen[jb.mol] = need_eigen[-1] = 1;
             } else {  // above the cluster Jacobi's size: the host runs the large-matrix eigensolver
                 big_stall[blockIdx.y] = 1;
                 atomicAdd(big_count, 1);

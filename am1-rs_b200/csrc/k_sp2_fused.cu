@@ -619,7 +619,7 @@ __device__ __forceinline__ void sp2_fused_body(const Sp2Job* __restrict__ jobs, 
         atomicAdd(&work[3], (double)steps * 16.0 * nd * nd);
         if (!converged) {
             atomicAdd(&work[2], 1.0);
-            need_eigen[jb.mol] = 1;
+            need_eigen[jb.mol] = need_eigen[-1] = 1;
         }
         Sp2State& s = sst[job];
         s.active = 0;

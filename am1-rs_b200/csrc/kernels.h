@@ -141,14 +141,13 @@ struct GraphLoop {
     int scf_iter;   // SCF iterations done in this launch
     int sp2_step;   // purification steps of the current iteration
     int sp2_total;  // purification steps of this launch
-    int eig_runs;   // iterations of this launch in which the stalled-purification eigensolver ran
+    int stalled;    // the loop ended because some purification stalled (the host takes over)
     int sp2_active; // channels still purifying, counted by the CTAs of the step's update
     int ticket;     // CTAs of the step's update that are done
 };
 __global__ void k_scf_arm(cudaGraphConditionalHandle h, GraphLoop* loop, int max_scf);
 __global__ void k_sp2_arm(cudaGraphConditionalHandle h, GraphLoop* loop);
-__global__ void k_stall_arm(cudaGraphConditionalHandle h, GraphLoop* loop, const int* need_eigen, int nmol);
-__global__ void k_scf_cond(cudaGraphConditionalHandle h, GraphLoop* loop, const int* active, int max_scf);
+__global__ void k_scf_cond(cudaGraphConditionalHandle h, GraphLoop* loop, const int* active, const int* need_eigen, int max_scf);
 
 struct ScfParams {
     int max_scf, use_diis, accelerator;
@@ -182,7 +181,9 @@ __global__ void k_fock(const MolDesc* mols, const int* atom_mol, int natoms_tota
 // grid (n, count), 128 threads: a CTA per row
 __global__ void k_permute_square(const double* in, long long si, double* out, long long so, const int* map, int n);
 // C = alpha A B (A row-major M x K) and C = alpha A^T B (A stored K x M)
-// mask (optional): only molecules with mask[mol] != 0 take part
+// mask (optional): only molecules with mask[mol] != 0 take part, and nothing at all when mask[-1] == 0 (so the
+// array of stalled purifications, need_eigen, starts with a word that says whether there is any); a CTA per tile,
+// or fewer that stride over them
 __global__ void k_gemm_nn(const GemmJob* jobs, const GemmTile* tiles, int ntiles, const MolState* st, int force, const int* mask);
 __global__ void k_gemm_tn(const GemmJob* jobs, const GemmTile* tiles, int ntiles, const MolState* st, int force, const int* mask);
 __global__ void k_jacobi(const EigJob* jobs, const MolState* st, int* mol_status, int force, const int* mask);
@@ -404,9 +405,10 @@ constexpr int RESULT_THREADS = 128;
 __global__ void k_diis_solve(const MolDesc* mols, const ChanJob* jobs, const int* mol_job0, int nmol, MolState* st,
                              int* mol_status, int nblk, ScfParams prm);
 __global__ void k_combine(const ChanJob* jobs, const MolState* st, int force);
-__global__ void k_density_post(const ChanJob* jobs, const MolState* st, int nblk);
+// mask (optional): only molecules with (mask[mol] != 0) == want
+__global__ void k_density_post(const ChanJob* jobs, const MolState* st, int nblk, const int* mask, int want);
 __global__ void k_converge(const MolDesc* mols, const ChanJob* jobs, const int* mol_job0, int nmol, MolState* st,
-                           int* mol_status, int nblk, ScfParams prm, int* active_count);
+                           int* mol_status, int nblk, ScfParams prm, int* active_count, const int* mask, int want);
 __global__ void k_final_energy(const MolDesc* mols, const ChanJob* jobs, const int* mol_job0, int nmol, MolState* st,
                                int nblk);
 // Per-molecule result record (doubles), see RES_* below; charges in internal atom order.
