@@ -298,6 +298,9 @@ struct Mem {
     cudaStream_t cap_stream = nullptr;  // stream the SCF graph is captured on, and the one-launch purifications' own in the host-driven loop
     cudaEvent_t fork = nullptr, join = nullptr;  // order the two streams in the host-driven loop
     std::vector<cudaStream_t> pipes;  // streams of the transfer pipelines (g_matrix_batch)
+    cudaGraphExec_t graph_exec = nullptr;  // the captured SCF loop of the last layout (scf_loop_graph), and what it was captured for
+    std::vector<uint64_t> graph_key;
+    int64_t graph_counts[3] = {0, 0, 0};  // its Batch::graph_counts
 };
 
 // Stream priority asked for by the calling host thread (am1gpu_set_stream_priority).
@@ -334,6 +337,7 @@ void mem_release(Mem& w) {
     if (w.hpin) cudaFreeHost(w.hpin);
     for (auto e : w.events) cudaEventDestroy(e);
     if (w.stream) cudaStreamDestroy(w.stream);
+    if (w.graph_exec) cudaGraphExecDestroy(w.graph_exec);
     if (w.cap_stream) cudaStreamDestroy(w.cap_stream);
     for (auto q : w.pipes) cudaStreamDestroy(q);
     if (w.fork) cudaEventDestroy(w.fork);
@@ -744,12 +748,6 @@ int plan_molecule(const am1gpu_molecule& m, const am1gpu_options& o, int user, M
 }
 
 struct Batch {
-    Batch() = default;
-    Batch(const Batch&) = delete;
-    Batch& operator=(const Batch&) = delete;
-    ~Batch() {
-        if (graph_exec) cudaGraphExecDestroy(graph_exec);  // one still running is freed once it completes
-    }
     int nmol = 0, natoms = 0, nblk = 1, maxn = 0, maxheavy = 0;
     long long npairs = 0;
     std::vector<MolPlan> plans;
@@ -835,7 +833,6 @@ struct Batch {
     char *d_extra = nullptr, *h_extra = nullptr;  // the caller's own regions (build_batch's extra_dev, extra_host)
     // kernels per captured head (+ arm), step and tail (+ condition)
     int64_t graph_counts[3] = {0, 0, 0};
-    cudaGraphExec_t graph_exec = nullptr;  // the captured loop; a resident batch keeps it across runs
 };
 
 // Lays out the batch in one device pool and one pinned staging area, copies inputs.
@@ -1924,6 +1921,38 @@ int add_while(cudaGraph_t g, cudaGraphNode_t dep, cudaGraphConditionalHandle h, 
     return AM1GPU_OK;
 }
 
+// Everything the captured kernels are given: pointers into the workspace's own pool, counts, launch shapes and
+// options; the library's switches (constant in a process) are left out.  What the molecules are (elements,
+// coordinates, tiles) lies behind those pointers and is written anew by each call.  Two solves with equal lists
+// are the same graph, so a thread that solves molecules of one layout one after the other (a geometry
+// optimisation, molecular dynamics, a resident batch) captures once: a solve of methane 1.14 -> 0.89 ms, of 32 waters
+// 3.85 -> 3.59 ms.  One graph per workspace, the last layout's.
+std::vector<uint64_t> graph_args(const IterEnq& e, const am1gpu_options& o) {
+    const Batch& b = e.b;
+    std::vector<uint64_t> k;
+    for (const void* p : {(const void*)b.d_mols, (const void*)b.d_atom_mol, (const void*)e.dp, (const void*)b.d_atom_z,
+                          (const void*)b.d_wstore, (const void*)b.d_arena, (const void*)b.d_st, (const void*)b.d_jobs,
+                          (const void*)b.d_sp2_tiles, (const void*)b.d_oz_tiles, (const void*)b.d_sp2_maps, (const void*)b.d_sp2_active,
+                          (const void*)b.d_job0, (const void*)b.d_status, (const void*)b.d_need_eigen, (const void*)b.d_sp2,
+                          (const void*)b.d_sp2_state, (const void*)b.d_fused, (const void*)b.d_work, (const void*)b.d_big_stall,
+                          (const void*)b.d_active, (const void*)b.d_loop, (const void*)e.ws->cap_stream})
+        k.push_back((uint64_t)(uintptr_t)p);
+    for (long long v : {(long long)b.nmol, (long long)b.natoms, (long long)b.maxn, (long long)b.maxheavy, (long long)e.nblk,
+                        (long long)e.rowblk, (long long)e.njobs, (long long)b.sp2_nblk, (long long)b.nt_sp2, (long long)b.nt_sp2_pairs,
+                        (long long)b.nt_step_pairs, (long long)b.nt_step_other, (long long)b.nt_oz, (long long)b.sp2_tma,
+                        (long long)b.unfused, (long long)o.max_scf, (long long)sp2_max_steps(), (long long)e.prm.max_scf,
+                        (long long)e.prm.use_diis, (long long)e.prm.accelerator, (long long)e.prm.lowp_max_iter})
+        k.push_back((uint64_t)v);
+    for (double v : {e.prm.e_tol, e.prm.p_tol, e.prm.adiis_switch, e.prm.lowp_switch}) {
+        uint64_t u;
+        std::memcpy(&u, &v, sizeof u);
+        k.push_back(u);
+    }
+    for (const auto& g : b.fused_groups)
+        for (long long v : {(long long)g.off, (long long)g.count, (long long)g.C, (long long)g.smem}) k.push_back((uint64_t)v);
+    return k;
+}
+
 // The SCF loop of run_device as one graph launch:
 //   k_scf_arm -> WHILE(scf) { head -> [one-launch purifications | start -> k_sp2_arm -> WHILE(sp2) { step }]
 //                             -> tail -> k_scf_cond }
@@ -1943,12 +1972,17 @@ int scf_loop_graph(IterEnq& e, const am1gpu_options& o, bool* launched) {
     const int sp2_max = sp2_max_steps();
     if (int rc0 = mem_side_stream(m)) return rc0;
     const cudaStream_t cs = m.cap_stream;
-    if (b.graph_exec) {  // captured on the batch's first run
+    std::vector<uint64_t> key = graph_args(e, o);
+    if (m.graph_exec && m.graph_key == key) {
         *launched = true;
-        CK(cudaGraphLaunch(b.graph_exec, e.s));
+        CK(cudaGraphLaunch(m.graph_exec, e.s));
         CK(cudaMemcpyAsync(b.h_loop, b.d_loop, sizeof(GraphLoop), cudaMemcpyDeviceToHost, e.s));
+        for (int k = 0; k < 3; ++k) b.graph_counts[k] = m.graph_counts[k];
         return AM1GPU_OK;
     }
+    if (m.graph_exec) cudaGraphExecDestroy(m.graph_exec);  // nothing of it runs between calls
+    m.graph_exec = nullptr;
+    m.graph_key.clear();
     am1gpu_call_stats cnt{};  // launches per captured sequence
     Run crun{e.ws, &cnt, false};
     IterEnq ce = e;
@@ -2014,13 +2048,14 @@ int scf_loop_graph(IterEnq& e, const am1gpu_options& o, bool* launched) {
     const int64_t per_tail = cnt.kernel_launches - tail0 + 1;
     cudaGraphExec_t ge = nullptr;
     CK(cudaGraphInstantiate(&ge, g, 0));
-    b.graph_exec = ge;
+    m.graph_exec = ge;
     *launched = true;
     CK(cudaGraphLaunch(ge, e.s));
     CK(cudaMemcpyAsync(b.h_loop, b.d_loop, sizeof(GraphLoop), cudaMemcpyDeviceToHost, e.s));
-    b.graph_counts[0] = per_head;
-    b.graph_counts[1] = per_step;
-    b.graph_counts[2] = per_tail;
+    m.graph_counts[0] = b.graph_counts[0] = per_head;
+    m.graph_counts[1] = b.graph_counts[1] = per_step;
+    m.graph_counts[2] = b.graph_counts[2] = per_tail;
+    m.graph_key = std::move(key);  // last: a graph without its key is captured anew
     return AM1GPU_OK;
 }
 
@@ -3588,11 +3623,7 @@ int am1gpu_batch_results(am1gpu_batch* h, am1gpu_result* results, int32_t* statu
 
 void am1gpu_batch_destroy(am1gpu_batch* h) {
     if (!h) return;
-    if (h->b.graph_exec) {
-        cudaStreamSynchronize(h->mem.stream);
-        cudaGraphExecDestroy(h->b.graph_exec);
-        h->b.graph_exec = nullptr;
-    }
+    if (h->mem.stream) cudaStreamSynchronize(h->mem.stream);
     am1::mem_release(h->mem);
     delete h;
 }
@@ -3612,6 +3643,9 @@ int am1gpu_set_stream_priority(int32_t priority) {
         w.stream = nullptr;
         CK(cudaStreamCreateWithPriority(&w.stream, cudaStreamNonBlocking, p));
         w.priority = p;
+        if (w.graph_exec) CK(cudaGraphExecDestroy(w.graph_exec));  // its kernels carry the old priority
+        w.graph_exec = nullptr;
+        w.graph_key.clear();
         if (w.cap_stream) {
             CK(cudaStreamSynchronize(w.cap_stream));
             CK(cudaStreamDestroy(w.cap_stream));
