@@ -822,6 +822,7 @@ struct Batch {
     double* h_charges;
     double* d_eps;  // every channel's orbital energies, contiguous (job order)
     double* h_eps;  // their pinned host copy
+    double* d_hist;  // the packed DIIS histories
     double* d_grad;  // nuclear gradient, 3 per atom (internal atom order), when asked for
     double* h_grad;
     long long eps_total = 0;
@@ -1019,6 +1020,7 @@ int build_batch(const am1gpu_molecule* in, const am1gpu_options& o, std::vector<
     b.d_ecc = (double*)dptr(o_ecc);
     b.d_arena = (double*)dptr(o_arena);
     double* d_hist = (double*)dptr(o_hist);
+    b.d_hist = d_hist;  // at least 8 n^2 doubles per molecule: 3 per atom pair fit several times
     double* d_misc = (double*)dptr(o_misc);
     int* d_colid = (int*)dptr(o_colid);
     b.d_res = (double*)dptr(o_res);
@@ -2205,8 +2207,18 @@ int run_device(Batch& b, Mem& mem, const DevElem* dp, const am1gpu_options& o, a
 int run_gradient(Batch& b, Mem& mem, const DevElem* dp, am1gpu_call_stats* stats) {
     cudaStream_t s = mem.stream;
     if (b.natoms > 0) {
-        k_gradient<<<cdiv(b.natoms, 8), 256, 0, s>>>(b.d_mols, b.d_atom_mol, b.natoms, dp, b.d_atom_z, b.d_atom_xyz, b.d_jobs, b.d_job0,
-                                                     b.d_grad, b.d_status);
+        if (b.npairs > 0) {  // the pairs' forces in the DIIS history's room, which the solve no longer needs
+            if (b.npairs <= GRAD_SPLIT_PAIRS * g_sms)
+                k_pair_gradient_split<<<cdiv(b.npairs, 32), 128, 0, s>>>(b.d_mols, b.nmol, b.d_pair_prefix, b.npairs, dp, b.d_atom_z,
+                                                                         b.d_atom_xyz, b.d_jobs, b.d_job0, b.d_hist, b.d_status);
+            else
+                k_pair_gradient<<<cdiv(b.npairs, GRAD_THREADS), GRAD_THREADS, 0, s>>>(b.d_mols, b.nmol, b.d_pair_prefix, b.npairs, dp,
+                                                                                      b.d_atom_z, b.d_atom_xyz, b.d_jobs, b.d_job0,
+                                                                                      b.d_hist, b.d_status);
+            CK(cudaGetLastError());
+            stats->kernel_launches += 1;
+        }
+        k_gradient<<<cdiv(b.natoms, 8), 256, 0, s>>>(b.d_mols, b.d_atom_mol, b.natoms, b.d_hist, b.d_grad);
         CK(cudaGetLastError());
         stats->kernel_launches += 1;
     }

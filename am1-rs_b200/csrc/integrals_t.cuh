@@ -1,7 +1,8 @@
 // The two-centre formulas of the NDDO model as templates over the scalar type: double for the
-// integrals, overlap and core-core energy the SCF uses (k_integrals.cu), D3 (dual3.cuh) for their
-// exact derivatives with respect to the pair displacement (k_gradient.cu).  Both instantiations
-// run the same expressions in the same order; the double one is what the SCF has always used.
+// integrals, overlap and core-core energy the SCF uses (k_integrals.cu), dual numbers (dual3.cuh) for
+// their exact derivatives with respect to the pair displacement (k_gradient.cu): T the type of what depends on
+// the direction (D3), R of what depends on the distance alone (D1), u the unit displacement (unused
+// for double).  Both instantiations run the same expressions in the same order.
 //
 // Formulas follow am1-rs:
 //   local integrals        src/integrals.rs:309-484 (Dewar-Sabelli-Klopman multipoles)
@@ -21,17 +22,9 @@
 namespace am1 {
 
 template <class T>
-__device__ __forceinline__ T zero();
-template <>
-__device__ __forceinline__ double zero<double>() { return 0.0; }
-template <>
-__device__ __forceinline__ D3 zero<D3>() { return d3c(0.0); }
+__device__ __forceinline__ T zero() { return T{0.0}; }
 template <class T>
-__device__ __forceinline__ T one();
-template <>
-__device__ __forceinline__ double one<double>() { return 1.0; }
-template <>
-__device__ __forceinline__ D3 one<D3>() { return d3c(1.0); }
+__device__ __forceinline__ T one() { return T{1.0}; }
 
 template <class T>
 __device__ __forceinline__ T rinv(const T& x) { return 1.0 / sqrt(x); }
@@ -89,7 +82,7 @@ __device__ void bint7(const T& x, T b[7]) {
 // Overlap of two Slater orbitals in the local diatomic frame (b at +z, distance r),
 // <n_a l_a m; z_a | n_b l_b m; z_b> with m = 0 (sigma) or 1 (pi), by Gauss-Legendre quadrature in
 // prolate-spheroidal coordinates: xi in [1, xi_max] (48 nodes), eta in [-1, 1] (40 nodes).  The
-// domain and the angular factors depend on r's value only; the radial factor carries r, so a D3
+// domain and the angular factors depend on r's value only; the radial factor carries r, so a D1
 // r gives the exact derivative of this quadrature (the boundary term at xi_max is negligible:
 // the integrand has decayed by e^-60 there).
 template <class T>
@@ -228,11 +221,14 @@ __device__ bool overlap_local(const DevElem& ea, const DevElem& eb, const T& r, 
 }
 
 // Global-frame 4x4 overlap S[i-orbital][j-orbital]; dir = unit vector i -> j.
-template <class T>
-__device__ bool overlap_block(const DevElem& ei, const DevElem& ej, const T& r, const T dir[3], T S[4][4]) {
-    T s[5];
+template <class T, class R>
+__device__ bool overlap_block(const DevElem& ei, const DevElem& ej, const R& r, const T dir[3], const double* u, T S[4][4]) {
+    R sr[5];
     const bool swap = ei.n < ej.n;
-    if (!overlap_local(swap ? ej : ei, swap ? ei : ej, r, s)) return false;
+    if (!overlap_local(swap ? ej : ei, swap ? ei : ej, r, sr)) return false;
+    T s[5];
+#pragma unroll
+    for (int k = 0; k < 5; ++k) s[k] = lift(sr[k], u);
     const double sg = swap ? -1.0 : 1.0;
     const T d[3] = {dir[0] * sg, dir[1] * sg, dir[2] * sg};
     T di[4][4];
@@ -339,14 +335,19 @@ __device__ void local_xx(const DevElem& ei, const DevElem& ej, const T& r, T ri[
 
 // Integrals of one pair (i = heavy or lower index, j), each handed to sink(kk, ll, mm, nn, value)
 // as it is formed: (kk ll | mm nn) with kk >= ll the orbitals on i and mm >= nn those on j
-// (0 = s, 1-3 = p), in the store's order (row pack(kk, ll), column pack(mm, nn)).
-template <class T, class Sink>
-__device__ void pair_integrals_each(const DevElem& ei, const DevElem& ej, const T dv[3], const T& r, Sink&& sink) {
-    const T inv = 1.0 / r;
+// (0 = s, 1-3 = p), in the store's order (row pack(kk, ll), column pack(mm, nn)).  rows(row): whether the row
+// of a heavy-heavy pair is wanted.
+struct AllRows {
+    __device__ constexpr bool operator()(int) const { return true; }
+};
+template <class T, class R, class Rows, class Sink>
+__device__ void pair_integrals_each(const DevElem& ei, const DevElem& ej, const T dv[3], const R& r, const double* u, Rows rows,
+                                    Sink&& sink) {
+    const T inv = lift(1.0 / r, u);
     const T n[3] = {-(dv[0] * inv), -(dv[1] * inv), -(dv[2] * inv)};  // frame axis, = -x_ij
     const bool hi = ei.norb == 4, hj = ej.norb == 4;
     if (!hi && !hj) {
-        sink(0, 0, 0, 0, rinv(r * r + (ei.rho0 + ej.rho0) * (ei.rho0 + ej.rho0)) * AM1_EV);
+        sink(0, 0, 0, 0, lift(rinv(r * r + (ei.rho0 + ej.rho0) * (ei.rho0 + ej.rho0)) * AM1_EV, u));
         return;
     }
     // p = I - n n^T
@@ -361,25 +362,28 @@ __device__ void pair_integrals_each(const DevElem& ei, const DevElem& ej, const 
         const double aee = (ei.rho0 + ej.rho0) * (ei.rho0 + ej.rho0);
         const double ade = (ei.rho1 + ej.rho0) * (ei.rho1 + ej.rho0);
         const double aqe = (ei.rho2 + ej.rho0) * (ei.rho2 + ej.rho0);
-        const T ee = rinv(r * r + aee) * AM1_EV;
-        const T q6 = rinv(r * r + aqe) * ev1;
-        const T r1 = rinv((r + da) * (r + da) + ade) * ev1 - rinv((r - da) * (r - da) + ade) * ev1;
-        const T r2 = ee + rinv((r + qa) * (r + qa) + aqe) * ev2 + rinv((r - qa) * (r - qa) + aqe) * ev2 - q6;
-        const T r3 = ee + rinv(r * r + qa * qa + aqe) * ev1 - q6;
-        sink(0, 0, 0, 0, ee);
+        const R ee = rinv(r * r + aee) * AM1_EV;
+        const R q6 = rinv(r * r + aqe) * ev1;
+        const R r1 = rinv((r + da) * (r + da) + ade) * ev1 - rinv((r - da) * (r - da) + ade) * ev1;
+        const R r2 = ee + rinv((r + qa) * (r + qa) + aqe) * ev2 + rinv((r - qa) * (r - qa) + aqe) * ev2 - q6;
+        const R r3 = ee + rinv(r * r + qa * qa + aqe) * ev1 - q6;
+        const T t1 = lift(r1, u), t2 = lift(r2, u), t3 = lift(r3, u);
+        sink(0, 0, 0, 0, lift(ee, u));
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
-            sink(k + 1, 0, 0, 0, r1 * n[k]);
+            sink(k + 1, 0, 0, 0, t1 * n[k]);
 #pragma unroll
-            for (int l = 0; l <= k; ++l) sink(k + 1, l + 1, 0, 0, r2 * (n[k] * n[l]) + r3 * p[k][l]);
+            for (int l = 0; l <= k; ++l) sink(k + 1, l + 1, 0, 0, t2 * (n[k] * n[l]) + t3 * p[k][l]);
         }
         return;
     }
-    T ri[22];
-    local_xx(ei, ej, r, ri);
+    R rr[22];
+    local_xx(ei, ej, r, rr);
+    const auto ri = [&](int k) { return lift(rr[k], u); };
 #pragma unroll 1
     for (int kk = 0; kk < 4; ++kk)
-        for (int ll = 0; ll <= kk; ++ll)
+        for (int ll = 0; ll <= kk; ++ll) {
+            if (!rows(kk * (kk + 1) / 2 + ll)) continue;
 #pragma unroll
             for (int mm = 0; mm < 4; ++mm)
 #pragma unroll
@@ -387,31 +391,32 @@ __device__ void pair_integrals_each(const DevElem& ei, const DevElem& ej, const 
                     const int k = kk - 1, l = ll - 1, m = mm - 1, q = nn - 1;
                     T v;
                     if (kk == 0) {
-                        if (mm == 0) v = ri[0];
-                        else if (nn == 0) v = ri[4] * n[m];
-                        else v = ri[10] * (n[m] * n[q]) + ri[11] * p[m][q];
+                        if (mm == 0) v = ri(0);
+                        else if (nn == 0) v = ri(4) * n[m];
+                        else v = ri(10) * (n[m] * n[q]) + ri(11) * p[m][q];
                     } else if (ll == 0) {
-                        if (mm == 0) v = ri[1] * n[k];
-                        else if (nn == 0) v = ri[5] * (n[k] * n[m]) + ri[6] * p[k][m];
-                        else v = ri[12] * (n[k] * n[m] * n[q]) + ri[13] * (p[m][q] * n[k]) + ri[14] * (p[k][q] * n[m] + p[k][m] * n[q]);
+                        if (mm == 0) v = ri(1) * n[k];
+                        else if (nn == 0) v = ri(5) * (n[k] * n[m]) + ri(6) * p[k][m];
+                        else v = ri(12) * (n[k] * n[m] * n[q]) + ri(13) * (p[m][q] * n[k]) + ri(14) * (p[k][q] * n[m] + p[k][m] * n[q]);
                     } else if (mm == 0) {
-                        v = ri[2] * (n[k] * n[l]) + ri[3] * p[k][l];
+                        v = ri(2) * (n[k] * n[l]) + ri(3) * p[k][l];
                     } else if (nn == 0) {
-                        v = ri[7] * (n[k] * n[l] * n[m]) + ri[8] * (p[k][l] * n[m]) + ri[9] * (p[l][m] * n[k] + p[k][m] * n[l]);
+                        v = ri(7) * (n[k] * n[l] * n[m]) + ri(8) * (p[k][l] * n[m]) + ri(9) * (p[l][m] * n[k] + p[k][m] * n[l]);
                     } else {
-                        v = ri[15] * (n[k] * n[l] * n[m] * n[q]) + ri[16] * (p[k][l] * n[m] * n[q]) + ri[17] * (p[m][q] * n[k] * n[l]) +
-                            ri[19] * (n[k] * (p[l][q] * n[m] + p[l][m] * n[q]) + n[l] * (p[k][q] * n[m] + p[k][m] * n[q])) +
-                            ri[20] * (p[k][l] * p[m][q]) + ri[21] * (p[k][m] * p[l][q] + p[k][q] * p[l][m]);
+                        v = ri(15) * (n[k] * n[l] * n[m] * n[q]) + ri(16) * (p[k][l] * n[m] * n[q]) + ri(17) * (p[m][q] * n[k] * n[l]) +
+                            ri(19) * (n[k] * (p[l][q] * n[m] + p[l][m] * n[q]) + n[l] * (p[k][q] * n[m] + p[k][m] * n[q])) +
+                            ri(20) * (p[k][l] * p[m][q]) + ri(21) * (p[k][m] * p[l][q] + p[k][q] * p[l][m]);
                     }
                     sink(kk, ll, mm, nn, v);
                 }
+        }
 }
 
 // pair_integrals_each written to the store: XX 10 x 10 row-major, XH 10, HH 1.
 template <class T>
 __device__ void pair_integrals(const DevElem& ei, const DevElem& ej, const T dv[3], const T& r, T* __restrict__ w) {
     const int nwb = ej.norb == 4 ? 10 : 1;
-    pair_integrals_each(ei, ej, dv, r, [&](int kk, int ll, int mm, int nn, const T& v) {
+    pair_integrals_each(ei, ej, dv, r, nullptr, AllRows(), [&](int kk, int ll, int mm, int nn, const T& v) {
         w[(kk * (kk + 1) / 2 + ll) * nwb + mm * (mm + 1) / 2 + nn] = v;
     });
 }

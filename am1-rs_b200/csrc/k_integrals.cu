@@ -16,28 +16,6 @@
 
 namespace am1 {
 
-// Locate the molecule and the (i, j) pair of a flat pair index.
-__device__ __forceinline__ int find_mol(const long long* __restrict__ prefix, int nmol, long long g) {
-    int lo = 0, hi = nmol - 1;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (prefix[mid] <= g) lo = mid;
-        else hi = mid - 1;
-    }
-    return lo;
-}
-
-__device__ __forceinline__ void pair_ij(long long p, int n, int& i, int& j) {
-    // rows i hold n-1-i pairs; S(i) = i*n - i(i+1)/2 pairs precede row i
-    const double nn = n - 0.5;
-    int ii = (int)floor(nn - sqrt(fmax(nn * nn - 2.0 * (double)p, 0.0)));
-    ii = max(0, min(ii, n - 2));
-    while (ii > 0 && (long long)ii * n - (long long)ii * (ii + 1) / 2 > p) --ii;
-    while ((long long)(ii + 1) * n - (long long)(ii + 1) * (ii + 2) / 2 <= p) ++ii;
-    i = ii;
-    j = (int)(p - ((long long)ii * n - (long long)ii * (ii + 1) / 2)) + ii + 1;
-}
-
 __global__ void k_pair_integrals(const MolDesc* __restrict__ mols, int nmol, const long long* __restrict__ pair_prefix,
                                  long long npairs, const DevElem* __restrict__ params, const int* __restrict__ atom_z,
                                  const double* __restrict__ atom_xyz, double* __restrict__ wstore, double* __restrict__ hmat,
@@ -84,7 +62,7 @@ __global__ void k_pair_integrals(const MolDesc* __restrict__ mols, int nmol, con
             for (int b = 0; b < 4; ++b) S[a][b] = a == b ? 1.0 : 0.0;
     } else {
         const double dir[3] = {e0 / rs, e1 / rs, e2 / rs};
-        if (!overlap_block(ei, ej, rs, dir, S)) {
+        if (!overlap_block(ei, ej, rs, dir, nullptr, S)) {
             atomicExch(&mol_status[m], 6);  // AM1GPU_UNSUPPORTED
             return;
         }

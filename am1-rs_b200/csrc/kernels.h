@@ -165,10 +165,21 @@ constexpr int CORE_DIAG_LANES = 16;  // lanes per atom of k_core_diag
 __global__ void k_core_diag(const MolDesc* mols, const int* atom_mol, int natoms_total, const DevElem* params,
                             const int* atom_z, const double* wstore, double* hmat);
 __global__ void k_core_energy(const MolDesc* mols, const double* ecc, MolState* st);
-// nuclear gradient at the current densities (jobs[].P), a warp per atom (8 per block); gradient:
-// 3 doubles per atom, internal atom order
-__global__ void k_gradient(const MolDesc* mols, const int* atom_mol, int natoms_total, const DevElem* params, const int* atom_z,
-                           const double* atom_xyz, const ChanJob* jobs, const int* mol_job0, double* gradient, int* mol_status);
+// nuclear gradient at the current densities (jobs[].P): every pair's force (a thread per pair, GRAD_THREADS per
+// CTA) to pairf (3 doubles per pair, pair-index order), then their sums per atom (a warp each, 8 per CTA) to
+// gradient: 3 doubles per atom, internal atom order
+constexpr int GRAD_THREADS = 64;
+// pairs per SM up to which four warps share 32 pairs: what an SM holds of that kernel at a time (two CTAs), 120 us;
+// a thread per pair takes 208 us for up to four times as many
+constexpr long long GRAD_SPLIT_PAIRS = 64;
+__global__ void k_pair_gradient(const MolDesc* mols, int nmol, const long long* pair_prefix, long long npairs, const DevElem* params,
+                                const int* atom_z, const double* atom_xyz, const ChanJob* jobs, const int* mol_job0, double* pairf,
+                                int* mol_status);
+// the same by 32 pairs per CTA of 128 threads, for few pairs
+__global__ void k_pair_gradient_split(const MolDesc* mols, int nmol, const long long* pair_prefix, long long npairs,
+                                      const DevElem* params, const int* atom_z, const double* atom_xyz, const ChanJob* jobs,
+                                      const int* mol_job0, double* pairf, int* mol_status);
+__global__ void k_gradient(const MolDesc* mols, const int* atom_mol, int natoms_total, const double* pairf, double* gradient);
 // grid fock_grid(...), 32 FOCK_WARPS threads
 constexpr int FOCK_WARPS = 4, FOCK_XX_CHUNK = 16, FOCK_SPLIT_ATOMS = 32768;
 inline dim3 fock_grid(long long natoms, int most_heavy) {  // atoms of the launch, most heavy atoms of a molecule
@@ -370,6 +381,28 @@ __global__ void k_dgemm8(const double* A, int lda, long long sA, const double* B
                          long long sC, int M, int N, int K, int sub);
 
 #ifdef __CUDACC__
+// Locate the molecule and the (i, j) pair of a flat pair index.
+__device__ __forceinline__ int find_mol(const long long* __restrict__ prefix, int nmol, long long g) {
+    int lo = 0, hi = nmol - 1;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (prefix[mid] <= g) lo = mid;
+        else hi = mid - 1;
+    }
+    return lo;
+}
+
+__device__ __forceinline__ void pair_ij(long long p, int n, int& i, int& j) {
+    // rows i hold n-1-i pairs; S(i) = i*n - i(i+1)/2 pairs precede row i
+    const double nn = n - 0.5;
+    int ii = (int)floor(nn - sqrt(fmax(nn * nn - 2.0 * (double)p, 0.0)));
+    ii = max(0, min(ii, n - 2));
+    while (ii > 0 && (long long)ii * n - (long long)ii * (ii + 1) / 2 > p) --ii;
+    while ((long long)(ii + 1) * n - (long long)(ii + 1) * (ii + 2) / 2 <= p) ++ii;
+    i = ii;
+    j = (int)(p - ((long long)ii * n - (long long)ii * (ii + 1) / 2)) + ii + 1;
+}
+
 // FP32 -> nearest TF32 value (ties away from zero), kept in an FP32 register
 __device__ __forceinline__ float tf32_round(float x) {
     unsigned u;
