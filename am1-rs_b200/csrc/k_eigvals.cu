@@ -21,14 +21,19 @@ namespace cg = cooperative_groups;
 // share fits one CTA.  Reflector s (GVL Alg. 8.3.1) zeroes row/column s below the subdiagonal:
 // v_s = x + sign(x0)|x| e1 from x = A[s, s+1:], beta_s = 1/(|x|(|x| + |x0|)), and the trailing
 // block takes the rank-2 update A -= v w^T + w v^T with p = beta A v, w = p - (beta/2)(p.v) v.
-// Iteration s of the loop:
-//   (a) one warp of the owner of row s applies update s-1 to row s and derives reflector s
-//   cluster barrier: v_s ready; the other CTAs copy it (distributed shared memory)
-//   (b) one fused pass over the CTA's rows > s, a thread per column > s: apply update s-1 and
-//       accumulate this CTA's share of A v_s (A symmetric: column r of the share is a dot product
+// Iteration s of the loop (update s-1 is on row s, reflector s is in row s's owner):
+//   cluster barrier; the other CTAs copy v_s (distributed shared memory)
+//   (b) one fused pass over the CTA's rows > s, a thread per pair of columns and group of rows: apply update
+//       s-1 and accumulate this CTA's share of A v_s (A symmetric: column r of the share is a dot product
 //       down the rows, so consecutive threads read consecutive words)
-//   cluster barrier: every CTA's share ready; each CTA sums the C shares itself -> p, w_s
-// Column s below the diagonal is never updated: row s holds the same numbers and is the one read.
+//   cluster barrier: every CTA's share ready; each CTA sums the C shares itself -> p, w_s, a thread per column
+//   (a) the owner of row s+1 applies update s to it, the same threads on the same columns, and derives
+//       reflector s+1
+// Bound by shared memory traffic in (b) and by the latency of the four reductions and barriers elsewhere: with two
+// columns to a thread and (v, w) in one word a row of 64 columns takes 10 wavefronts, against 14 with a column
+// and three vectors; (a) by all threads follows (p.v) without a barrier of its own (a warp took 1440 cycles).
+// One 192-row matrix (two CTAs, then one from 166 rows on) 768 -> 651 us, 192 molecules of 79 atoms 3.83 -> 3.29 ms.
+// Column s below the diagonal is never read again: row s holds the same numbers and is the one read.
 // All control flow is uniform over the cluster, so every CTA takes the same barriers.
 // With job.stop > 0 the loop ends after reflector stop - 1: the trailing block (rows and columns
 // >= stop) with update stop - 1 applied goes to job.W (row-major, n - stop rows), and a job on fewer
@@ -37,34 +42,23 @@ namespace cg = cooperative_groups;
 constexpr int TRI_THREADS = 512;
 constexpr int TRI_WARPS = TRI_THREADS / 32;
 
-// Dynamic shared memory of one CTA: local rows, v and w (two buffers each), the share of A v,
-// beta (two buffers) and two reduction scratches.
+// Dynamic shared memory of one CTA: local rows (even length), (v, w) (two buffers), the share of A v, 1 / beta (two
+// buffers), beta and p of the next reflector's first column, two reduction scratches and the row groups' column sums.
 size_t tridiag_smem_bytes(int n, int C) {
-    const size_t rows = (size_t)(n + C - 1) / C;
-    return sizeof(double) * (rows * n + 5 * (size_t)n + 2 + TRI_WARPS + TRI_THREADS);
+    const size_t rows = (size_t)(n + C - 1) / C, ld = (size_t)n + (n & 1);
+    return sizeof(double) * (rows * ld + 5 * ld + 4 + 2 * TRI_WARPS + TRI_THREADS);
 }
 
-// Householder vector of row `row` (the trailing part from column s + 1), computed by one warp:
-// v into vbuf, beta into *beta, and d[s], e[s].
-__device__ __forceinline__ void tri_reflector(const double* row, int s, int n, double* vbuf, double* beta, double* d, double* e) {
-    const int lane = threadIdx.x & 31, c0 = s + 1;
-    double nrm = 0.0;
-    for (int c = c0 + lane; c < n; c += 32) {
-        const double x = row[c];
-        vbuf[c] = x;
-        nrm += x * x;
-    }
-    for (int o = 16; o > 0; o >>= 1) nrm += __shfl_xor_sync(0xffffffffu, nrm, o);
-    const double alpha = sqrt(nrm);
-    const double x0 = row[c0];
-    const double sg = x0 >= 0.0 ? 1.0 : -1.0;
-    __syncwarp();
-    if (lane == 0) {
-        d[s] = row[s];
-        e[s] = alpha == 0.0 ? 0.0 : -sg * alpha;
-        *beta = alpha == 0.0 ? 0.0 : 1.0 / (alpha * (alpha + fabs(x0)));
-        if (alpha != 0.0) vbuf[c0] = x0 + sg * alpha;
-    }
+// The sum of the warps' partial sums in a tree: 16 dependent additions would be 130 cycles of every step, twice.
+__device__ __forceinline__ double tri_warp_sums(const double* red) {
+    double t[TRI_WARPS];
+#pragma unroll
+    for (int q = 0; q < TRI_WARPS; ++q) t[q] = red[q];
+#pragma unroll
+    for (int h = TRI_WARPS / 2; h > 0; h >>= 1)
+#pragma unroll
+        for (int q = 0; q < h; ++q) t[q] += t[q + h];
+    return t[0];
 }
 
 __global__ void __launch_bounds__(TRI_THREADS) k_tridiag(const TriJob* __restrict__ jobs, const int* __restrict__ mask) {
@@ -74,139 +68,182 @@ __global__ void __launch_bounds__(TRI_THREADS) k_tridiag(const TriJob* __restric
     const TriJob jb = jobs[blockIdx.x / C];
     if (mask && !mask[jb.mol]) return;  // uniform over the cluster
     const int n = jb.n;
+    const int ld = n + (n & 1);
     const int R = (n + C - 1) / C;
-    extern __shared__ double sh[];
-    double* A = sh;                    // R x n: global row lr * C + crank at local row lr
-    double* vb = A + (size_t)R * n;    // v, two buffers of n (global column index)
-    double* wb = vb + 2 * (size_t)n;   // w, two buffers of n
-    double* pp = wb + 2 * (size_t)n;   // this CTA's share of A v
-    double* bb = pp + n;               // beta, two buffers
-    double* red = bb + 2;              // [TRI_WARPS]
-    double* red2 = red + TRI_WARPS;    // [TRI_THREADS] partial column sums of the row groups
+    extern __shared__ double2 tri_sh[];
+    double* A = (double*)tri_sh;                      // R x ld: global row lr * C + crank at local row lr
+    double2* vwb = (double2*)(A + (size_t)R * ld);    // (v, w), two buffers of ld (global column index)
+    double* pp = (double*)(vwb + 2 * (size_t)ld);     // this CTA's share of A v
+    double* bb = pp + ld;                             // 1 / beta, two buffers
+    double* p1 = bb + 2;                              // beta_s, p of column s + 1
+    double* red = p1 + 2;                             // [TRI_WARPS] p.v
+    double* redn = red + TRI_WARPS;                   // [TRI_WARPS] |x|^2
+    double* red2 = redn + TRI_WARPS;                  // [TRI_THREADS] column sums of the row groups
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     auto csync = [&]() {
         if (C > 1) cluster.sync();
         else __syncthreads();
     };
+    // Row s (in its owner): the update with (v, w) = vw, whose entries of column s are vs, ws, and the reflector s
+    // of the result into vn, d[s], e[s], with 1 / beta in *rb (0: no reflection).  A thread per column, s + tid; ends
+    // with thread 1's vn[s + 1] and *rb not yet visible.
+    auto reflect = [&](int s, const double2* vw, double vs, double ws, double2* vn, double* rb) {
+        double* row = A + (size_t)(s / C) * ld;
+        const bool has_next = s + 2 < n;
+        double nrm = 0.0;
+        for (int c = s + tid; c < n; c += TRI_THREADS) {
+            const double2 q = vw[c];
+            const double y = row[c] - vs * q.y - ws * q.x;
+            row[c] = y;
+            if (c > s) {
+                vn[c].x = y;
+                nrm = fma(y, y, nrm);
+            }
+        }
+        if (!has_next) return;  // uniform over the CTA
+        for (int o = 16; o > 0; o >>= 1) nrm += __shfl_xor_sync(0xffffffffu, nrm, o);
+        if (lane == 0) redn[warp] = nrm;
+        __syncthreads();
+        if (tid == 0) jb.d[s] = row[s];
+        if (tid == 1) {
+            const double alpha = sqrt(tri_warp_sums(redn)), x0 = row[s + 1];
+            const double sg = x0 >= 0.0 ? 1.0 : -1.0;
+            if (alpha != 0.0) vn[s + 1].x = x0 + sg * alpha;
+            *rb = alpha * (alpha + fabs(x0));
+            jb.e[s] = alpha == 0.0 ? 0.0 : -sg * alpha;
+        }
+    };
     for (int lr = warp; lr < R; lr += TRI_WARPS) {
         const int r = lr * C + crank;
         if (r >= n) break;
-        for (int c = lane; c < n; c += 32) A[(size_t)lr * n + c] = jb.A[(size_t)r * n + c];
+        for (int c = lane; c < ld; c += 32) A[(size_t)lr * ld + c] = c < n ? jb.A[(size_t)r * n + c] : 0.0;
     }
-    for (int c = tid; c < n; c += TRI_THREADS) {  // update "-1" is the identity
-        vb[n + c] = 0.0;
-        wb[n + c] = 0.0;
-    }
+    for (int c = tid; c < 2 * ld; c += TRI_THREADS) vwb[c] = double2{0.0, 0.0};  // update "-1" is the identity
     __syncthreads();
+    if (crank == 0) reflect(0, vwb + ld, 0.0, 0.0, vwb, bb);
     for (int s = 0; s + 1 < n; ++s) {
-        const int cur = (s + 1) & 1, nxt = s & 1;
-        const double* v = vb + (size_t)cur * n;  // reflector s - 1
-        const double* w = wb + (size_t)cur * n;
-        double* vn = vb + (size_t)nxt * n;       // reflector s
+        const int nxt = s & 1;
+        const double2* vw = vwb + (size_t)(1 - nxt) * ld;  // v, w of step s - 1
+        double2* vn = vwb + (size_t)nxt * ld;              // of step s
         const bool has_next = s + 2 < n;
         const int owner = s % C;
-        if (crank == owner && warp == 0) {  // (a)
-            double* row = A + (size_t)(s / C) * n;
-            const double vs = v[s], ws = w[s];
-            for (int c = s + lane; c < n; c += 32) row[c] -= vs * w[c] + ws * v[c];
-            __syncwarp();
-            if (has_next) tri_reflector(row, s, n, vn, bb + nxt, jb.d, jb.e);
-        }
-        csync();  // v_s ready in the owner
+        // (b) columns > s in pairs from an even one on (column s among them for an even s: written, not read), rows
+        // c > s of this CTA.  Threads in G groups of a thread per pair; group g takes rows lr0 + g, lr0 + g + G, ...
+        // (more groups when there are few columns, as many as red2 holds the sums of)
+        const int lr0 = (s + 1 - crank + C - 1) / C;  // first local row with global index > s
+        const int lre = (n - crank + C - 1) / C;      // local rows with global index < n
+        const int q0 = (s + 1) & ~1;
+        const int ncp = (n - q0 + 1) / 2;
+        const int G = max(1, min(16, TRI_THREADS / (2 * ncp)));
+        const int g = tid / ncp;
+        csync();  // v_s ready in the owner, w_{s-1} everywhere
         if (has_next && crank != owner) {
-            const double* rv = cluster.map_shared_rank(vn, owner);
-            for (int c = s + 1 + tid; c < n; c += TRI_THREADS) vn[c] = rv[c];
+            const double2* rv = cluster.map_shared_rank(vn, owner);
+            for (int c = s + 1 + tid; c < n; c += TRI_THREADS) vn[c].x = rv[c].x;
             if (tid == 0) bb[nxt] = *cluster.map_shared_rank(bb + nxt, owner);
             __syncthreads();
         }
-        // (b) columns r > s, rows c > s of this CTA: threads in G groups of cpg; thread (g, j) owns
-        // column s + 1 + j and rows lr0 + g, lr0 + g + G, ... (more groups when there are few columns)
-        const int lr0 = (s + 1 - crank + C - 1) / C;  // first local row with global index > s
-        const int lre = (n - crank + C - 1) / C;      // local rows with global index < n
-        const int ncol = n - (s + 1);
-        const int G = max(1, min(16, TRI_THREADS / (((ncol + 31) / 32) * 32)));
-        const int cpg = TRI_THREADS / G;
-        const int g = tid / cpg, j = tid - g * cpg;
-        // columns s + 1 + j, j = this thread's index in its group, then strided by the group size
-        // (more columns than threads take several trips; more groups only when columns are few)
-        for (int jj = j; jj < ncol || (G > 1 && jj == j); jj += cpg) {
-            double acc = 0.0;
-            if (g < G && jj < ncol) {
-                const int r = s + 1 + jj;
-                const double vr = v[r], wr = w[r];
-                int lr = lr0 + g;
-                for (; lr + 3 * G < lre; lr += 4 * G) {  // four independent rows per trip
-                    double* a0 = A + (size_t)lr * n + r;
-                    double* a1 = a0 + (size_t)G * n;
-                    double* a2 = a1 + (size_t)G * n;
-                    double* a3 = a2 + (size_t)G * n;
-                    const int c0 = lr * C + crank, c1 = c0 + G * C, c2 = c1 + G * C, c3 = c2 + G * C;
-                    const double x0 = *a0, x1 = *a1, x2 = *a2, x3 = *a3;
-                    const double y0 = x0 - v[c0] * wr - w[c0] * vr, y1 = x1 - v[c1] * wr - w[c1] * vr;
-                    const double y2 = x2 - v[c2] * wr - w[c2] * vr, y3 = x3 - v[c3] * wr - w[c3] * vr;
-                    *a0 = y0;
-                    *a1 = y1;
-                    *a2 = y2;
-                    *a3 = y3;
-                    acc = fma(y0, vn[c0], acc);
-                    acc = fma(y1, vn[c1], acc);
-                    acc = fma(y2, vn[c2], acc);
-                    acc = fma(y3, vn[c3], acc);
+        if (tid == TRI_THREADS - 1 && has_next) *p1 = bb[nxt] == 0.0 ? 0.0 : 1.0 / bb[nxt];  // a thread (b) has no pair for
+        for (int j = G > 1 ? tid - g * ncp : tid; j < ncp && (G == 1 || g < G); j += TRI_THREADS) {
+            const int r = q0 + 2 * j;
+            const double2 q = vw[r], q1 = vw[r + 1];
+            double acc0 = 0.0, acc1 = 0.0;
+            auto row2 = [&](double2 x, double2 m) {  // m: (v, w) of the row
+                x.x = x.x - m.x * q.y - m.y * q.x;
+                x.y = x.y - m.x * q1.y - m.y * q1.x;
+                return x;
+            };
+            int lr = lr0 + (G > 1 ? g : 0);
+            double2* ap = (double2*)(A + (size_t)lr * ld + r);
+            const size_t step = (size_t)G * ld / 2;
+            for (; lr + 3 * G < lre; lr += 4 * G, ap += 4 * step) {  // four independent rows per trip
+                const int c0 = lr * C + crank, c1 = c0 + G * C, c2 = c1 + G * C, c3 = c2 + G * C;
+                const double2 x0 = ap[0], x1 = ap[step], x2 = ap[2 * step], x3 = ap[3 * step];
+                const double2 m0 = vw[c0], m1 = vw[c1], m2 = vw[c2], m3 = vw[c3];
+                const double n0 = vn[c0].x, n1 = vn[c1].x, n2 = vn[c2].x, n3 = vn[c3].x;
+                const double2 y0 = row2(x0, m0), y1 = row2(x1, m1), y2 = row2(x2, m2), y3 = row2(x3, m3);
+                ap[0] = y0;
+                ap[step] = y1;
+                ap[2 * step] = y2;
+                ap[3 * step] = y3;
+                acc0 = fma(y0.x, n0, acc0), acc1 = fma(y0.y, n0, acc1);
+                acc0 = fma(y1.x, n1, acc0), acc1 = fma(y1.y, n1, acc1);
+                acc0 = fma(y2.x, n2, acc0), acc1 = fma(y2.y, n2, acc1);
+                acc0 = fma(y3.x, n3, acc0), acc1 = fma(y3.y, n3, acc1);
+            }
+            if (lr < lre) {  // up to three more, their loads together
+                const int k1 = lr + G < lre ? 1 : 0, k2 = lr + 2 * G < lre ? 2 : 0;
+                const int c0 = lr * C + crank, c1 = c0 + k1 * G * C, c2 = c0 + k2 * G * C;
+                const double2 x0 = ap[0], x1 = ap[k1 * step], x2 = ap[k2 * step];
+                const double2 m0 = vw[c0], m1 = vw[c1], m2 = vw[c2];
+                const double n0 = vn[c0].x, n1 = vn[c1].x, n2 = vn[c2].x;
+                const double2 y0 = row2(x0, m0), y1 = row2(x1, m1), y2 = row2(x2, m2);
+                ap[0] = y0;
+                acc0 = fma(y0.x, n0, acc0), acc1 = fma(y0.y, n0, acc1);
+                if (k1) {
+                    ap[step] = y1;
+                    acc0 = fma(y1.x, n1, acc0), acc1 = fma(y1.y, n1, acc1);
                 }
-                for (; lr < lre; lr += G) {
-                    const int c = lr * C + crank;
-                    double* ap = A + (size_t)lr * n + r;
-                    const double y = *ap - v[c] * wr - w[c] * vr;
-                    *ap = y;
-                    acc = fma(y, vn[c], acc);
+                if (k2) {
+                    ap[2 * step] = y2;
+                    acc0 = fma(y2.x, n2, acc0), acc1 = fma(y2.y, n2, acc1);
                 }
             }
-            if (G == 1) {
-                if (jj < ncol) pp[s + 1 + jj] = acc;
-            } else {  // one trip only (ncol <= cpg), uniform over the CTA
-                red2[tid] = acc;
-                __syncthreads();
-                if (g == 0 && jj < ncol) {
-                    double t = 0.0;
-                    for (int q = 0; q < G; ++q) t += red2[q * cpg + jj];
-                    pp[s + 1 + jj] = t;
-                }
-                break;
-            }
+            double* o = G > 1 ? red2 + 2 * (g * ncp + j) : pp + r;
+            o[0] = acc0;
+            o[1] = acc1;
+            if (G > 1) break;
         }
         if (!has_next) break;
-        csync();  // every CTA's share of A v_s ready
-        const double beta = bb[nxt];
+        if (G > 1) {
+            __syncthreads();
+            for (int r = s + 1 + tid; r < n; r += TRI_THREADS) {  // the loop below: the same thread's columns
+                const double* col = red2 + r - q0;
+                double t[4] = {0.0, 0.0, 0.0, 0.0};
+                for (int q = 0; q < G; q += 4)
+#pragma unroll
+                    for (int k = 0; k < 4; ++k)
+                        if (q + k < G) t[k] += col[2 * (q + k) * ncp];
+                pp[r] = (t[0] + t[1]) + (t[2] + t[3]);
+            }
+        }
+        if (C > 1 || G == 1) csync();  // every CTA's share of A v_s ready
+        const double beta = *p1;
         double part = 0.0;
         for (int r = s + 1 + tid; r < n; r += TRI_THREADS) {
             double sum = 0.0;
-            for (int q = 0; q < C; ++q) sum += *cluster.map_shared_rank(pp + r, q);
+            if (C == 1) sum = pp[r];
+            else
+                for (int q = 0; q < C; ++q) sum += *cluster.map_shared_rank(pp + r, q);
             const double p = beta * sum;
-            wb[(size_t)nxt * n + r] = p;  // p for now, w below
-            part += p * vn[r];
+            if (r == s + 1) p1[1] = p;
+            vn[r].y = p;  // p for now, w below
+            part = fma(p, vn[r].x, part);
         }
         for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
         if (lane == 0) red[warp] = part;
         __syncthreads();
-        double pv = 0.0;
-        for (int q = 0; q < TRI_WARPS; ++q) pv += red[q];
-        const double kk = 0.5 * beta * pv;
-        for (int r = s + 1 + tid; r < n; r += TRI_THREADS) wb[(size_t)nxt * n + r] -= kk * vn[r];
-        __syncthreads();
+        const double kk = 0.5 * beta * tri_warp_sums(red);
+        for (int r = s + 1 + tid; r < n; r += TRI_THREADS) vn[r].y = fma(-kk, vn[r].x, vn[r].y);
         if (s + 1 == jb.stop) {  // uniform over the cluster
             // hand-off: the trailing block with update s applied, to W (m x m, row-major)
+            __syncthreads();
             const int s0 = s + 1, m = n - s0;
-            const double* wv = wb + (size_t)nxt * n;
             for (int lr = (s0 - crank + C - 1) / C + warp; lr < R; lr += TRI_WARPS) {
                 const int c = lr * C + crank;
                 if (c >= n) break;
-                const double vc = vn[c], wc = wv[c];
-                const double* arow = A + (size_t)lr * n;
+                const double2 m2 = vn[c];
+                const double* arow = A + (size_t)lr * ld;
                 double* out = jb.W + (size_t)(c - s0) * m - s0;
-                for (int r = s0 + lane; r < n; r += 32) out[r] = arow[r] - vc * wv[r] - wc * vn[r];
+                for (int r = s0 + lane; r < n; r += 32) out[r] = arow[r] - m2.x * vn[r].y - m2.y * vn[r].x;
             }
             csync();  // no CTA leaves while another may still address its shared memory
             return;
+        }
+        // (a) row s + 1: its columns are those of w this thread wrote
+        if (crank == (s + 1) % C) {
+            const double v1 = vn[s + 1].x;
+            reflect(s + 1, vn, v1, fma(-kk, v1, p1[1]), vwb + (size_t)(1 - nxt) * ld, bb + (1 - nxt));
         }
     }
     __syncthreads();
@@ -214,10 +251,10 @@ __global__ void __launch_bounds__(TRI_THREADS) k_tridiag(const TriJob* __restric
     if (tid == 0) {
         if (n >= 2) {
             if ((n - 2) % C == crank) {
-                jb.d[n - 2] = A[(size_t)((n - 2) / C) * n + n - 2];
-                jb.e[n - 2] = A[(size_t)((n - 2) / C) * n + n - 1];
+                jb.d[n - 2] = A[(size_t)((n - 2) / C) * ld + n - 2];
+                jb.e[n - 2] = A[(size_t)((n - 2) / C) * ld + n - 1];
             }
-            if ((n - 1) % C == crank) jb.d[n - 1] = A[(size_t)((n - 1) / C) * n + n - 1];
+            if ((n - 1) % C == crank) jb.d[n - 1] = A[(size_t)((n - 1) / C) * ld + n - 1];
         } else if (crank == 0) {
             jb.d[0] = A[0];
         }
