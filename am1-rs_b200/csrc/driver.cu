@@ -251,6 +251,9 @@ int device_ctx(DeviceCtx** out) {
         for (const void* f : {(const void*)k_sp2_step_tma, (const void*)k_commutator_tma})
             if ((err = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dgemm_tma_smem_bytes())) != cudaSuccess)
                 return bad("tensor-map tile kernel smem attribute", err);
+        for (const void* f : {(const void*)k_sp2_step_both, (const void*)k_commutator_both})
+            if ((err = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dgemm_both_smem_bytes())) != cudaSuccess)
+                return bad("tensor-map tile kernel smem attribute", err);
         if ((err = cudaFuncSetAttribute(k_sp2_step_tf32, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tf32_smem_bytes())) !=
             cudaSuccess)
             return bad("tf32 tile kernel smem attribute", err);
@@ -1701,14 +1704,20 @@ int enq_head(IterEnq& e) {
     k_fock<<<fock_grid(b.natoms, b.maxheavy), 32 * FOCK_WARPS, 0, s>>>(b.d_mols, b.d_atom_mol, b.natoms, e.dp, b.d_atom_z, b.d_wstore, b.d_arena, b.d_st, 0);
     run.launched(AM1GPU_PHASE_FOCK);
     if ((rc = run.end(AM1GPU_PHASE_FOCK, e.ph)) || (rc = run.begin(&e.ph))) return rc;
-    launch_tiles(b, false, [&](const GemmTile* t, int nt, bool pairs) {
-        if (pairs && b.sp2_tma)
-            k_commutator_tma<<<nt, 128, dgemm_tma_smem_bytes(), s>>>(b.d_jobs, t, nt, b.d_st, b.d_sp2_maps, b.d_sp2_active + 2);
-        else if (pairs)
-            k_commutator16<<<nt, 128, dgemm_smem_bytes(), s>>>(b.d_jobs, t, nt, b.d_st);
-        else
-            k_commutator8<<<nt, 128, dgemm_smem_bytes(), s>>>(b.d_jobs, t, nt, b.d_st);
-    });
+    const int nt_other = b.nt_sp2 - b.nt_sp2_pairs;
+    if (b.sp2_tma && b.nt_sp2_pairs > 0 && nt_other > 0)
+        k_commutator_both<<<b.nt_sp2, 128, dgemm_both_smem_bytes(), s>>>(b.d_jobs, b.d_sp2_tiles, b.nt_sp2_pairs,
+                                                                        b.d_sp2_tiles + b.nt_sp2_pairs, nt_other, b.d_st, b.d_sp2_maps,
+                                                                        b.d_sp2_active + 2);
+    else
+        launch_tiles(b, false, [&](const GemmTile* t, int nt, bool pairs) {
+            if (pairs && b.sp2_tma)
+                k_commutator_tma<<<nt, 128, dgemm_tma_smem_bytes(), s>>>(b.d_jobs, t, nt, b.d_st, b.d_sp2_maps, b.d_sp2_active + 2);
+            else if (pairs)
+                k_commutator16<<<nt, 128, dgemm_smem_bytes(), s>>>(b.d_jobs, t, nt, b.d_st);
+            else
+                k_commutator8<<<nt, 128, dgemm_smem_bytes(), s>>>(b.d_jobs, t, nt, b.d_st);
+        });
     k_post_fock<<<dim3(e.nblk, e.njobs), 256, 0, s>>>(b.d_jobs, b.d_mols, b.d_st, e.nblk, 0, 0);
     run.launched(AM1GPU_PHASE_COMMUTATOR, 2);
     if ((rc = run.end(AM1GPU_PHASE_COMMUTATOR, e.ph)) || (rc = run.begin(&e.ph))) return rc;
@@ -1754,15 +1763,22 @@ int enq_step(IterEnq& e, int sp2_max, bool lowp_left, bool zero_count, const cud
     size_t pc;
     if ((rc = run.begin(&pc))) return rc;
     int nl = 0;
-    launch_tiles(b, true, [&](const GemmTile* t, int nt, bool pairs) {
-        if (pairs && b.sp2_tma)
-            k_sp2_step_tma<<<nt, 128, dgemm_tma_smem_bytes(), s>>>(b.d_sp2, t, nt, b.d_sp2_state, b.d_sp2_maps, b.d_sp2_active + 2);
-        else if (pairs)
-            k_sp2_step16<<<nt, 128, dgemm_smem_bytes(), s>>>(b.d_sp2, t, nt, b.d_sp2_state);
-        else
-            k_sp2_step8<<<nt, 128, dgemm_smem_bytes(), s>>>(b.d_sp2, t, nt, b.d_sp2_state);
+    if (b.sp2_tma && b.nt_step_pairs > 0 && b.nt_step_other > 0) {
+        k_sp2_step_both<<<b.nt_step_pairs + b.nt_step_other, 128, dgemm_both_smem_bytes(), s>>>(
+            b.d_sp2, b.d_sp2_tiles, b.nt_step_pairs, b.d_sp2_tiles + b.nt_sp2_pairs, b.nt_step_other, b.d_sp2_state, b.d_sp2_maps,
+            b.d_sp2_active + 2);
         ++nl;
-    });
+    } else {
+        launch_tiles(b, true, [&](const GemmTile* t, int nt, bool pairs) {
+            if (pairs && b.sp2_tma)
+                k_sp2_step_tma<<<nt, 128, dgemm_tma_smem_bytes(), s>>>(b.d_sp2, t, nt, b.d_sp2_state, b.d_sp2_maps, b.d_sp2_active + 2);
+            else if (pairs)
+                k_sp2_step16<<<nt, 128, dgemm_smem_bytes(), s>>>(b.d_sp2, t, nt, b.d_sp2_state);
+            else
+                k_sp2_step8<<<nt, 128, dgemm_smem_bytes(), s>>>(b.d_sp2, t, nt, b.d_sp2_state);
+            ++nl;
+        });
+    }
     if (b.nt_oz > 0) {
         k_sp2_step_oz<<<b.nt_oz, 128, oz_smem_bytes(), s>>>(b.d_sp2, b.d_oz_tiles, b.nt_oz, b.d_sp2_state, b.d_sp2_active + 2);
         ++nl;

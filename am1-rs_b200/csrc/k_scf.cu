@@ -175,11 +175,9 @@ __global__ void __launch_bounds__(32 * POST_WARPS) k_post_fock(const ChanJob* __
 constexpr int CT_LD = DG_TILE + 1;  // row stride of the staged commutator tile (doubles)
 
 template <int COPY>
-__device__ __forceinline__ void commutator_body(const ChanJob* __restrict__ jobs, const GemmTile* __restrict__ tiles, int ntiles,
-                                                const MolState* __restrict__ st, const TmaDesc* __restrict__ maps, int* __restrict__ err) {
-    __shared__ double red[CP_N][4];
-    const int t = blockIdx.x;
-    if (t >= ntiles) return;
+__device__ __forceinline__ void commutator_body(const ChanJob* __restrict__ jobs, const GemmTile* __restrict__ tiles, int t,
+                                                const MolState* __restrict__ st, const TmaDesc* __restrict__ maps, int* __restrict__ err,
+                                                double red[CP_N][4]) {
     const GemmTile tl = tiles[t];
     const ChanJob jb = jobs[tl.job];
     const MolState& s = st[jb.mol];
@@ -196,7 +194,7 @@ __device__ __forceinline__ void commutator_body(const ChanJob* __restrict__ jobs
     double acc[2][4][4];
     double* T;  // the tile staged for the epilogue, in the pipeline's shared memory (free after the k-loop)
     if constexpr (COPY == 2) {
-        extern __shared__ __align__(1024) unsigned char ctsm[];
+        extern __shared__ __align__(16) unsigned char ctsm[];
         __shared__ DtBars bars;
         const TmaDesc* mp = maps + 4 * tl.job;  // F and P are symmetric: B = F or P read by rows
         const int shape = dg_quarter_shape(m0, n0, n, n, tl.tm == tl.tn);
@@ -273,16 +271,29 @@ __device__ __forceinline__ void commutator_body(const ChanJob* __restrict__ jobs
 
 __global__ void __launch_bounds__(DG_THREADS, 4) k_commutator16(const ChanJob* __restrict__ jobs, const GemmTile* __restrict__ tiles,
                                                                 int ntiles, const MolState* __restrict__ st) {
-    commutator_body<1>(jobs, tiles, ntiles, st, nullptr, nullptr);
+    __shared__ double red[CP_N][4];
+    if ((int)blockIdx.x < ntiles) commutator_body<1>(jobs, tiles, (int)blockIdx.x, st, nullptr, nullptr, red);
 }
 __global__ void __launch_bounds__(DG_THREADS, 4) k_commutator8(const ChanJob* __restrict__ jobs, const GemmTile* __restrict__ tiles,
                                                                int ntiles, const MolState* __restrict__ st) {
-    commutator_body<0>(jobs, tiles, ntiles, st, nullptr, nullptr);
+    __shared__ double red[CP_N][4];
+    if ((int)blockIdx.x < ntiles) commutator_body<0>(jobs, tiles, (int)blockIdx.x, st, nullptr, nullptr, red);
 }
 __global__ void __launch_bounds__(DG_THREADS, 4) k_commutator_tma(const ChanJob* __restrict__ jobs, const GemmTile* __restrict__ tiles,
                                                                   int ntiles, const MolState* __restrict__ st,
                                                                   const TmaDesc* __restrict__ maps, int* __restrict__ err) {
-    commutator_body<2>(jobs, tiles, ntiles, st, maps, err);
+    __shared__ double red[CP_N][4];
+    if ((int)blockIdx.x < ntiles) commutator_body<2>(jobs, tiles, (int)blockIdx.x, st, maps, err, red);
+}
+// The first nother CTAs take the tiles of odd n, as k_commutator8 (k_sp2_step_both says why).
+__global__ void __launch_bounds__(DG_THREADS, 4) k_commutator_both(const ChanJob* __restrict__ jobs, const GemmTile* __restrict__ tiles,
+                                                                   int ntiles, const GemmTile* __restrict__ other, int nother,
+                                                                   const MolState* __restrict__ st,
+                                                                   const TmaDesc* __restrict__ maps, int* __restrict__ err) {
+    __shared__ double red[CP_N][4];
+    const int t = (int)blockIdx.x - nother;
+    if (t < 0) commutator_body<0>(jobs, other, (int)blockIdx.x, st, nullptr, nullptr, red);
+    else if (t < ntiles) commutator_body<2>(jobs, tiles, t, st, maps, err, red);
 }
 
 // ---- the extrapolation, a warp per molecule.  The kernel is a handful of tiny dense problems behind

@@ -559,12 +559,8 @@ __device__ __forceinline__ void sp2_step_epilogue(const Sp2Job* __restrict__ jp,
 // One SP2 step over all upper-triangle 64x64 tiles of every active channel (operands copied by
 // cp.async: k_sp2_step8 for odd n, and k_sp2_step16 where the tensor-map kernel is not used).
 template <bool PAIRS>
-__device__ __forceinline__ void sp2_step_body(const Sp2Job* __restrict__ jobs, const GemmTile* __restrict__ tiles, int ntiles,
-                                              const Sp2State* __restrict__ sst) {
-    extern __shared__ __align__(16) double dsm[];
-    __shared__ double red[2][4];
-    const int t = blockIdx.x;
-    if (t >= ntiles) return;
+__device__ __forceinline__ void sp2_step_body(const Sp2Job* __restrict__ jobs, const GemmTile* __restrict__ tiles, int t,
+                                              const Sp2State* __restrict__ sst, double* dsm, double red[2][4]) {
     const GemmTile tl = tiles[t];
     const Sp2State* sp = sst + tl.job;
     const Sp2Job* jp = jobs + tl.job;
@@ -584,14 +580,9 @@ __device__ __forceinline__ void sp2_step_body(const Sp2Job* __restrict__ jobs, c
 // job's tensor maps (maps[4 job + cur] describes the current iterate), through the mbarrier
 // pipeline of dg_mainloop_tma: bit-identical to k_sp2_step16.  A copy wait that runs out sets bit
 // 11 of *err and the tile is left unwritten.
-__global__ void __launch_bounds__(DG_THREADS, 4) k_sp2_step_tma(const Sp2Job* __restrict__ jobs, const GemmTile* __restrict__ tiles,
-                                                               int ntiles, const Sp2State* __restrict__ sst,
-                                                               const TmaDesc* __restrict__ maps, int* __restrict__ err) {
-    extern __shared__ __align__(1024) unsigned char dtsm[];
-    __shared__ DtBars bars;
-    __shared__ double red[2][4];
-    const int t = blockIdx.x;
-    if (t >= ntiles) return;
+__device__ __forceinline__ void sp2_step_tma_body(const Sp2Job* __restrict__ jobs, const GemmTile* __restrict__ tiles, int t,
+                                                  const Sp2State* __restrict__ sst, const TmaDesc* __restrict__ maps,
+                                                  int* __restrict__ err, unsigned char* dtsm, DtBars& bars, double red[2][4]) {
     const GemmTile tl = tiles[t];
     const Sp2State* sp = sst + tl.job;
     const Sp2Job* jp = jobs + tl.job;
@@ -607,6 +598,31 @@ __global__ void __launch_bounds__(DG_THREADS, 4) k_sp2_step_tma(const Sp2Job* __
         return;
     }
     sp2_step_epilogue(jp, sp, t, n, m0, n0, acc, compute, red);
+}
+
+__global__ void __launch_bounds__(DG_THREADS, 4) k_sp2_step_tma(const Sp2Job* __restrict__ jobs, const GemmTile* __restrict__ tiles,
+                                                               int ntiles, const Sp2State* __restrict__ sst,
+                                                               const TmaDesc* __restrict__ maps, int* __restrict__ err) {
+    extern __shared__ __align__(16) unsigned char dtsm[];
+    __shared__ DtBars bars;
+    __shared__ double red[2][4];
+    if ((int)blockIdx.x < ntiles) sp2_step_tma_body(jobs, tiles, (int)blockIdx.x, sst, maps, err, dtsm, bars, red);
+}
+
+// Both kinds of tiles in one launch: the first nother CTAs take those of odd n, as k_sp2_step8.  Alone these are a
+// launch of less than a wave that lasts as long as its largest matrix' k-loop, with the GPU half empty; here
+// the even ones fill it (64 molecules of mixed sizes 137 -> 128 ms, 1152 with one radical in nine 163 -> 159).  A kernel of
+// its own, since the TMA path takes 7 registers more beside the other (0.4% of a batch of even orders).
+__global__ void __launch_bounds__(DG_THREADS, 4) k_sp2_step_both(const Sp2Job* __restrict__ jobs, const GemmTile* __restrict__ tiles,
+                                                                int ntiles, const GemmTile* __restrict__ other, int nother,
+                                                                const Sp2State* __restrict__ sst,
+                                                                const TmaDesc* __restrict__ maps, int* __restrict__ err) {
+    extern __shared__ __align__(16) unsigned char dtsm[];
+    __shared__ DtBars bars;
+    __shared__ double red[2][4];
+    const int t = (int)blockIdx.x - nother;
+    if (t < 0) sp2_step_body<false>(jobs, other, (int)blockIdx.x, sst, (double*)dtsm, red);
+    else if (t < ntiles) sp2_step_tma_body(jobs, tiles, t, sst, maps, err, dtsm, bars, red);
 }
 
 // After a step: reduce the tile partials (in tile order), test idempotency, choose the next branch.
@@ -743,14 +759,19 @@ __global__ void k_sp2_finish(const Sp2Job* __restrict__ jobs, const Sp2State* __
 
 size_t dgemm_smem_bytes() { return DG_SMEM; }
 size_t dgemm_tma_smem_bytes() { return DT_SMEM; }
+size_t dgemm_both_smem_bytes() { return DG_SMEM > DT_SMEM ? DG_SMEM : DT_SMEM; }  // four CTAs still fit an SM
 
 __global__ void __launch_bounds__(DG_THREADS, 4) k_sp2_step16(const Sp2Job* __restrict__ jobs, const GemmTile* __restrict__ tiles,
                                                               int ntiles, const Sp2State* __restrict__ sst) {
-    sp2_step_body<true>(jobs, tiles, ntiles, sst);
+    extern __shared__ __align__(16) double dsm[];
+    __shared__ double red[2][4];
+    if ((int)blockIdx.x < ntiles) sp2_step_body<true>(jobs, tiles, (int)blockIdx.x, sst, dsm, red);
 }
 __global__ void __launch_bounds__(DG_THREADS, 4) k_sp2_step8(const Sp2Job* __restrict__ jobs, const GemmTile* __restrict__ tiles,
                                                              int ntiles, const Sp2State* __restrict__ sst) {
-    sp2_step_body<false>(jobs, tiles, ntiles, sst);
+    extern __shared__ __align__(16) double dsm[];
+    __shared__ double red[2][4];
+    if ((int)blockIdx.x < ntiles) sp2_step_body<false>(jobs, tiles, (int)blockIdx.x, sst, dsm, red);
 }
 
 }  // namespace am1

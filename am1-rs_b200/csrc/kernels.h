@@ -244,7 +244,11 @@ __global__ void k_sp2_step8(const Sp2Job* jobs, const GemmTile* tiles, int ntile
 // wait that runs out sets bit 11 of *err
 __global__ void k_sp2_step_tma(const Sp2Job* jobs, const GemmTile* tiles, int ntiles, const Sp2State* sst, const TmaDesc* maps,
                                int* err);
+// the same with nother CTAs more, the first, for tiles of odd n (k_sp2_step8's); dgemm_both_smem_bytes()
+__global__ void k_sp2_step_both(const Sp2Job* jobs, const GemmTile* tiles, int ntiles, const GemmTile* other, int nother,
+                                const Sp2State* sst, const TmaDesc* maps, int* err);
 size_t dgemm_tma_smem_bytes();
+size_t dgemm_both_smem_bytes();
 // the TF32 step of the mixed path's reduced-precision iterations (jobs with Sp2State::lowp);
 // tf32_smem_bytes() of dynamic shared memory, same tile lists
 __global__ void k_sp2_step_tf32(const Sp2Job* jobs, const GemmTile* tiles, int ntiles, const Sp2State* sst);
@@ -252,9 +256,11 @@ size_t tf32_smem_bytes();
 // E = F.P - P.F over the upper-triangle tiles: history push of E and its CDIIS Gram row
 __global__ void k_commutator16(const ChanJob* jobs, const GemmTile* tiles, int ntiles, const MolState* st);
 __global__ void k_commutator8(const ChanJob* jobs, const GemmTile* tiles, int ntiles, const MolState* st);
-// the *16 tiles from the tensor maps of F and P (maps[4 job + 2], [4 job + 3]); dgemm_tma_smem_bytes()
+// the *16 tiles from the tensor maps of F and P (maps[4 job + 2], [4 job + 3]); dgemm_tma_smem_bytes(), ..._both: dgemm_both_smem_bytes()
 __global__ void k_commutator_tma(const ChanJob* jobs, const GemmTile* tiles, int ntiles, const MolState* st, const TmaDesc* maps,
                                  int* err);
+__global__ void k_commutator_both(const ChanJob* jobs, const GemmTile* tiles, int ntiles, const GemmTile* other, int nother,
+                                  const MolState* st, const TmaDesc* maps, int* err);
 size_t dgemm_smem_bytes();
 __global__ void k_sp2_update(const Sp2Job* jobs, Sp2State* sst, int njobs, int max_steps, int* active_count, double* work);
 __global__ void k_sp2_update_cond(const Sp2Job* jobs, Sp2State* sst, int njobs, int max_steps, double* work, cudaGraphConditionalHandle h,
