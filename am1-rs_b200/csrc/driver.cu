@@ -1784,10 +1784,10 @@ int enq_step(IterEnq& e, int sp2_max, bool lowp_left, bool zero_count, const cud
         ++nl;
     }
     if (lowp_left) {
-        launch_tiles(b, false, [&](const GemmTile* t, int nt, bool) {
-            k_sp2_step_tf32<<<nt, 128, tf32_smem_bytes(), s>>>(b.d_sp2, t, nt, b.d_sp2_state);
+        if (b.nt_sp2 > 0) {  // one kernel for both kinds of tiles
+            k_sp2_step_tf32<<<b.nt_sp2, 128, tf32_smem_bytes(), s>>>(b.d_sp2, b.d_sp2_tiles, b.nt_sp2_pairs, b.nt_sp2, b.d_sp2_state);
             ++nl;
-        });
+        }
         if (b.nt_tc > 0 && b.has_tc3) {
             k_sp2_step_tc<<<b.nt_tc, 128, tc_smem_bytes(), s>>>(b.d_sp2, b.d_tc_tiles, b.nt_tc, b.d_sp2_state, b.d_sp2_active + 2);
             ++nl;
@@ -3101,7 +3101,7 @@ int density_purify_one(int n, const double* F, double nocc, double weight, int p
             if (precision == 3) {
                 k_sp2_step_oz<<<ntoz, 128, oz_smem_bytes(), s>>>(dj, (const GemmTile*)(D + o_toz), ntoz, dsst, dact + 2);
             } else if (precision == 2) {
-                k_sp2_step_tf32<<<nt64, 128, tf32_smem_bytes(), s>>>(dj, d64, nt64, dsst);
+                k_sp2_step_tf32<<<nt64, 128, tf32_smem_bytes(), s>>>(dj, d64, nt64, nt64, dsst);
             } else if (precision == 4) {
                 k_sp2_step_tc1<<<nt128, 128, tc1_smem_bytes(), s>>>(dj, d128, nt128, dsst, (const TmaDesc*)(D + o_xfmaps), dact + 2);
             } else {

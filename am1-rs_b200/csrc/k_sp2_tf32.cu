@@ -69,12 +69,13 @@ __device__ __forceinline__ void tf_load(float* smem, int st, const float* __rest
 }
 
 __global__ void __launch_bounds__(TF_THREADS, 4) k_sp2_step_tf32(const Sp2Job* __restrict__ jobs, const GemmTile* __restrict__ tiles,
-                                                                 int ntiles, const Sp2State* __restrict__ sst) {
+                                                                 int npairs, int ntiles, const Sp2State* __restrict__ sst) {
     extern __shared__ __align__(16) float fsm[];
     __shared__ double red[2][4];
-    const int t = blockIdx.x;
-    if (t >= ntiles) return;
-    const GemmTile tl = tiles[t];
+    const int at = blockIdx.x;
+    if (at >= ntiles) return;
+    const GemmTile tl = tiles[at];
+    const int t = at < npairs ? at : at - npairs;  // index among its kind, as the FP64 launches count
     const Sp2State* sp = sst + tl.job;
     const Sp2Job* jp = jobs + tl.job;
     if (!sp->active || !sp->lowp || jp->lowp_tc) return;  // FP64 runs: k_sp2_step_tma / 16 / 8; tcgen05: k_sp2_step_tc / _tc1

@@ -250,8 +250,8 @@ __global__ void k_sp2_step_both(const Sp2Job* jobs, const GemmTile* tiles, int n
 size_t dgemm_tma_smem_bytes();
 size_t dgemm_both_smem_bytes();
 // the TF32 step of the mixed path's reduced-precision iterations (jobs with Sp2State::lowp);
-// tf32_smem_bytes() of dynamic shared memory, same tile lists
-__global__ void k_sp2_step_tf32(const Sp2Job* jobs, const GemmTile* tiles, int ntiles, const Sp2State* sst);
+// tf32_smem_bytes() of dynamic shared memory, the tiles of both kinds: npairs *16 tiles, then the rest
+__global__ void k_sp2_step_tf32(const Sp2Job* jobs, const GemmTile* tiles, int npairs, int ntiles, const Sp2State* sst);
 size_t tf32_smem_bytes();
 // E = F.P - P.F over the upper-triangle tiles: history push of E and its CDIIS Gram row
 __global__ void k_commutator16(const ChanJob* jobs, const GemmTile* tiles, int ntiles, const MolState* st);
