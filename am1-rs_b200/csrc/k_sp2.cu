@@ -245,6 +245,10 @@ __device__ void lz_interval(const double* alpha, const double* beta, int m, doub
 // purification starts) and every CTA keeps the same alpha, beta (sums of the per-CTA shares in one
 // fixed order).  Three group barriers per step; cross-CTA data is read through L2 (__ldcg).
 // Scratch: q[3][n] | share[2][G].
+// Bound by L2 latency: a lane loads LZ_AHEAD elements of two rows before it uses any, and the vector updates take a
+// row per lane (14 matrices above 448 orbitals, a cluster each: 394 -> 336 us a launch).
+constexpr int LZ_AHEAD = 4;
+
 template <class Sync>
 __device__ void sp2_bounds_group(const Sp2Job& jb, int G, int gi, Sync sync) {
     const int n = jb.n;
@@ -304,14 +308,38 @@ __device__ void sp2_bounds_group(const Sp2Job& jb, int G, int gi, Sync sync) {
         double* wq = qb + (size_t)nxt * n;
         // w_r = F[r, :] . q for own rows (a warp per row) and the CTA's share of q . w
         double part = 0.0;
-        for (int r = gi + warp * G; r < n; r += NW * G) {
+        for (int r = gi + warp * G; r < n; r += 2 * NW * G) {
+            const int r2 = r + NW * G;
+            const bool two = r2 < n;  // uniform over the warp
             const double* Fr = jb.F + (long long)r * n;
-            double acc = 0.0;
-#pragma unroll 4
-            for (int c = lane; c < n; c += 32) acc = fma(Fr[c], __ldcg(q + c), acc);
-            for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-            if (lane == 0) wq[r] = acc;
+            const double* Fs = jb.F + (long long)(two ? r2 : r) * n;
+            double acc = 0.0, acc2 = 0.0;
+            for (int c0 = lane; c0 < n; c0 += 32 * LZ_AHEAD) {
+                double x[LZ_AHEAD], y[LZ_AHEAD], v[LZ_AHEAD];
+#pragma unroll
+                for (int u = 0; u < LZ_AHEAD; ++u) {
+                    const int c = c0 + 32 * u;
+                    x[u] = c < n ? Fr[c] : 0.0;
+                    y[u] = two && c < n ? Fs[c] : 0.0;
+                    v[u] = c < n ? __ldcg(q + c) : 0.0;
+                }
+#pragma unroll
+                for (int u = 0; u < LZ_AHEAD; ++u)
+                    if (c0 + 32 * u < n) {
+                        acc = fma(x[u], v[u], acc);
+                        acc2 = fma(y[u], v[u], acc2);
+                    }
+            }
+            for (int o = 16; o > 0; o >>= 1) {
+                acc += __shfl_xor_sync(0xffffffffu, acc, o);
+                acc2 += __shfl_xor_sync(0xffffffffu, acc2, o);
+            }
+            if (lane == 0) {
+                wq[r] = acc;
+                if (two) wq[r2] = acc2;
+            }
             part += acc * __ldcg(q + r);
+            if (two) part += acc2 * __ldcg(q + r2);
         }
         part = bsum(lane == 0 ? part : 0.0);
         if (tid == 0) share[gi] = part;
@@ -319,13 +347,20 @@ __device__ void sp2_bounds_group(const Sp2Job& jb, int G, int gi, Sync sync) {
         const double a = group_share_sum(share, G);
         // w <- w - a q - b_prev q_prev on own rows, the CTA's share of |w|^2
         part = 0.0;
-        for (int r = gi + warp * G; r < n; r += NW * G) {
-            if (lane == 0) {
-                const double x = __ldcg(wq + r) - a * __ldcg(q + r) - bprev * __ldcg(qp + r);
+        for (int r0 = gi + warp * G; r0 < n; r0 += 32 * NW * G) {  // a row per lane, summed in row order
+            const int r = r0 + lane * NW * G;
+            double x = 0.0;
+            if (r < n) {
+                x = __ldcg(wq + r) - a * __ldcg(q + r) - bprev * __ldcg(qp + r);
                 wq[r] = x;
-                part += x * x;
+            }
+            const int rows = min(32, (n - r0 + NW * G - 1) / (NW * G));
+            for (int k = 0; k < rows; ++k) {
+                const double xk = __shfl_sync(0xffffffffu, x, k);
+                part += xk * xk;
             }
         }
+        if (lane != 0) part = 0.0;
         part = bsum(part);
         if (tid == 0) share[G + gi] = part;
         sync();
@@ -337,8 +372,7 @@ __device__ void sp2_bounds_group(const Sp2Job& jb, int G, int gi, Sync sync) {
         m = j + 1;
         if (!(bnorm > 1e-12 * fmax(fabs(a), 1.0))) break;  // invariant subspace: T is exact (uniform)
         const double ib = 1.0 / bnorm;
-        for (int r = gi + warp * G; r < n; r += NW * G)
-            if (lane == 0) wq[r] = __ldcg(wq + r) * ib;
+        for (int r = gi + (warp + lane * NW) * G; r < n; r += 32 * NW * G) wq[r] = __ldcg(wq + r) * ib;
         bprev = bnorm;
         prv = cur;
         cur = nxt;
