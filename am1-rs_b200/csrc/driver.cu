@@ -634,14 +634,15 @@ long long vs_rows(const MolPlan& p) { return std::max<long long>(p.npad, ((p.nao
 // CTA's shared memory allow) always: alone the launch-per-step form of so small a matrix is all latency (methane 2.54
 // against 1.14 ms a solve; 192 gradients 45.2 against 44.5).  Only with kResPerSm channels per SM and more (a batch
 // of thousands) do the tiles fill the GPU as well (4096 molecules: 526.5-529.1 ms with tiles, 528.9-529.4 with one
-// launch), and the batch takes the tiles throughout.  Above FU_RES_MAX (to 448) while the whole batch's clusters are resident at once
+// launch), and the batch takes the tiles throughout.  Above FU_RES_MAX, to FU_CLU_MAX, while the whole batch's clusters are resident at once
 // (sp2_cluster_for); past that the tiles of the launch-per-step kernels fill the GPU, while a cluster's rate does not
 // grow with the batch (n = 384: 32 us a product on 16 SMs against 30 on 21 tiles' SMs plus 11 of update and launches).
+// FU_CLU_MAX is that kernel's own limit, a little below the cluster Jacobi's (choose_cluster).
 constexpr int kResPerSm = 4;
 constexpr int kResSmall = 72;  // two CTAs of k_sp2_res per SM up to here
 int sp2_fused_kind(const MolPlan& p) {
     if (density_mode() != 0 || p.cluster <= 0 || fp64_oz_for(p.nao) || p.nao < 1) return FU_NONE;
-    return p.nao <= FU_RES_MAX ? FU_RES : FU_CLU;
+    return p.nao <= FU_RES_MAX ? FU_RES : p.nao <= FU_CLU_MAX ? FU_CLU : FU_NONE;
 }
 int sp2_cluster_for(int channels) { return channels < 1 ? 0 : channels <= 8 ? 16 : channels <= 16 ? 8 : 0; }
 

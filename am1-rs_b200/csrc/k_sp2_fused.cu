@@ -4,7 +4,7 @@
 // a small matrix anywhere, is bound by latency there: a product of a few microseconds, an update of as
 // many, and the gaps between launches, 12 to 20 times per SCF iteration.  Here the loop stays on chip:
 //   k_sp2_res  one CTA per matrix of up to FU_RES_MAX orbitals, both iterates in shared memory
-//   k_sp2_clu  one cluster per matrix of up to 448 orbitals, the iterates in L2 (scratch rows padded to 32),
+//   k_sp2_clu  one cluster per matrix of up to FU_CLU_MAX orbitals, the iterates in L2 (scratch rows padded to 32),
 //              32-row panels fetched by cp.async; one cluster barrier per product
 // The products are DMMA m16n8k8 blocks over ascending k, and every sum (Lanczos dots, start, tile sums) is
 // taken in the order of the launch-per-step kernels, whose unit is the 32 x 32 quarter of a 64 x 64 tile,
@@ -35,10 +35,8 @@ constexpr int FU_LD = FU_KC + 4;  // its row stride in shared memory (conflict-f
 constexpr int FU_STAGES = 4, FU_PANEL = 32 * FU_LD, FU_STAGE = 2 * FU_PANEL;  // per group of four warps: rows R and columns C
 constexpr int FU_GROUPS = FU_WARPS / 4;
 
-__host__ __device__ inline int fu_tiles(int n) {
-    const int t = (n + 63) / 64;
-    return t * (t + 1) / 2;
-}
+__host__ __device__ constexpr int fu_tiles(int n) { return (n + 63) / 64 * ((n + 63) / 64 + 1) / 2; }
+static_assert(FU_RES_MAX <= FU_CLU_MAX && fu_tiles(FU_CLU_MAX) <= 32, "a lane per tile in the update");
 __host__ __device__ inline int fu_res_ld(int n) { return ((n + 7) & ~7) + 4; }
 __host__ __device__ inline int fu_clu_ld(int n) { return (n + FU_KC - 1) / FU_KC * FU_KC; }
 // doubles of the two scratch iterates of a k_sp2_clu channel: rows padded to 32, columns to whole chunks
@@ -122,6 +120,7 @@ __device__ __forceinline__ void sp2_fused_body(const Sp2Job* __restrict__ jobs, 
     __shared__ double red[16], gred[2][FU_WARPS], alpha[SP2_LANCZOS], beta[SP2_LANCZOS], ritz[2], comp[2];
     __shared__ double chain[FU_GROUPS][32][2];
     __shared__ unsigned short item[128];  // res: 16 x 16 sub-blocks; clu: quarters (R, C)
+    static_assert((FU_CLU_MAX + 31) / 32 * ((FU_CLU_MAX + 31) / 32 + 1) / 2 <= 128, "item holds every quarter");
     __shared__ int nitem;
     int C = 1, crank = 0;
     if constexpr (!RES) {

@@ -268,6 +268,7 @@ __global__ void k_sp2_update_cond(const Sp2Job* jobs, Sp2State* sst, int njobs, 
 // one whole FP64 purification per channel job of list[] (k_sp2_res: grid count; k_sp2_clu: grid (C, count) in
 // clusters of C CTAs), sp2_fused_smem_bytes(largest n, res) of dynamic shared memory, 256 threads
 constexpr int FU_RES_MAX = 112;
+constexpr int FU_CLU_MAX = 448;  // its update sums a 64 x 64 tile per lane of a warp: at most 32 tiles
 __global__ void k_sp2_res(const Sp2Job* jobs, const int* list, Sp2State* sst, const MolState* st, int* need_eigen, double* work, int max_steps);
 __global__ void k_sp2_clu(const Sp2Job* jobs, const int* list, Sp2State* sst, const MolState* st, int* need_eigen, double* work, int max_steps);
 size_t sp2_fused_smem_bytes(int n, bool res);
