@@ -144,6 +144,7 @@ struct DeviceCtx {
     int jacobi_smem = 0;  // dynamic shared memory available to one eigensolver CTA
     int tridiag_smem = 0;  // ... and to one tridiagonalisation CTA
     int sp2b_grid = 0;     // CTAs of the grid-wide Lanczos bounds (all co-resident)
+    int clu_resident[2] = {0, 0};  // clusters of 16 and of 8 CTAs of k_sp2_clu that are resident at once
 };
 
 // Shared-memory budgets the planner sizes eigensolver and tridiagonalisation clusters for (set
@@ -152,6 +153,7 @@ int g_jacobi_budget = 232448 - 1024;
 int g_tridiag_budget = 232448 - 1024;
 int g_sp2b_grid = 148;  // CTAs of the grid-wide Lanczos bounds (set when a device is opened)
 int g_sms = 148;        // SMs of the current device
+int g_clu_resident[2] = {7, 15};  // DeviceCtx::clu_resident of the current device
 
 // Smallest cluster (1, 2, 4, 8, 16 CTAs) whose row share of an n x n matrix fits one CTA's
 // shared memory; 0 when none does.
@@ -174,6 +176,22 @@ int tridiag_cluster(int n) {
     for (int C = 1; C <= 16; C *= 2)
         if (tridiag_smem_bytes(n, C) <= (size_t)g_tridiag_budget) return C;
     return 0;
+}
+
+// A launch of `count` clusters of C CTAs along x (grid (C, count)); attr holds the cluster's shape.
+cudaLaunchConfig_t cluster_config(int C, int count, int threads, size_t smem, cudaStream_t s, cudaLaunchAttribute attr[1]) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(C, count, 1);
+    cfg.blockDim = dim3(threads, 1, 1);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = C;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cfg;
 }
 
 DeviceCtx g_dev[64];
@@ -248,6 +266,13 @@ int device_ctx(DeviceCtx** out) {
         }
         if ((err = cudaFuncSetAttribute(k_sp2_clu, cudaFuncAttributeNonPortableClusterSizeAllowed, 1)) != cudaSuccess)
             return bad("one-launch purification cluster attribute", err);
+        for (int k = 0; k < 2; ++k) {
+            const int C = k == 0 ? 16 : 8;
+            cudaLaunchAttribute at[1];
+            cudaLaunchConfig_t cfg = cluster_config(C, 1, 256, sp2_fused_smem_bytes(FU_CLU_MAX, false), nullptr, at);
+            if ((err = cudaOccupancyMaxActiveClusters(&c.clu_resident[k], k_sp2_clu, &cfg)) != cudaSuccess)
+                return bad("one-launch purification occupancy", err);
+        }
         for (const void* f : {(const void*)k_sp2_step_tma, (const void*)k_commutator_tma})
             if ((err = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dgemm_tma_smem_bytes())) != cudaSuccess)
                 return bad("tensor-map tile kernel smem attribute", err);
@@ -281,6 +306,7 @@ int device_ctx(DeviceCtx** out) {
     g_tridiag_budget = c.tridiag_smem;
     g_sms = c.sms;
     g_sp2b_grid = c.sp2b_grid;
+    std::copy(c.clu_resident, c.clu_resident + 2, g_clu_resident);
     *out = &c;
     return AM1GPU_OK;
 }
@@ -630,25 +656,71 @@ struct MolPlan {
 // mixed path's two FP32 iterates of n rows of (n rounded up to 4) floats plus 16-byte alignment.
 long long vs_rows(const MolPlan& p) { return std::max<long long>(p.npad, ((p.nao + 3) & ~3) + 2); }
 
+// Largest molecule (orbitals) the purification path takes: the Lanczos bounds and the bisection hold
+// 3 n and 2 n doubles in one CTA's shared memory.
+constexpr int kMaxAo = 8192;
+
 // Which channels purify in one launch (k_sp2_fused.cu).  Up to FU_RES_MAX orbitals (what two iterates in one
 // CTA's shared memory allow) always: alone the launch-per-step form of so small a matrix is all latency (methane 2.54
 // against 1.14 ms a solve; 192 gradients 45.2 against 44.5).  Only with kResPerSm channels per SM and more (a batch
 // of thousands) do the tiles fill the GPU as well (4096 molecules: 526.5-529.1 ms with tiles, 528.9-529.4 with one
-// launch), and the batch takes the tiles throughout.  Above FU_RES_MAX, to FU_CLU_MAX, while the whole batch's clusters are resident at once
-// (sp2_cluster_for); past that the tiles of the launch-per-step kernels fill the GPU, while a cluster's rate does not
-// grow with the batch (n = 384: 32 us a product on 16 SMs against 30 on 21 tiles' SMs plus 11 of update and launches).
-// FU_CLU_MAX is that kernel's own limit, a little below the cluster Jacobi's (choose_cluster).
+// launch), and the batch takes the tiles throughout.  Above FU_RES_MAX, to FU_CLU_MAX (that kernel's own limit, a little
+// below the cluster Jacobi's): sp2_cluster_for.
 constexpr int kResPerSm = 4;
 constexpr int kResSmall = 72;  // two CTAs of k_sp2_res per SM up to here
 int sp2_fused_kind(const MolPlan& p) {
     if (density_mode() != 0 || p.cluster <= 0 || fp64_oz_for(p.nao) || p.nao < 1) return FU_NONE;
     return p.nao <= FU_RES_MAX ? FU_RES : p.nao <= FU_CLU_MAX ? FU_CLU : FU_NONE;
 }
-int sp2_cluster_for(int channels) { return channels < 1 ? 0 : channels <= 8 ? 16 : channels <= 16 ? 8 : 0; }
-
-// Largest molecule (orbitals) the purification path takes: the Lanczos bounds and the bisection hold
-// 3 n and 2 n doubles in one CTA's shared memory.
-constexpr int kMaxAo = 8192;
+// CTAs of the cluster in which each of a batch's channels `clu` (their orders, FU_RES_MAX < n <= FU_CLU_MAX) purifies, 0
+// for the tiles of the launch-per-step kernels, which the channels `tiled` take anyway.  Up to as many channels as are
+// resident in clusters of 16 at once (7 on a B200): those (2.1 times the tiles' solve at 114 orbitals, 1.9 at 192, 1.13
+// at 384, 0.97 to 1 at 445).  To 16 channels: whichever is estimated least of two or more waves of them, of clusters of 8 (15
+// resident) and of the tiles.  The microseconds of a purification are fitted to solves of 1 to 16 equal molecules of
+// 114 to 445 orbitals forced to each form, and the choice checked on 90 mixed batches (0.1% over the best on average, 3% at most):
+// a cluster takes its quarters in turns of two a CTA, 16 us per 32 columns of a turn; the tiles a launch's
+// latency and their longest k-loop, again for every further tile an SM gets (8 x 288 orbitals 10.1, 8.7 and 9.9 ms a
+// solve in clusters of 16, of 8 and as tiles, 8 x 384 16.9, 15.3, 14.1, 16 x 444 36, 41, 26).  More channels: the tiles, whose
+// rate grows with the batch.
+int sp2_cluster_for(std::vector<int> clu, const std::vector<int>& tiled) {
+    const int count = (int)clu.size();
+    if (count < 1 || count > 16) return 0;
+    if (count <= g_clu_resident[0]) return 16;
+    std::sort(clu.begin(), clu.end(), std::greater<int>());
+    auto clusters_us = [&](int C, int resident) {  // largest first, each where a place is free first
+        std::vector<double> place(resident, 0.0);
+        for (int n : clu) {
+            const int q = (n + 31) / 32, turns = (q * (q + 1) / 2 + 2 * C - 1) / (2 * C);
+            *std::min_element(place.begin(), place.end()) += 50.0 + (C == 16 ? 15.5 : 16.5) * q * turns;
+        }
+        return *std::max_element(place.begin(), place.end());
+    };
+    auto tiles_us = [](std::initializer_list<const std::vector<int>*> lists) {
+        int tiles = 0, nmax = 0, nmin = kMaxAo;
+        for (const auto* l : lists)
+            for (int n : *l) {
+                const int t = (n + 63) / 64;
+                tiles += t * (t + 1) / 2;
+                nmax = std::max(nmax, n);
+                nmin = std::min(nmin, n);
+            }
+        const int per_sm = (tiles + g_sms - 1) / g_sms;
+        const double products = nmax > 1.05 * nmin ? 17.0 : 15.2;  // as many as the channel that needs most
+        return tiles ? products * (12.0 + nmax * (0.105 + 0.034 * (per_sm - 1))) : 0.0;
+    };
+    int best = 0;
+    double least = tiles_us({&clu, &tiled});
+    for (int k = 0; k < 2; ++k) {
+        const int C = k == 0 ? 16 : 8, resident = g_clu_resident[k];
+        if (resident < 1) continue;
+        const double us = std::max(clusters_us(C, resident), tiles_us({&tiled}));
+        if (us < least) {
+            least = us;
+            best = C;
+        }
+    }
+    return best;
+}
 
 int choose_cluster(int n, int* npad_out, int* c_out) {
     static const int cs[5] = {1, 2, 4, 8, 16};
@@ -884,16 +956,18 @@ int build_batch(const am1gpu_molecule* in, const am1gpu_options& o, std::vector<
             dq_bytes += p.nch * (2LL * kOzPlanes * p.nao * oz_ldq(p.nao) + 256);
         }
     }
-    // clusters of the one-launch purification: only while every such channel's cluster is resident at once
-    int clu_jobs = 0, res_jobs = 0;
+    // the one-launch purifications of the batch
+    int res_jobs = 0;
     long long clu_doubles = 0;
+    std::vector<int> clu_orders, tiled_orders;
     for (auto& p : b.plans) {
         const int kind = sp2_fused_kind(p);
-        clu_jobs += kind == FU_CLU ? p.nch : 0;
         res_jobs += kind == FU_RES ? p.nch : 0;
+        if (kind != FU_RES)
+            for (int c = 0; c < p.nch; ++c) (kind == FU_CLU ? clu_orders : tiled_orders).push_back(p.nao);
     }
     const bool one_launch = res_jobs <= kResPerSm * g_sms;
-    const int clu_size = one_launch ? sp2_cluster_for(clu_jobs) : 0;
+    const int clu_size = one_launch ? sp2_cluster_for(clu_orders, tiled_orders) : 0;
     if (clu_size)
         for (auto& p : b.plans)
             if (sp2_fused_kind(p) == FU_CLU) clu_doubles += p.nch * sp2_clu_doubles(p.nao);
@@ -1508,18 +1582,8 @@ int big_split(int count, NOf n_of) {
 int big_launches(int grid_count, int count) { return grid_count + (count > grid_count ? 1 : 0); }
 
 cudaError_t launch_clusters(const void* f, int C, int count, int threads, size_t smem, cudaStream_t s, void** args) {
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(C, count, 1);
-    cfg.blockDim = dim3(threads, 1, 1);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = s;
     cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = C;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    const cudaLaunchConfig_t cfg = cluster_config(C, count, threads, smem, s, attr);
     return cudaLaunchKernelExC(&cfg, f, args);
 }
 
@@ -3091,7 +3155,7 @@ int density_purify_one(int n, const double* F, double nocc, double weight, int p
             CK(cudaGetLastError());
         } else {
             void* args[] = {&dj, &list, &dsst, &dms, &need, &work, &max_steps};
-            CK(launch_clusters((const void*)k_sp2_clu, sp2_cluster_for(1), 1, 256, smem, s, args));
+            CK(launch_clusters((const void*)k_sp2_clu, 16, 1, 256, smem, s, args));
         }
     } else {
         k_sp2_bounds<<<1, 512, 3 * sizeof(double) * n, s>>>(dj, dms);
