@@ -3295,12 +3295,12 @@ int jacobi_eigen_small(std::vector<SmallEig>& items, Mem& mem) {
         for (int k = k0; k < k0 + cnt; ++k) std::memcpy(H + o_a[k], items[k].a, sizeof(double) * items[k].n * items[k].n);
         CK(cudaMemcpyAsync(D + gr.in0, H + gr.in0, gr.in1 - gr.in0, cudaMemcpyHostToDevice, s));
         const unsigned tiles = cdiv(gr.nmax, 32);
-        k_eig_mirror<<<dim3(tiles, tiles, cnt), dim3(32, 8), 0, s>>>(dp + k0, bad + k0);
-        k_eig_rowmin<<<dim3(cdiv(gr.nmax, 128), cnt), 128, 0, s>>>(dp + k0);
+        k_eig_mirror<<<dim3(cnt, tiles, tiles), dim3(32, 8), 0, s>>>(dp + k0, bad + k0);
+        k_eig_rowmin<<<dim3(cnt, cdiv(gr.nmax, 128)), 128, 0, s>>>(dp + k0);
         CK(cudaGetLastError());
         if (int r = launch_jacobi_bucket(gr.bk, dj, (const MolState*)(D + o_st), status, 1, nullptr, s)) return r;
         k_eig_sort<<<cnt, 512, 0, s>>>(dj + k0, (const MolState*)(D + o_st), 1, nullptr);
-        k_eig_columns<<<dim3(tiles, tiles, cnt), dim3(32, 8), 0, s>>>(dp + k0);
+        k_eig_columns<<<dim3(cnt, tiles, tiles), dim3(32, 8), 0, s>>>(dp + k0);
         CK(cudaGetLastError());
         CK(cudaMemcpyAsync(H + gr.out0, D + gr.out0, gr.out1 - gr.out0, cudaMemcpyDeviceToHost, s));
         CK(cudaMemcpyAsync(H + o_code + sizeof(int) * k0, bad + k0, sizeof(int) * cnt, cudaMemcpyDeviceToHost, s));

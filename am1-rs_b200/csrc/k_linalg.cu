@@ -439,11 +439,12 @@ __global__ void __launch_bounds__(512) k_eig_sort(const EigJob* __restrict__ job
 // ---------------------------------------------------------------------------------------
 // Caller's matrices to the eigensolver's inputs, and its vectors back to columns
 // ---------------------------------------------------------------------------------------
-// 32 x 32 tiles through shared memory, each element read and written in runs of 32: bound by memory.
+// 32 x 32 tiles through shared memory, each element read and written in runs of 32: bound by memory.  The matrix is
+// the grid's x, the only extent that takes more than 65535 of them.
 __global__ void __launch_bounds__(256) k_eig_mirror(const EigPrep* __restrict__ prep, int* __restrict__ bad) {
     __shared__ double t[32][33];
-    const EigPrep p = prep[blockIdx.z];
-    const int n = p.n, bx = blockIdx.x, by = blockIdx.y;
+    const EigPrep p = prep[blockIdx.x];
+    const int n = p.n, bx = blockIdx.y, by = blockIdx.z;
     if (32 * by >= n || bx > by) return;  // tiles of the lower triangle
     const int x = threadIdx.x;
     bool fin = true;
@@ -469,13 +470,13 @@ __global__ void __launch_bounds__(256) k_eig_mirror(const EigPrep* __restrict__ 
             p.ct[(size_t)rt * n + ct] = 0.0;
         }
     }
-    if (__syncthreads_or(!fin) && threadIdx.x == 0 && threadIdx.y == 0) bad[blockIdx.z] = 1;
+    if (__syncthreads_or(!fin) && threadIdx.x == 0 && threadIdx.y == 0) bad[blockIdx.x] = 1;
 }
 
 // A thread per row; column by column of the symmetric matrix, so a warp reads 32 consecutive words.
 __global__ void __launch_bounds__(128) k_eig_rowmin(const EigPrep* __restrict__ prep) {
-    const EigPrep p = prep[blockIdx.y];
-    const int n = p.n, r = blockIdx.x * 128 + threadIdx.x;
+    const EigPrep p = prep[blockIdx.x];
+    const int n = p.n, r = blockIdx.y * 128 + threadIdx.x;
     if (r >= n) return;
     double bound = 0.0;
     for (int c0 = 0; c0 < n; c0 += 16) {
@@ -491,8 +492,8 @@ __global__ void __launch_bounds__(128) k_eig_rowmin(const EigPrep* __restrict__ 
 
 __global__ void __launch_bounds__(256) k_eig_columns(const EigPrep* __restrict__ prep) {
     __shared__ double t[32][33];
-    const EigPrep p = prep[blockIdx.z];
-    const int n = p.n, r0 = 32 * blockIdx.y, c0 = 32 * blockIdx.x, x = threadIdx.x;
+    const EigPrep p = prep[blockIdx.x];
+    const int n = p.n, r0 = 32 * blockIdx.z, c0 = 32 * blockIdx.y, x = threadIdx.x;
     if (r0 >= n || c0 >= n) return;
     for (int y = threadIdx.y; y < 32; y += 8)
         if (r0 + y < n && c0 + x < n) t[y][x] = p.ct[(size_t)(r0 + y) * n + c0 + x];

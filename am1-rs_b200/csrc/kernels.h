@@ -200,8 +200,8 @@ __global__ void k_gemm_tn(const GemmJob* jobs, const GemmTile* tiles, int ntiles
 __global__ void k_jacobi(const EigJob* jobs, const MolState* st, int* mol_status, int force, const int* mask);
 // The inputs of k_jacobi from count matrices in the caller's order (one EigPrep each): Gt the matrix with its
 // lower triangle mirrored, Ct the identity, rowmin the Gershgorin row minima (each row's sum over ascending
-// columns); bad[i] is set when matrix i has an element that is not finite.  k_eig_mirror: grid (ceil(nmax / 32),
-// ceil(nmax / 32), count), block (32, 8); then k_eig_rowmin: grid (ceil(nmax / 128), count), 128 threads.
+// columns); bad[i] is set when matrix i has an element that is not finite.  k_eig_mirror: grid (count,
+// ceil(nmax / 32), ceil(nmax / 32)), block (32, 8); then k_eig_rowmin: grid (count, ceil(nmax / 128)), 128 threads.
 // k_eig_columns: v = Ct_out transposed, the eigenvectors as columns (grid and block of k_eig_mirror).
 struct EigPrep {
     const double* a;  // n x n as the caller holds it (its lower triangle is read)
