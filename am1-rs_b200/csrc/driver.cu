@@ -3436,38 +3436,47 @@ int symmetric_eigen_batch(int count, const int32_t* ns, const double* const* a, 
             first_msg = msg;
         }
     };
-    DeviceCtx* ctx = nullptr;
     std::vector<SmallEig> items;
     std::vector<int> large;
-    std::vector<std::pair<int, std::string>> refused(std::max(count, 0), {AM1GPU_OK, std::string()});
-    for (int i = 0; i < count; ++i) {
-        const int n = ns[i];
-        if (n < 0 || (n > 0 && (!a[i] || !w[i] || !v[i]))) {
-            refused[i] = {AM1GPU_INVALID_INPUT, ": null argument or negative size"};
-            continue;
-        }
-        if (n == 0) continue;
-        if (!ctx)
-            if (const int rc = device_ctx(&ctx)) return rc;
-        SmallEig it{i, n, 0, 0, a[i], w[i], v[i]};
-        if (choose_cluster(n, &it.npad, &it.C)) {
-            items.push_back(it);
-            continue;
-        }
+    std::vector<std::pair<int, std::string>> refused(count, {AM1GPU_OK, std::string()});
+    auto refuse_large = [&](int i) {  // what the device does not check
         bool finite = true;
-        for (long long k = 0; k < (long long)n * n && finite; ++k) finite = std::isfinite(a[i][k]);
+        for (long long k = 0; k < (long long)ns[i] * ns[i] && finite; ++k) finite = std::isfinite(a[i][k]);
         if (!finite)
             refused[i] = {AM1GPU_LINALG, " handed to the eigensolver is not finite"};
-        else if (n > kMaxAo)
+        else if (ns[i] > kMaxAo)
             refused[i] = {AM1GPU_UNSUPPORTED, " has more than " + std::to_string(kMaxAo) + " rows"};
+        return refused[i].first != AM1GPU_OK;
+    };
+    // a device that fails: every matrix' code is still whether it is refused
+    auto device_failed = [&](int rc) {
+        for (int i = 0; i < count && status; ++i) {
+            if (!refused[i].first && ns[i] > 0) refuse_large(i);
+            status[i] = refused[i].first;
+        }
+        return rc;
+    };
+    bool any = false;
+    for (int i = 0; i < count; ++i) {
+        if (ns[i] < 0 || (ns[i] > 0 && (!a[i] || !w[i] || !v[i])))
+            refused[i] = {AM1GPU_INVALID_INPUT, ": null argument or negative size"};
         else
-            large.push_back(i);  // past the cluster Jacobi: the large-matrix path, one at a time, after the batch
+            any |= ns[i] > 0;
+    }
+    DeviceCtx* ctx;
+    if (any)
+        if (const int rc = device_ctx(&ctx)) return device_failed(rc);
+    for (int i = 0; i < count; ++i) {
+        if (ns[i] == 0 || refused[i].first) continue;
+        SmallEig it{i, ns[i], 0, 0, a[i], w[i], v[i]};
+        if (choose_cluster(ns[i], &it.npad, &it.C)) items.push_back(it);
+        else if (!refuse_large(i)) large.push_back(i);  // past the cluster Jacobi: the large-matrix path, one at a time, after the batch
     }
     if (!items.empty()) {
         Workspace* ws;
         int rc = workspace(&ws, 0, 0);
         if (!rc) rc = jacobi_eigen_small(items, *ws);
-        if (rc) return rc;
+        if (rc) return device_failed(rc);
         for (const SmallEig& it : items)
             if (it.bad) refused[it.i] = {AM1GPU_LINALG, " handed to the eigensolver is not finite"};
     }
