@@ -3229,17 +3229,18 @@ int jacobi_eigen_small(std::vector<SmallEig>& items, Mem& mem) {
         off += bytes;
         return o2;
     };
-    // staged: records, then the matrices; fetched: two codes per matrix, then w and v; device only: the rest
+    // staged: records, then the matrices (mirrored in place, Gt); fetched: two codes per matrix, then w and v (npad rows of n,
+    // which hold the eigensolver's Vs before); device only: the rest.  Three matrices' room each on the device.
     const size_t o_job = take(sizeof(EigJob) * m), o_prep = take(sizeof(EigPrep) * m), o_st = take(sizeof(MolState) * m),
                  records = align256(off);
     std::vector<size_t> o_a(m), o_out(m), o_dev(m);
     for (int k = 0; k < m; ++k) o_a[k] = take(sizeof(double) * items[k].n * items[k].n);
     const size_t o_code = take(sizeof(int) * 2 * m);
-    for (int k = 0; k < m; ++k) o_out[k] = take(sizeof(double) * ((size_t)items[k].n * items[k].n + items[k].n));
+    for (int k = 0; k < m; ++k) o_out[k] = take(sizeof(double) * ((size_t)items[k].n * items[k].npad + items[k].n));
     const size_t host_bytes = align256(off);
     for (int k = 0; k < m; ++k) {
         const size_t n = items[k].n, np = items[k].npad;
-        o_dev[k] = take(sizeof(double) * (2 * n * n + np * n + 2 * np + n));  // Gt, Ct, Vs, lam, column ids, rowmin
+        o_dev[k] = take(sizeof(double) * (n * n + 2 * np + n));  // Ct, lam, column ids, rowmin
     }
     int rc = mem_ensure(mem, align256(off), host_bytes);
     if (rc) return rc;
@@ -3251,10 +3252,12 @@ int jacobi_eigen_small(std::vector<SmallEig>& items, Mem& mem) {
     for (int k = 0; k < m; ++k) {
         const SmallEig& it = items[k];
         const size_t n = it.n, np = it.npad;
-        double* gt = (double*)(D + o_dev[k]);
-        double *ct = gt + n * n, *vs = ct + n * n, *lam = vs + np * n, *ids = lam + np, *rmin = ids + np;
+        double* gt = (double*)(D + o_a[k]);
+        double* ct = (double*)(D + o_dev[k]);
+        double *lam = ct + n * n, *ids = lam + np, *rmin = ids + np;
         double* out = (double*)(D + o_out[k]);
-        hp[k] = EigPrep{(const double*)(D + o_a[k]), gt, ct, rmin, out + n, it.n};
+        double* vs = out + n;
+        hp[k] = EigPrep{gt, ct, rmin, vs, it.n};
         hj[k] = EigJob{};
         hj[k].Gt = gt;
         hj[k].Ct = ct;
@@ -3274,7 +3277,7 @@ int jacobi_eigen_small(std::vector<SmallEig>& items, Mem& mem) {
         gr.bk.add(it.n, it.npad);
         gr.nmax = std::max(gr.nmax, it.n);
         gr.in1 = o_a[k] + sizeof(double) * n * n;
-        gr.out1 = o_out[k] + sizeof(double) * (n * n + n);
+        gr.out1 = o_out[k] + sizeof(double) * (n * np + n);
     }
     while (mem.pipes.size() < groups.size()) {
         cudaStream_t q;

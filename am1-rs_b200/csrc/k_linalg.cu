@@ -439,7 +439,8 @@ __global__ void __launch_bounds__(512) k_eig_sort(const EigJob* __restrict__ job
 // ---------------------------------------------------------------------------------------
 // Caller's matrices to the eigensolver's inputs, and its vectors back to columns
 // ---------------------------------------------------------------------------------------
-// 32 x 32 tiles through shared memory, each element read and written in runs of 32: bound by memory.  The matrix is
+// 32 x 32 tiles through shared memory, each element read and written in runs of 32: bound by memory.  A CTA reads
+// and writes one tile and its mirror, so k_eig_mirror works in place.  The matrix is
 // the grid's x, the only extent that takes more than 65535 of them.
 __global__ void __launch_bounds__(256) k_eig_mirror(const EigPrep* __restrict__ prep, int* __restrict__ bad) {
     __shared__ double t[32][33];
@@ -451,9 +452,9 @@ __global__ void __launch_bounds__(256) k_eig_mirror(const EigPrep* __restrict__ 
     for (int y = threadIdx.y; y < 32; y += 8) {
         const int r = 32 * by + y, c = 32 * bx + x, ru = 32 * bx + y, cu = 32 * by + x;
         double v = 0.0;
-        if (r < n && c < n) v = p.a[(size_t)r * n + c];
+        if (r < n && c < n) v = p.gt[(size_t)r * n + c];
         fin = fin && isfinite(v);
-        if (bx < by && ru < n && cu < n) fin = fin && isfinite(p.a[(size_t)ru * n + cu]);  // the unread triangle too
+        if (bx < by && ru < n && cu < n) fin = fin && isfinite(p.gt[(size_t)ru * n + cu]);  // the unread triangle too
         t[y][x] = v;
     }
     __syncthreads();

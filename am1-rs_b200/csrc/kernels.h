@@ -198,13 +198,12 @@ __global__ void k_permute_square(const double* in, long long si, double* out, lo
 __global__ void k_gemm_nn(const GemmJob* jobs, const GemmTile* tiles, int ntiles, const MolState* st, int force, const int* mask);
 __global__ void k_gemm_tn(const GemmJob* jobs, const GemmTile* tiles, int ntiles, const MolState* st, int force, const int* mask);
 __global__ void k_jacobi(const EigJob* jobs, const MolState* st, int* mol_status, int force, const int* mask);
-// The inputs of k_jacobi from count matrices in the caller's order (one EigPrep each): Gt the matrix with its
-// lower triangle mirrored, Ct the identity, rowmin the Gershgorin row minima (each row's sum over ascending
+// The inputs of k_jacobi from count matrices (one EigPrep each): Gt, which holds the caller's matrix, gets its
+// lower triangle mirrored, Ct becomes the identity, rowmin the Gershgorin row minima (each row's sum over ascending
 // columns); bad[i] is set when matrix i has an element that is not finite.  k_eig_mirror: grid (count,
 // ceil(nmax / 32), ceil(nmax / 32)), block (32, 8); then k_eig_rowmin: grid (count, ceil(nmax / 128)), 128 threads.
 // k_eig_columns: v = Ct_out transposed, the eigenvectors as columns (grid and block of k_eig_mirror).
 struct EigPrep {
-    const double* a;  // n x n as the caller holds it (its lower triangle is read)
     double *gt, *ct, *rowmin, *v;
     int n;
 };
