@@ -126,12 +126,12 @@ __device__ __forceinline__ int rotate_pair(double* __restrict__ gp, double* __re
     al = warp_sum(al);
     be = warp_sum(be);
     ga = warp_sum(ga);
-    // the angle beside the test, not behind it: both are chains of square roots and divisions
-    const double thr = tol * sqrt(al * be);
+    // The test first: the angle beside its square root shortens the chain of a pair that rotates, but costs every
+    // pair that does not more than that (64 rows 1069 us so, 1124 with the first division alone beside the test)
+    if (!(fabs(ga) > tol * sqrt(al * be)) || al == 0.0 || be == 0.0) return 0;
     const double zeta = (be - al) / (2.0 * ga);
     const double tt = copysign(1.0, zeta) / (fabs(zeta) + sqrt(1.0 + zeta * zeta));
     const double c = 1.0 / sqrt(1.0 + tt * tt), s = c * tt;
-    if (!(fabs(ga) > thr) || al == 0.0 || be == 0.0) return 0;
     for (int i = lane; i < n; i += 32) {
         const double x = gp[i], y = gq[i];
         gp[i] = c * x - s * y;
