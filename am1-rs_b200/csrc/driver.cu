@@ -3212,6 +3212,10 @@ struct SmallEig {
 // there, and fetched, so one group's copies and host staging run under the others' solves and the groups share the
 // SMs.  One group after the other on one stream, prepared and transposed on the host, took 94 ms for 96
 // matrices of 24 to 320 rows; now 30.
+// Up to kEigHostElements elements in all, the host prepares and transposes after all, with one copy each way on the one
+// stream: three small kernels, an event and four more copies cost more than they save (2 matrices of 5 rows 104 us
+// on the device, 83 so, 10 of 40 668 and 655; 80 of 16, past the line, 705 and 710).
+constexpr size_t kEigHostElements = 16000;
 int jacobi_eigen_small(std::vector<SmallEig>& items, Mem& mem) {
     if (items.empty()) return AM1GPU_OK;
     std::stable_sort(items.begin(), items.end(), [](const SmallEig& x, const SmallEig& y) { return x.C != y.C ? x.C > y.C : x.n > y.n; });
@@ -3242,9 +3246,13 @@ int jacobi_eigen_small(std::vector<SmallEig>& items, Mem& mem) {
         const size_t n = items[k].n, np = items[k].npad;
         o_dev[k] = take(sizeof(double) * (n * n + 2 * np + n));  // Ct, lam, column ids, rowmin
     }
-    int rc = mem_ensure(mem, align256(off), host_bytes);
+    // few elements: prepared and transposed on the host, everything in one copy each way
+    size_t elements = 0;
+    for (const SmallEig& it : items) elements += (size_t)it.n * it.n;
+    const bool on_host = elements <= kEigHostElements;
+    int rc = mem_ensure(mem, align256(off), on_host ? align256(off) : host_bytes);
     if (rc) return rc;
-    if ((rc = mem_side_stream(mem))) return rc;
+    if (!on_host && (rc = mem_side_stream(mem))) return rc;
     char *D = mem.dpool, *H = mem.hpin;
     EigJob* hj = (EigJob*)(H + o_job);
     EigPrep* hp = (EigPrep*)(H + o_prep);
@@ -3279,14 +3287,57 @@ int jacobi_eigen_small(std::vector<SmallEig>& items, Mem& mem) {
         gr.in1 = o_a[k] + sizeof(double) * n * n;
         gr.out1 = o_out[k] + sizeof(double) * (n * np + n);
     }
+    const EigJob* dj = (const EigJob*)(D + o_job);
+    const EigPrep* dp = (const EigPrep*)(D + o_prep);
+    int *bad = (int*)(D + o_code), *status = bad + m;
+    if (on_host) {
+        int* code = (int*)(H + o_code);
+        for (int k = 0; k < m; ++k) {
+            const SmallEig& it = items[k];
+            const int n = it.n;
+            double *g = (double*)(H + o_a[k]), *c = (double*)(H + o_dev[k]), *rmin = c + (size_t)n * n + 2 * it.npad;
+            bool finite = true;
+            for (int i = 0; i < n; ++i) {
+                double bound = 0.0;
+                for (int j = 0; j < n; ++j) {
+                    const double x = i >= j ? it.a[(size_t)i * n + j] : it.a[(size_t)j * n + i];  // lower triangle
+                    finite = finite && std::isfinite(it.a[(size_t)i * n + j]);
+                    g[(size_t)i * n + j] = x;
+                    c[(size_t)i * n + j] = i == j ? 1.0 : 0.0;
+                    if (i != j) bound += std::fabs(x);
+                }
+                rmin[i] = g[(size_t)i * n + i] - bound;
+            }
+            code[k] = !finite;
+            code[m + k] = 0;
+        }
+        CK(cudaMemcpyAsync(D, H, align256(off), cudaMemcpyHostToDevice, mem.stream));
+        for (const Group& gr : groups)
+            if ((rc = launch_jacobi_bucket(gr.bk, dj, (const MolState*)(D + o_st), status, 1, nullptr, mem.stream))) return rc;
+        k_eig_sort<<<m, 512, 0, mem.stream>>>(dj, (const MolState*)(D + o_st), 1, nullptr);
+        CK(cudaGetLastError());
+        CK(cudaMemcpyAsync(H + o_code, D + o_code, align256(off) - o_code, cudaMemcpyDeviceToHost, mem.stream));
+        CK(cudaStreamSynchronize(mem.stream));
+        for (int k = 0; k < m; ++k) {
+            SmallEig& it = items[k];
+            const int n = it.n;
+            it.bad = code[k] != 0;
+            if (it.bad || code[m + k]) {
+                it.code = AM1GPU_LINALG;
+                continue;
+            }
+            std::memcpy(it.w, H + o_out[k], sizeof(double) * n);
+            const double* ct = (const double*)(H + o_dev[k]);
+            for (int q = 0; q < n; ++q)
+                for (int i = 0; i < n; ++i) it.v[(size_t)i * n + q] = ct[(size_t)q * n + i];
+        }
+        return AM1GPU_OK;
+    }
     while (mem.pipes.size() < groups.size()) {
         cudaStream_t q;
         CK(cudaStreamCreateWithPriority(&q, cudaStreamNonBlocking, mem.priority));
         mem.pipes.push_back(q);
     }
-    const EigJob* dj = (const EigJob*)(D + o_job);
-    const EigPrep* dp = (const EigPrep*)(D + o_prep);
-    int *bad = (int*)(D + o_code), *status = bad + m;
     CK(cudaMemcpyAsync(D, H, records, cudaMemcpyHostToDevice, mem.stream));
     CK(cudaMemsetAsync(bad, 0, sizeof(int) * 2 * m, mem.stream));
     CK(cudaEventRecord(mem.fork, mem.stream));
