@@ -549,19 +549,19 @@ __global__ void k_bisect(const TriJob* __restrict__ jobs, const int* __restrict_
                 else h = mid;
                 mid = 0.5 * (l + h);
             }
-            const bool up = lane < 31 && mid > l && mid < h && sturm_count(de, n, mid) <= k;
-            const unsigned ball = __ballot_sync(0xffffffffu, up);
-            for (int step = 0, at = 1; step < 5; ++step) {
-                mid = 0.5 * (lo + hi);
-                if (!(mid > lo && mid < hi) || hi - lo <= 4.0 * 2.220446049250313e-16 * fmax(fabs(lo), fabs(hi))) {
-                    done = true;
-                    break;
-                }
-                const bool above = ball >> (at - 1) & 1;
-                if (above) lo = mid;
-                else hi = mid;
-                at = 2 * at + (above ? 1 : 0);
+            const bool halt = !(mid > l && mid < h) || h - l <= 4.0 * 2.220446049250313e-16 * fmax(fabs(l), fabs(h));
+            const bool up = lane < 31 && !halt && sturm_count(de, n, mid) <= k;
+            const unsigned halts = __ballot_sync(0xffffffffu, halt), ups = __ballot_sync(0xffffffffu, up);
+            // the steps, on the nodes' bits alone (each step's own arithmetic cost a matrix of 5 rows 5 of 45 us): to the
+            // node where bisection ends, or past the last of five
+            int at = 1, last = 1;
+            for (int step = 0; step < 5 && !done; ++step) {
+                done = halts >> (at - 1) & 1;
+                last = at;
+                at = 2 * at + (ups >> (at - 1) & 1);
             }
+            lo = __shfl_sync(0xffffffffu, !done && up ? mid : l, last - 1);
+            hi = __shfl_sync(0xffffffffu, done || up ? h : mid, last - 1);
         }
         if (lane == 0) jb.eps[k] = 0.5 * (lo + hi);
         return;
