@@ -2156,8 +2156,8 @@ int run_device(Batch& b, Mem& mem, const DevElem* dp, const am1gpu_options& o, a
     CK(cudaMemsetAsync(b.d_status, 0, sizeof(int) * b.nmol, s));
     CK(cudaMemsetAsync(b.d_work, 0, sizeof(double) * kWorkN, s));
     CK(cudaMemsetAsync(b.d_sp2_active, 0, 4 * sizeof(int), s));  // [2]: error word of the tensor-core steps
-    // P (zero) and the eigensolver's warm start (the identity); every other slot is written before it is read
-    k_slots_init<<<dim3(std::max(1u, cdiv(2LL * b.maxn * b.maxn, 16384)), (unsigned)b.jobs.size()), 256, 0, s>>>(b.d_jobs);
+    // F* and P (zero) and the eigensolver's warm start (the identity); every other slot is written before it is read
+    k_slots_init<<<dim3(std::max(1u, cdiv(3LL * b.maxn * b.maxn, 16384)), (unsigned)b.jobs.size()), 256, 0, s>>>(b.d_jobs);
     // mixed precision: every molecule starts with TF32 purification (k_converge ends that phase)
     const bool mixed = o.precision == AM1GPU_PRECISION_MIXED && density_mode() == 0;
     bool lowp_left = mixed;  // some molecule may still be in its TF32 phase

@@ -67,17 +67,18 @@ __global__ void k_state_init(MolState* __restrict__ st, const MolDesc* __restric
     st[i] = s;
 }
 
-// P = 0 (k_sad_init then sets its diagonal) and the eigensolver's warm start C^T = I, the two slots a run reads
-// before it writes them.  Bound by the writes; the whole arena, six slots and more a channel, was zeroed for these
-// two, and twice in a batched call (25 GB each time for 4096 molecules, 7 ms a call).
+// F* = 0 (what the final spectrum is of where no iteration formed one: none allowed, or an energy that is not finite in the
+// first), P = 0 (k_sad_init then sets its diagonal) and the eigensolver's warm start C^T = I: the three slots a run reads before
+// it writes them.  Bound by the writes; the whole arena, six slots and more a channel, was zeroed for these, and twice in a
+// batched call (25 GB each time for 4096 molecules, 7 ms a call).
 __global__ void __launch_bounds__(256) k_slots_init(const ChanJob* __restrict__ jobs) {
-    static_assert(SLOT_CT == SLOT_P + 1, "P and Ct adjacent");
+    static_assert(SLOT_P == SLOT_FX + 1 && SLOT_CT == SLOT_P + 1, "F*, P and Ct adjacent");
     const ChanJob& jb = jobs[blockIdx.y];
     const int n = jb.n;
-    double* P = jb.P;
+    double* X = jb.Fx;
     const long long nn = (long long)n * n;
-    for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < 2 * nn; i += (long long)gridDim.x * 256)
-        P[i] = i >= nn && (i - nn) % (n + 1) == 0 ? 1.0 : 0.0;
+    for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < 3 * nn; i += (long long)gridDim.x * 256)
+        X[i] = i >= 2 * nn && (i - 2 * nn) % (n + 1) == 0 ? 1.0 : 0.0;
 }
 
 __device__ __forceinline__ void live_slots(const MolState& s, int& newslot, unsigned& live_mask) {

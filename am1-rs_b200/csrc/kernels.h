@@ -431,7 +431,7 @@ __device__ __forceinline__ double group_share_sum(const double* share, int G) {
 
 __global__ void k_sad_init(const MolDesc* mols, const int* atom_mol, int natoms_total, const DevElem* params,
                            const int* atom_z, double* arena);
-// P = 0, Ct = I of every channel (adjacent slots); grid (any, channels)
+// F* = 0, P = 0, Ct = I of every channel (adjacent slots); grid (any, channels)
 __global__ void k_slots_init(const ChanJob* jobs);
 // largest open-shell molecule (orbitals) that takes the mixed path's TF32 phase
 constexpr int kLowpMaxOpenShellAo = 448;
