@@ -2715,6 +2715,7 @@ int g_matrix_batch(const am1gpu_molecule* mol, int method, int nrhs, const doubl
     rc = plan_molecule(m, o, 0, p);
     if (rc) return rc;
     const int n = p.nao, natoms = p.natoms;
+    if (n == 0) return fail(AM1GPU_DEVICE_ERROR, "G(P) of a molecule without orbitals: nothing to launch");
     const size_t nn = (size_t)n * n, bytes = sizeof(double) * nn;
     // matrices per chunk, and pipelines
     const int R = (int)std::max<size_t>(1, std::min<size_t>({(size_t)nrhs, kGChunkBytes / bytes, (size_t)64}));
