@@ -2689,7 +2689,8 @@ int build_fock_one(const am1gpu_molecule* mol, int method, const double* p_tot, 
 // pipeline's copies to and from its slot overlap the others' transfers and kernels, and the reordering to and from
 // the internal AO order runs on the device.  One matrix at a time, reordered on the host with a pageable
 // copy and a synchronisation each, took 60 ms for those 288; now 15, most of it the first touch of the result's
-// pages (4 to 16 pipelines, chunks of 1 to 4 MB: 14.9 to 16.7 ms).
+// pages (4 to 16 pipelines, chunks of 1 to 4 MB: 14.9 to 16.7 ms).  A single chunk has nothing to overlap: no stream, no
+// event, no thread of its own (one density of two waters 132 us, 145 with them and with the core terms it does not need).
 constexpr size_t kGChunkBytes = 2u << 20;
 constexpr int kGPipes = 8;
 constexpr size_t kGPinnedMax = 64u << 20;  // pinned memory of all slots; larger matrices go straight from and to the caller's
@@ -2741,14 +2742,15 @@ int g_matrix_batch(const am1gpu_molecule* mol, int method, int nrhs, const doubl
     if (rc) return rc;
     std::vector<MolPlan> plans{p};
     Batch b;
-    rc = build_batch(&m, o, std::move(plans), b, *ws, &tl_stats, -1.0, nullptr, align256(off), records + (pinned ? bytes * R * pipes : 0));
+    rc = build_batch(&m, o, std::move(plans), b, *ws, &tl_stats, -1.0, nullptr, align256(off), records + (pinned ? bytes * R * pipes : 0), false);
     if (rc) return rc;
-    while ((int)ws->pipes.size() < pipes) {
+    // one pipeline runs on the workspace's own stream, several on streams of their own behind it
+    while (pipes > 1 && (int)ws->pipes.size() < pipes) {
         cudaStream_t q;
         CK(cudaStreamCreateWithPriority(&q, cudaStreamNonBlocking, ws->priority));
         ws->pipes.push_back(q);
     }
-    if ((rc = mem_side_stream(*ws))) return rc;
+    if (pipes > 1 && (rc = mem_side_stream(*ws))) return rc;
     {
         MolDesc* hm = (MolDesc*)(b.h_extra + o_mols);
         int *ham = (int*)(b.h_extra + o_am), *hz = (int*)(b.h_extra + o_z), *hmap = (int*)(b.h_extra + o_map);
@@ -2769,8 +2771,12 @@ int g_matrix_batch(const am1gpu_molecule* mol, int method, int nrhs, const doubl
         CK(cudaMemcpyAsync(b.d_extra, b.h_extra, records, cudaMemcpyHostToDevice, ws->stream));
         tl_stats.h2d_bytes += (int64_t)records;
     }
-    if ((rc = launch_core(b, ws, ctx->d_params, nullptr))) return rc;
-    CK(cudaEventRecord(ws->fork, ws->stream));
+    if (b.npairs > 0) {  // the integrals are all that is needed
+        k_pair_integrals<<<cdiv(b.npairs, 128), 128, 0, ws->stream>>>(b.d_mols, b.nmol, b.d_pair_prefix, b.npairs, ctx->d_params, b.d_atom_z,
+                                                                     b.d_atom_xyz, b.d_wstore, b.d_arena, b.d_ecc, b.d_status);
+        CK(cudaGetLastError());
+    }
+    if (pipes > 1) CK(cudaEventRecord(ws->fork, ws->stream));
     const MolDesc* dm = (const MolDesc*)(b.d_extra + o_mols);
     const int *dam = (const int*)(b.d_extra + o_am), *dz = (const int*)(b.d_extra + o_z), *dmap = (const int*)(b.d_extra + o_map);
     int dev = 0;
@@ -2781,8 +2787,8 @@ int g_matrix_batch(const am1gpu_molecule* mol, int method, int nrhs, const doubl
     // one pipeline: takes chunks until none is left
     auto pipeline = [&](int k) -> int {
         CK(cudaSetDevice(dev));
-        const cudaStream_t s = ws->pipes[k];
-        CK(cudaStreamWaitEvent(s, ws->fork, 0));
+        const cudaStream_t s = pipes > 1 ? ws->pipes[k] : ws->stream;
+        if (pipes > 1) CK(cudaStreamWaitEvent(s, ws->fork, 0));
         double* arena = (double*)(b.d_extra + o_pipe) + pipe_doubles * k;
         double* raw = arena + arena_doubles;
         double* slot = (double*)(b.h_extra + records) + nn * R * k;
@@ -2809,7 +2815,7 @@ int g_matrix_batch(const am1gpu_molecule* mol, int method, int nrhs, const doubl
             std::lock_guard<std::mutex> lock(mu);
             if (!failed.exchange(r)) msg = g_err;
         }
-        cudaStreamSynchronize(ws->pipes[k]);
+        cudaStreamSynchronize(pipes > 1 ? ws->pipes[k] : ws->stream);
     };
     std::vector<std::thread> pool;
     for (int k = 1; k < pipes; ++k) {
