@@ -526,13 +526,13 @@ bool encode_rows_map_f32(TmaDesc* out, const float* base, int ldf, int n) {
 // within about four waves of resident threads (one molecule, one large matrix, small batches), a thread per
 // eigenvalue otherwise (the warp form does about seven times the work, so it only pays when the GPU is
 // idle).  The eigenvalues are the same.
-void bisect_launch(const TriJob* jobs, int njobs, int maxn, cudaStream_t s) {
+void bisect_launch(const TriJob* jobs, int njobs, int maxn, cudaStream_t s, const int* skip = nullptr) {
     constexpr long long kFourWaves = 4LL * 148 * 2048;  // resident threads of four waves on a B200
     const int lanes = (long long)njobs * maxn * 32 <= kFourWaves ? 32 : 1;
     // few warps: small blocks, so that they spread over the SMs
     const long long warps = (long long)njobs * maxn;
     const int threads = lanes == 1 || warps > 148 * 16 ? 512 : warps > 148 * 4 ? 128 : 64, per_block = threads / lanes;
-    k_bisect<<<dim3(njobs, (maxn + per_block - 1) / per_block), threads, 2 * sizeof(double) * maxn, s>>>(jobs, nullptr, lanes);
+    k_bisect<<<dim3(njobs, (maxn + per_block - 1) / per_block), threads, 2 * sizeof(double) * maxn, s>>>(jobs, skip, lanes);
 }
 
 inline int oz_ldq(int n) { return (n + 15) & ~15; }
@@ -1551,7 +1551,7 @@ int launch_core(Batch& b, Mem* ws, const DevElem* dp, Run* run) {
 }
 
 // One cluster of C CTAs per matrix, one launch per cluster size.
-int launch_tridiag(Batch& b, Mem* ws) {
+int launch_tridiag(Batch& b, Mem* ws, const int* skip = nullptr) {
     for (auto& bk : b.tri_buckets) {
         cudaLaunchConfig_t cfg{};
         cfg.gridDim = dim3(bk.count * bk.C, 1, 1);
@@ -1565,7 +1565,7 @@ int launch_tridiag(Batch& b, Mem* ws) {
         attr[0].val.clusterDim.z = 1;
         cfg.attrs = attr;
         cfg.numAttrs = 1;
-        CK(cudaLaunchKernelEx(&cfg, k_tridiag, (const TriJob*)(b.d_tri + bk.off), (const int*)nullptr));
+        CK(cudaLaunchKernelEx(&cfg, k_tridiag, (const TriJob*)(b.d_tri + bk.off), skip));
     }
     return AM1GPU_OK;
 }
@@ -1766,7 +1766,7 @@ int enq_head(IterEnq& e) {
     int rc;
     CK(cudaMemsetAsync(b.d_active, 0, 4 * sizeof(int), s));
     if ((rc = run.begin(&e.ph))) return rc;
-    k_fock<<<fock_grid(b.natoms, b.maxheavy), 32 * FOCK_WARPS, 0, s>>>(b.d_mols, b.d_atom_mol, b.natoms, e.dp, b.d_atom_z, b.d_wstore, b.d_arena, b.d_st, 0);
+    k_fock<<<fock_grid(b.natoms, b.maxheavy), 32 * FOCK_WARPS, 0, s>>>(b.d_mols, b.d_atom_mol, b.natoms, e.dp, b.d_atom_z, b.d_wstore, b.d_arena, b.d_st, 0, nullptr);
     run.launched(AM1GPU_PHASE_FOCK);
     if ((rc = run.end(AM1GPU_PHASE_FOCK, e.ph)) || (rc = run.begin(&e.ph))) return rc;
     const int nt_other = b.nt_sp2 - b.nt_sp2_pairs;
@@ -1783,7 +1783,7 @@ int enq_head(IterEnq& e) {
             else
                 k_commutator8<<<nt, 128, dgemm_smem_bytes(), s>>>(b.d_jobs, t, nt, b.d_st);
         });
-    k_post_fock<<<dim3(e.nblk, e.njobs), 256, 0, s>>>(b.d_jobs, b.d_mols, b.d_st, e.nblk, 0, 0);
+    k_post_fock<<<dim3(e.nblk, e.njobs), 256, 0, s>>>(b.d_jobs, b.d_mols, b.d_st, e.nblk, 0, 0, nullptr);
     run.launched(AM1GPU_PHASE_COMMUTATOR, 2);
     if ((rc = run.end(AM1GPU_PHASE_COMMUTATOR, e.ph)) || (rc = run.begin(&e.ph))) return rc;
     k_diis_solve<<<cdiv(b.nmol, SCF_MOL_WARPS), 32 * SCF_MOL_WARPS, 0, s>>>(b.d_mols, b.d_jobs, b.d_job0, b.nmol, b.d_st, b.d_status, e.nblk, e.prm);
@@ -2120,6 +2120,7 @@ int scf_loop_graph(IterEnq& e, const am1gpu_options& o, bool* launched) {
     const int64_t per_step = cnt.kernel_launches - step0;
     const int64_t tail0 = cnt.kernel_launches;
     ce.mask = b.d_need_eigen;  // molecules whose purification stalled wait for the host
+    ce.want = 0;
     if ((rc = capture_into(cs, body, purified.data(), purified.size(), &tail, [&]() -> int {
              int r = enq_tail_finish(ce, false);
              if (!r) r = enq_tail_rest(ce);
@@ -2228,21 +2229,26 @@ int run_device(Batch& b, Mem& mem, const DevElem* dp, const am1gpu_options& o, a
     }
     const int nblk = b.nblk;
     size_t t1;
+    // Behind a captured loop that ended on a stalled purification the final phase, launched before the host knows, does nothing
+    // (a flag that its kernels read), so such an iteration costs those launches, the eigensolver and a second launch of the
+    // graph, not the phase: 4096 water clusters 260 ms, with one molecule that stalls in each of its 13 iterations 275 (506
+    // with the phase run and thrown away each time).
+    const int* skip = graph ? &b.d_loop->stalled : nullptr;
     for (bool again = true; again;) {
         again = false;
         // final energy at the final density (src/scf.rs:698-701, 835-839) and the result records
         if ((rc = run.begin(&ph))) return rc;
         k_fock<<<fock_grid(b.natoms, b.maxheavy), 32 * FOCK_WARPS, 0, s>>>(b.d_mols, b.d_atom_mol, b.natoms, dp, b.d_atom_z, b.d_wstore,
-                                                                           b.d_arena, b.d_st, 1);
-        k_post_fock<<<dim3(nblk, njobs), 256, 0, s>>>(b.d_jobs, b.d_mols, b.d_st, nblk, 1, 1);
-        k_final_energy<<<cdiv(b.nmol, SCF_MOL_WARPS), 32 * SCF_MOL_WARPS, 0, s>>>(b.d_mols, b.d_jobs, b.d_job0, b.nmol, b.d_st, nblk);
+                                                                           b.d_arena, b.d_st, 1, skip);
+        k_post_fock<<<dim3(nblk, njobs), 256, 0, s>>>(b.d_jobs, b.d_mols, b.d_st, nblk, 1, 1, skip);
+        k_final_energy<<<cdiv(b.nmol, SCF_MOL_WARPS), 32 * SCF_MOL_WARPS, 0, s>>>(b.d_mols, b.d_jobs, b.d_job0, b.nmol, b.d_st, nblk, skip);
         // eigenvalues of the last F* (mo_energies, HOMO/LUMO): tridiagonalisation + bisection
-        if ((rc = launch_tridiag(b, ws))) return rc;
+        if ((rc = launch_tridiag(b, ws, skip))) return rc;
         int64_t big_tri_launches = 0;
         if ((rc = launch_big_tridiag(b, s, &big_tri_launches))) return rc;
-        bisect_launch(b.d_tri, njobs, b.maxn, s);
+        bisect_launch(b.d_tri, njobs, b.maxn, s, skip);
         k_results<<<b.nmol, RESULT_THREADS, 0, s>>>(b.d_mols, b.d_jobs, b.d_job0, b.nmol, b.d_st, b.d_status, dp, b.d_atom_z,
-                                                     b.d_atom_xyz, b.d_res, b.d_charges);
+                                                     b.d_atom_xyz, b.d_res, b.d_charges, skip);
         run.launched(AM1GPU_PHASE_FINAL, 5 + (int)b.tri_buckets.size() + (int)big_tri_launches);
         CK(cudaGetLastError());
         if ((rc = run.end(AM1GPU_PHASE_FINAL, ph))) return rc;
@@ -2253,8 +2259,7 @@ int run_device(Batch& b, Mem& mem, const DevElem* dp, const am1gpu_options& o, a
         if (b.h_active[2] & (1 << 10)) return fail(AM1GPU_LINALG, "a purification iterate left the range of its digit planes (|x| >= 2)");
         if (b.h_active[2]) return fail(AM1GPU_DEVICE_ERROR, "a tensor-core step gave up waiting for its MMAs or operand copies");
         if (!graph) break;
-        // what the captured loops launched, and whether they ended on a stalled purification (the results
-        // just formed are then of an unfinished solve, and are formed again)
+        // what the captured loops launched, and whether they ended on a stalled purification
         const GraphLoop lp = *b.h_loop;
         b.h_loop->stalled = b.h_loop->scf_iter = b.h_loop->sp2_total = 0;
         done += lp.scf_iter;
@@ -2267,7 +2272,8 @@ int run_device(Batch& b, Mem& mem, const DevElem* dp, const am1gpu_options& o, a
             CK(cudaMemcpyAsync(b.h_active, b.d_active, sizeof(int), cudaMemcpyDeviceToHost, s));
             CK(cudaStreamSynchronize(s));
             bool launched = false;
-            if (b.h_active[0] > 0 && (rc = scf_loop_graph(e, o, &launched))) return rc;
+            if (b.h_active[0] == 0) CK(cudaMemsetAsync(&b.d_loop->stalled, 0, sizeof(int), s));  // else the loop's start clears it
+            else if ((rc = scf_loop_graph(e, o, &launched))) return rc;
         }
     }
     stats->scf_cycles = done;
@@ -2668,7 +2674,7 @@ int build_fock_one(const am1gpu_molecule* mol, int method, const double* p_tot, 
     CK(cudaMemcpyAsync(b.jobs[0].P, p0.data(), sizeof(double) * n * n, cudaMemcpyHostToDevice, ws->stream));
     CK(cudaMemcpyAsync(b.jobs[1].P, p1.data(), sizeof(double) * n * n, cudaMemcpyHostToDevice, ws->stream));
     k_fock<<<fock_grid(b.natoms, b.maxheavy), 32 * FOCK_WARPS, 0, ws->stream>>>(b.d_mols, b.d_atom_mol, b.natoms, ctx->d_params, b.d_atom_z, b.d_wstore,
-                                                      b.d_arena, b.d_st, 1);
+                                                      b.d_arena, b.d_st, 1, nullptr);
     CK(cudaGetLastError());
     std::vector<double> t;
     rc = fetch_matrix(ws, b.jobs[0].F, n, t);
@@ -2800,7 +2806,7 @@ int g_matrix_batch(const am1gpu_molecule* mol, int method, int nrhs, const doubl
             if (pinned) std::memcpy(slot, src, bytes * cnt);
             CK(cudaMemcpyAsync(raw, pinned ? slot : src, bytes * cnt, cudaMemcpyHostToDevice, s));
             k_permute_square<<<dim3(n, cnt), 128, 0, s>>>(raw, (long long)nn, arena + nn * (1 + SLOT_P), (long long)(3 * nn), dmap, n);
-            k_fock<<<fock_grid((long long)cnt * natoms, b.maxheavy), 32 * FOCK_WARPS, 0, s>>>(dm, dam, cnt * natoms, ctx->d_params, dz, b.d_wstore, arena, b.d_st, 1);
+            k_fock<<<fock_grid((long long)cnt * natoms, b.maxheavy), 32 * FOCK_WARPS, 0, s>>>(dm, dam, cnt * natoms, ctx->d_params, dz, b.d_wstore, arena, b.d_st, 1, nullptr);
             k_permute_square<<<dim3(n, cnt), 128, 0, s>>>(arena + nn * (1 + SLOT_F), (long long)(3 * nn), raw, (long long)nn, dmap + n, n);
             CK(cudaGetLastError());
             CK(cudaMemcpyAsync(pinned ? slot : dst, raw, bytes * cnt, cudaMemcpyDeviceToHost, s));

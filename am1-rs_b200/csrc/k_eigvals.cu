@@ -61,12 +61,12 @@ __device__ __forceinline__ double tri_warp_sums(const double* red) {
     return t[0];
 }
 
-__global__ void __launch_bounds__(TRI_THREADS) k_tridiag(const TriJob* __restrict__ jobs, const int* __restrict__ mask) {
+__global__ void __launch_bounds__(TRI_THREADS) k_tridiag(const TriJob* __restrict__ jobs, const int* __restrict__ skip) {
     cg::cluster_group cluster = cg::this_cluster();
     const int C = (int)cluster.num_blocks();
     const int crank = (int)cluster.block_rank();
     const TriJob jb = jobs[blockIdx.x / C];
-    if (mask && !mask[jb.mol]) return;  // uniform over the cluster
+    if (skip && *skip) return;  // uniform over the cluster
     const int n = jb.n;
     const int ld = n + (n & 1);
     const int R = (n + C - 1) / C;
@@ -499,9 +499,9 @@ __device__ __forceinline__ int sturm_count(const double2* de, int n, double x) {
 // of one thread's ~50 dependent counts is the cost.  The midpoints, the counts and so
 // the eigenvalues are the same either way.  n = 1501: 5.0 -> 0.7 ms, 192 orbitals alone 107 -> 83 us (32-way multisection
 // before, whose eigenvalues differed from the thread form's in the last bits), a batch of 192 molecules 1.07 -> 0.83 ms.
-__global__ void k_bisect(const TriJob* __restrict__ jobs, const int* __restrict__ mask, int lanes) {
+__global__ void k_bisect(const TriJob* __restrict__ jobs, const int* __restrict__ skip, int lanes) {
     const TriJob jb = jobs[blockIdx.x];
-    if (mask && !mask[jb.mol]) return;
+    if (skip && *skip) return;
     const int n = jb.n;
     extern __shared__ __align__(16) double sh[];
     double2* de = reinterpret_cast<double2*>(sh);  // d_i, e_{i-1}^2

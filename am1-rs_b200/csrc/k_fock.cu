@@ -45,7 +45,9 @@ __host__ __device__ constexpr int pair_lo(int q) { return q - pair_hi(q) * (pair
 __global__ void __launch_bounds__(32 * FOCK_WARPS, 4) k_fock(const MolDesc* __restrict__ mols, const int* __restrict__ atom_mol,
                                                          int natoms_total, const DevElem* __restrict__ params,
                                                          const int* __restrict__ atom_z, const double* __restrict__ wstore,
-                                                         double* __restrict__ arena, const MolState* __restrict__ st, int force) {
+                                                         double* __restrict__ arena, const MolState* __restrict__ st, int force,
+                                                         const int* __restrict__ skip) {
+    if (skip && *skip) return;
     __shared__ double s_w[FOCK_WARPS][100 * FOCK_XX_ROUND];
     __shared__ double s_q[FOCK_WARPS][10];
     __shared__ double s_pab[FOCK_WARPS][FOCK_XX_ROUND][2][16];

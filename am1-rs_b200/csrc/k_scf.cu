@@ -96,7 +96,9 @@ __device__ __forceinline__ void live_slots(const MolState& s, int& newslot, unsi
 constexpr int POST_WARPS = 8;
 
 __global__ void __launch_bounds__(32 * POST_WARPS) k_post_fock(const ChanJob* __restrict__ jobs, const MolDesc* __restrict__ mols,
-                                                               const MolState* __restrict__ st, int nblk, int energy_only, int force) {
+                                                               const MolState* __restrict__ st, int nblk, int energy_only, int force,
+                                                               const int* __restrict__ skip) {
+    if (skip && *skip) return;
     const ChanJob jb = jobs[blockIdx.y];
     const MolState& s = st[jb.mol];
     if (!force && !s.active) return;
@@ -789,9 +791,9 @@ __global__ void __launch_bounds__(32 * SCF_MOL_WARPS) k_converge(const MolDesc* 
 // A warp per molecule: lanes 0 and 1 add the two energy traces, in block order.
 __global__ void __launch_bounds__(32 * SCF_MOL_WARPS) k_final_energy(const MolDesc* __restrict__ mols, const ChanJob* __restrict__ jobs,
                                                                      const int* __restrict__ mol_job0, int nmol,
-                                                                     MolState* __restrict__ st, int nblk) {
+                                                                     MolState* __restrict__ st, int nblk, const int* __restrict__ skip) {
     const int lane = threadIdx.x & 31, mi = blockIdx.x * SCF_MOL_WARPS + (threadIdx.x >> 5);
-    if (mi >= nmol) return;
+    if (mi >= nmol || (skip && *skip)) return;
     const int nch = mols[mi].nch, job0 = mol_job0[mi];
     double t = 0.0;
     for (int c = 0; c < nch; ++c) {
@@ -810,10 +812,11 @@ __global__ void __launch_bounds__(RESULT_THREADS) k_results(const MolDesc* __res
                                                             const int* __restrict__ mol_job0, int nmol, const MolState* __restrict__ st,
                                                             const int* __restrict__ mol_status, const DevElem* __restrict__ params,
                                                             const int* __restrict__ atom_z, const double* __restrict__ atom_xyz,
-                                                            double* __restrict__ res, double* __restrict__ charges) {
+                                                            double* __restrict__ res, double* __restrict__ charges,
+                                                            const int* __restrict__ skip) {
     __shared__ double part[5][RESULT_THREADS / 32];
     const int mi = blockIdx.x;
-    if (mi >= nmol) return;
+    if (mi >= nmol || (skip && *skip)) return;
     const MolDesc md = mols[mi];
     const MolState& s = st[mi];
     const int n = md.nao, h = md.nheavy, tid = threadIdx.x;

@@ -180,14 +180,15 @@ __global__ void k_pair_gradient_split(const MolDesc* mols, int nmol, const long 
                                       const DevElem* params, const int* atom_z, const double* atom_xyz, const ChanJob* jobs,
                                       const int* mol_job0, double* pairf, int* mol_status);
 __global__ void k_gradient(const MolDesc* mols, const int* atom_mol, int natoms_total, const double* pairf, double* gradient);
-// grid fock_grid(...), 32 FOCK_WARPS threads
+// grid fock_grid(...), 32 FOCK_WARPS threads.  skip (here and in the other kernels of a run's final phase, optional): nothing
+// is done where *skip is not zero
 constexpr int FOCK_WARPS = 4, FOCK_XX_CHUNK = 16, FOCK_SPLIT_ATOMS = 32768;
 inline dim3 fock_grid(long long natoms, int most_heavy) {  // atoms of the launch, most heavy atoms of a molecule
     const unsigned chunks = natoms >= FOCK_SPLIT_ATOMS || most_heavy < 2 ? 0u : (unsigned)((most_heavy - 1 + FOCK_XX_CHUNK - 1) / FOCK_XX_CHUNK);
     return dim3((unsigned)((natoms + FOCK_WARPS - 1) / FOCK_WARPS), 1 + chunks);
 }
 __global__ void k_fock(const MolDesc* mols, const int* atom_mol, int natoms_total, const DevElem* params,
-                       const int* atom_z, const double* wstore, double* arena, const MolState* st, int force);
+                       const int* atom_z, const double* wstore, double* arena, const MolState* st, int force, const int* skip);
 // out_r[i][j] = in_r[map[i]][map[j]] for matrices r = blockIdx.y, n x n, at strides so and si (doubles);
 // grid (n, count), 128 threads: a CTA per row
 __global__ void k_permute_square(const double* in, long long si, double* out, long long so, const int* map, int n);
@@ -305,11 +306,11 @@ __global__ void k_sp2_step_tc1(const Sp2Job* jobs, const GemmTile* tiles, int nt
 __global__ void k_sp2_finish(const Sp2Job* jobs, const Sp2State* sst, const MolState* st, int* need_eigen, double* work,
                              int* big_stall, int* big_count);
 // launched in clusters of C CTAs (one cluster per job), tridiag_smem_bytes(n, C) each
-__global__ void k_tridiag(const TriJob* jobs, const int* mask);
+__global__ void k_tridiag(const TriJob* jobs, const int* skip);
 size_t tridiag_smem_bytes(int n, int C);
 // lanes = 1: a thread per eigenvalue, blockIdx.y the block of blockDim eigenvalue indices; lanes =
 // 32: a warp per eigenvalue, blockIdx.y the block of blockDim / 32 indices (bisect_launch sizes both)
-__global__ void k_bisect(const TriJob* jobs, const int* mask, int lanes);
+__global__ void k_bisect(const TriJob* jobs, const int* skip, int lanes);
 // matrices too large for a cluster's shared memory, the matrix in global memory: one cooperative
 // launch over the whole GPU (grid <= co-resident CTAs of TRIB_THREADS threads), or a cluster of
 // C CTAs per matrix (grid (C, count), blockIdx.y indexes jobs); tridiag_big_smem_bytes(largest n)
@@ -437,7 +438,7 @@ __global__ void k_slots_init(const ChanJob* jobs);
 constexpr int kLowpMaxOpenShellAo = 448;
 __global__ void k_state_init(MolState* st, const MolDesc* mols, int nmol, int lowp);
 __global__ void k_post_fock(const ChanJob* jobs, const MolDesc* mols, const MolState* st, int nblk, int energy_only,
-                            int force);
+                            int force, const int* skip);
 // per-molecule bookkeeping: a warp per molecule, SCF_MOL_WARPS per CTA (k_results: a CTA per molecule)
 constexpr int SCF_MOL_WARPS = 4;
 constexpr int RESULT_THREADS = 128;
@@ -449,11 +450,11 @@ __global__ void k_density_post(const ChanJob* jobs, const MolState* st, int nblk
 __global__ void k_converge(const MolDesc* mols, const ChanJob* jobs, const int* mol_job0, int nmol, MolState* st,
                            int* mol_status, int nblk, ScfParams prm, int* active_count, const int* mask, int want);
 __global__ void k_final_energy(const MolDesc* mols, const ChanJob* jobs, const int* mol_job0, int nmol, MolState* st,
-                               int nblk);
+                               int nblk, const int* skip);
 // Per-molecule result record (doubles), see RES_* below; charges in internal atom order.
 __global__ void k_results(const MolDesc* mols, const ChanJob* jobs, const int* mol_job0, int nmol, const MolState* st,
                           const int* mol_status, const DevElem* params, const int* atom_z, const double* atom_xyz,
-                          double* res, double* charges);
+                          double* res, double* charges, const int* skip);
 constexpr int RES_ELEC = 0, RES_CORE = 1, RES_TOTAL = 2, RES_HOF = 3, RES_DIP = 4, RES_DIPMAG = 7, RES_HOMO = 8,
               RES_LUMO = 9, RES_HOMO_B = 10, RES_LUMO_B = 11, RES_RESID = 12, RES_ITER = 13, RES_CONV = 14,
               RES_STATUS = 15, RES_N = 16;
