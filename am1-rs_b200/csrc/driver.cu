@@ -1620,6 +1620,7 @@ bool tridiag_blocked() {
     return v;
 }
 
+// CTAs of a panel: two per SM, all co-resident; AM1GPU_TRIDIAG_CTAS takes fewer, as on a smaller GPU (for tests).
 int blocked_tridiag(TriJob tj, cudaStream_t s, int64_t* launches) {
     const int n = tj.n;
     tj.work = (double*)(((uintptr_t)tj.work + 15) & ~(uintptr_t)15);  // 16-byte copies of V, W
@@ -1627,8 +1628,13 @@ int blocked_tridiag(TriJob tj, cudaStream_t s, int64_t* launches) {
     const size_t smem = tridiag_panel_smem_bytes(n);
     int per_sm = 0;
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_tridiag_panel, TRIB_THREADS, smem));
-    const int grid = std::min(per_sm, 2) * g_sms;
-    if (per_sm < 1 || (long long)grid * 64 < n) return fail(AM1GPU_DEVICE_ERROR, "blocked tridiagonalisation does not fit the GPU");
+    static const int most = [] {
+        const char* e = std::getenv("AM1GPU_TRIDIAG_CTAS");
+        return e && std::atoi(e) > 0 ? std::atoi(e) : 1024;
+    }();
+    const int grid = std::min(std::min(per_sm, 2) * g_sms, most);
+    // a CTA keeps 64 rows at most, and its warps but one sum the 2 TRP_B slots of all CTAs
+    if (per_sm < 1 || (long long)grid * 64 < n || grid * (TRIB_THREADS / 32 - 1) < 2 * TRP_B) return fail(AM1GPU_DEVICE_ERROR, "blocked tridiagonalisation does not fit the GPU");
     for (int k = 0; k < n - 1; k += TRP_B) {
         int bw = std::min(TRP_B, n - 1 - k);
         void* args[] = {&tj, &k, &bw};

@@ -709,18 +709,20 @@ __global__ void __launch_bounds__(TRIB_THREADS) k_tridiag_panel(TriJob jb, int k
             for (int u = 0; u < 4; ++u)
                 if (i0 + u * TRIB_THREADS < n) sv[i0 + u * TRIB_THREADS] = v[u];
         }
-        // |x|^2 in warp 0; slot gi (W^T x or V^T x) of the shares in warp 1, summed for all CTAs
+        // |x|^2 in warp 0; the slots (W^T x or V^T x) of the shares one each in the CTAs' warps 1, then 2, and so on,
+        // summed for all CTAs: warp 1 alone where there are 2 B CTAs
         const double* V1 = VW + (size_t)(c + 1) * 2 * B;
-        const double sum = warp == 0 ? panel_share_sum(share, G)
-                           : warp == 1 && gi < 2 * j ? panel_share_sum(share + (size_t)(1 + gi) * G, G) : 0.0;
-        const double v1 = warp == 1 && gi < 2 * j ? __ldcg(V1 + (gi < j ? B + gi : gi - j)) : 0.0;
+        const int sl = gi + (warp - 1) * G;
+        const bool slot = warp > 0 && sl < 2 * j;
+        const double sum = warp == 0 ? panel_share_sum(share, G) : slot ? panel_share_sum(share + (size_t)(1 + sl) * G, G) : 0.0;
+        const double v1 = slot ? __ldcg(V1 + (sl < j ? B + sl : sl - j)) : 0.0;
         if (warp == 0 && lane == 0) red[0] = sum;
         __syncthreads();
         const double alpha = sqrt(red[0]);
         const double sg = x1 >= 0.0 ? 1.0 : -1.0;
         const double beta = alpha == 0.0 ? 0.0 : 1.0 / (alpha * (alpha + fabs(x1)));
-        if (warp == 1 && lane == 0 && gi < 2 * j)  // plus the e_{c+1} part of v = x + sg alpha e_{c+1}
-            sums[gi < j ? gi : B + gi - j] = sum + sg * alpha * v1;
+        if (slot && lane == 0)  // plus the e_{c+1} part of v = x + sg alpha e_{c+1}
+            sums[sl < j ? sl : B + sl - j] = sum + sg * alpha * v1;
         if (tid == 0) sv[c + 1] = x1 + sg * alpha;
         __syncthreads();
         // ---- phase 2a: u = A v on own rows i > c, this CTA's share of v . u.  Rows go in groups of
