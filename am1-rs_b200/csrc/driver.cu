@@ -382,6 +382,27 @@ int mem_side_stream(Mem& w) {
     return AM1GPU_OK;
 }
 
+// Streams of another priority: those the workspace has are replaced (nothing is in flight between calls), and the captured
+// loop goes with them (its kernels carry the old one); what is created on first use is created anew.
+int mem_set_priority(Mem& w, int p) {
+    if (!w.stream || w.priority == p) return AM1GPU_OK;
+    if (w.graph_exec) CK(cudaGraphExecDestroy(w.graph_exec));
+    w.graph_exec = nullptr;
+    w.graph_key.clear();
+    std::vector<cudaStream_t> old = std::move(w.pipes);
+    w.pipes.clear();
+    old.push_back(w.stream);
+    if (w.cap_stream) old.push_back(w.cap_stream);
+    w.stream = w.cap_stream = nullptr;
+    for (cudaStream_t q : old) {
+        CK(cudaStreamSynchronize(q));
+        CK(cudaStreamDestroy(q));
+    }
+    CK(cudaStreamCreateWithPriority(&w.stream, cudaStreamNonBlocking, p));
+    w.priority = p;
+    return AM1GPU_OK;
+}
+
 thread_local Mem tl_mem;
 using Workspace = Mem;
 
@@ -3811,23 +3832,8 @@ int am1gpu_set_stream_priority(int32_t priority) {
     CK(cudaDeviceGetStreamPriorityRange(&lo, &hi));  // lo: least (0), hi: greatest (negative)
     const int p = std::max(hi, std::min(lo, (int)priority));
     tl_priority = p;
-    Mem& w = tl_mem;
-    if (w.stream && w.priority != p) {  // the thread's stream so far: replace it (nothing is in flight between calls)
-        CK(cudaStreamSynchronize(w.stream));
-        CK(cudaStreamDestroy(w.stream));
-        w.stream = nullptr;
-        CK(cudaStreamCreateWithPriority(&w.stream, cudaStreamNonBlocking, p));
-        w.priority = p;
-        if (w.graph_exec) CK(cudaGraphExecDestroy(w.graph_exec));  // its kernels carry the old priority
-        w.graph_exec = nullptr;
-        w.graph_key.clear();
-        if (w.cap_stream) {
-            CK(cudaStreamSynchronize(w.cap_stream));
-            CK(cudaStreamDestroy(w.cap_stream));
-            w.cap_stream = nullptr;
-        }
-    }
-    return AM1GPU_OK;
+    if (const int rc = mem_set_priority(tl_mem, p)) return rc;
+    return mem_set_priority(tl_mem_eig, p);
 }
 
 int am1gpu_last_call_stats(am1gpu_call_stats* out) {
