@@ -270,8 +270,10 @@ int device_ctx(DeviceCtx** out) {
             const int C = k == 0 ? 16 : 8;
             cudaLaunchAttribute at[1];
             cudaLaunchConfig_t cfg = cluster_config(C, 1, 256, sp2_fused_smem_bytes(FU_CLU_MAX, false), nullptr, at);
-            if ((err = cudaOccupancyMaxActiveClusters(&c.clu_resident[k], k_sp2_clu, &cfg)) != cudaSuccess)
-                return bad("one-launch purification occupancy", err);
+            if (cudaOccupancyMaxActiveClusters(&c.clu_resident[k], k_sp2_clu, &cfg) != cudaSuccess) {
+                c.clu_resident[k] = 0;  // no such cluster on this device: the tiles take over
+                cudaGetLastError();
+            }
         }
         for (const void* f : {(const void*)k_sp2_step_tma, (const void*)k_commutator_tma})
             if ((err = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dgemm_tma_smem_bytes())) != cudaSuccess)
@@ -706,7 +708,7 @@ int sp2_fused_kind(const MolPlan& p) {
 int sp2_cluster_for(std::vector<int> clu, const std::vector<int>& tiled) {
     const int count = (int)clu.size();
     if (count < 1 || count > 16) return 0;
-    if (count <= g_clu_resident[0]) return 16;
+    if (count <= g_clu_resident[0]) return 16;  // (0 where a device holds none)
     std::sort(clu.begin(), clu.end(), std::greater<int>());
     auto clusters_us = [&](int C, int resident) {  // largest first, each where a place is free first
         std::vector<double> place(resident, 0.0);
@@ -2290,7 +2292,7 @@ int run_device(Batch& b, Mem& mem, const DevElem* dp, const am1gpu_options& o, a
         const GraphLoop lp = *b.h_loop;
         b.h_loop->stalled = b.h_loop->scf_iter = b.h_loop->sp2_total = 0;
         done += lp.scf_iter;
-        stats->kernel_launches += 1 + (int64_t)lp.scf_iter * (b.graph_counts[0] + b.graph_counts[2]) + (int64_t)lp.sp2_total * b.graph_counts[1];
+        stats->kernel_launches += (lp.scf_iter > 0) + (int64_t)lp.scf_iter * (b.graph_counts[0] + b.graph_counts[2]) + (int64_t)lp.sp2_total * b.graph_counts[1];
         if (lp.stalled) {
             again = true;
             e.mask = b.d_need_eigen;
@@ -3195,7 +3197,7 @@ int density_purify_one(int n, const double* F, double nocc, double weight, int p
             CK(cudaGetLastError());
         } else {
             void* args[] = {&dj, &list, &dsst, &dms, &need, &work, &max_steps};
-            CK(launch_clusters((const void*)k_sp2_clu, 16, 1, 256, smem, s, args));
+            CK(launch_clusters((const void*)k_sp2_clu, g_clu_resident[0] > 0 ? 16 : 8, 1, 256, smem, s, args));
         }
     } else {
         k_sp2_bounds<<<1, 512, 3 * sizeof(double) * n, s>>>(dj, dms);
