@@ -604,7 +604,9 @@ namespace am1 {
 // row c+1 of W and V; they are needed only after the second barrier, which sums v . A v, since
 // p . v = beta (v . A v - 2 (V^T v) . (W^T v)).  Two grid barriers per column: row c+1's newest
 // entries of V and W, which its owner writes after the second barrier, every CTA forms itself for
-// the next column's first phase.  Rows are cyclic over the CTAs (r % G).
+// the next column's first phase.  Rows are cyclic over G shares (r % G), the CTAs of a GPU that the matrix has to
+// itself; fewer CTAs take several shares each, with the same sums in the same order, so the results do not depend on
+// how many there are (blocked_tridiag).
 // Scratch (job.work, 16-byte aligned): VW[n][2B] = [V | W] | WVt[2B][n] = [W | V]^T | x[n] |
 // u[n] | share[2B + 2][G] | sums[2B]; dynamic shared memory: v (n doubles) and W^T v, V^T v.  As in
 // tridiag_group, row c of job.W ends holding reflector v_c in columns c+1..n-1.
@@ -635,11 +637,15 @@ __device__ __forceinline__ double panel_share_sum(const double* __restrict__ sha
 // column: 4.1k for the column, 15.7k for the reflector, 6.7k for A v, 8.7k for w).  Now a slot is summed by one CTA,
 // from consecutive words, while the others multiply, and A v's rows are reduced behind one barrier: 2.5k, 3.2k, 8.2k and
 // 2.3k; eigenvalues alone, with copies and bisection, 1501 rows 34.8 -> 17.5 ms, 3072 rows 92 -> 53 ms.
-__global__ void __launch_bounds__(TRIB_THREADS) k_tridiag_panel(TriJob jb, int k, int bw) {
+__global__ void __launch_bounds__(TRIB_THREADS) k_tridiag_panel(TriJob jb, int k, int bw, int G) {
     cg::grid_group grid = cg::this_grid();
-    const int G = (int)gridDim.x, gi = (int)blockIdx.x;
     const int n = jb.n;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    // the G shares of the work: CTA b takes b, b + gridDim.x, ..., L in all, 64 threads each for the work on single rows, S
+    // rows' room each
+    const int P = (int)gridDim.x, L = (G + P - 1) / P, S = 64 / L;
+    const int lg = tid >> 6, t = tid & 63, gi = (int)blockIdx.x + lg * P;
+    const bool act = lg < L && gi < G;
     constexpr int NW = TRIB_THREADS / 32;
     constexpr int B = TRP_B;
     double* A = jb.W;
@@ -652,47 +658,63 @@ __global__ void __launch_bounds__(TRIB_THREADS) k_tridiag_panel(TriJob jb, int k
     extern __shared__ double psh[];
     double* sv = psh;      // v, rows c+1..n-1
     double* st = psh + n;  // [0, B): W^T v;  [B, 2B): V^T v
-    __shared__ double xr[64];  // this CTA's x_i of the current column (its rows > c, at most 64 of them)
+    __shared__ double xr[64];  // this CTA's x_i of the current column (its rows >= c, at most 64 of them)
     __shared__ double red[NW];
-    // the panel's V and W on this CTA's own rows (row gi + q G in slot q), kept here as they are
+    // the panel's V and W on this CTA's own rows (row gi + q G of a share in its slot q), kept here as they are
     // formed: the per-column corrections read them from shared memory, not global
     __shared__ double svw[64][2 * TRP_B];
     __shared__ double srow[2 * TRP_B];  // V and W of row c (formed locally in the previous column, or read)
-    __shared__ double redr[64][NW];     // A v of the own rows, each warp's share of the columns
+    __shared__ double redr[64][NW];     // A v of the own rows, each warp's part of the columns
+    // rows >= c = cd G + cm of share g: the first, how many (<= S), the slot of the first, the index of the first > c
+    struct Rows {
+        int first, nr, q0, qa;
+    };
+    const int nd = n / G, nm = n % G;
+    int cd = k / G, cm = k % G;
+    auto rows = [&](int g) {
+        Rows r;
+        r.q0 = cd + (g < cm ? 1 : 0);
+        r.first = r.q0 * G + g;
+        r.nr = nd + (g < nm ? 1 : 0) - r.q0;
+        r.qa = g == cm ? 1 : 0;
+        return r;
+    };
     for (int j = 0; j < bw; ++j) {
         const int c = k + j;
+        if (j > 0 && ++cm == G) {
+            cm = 0;
+            ++cd;
+        }
         __syncthreads();  // own rows' V, W of the previous column, and srow, are written
         // ---- phase 1: column c for own rows i >= c, and this CTA's shares of |x|^2, W^T x, V^T x
-        const int first = c + ((gi - c % G) % G + G) % G;  // first own row >= c
-        const int nr = first < n ? (n - 1 - first) / G + 1 : 0;  // own rows >= c (<= 64: n <= 8192 and G >= 128)
-        const int q0 = (first - gi) / G;  // slot of the first own row >= c
-        const int qa = first > c ? 0 : 1;  // first own row > c
-        if (tid < nr) {
-            const int i = first + tid * G;
-            const double* Vi = svw[q0 + tid];
+        const Rows me = rows(gi);
+        const int row = me.first + t * G, slot0 = lg * S + me.q0, at = lg * S;  // this thread's own row (where t < nr)
+        if (act && t < me.nr) {
+            const int i = row;
+            const double* Vi = svw[slot0 + t];
             double x = __ldcg(A + (size_t)i * n + c);
             for (int l = 0; l < j; ++l) x -= Vi[l] * srow[B + l] + Vi[B + l] * srow[l];
-            xr[tid] = x;
+            xr[at + t] = x;
             xb[i] = x;
             if (i == c) jb.d[c] = x;
         }
         __syncthreads();
-        if (tid < 2 * j + 1) {  // share slot 0: |x_{>c}|^2; 1..j: W^T x; j+1..2j: V^T x
+        if (act && t < 2 * j + 1) {  // share slot 0: |x_{>c}|^2; 1..j: W^T x; j+1..2j: V^T x
             double s = 0.0;
-            for (int q = qa; q < nr; ++q) {
-                const double xq = xr[q];
-                if (tid == 0) s += xq * xq;
-                else if (tid <= j) s += svw[q0 + q][B + (tid - 1)] * xq;
-                else s += svw[q0 + q][tid - 1 - j] * xq;
+            for (int q = me.qa; q < me.nr; ++q) {
+                const double xq = xr[at + q];
+                if (t == 0) s += xq * xq;
+                else if (t <= j) s += svw[slot0 + q][B + (t - 1)] * xq;
+                else s += svw[slot0 + q][t - 1 - j] * xq;
             }
-            share[(size_t)tid * G + gi] = s;
+            share[(size_t)t * G + gi] = s;
         }
         grid.sync();
         // ---- the reflector (every CTA forms the same values: fixed-order sums of the shares)
         const bool has_next = c + 2 < n;
         const double x1 = __ldcg(xb + c + 1);
         if (!has_next) {  // the last 2 x 2 block: e[n-2], and d[n-1] with this panel's updates
-            if (gi == (n - 1) % G && tid == 0) {
+            if (act && gi == (nm == 0 ? G - 1 : nm - 1) && t == 0) {
                 jb.e[c] = x1;
                 double dn = __ldcg(A + (size_t)(n - 1) * n + n - 1);
                 const double* Vn = VW + (size_t)(n - 1) * 2 * B;
@@ -712,7 +734,7 @@ __global__ void __launch_bounds__(TRIB_THREADS) k_tridiag_panel(TriJob jb, int k
         // |x|^2 in warp 0; the slots (W^T x or V^T x) of the shares one each in the CTAs' warps 1, then 2, and so on,
         // summed for all CTAs: warp 1 alone where there are 2 B CTAs
         const double* V1 = VW + (size_t)(c + 1) * 2 * B;
-        const int sl = gi + (warp - 1) * G;
+        const int sl = (int)blockIdx.x + (warp - 1) * P;
         const bool slot = warp > 0 && sl < 2 * j;
         const double sum = warp == 0 ? panel_share_sum(share, G) : slot ? panel_share_sum(share + (size_t)(1 + sl) * G, G) : 0.0;
         const double v1 = slot ? __ldcg(V1 + (sl < j ? B + sl : sl - j)) : 0.0;
@@ -728,41 +750,44 @@ __global__ void __launch_bounds__(TRIB_THREADS) k_tridiag_panel(TriJob jb, int k
         // ---- phase 2a: u = A v on own rows i > c, this CTA's share of v . u.  Rows go in groups of
         // four; every thread takes a stride of the columns for all four (many loads in flight),
         // and the partial sums are reduced over the CTA in a fixed order.
-        for (int g0 = qa; g0 < nr; g0 += 4) {
-            const int gr = min(4, nr - g0);
-            const double* Ar[4];
+        for (int l = 0, g = (int)blockIdx.x; l < L && g < G; ++l, g += P) {
+            const Rows r = rows(g);
+            for (int g0 = r.qa; g0 < r.nr; g0 += 4) {
+                const int gr = min(4, r.nr - g0);
+                const double* Ar[4];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) Ar[u] = A + (size_t)(first + (g0 + (u < gr ? u : 0)) * G) * n;
-            double acc[4] = {0.0, 0.0, 0.0, 0.0};
+                for (int u = 0; u < 4; ++u) Ar[u] = A + (size_t)(r.first + (g0 + (u < gr ? u : 0)) * G) * n;
+                double acc[4] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll 2
-            for (int m = c + 1 + tid; m < n; m += TRIB_THREADS) {
-                const double vm = sv[m];
+                for (int m = c + 1 + tid; m < n; m += TRIB_THREADS) {
+                    const double vm = sv[m];
 #pragma unroll
-                for (int u = 0; u < 4; ++u) acc[u] = fma(__ldcg(Ar[u] + m), vm, acc[u]);
-            }
-#pragma unroll
-            for (int u = 0; u < 4; ++u)
-                for (int o = 16; o > 0; o >>= 1) acc[u] += __shfl_xor_sync(0xffffffffu, acc[u], o);
-            if (lane == 0)
+                    for (int u = 0; u < 4; ++u) acc[u] = fma(__ldcg(Ar[u] + m), vm, acc[u]);
+                }
 #pragma unroll
                 for (int u = 0; u < 4; ++u)
-                    if (u < gr) redr[g0 + u][warp] = acc[u];
+                    for (int o = 16; o > 0; o >>= 1) acc[u] += __shfl_xor_sync(0xffffffffu, acc[u], o);
+                if (lane == 0)
+#pragma unroll
+                    for (int u = 0; u < 4; ++u)
+                        if (u < gr) redr[l * S + g0 + u][warp] = acc[u];
+            }
         }
         __syncthreads();
+        const bool own = act && t >= me.qa && t < me.nr;
         double ui = 0.0;  // u of this thread's own row, kept for phase 2b
-        if (warp < 2) {   // at most 64 own rows
+        if (lg < L) {
             double part = 0.0;
-            if (tid >= qa && tid < nr) {
-                const int i = first + tid * G;
-                for (int w = 0; w < NW; ++w) ui += redr[tid][w];
-                if (i == c + 1) ub[i] = ui;
-                part = ui * sv[i];
+            if (own) {
+                for (int w = 0; w < NW; ++w) ui += redr[at + t][w];
+                if (row == c + 1) ub[row] = ui;
+                part = ui * sv[row];
             }
             for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
             if (lane == 0) red[1 + warp] = part;
         }
         __syncthreads();
-        if (tid == 0) share[(size_t)(2 * B + 1) * G + gi] = red[1] + red[2];
+        if (act && t == 0) share[(size_t)(2 * B + 1) * G + gi] = red[1 + 2 * lg] + red[2 + 2 * lg];
         grid.sync();
         // ---- phase 2b: p = beta (u - V (W^T v) - W (V^T v)), w = p - kk v for own rows i > c with
         // kk = (beta / 2) p . v, p . v = beta (v . u - 2 (V^T v) . (W^T v)); column j of V and W in both
@@ -779,21 +804,21 @@ __global__ void __launch_bounds__(TRIB_THREADS) k_tridiag_panel(TriJob jb, int k
         }
         const double u1 = tid == TRIB_THREADS - 1 ? __ldcg(ub + c + 1) : 0.0;
         __syncthreads();
-        const bool next_row = tid == TRIB_THREADS - 1, own = tid >= qa && tid < nr;
-        const double* Vi = next_row ? srow : svw[own ? q0 + tid : 0];
-        double t = next_row ? u1 : ui, vv = 0.0;
+        const bool next_row = tid == TRIB_THREADS - 1;  // (no share's: L < 8)
+        const double* Vi = next_row ? srow : svw[own ? slot0 + t : 0];
+        double pu = next_row ? u1 : ui, vv = 0.0;
         if (own || next_row) {
             for (int l = 0; l < j; ++l) {
-                t -= Vi[l] * st[l] + Vi[B + l] * st[B + l];
+                pu -= Vi[l] * st[l] + Vi[B + l] * st[B + l];
                 vv += st[l] * st[B + l];
             }
         }
-        const double p = beta * t, kk = 0.5 * beta * (beta * (red[0] - 2.0 * vv));
+        const double p = beta * pu, kk = 0.5 * beta * (beta * (red[0] - 2.0 * vv));
         if (own) {
-            const int i = first + tid * G;
+            const int i = row;
             const double v = sv[i], w = p - kk * v;
-            svw[q0 + tid][j] = v;
-            svw[q0 + tid][B + j] = w;
+            svw[slot0 + t][j] = v;
+            svw[slot0 + t][B + j] = w;
             VW[(size_t)i * 2 * B + j] = v;
             VW[(size_t)i * 2 * B + B + j] = w;
             WVt[(size_t)j * n + i] = w;
@@ -804,7 +829,7 @@ __global__ void __launch_bounds__(TRIB_THREADS) k_tridiag_panel(TriJob jb, int k
             srow[j] = sv[c + 1];
             srow[B + j] = p - kk * sv[c + 1];
         }
-        if (gi == c % G && tid == 0) jb.e[c] = alpha == 0.0 ? 0.0 : -sg * alpha;
+        if (act && gi == cm && t == 0) jb.e[c] = alpha == 0.0 ? 0.0 : -sg * alpha;
     }
 }
 
