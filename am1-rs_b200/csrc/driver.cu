@@ -3291,7 +3291,7 @@ struct SmallEig {
 // staged and copied, prepared (mirrored, bounds, identity) on the device, solved, sorted and turned into columns
 // there, and fetched, so one group's copies and host staging run under the others' solves and the groups share the
 // SMs.  One group after the other on one stream, prepared and transposed on the host, took 94 ms for 96
-// matrices of 24 to 320 rows; now 30.
+// matrices of 24 to 320 rows; now 36.
 // Up to kEigHostElements elements in all, the host prepares and transposes after all, with one copy each way on the one
 // stream: three small kernels, an event and four more copies cost more than they save (2 matrices of 5 rows 104 us
 // on the device, 83 so, 10 of 40 668 and 655; 80 of 16, past the line, 705 and 710).

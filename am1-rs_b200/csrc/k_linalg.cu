@@ -151,7 +151,7 @@ constexpr int JAC_MAX_SWEEPS = 60;
 // pair of the CTA (up to 32: blockDim.x is the launch's, jacobi_threads), where eight warps took the 20 pairs of
 // a CTA at 320 rows in three turns, and two landing zones used in turn where shared memory has room
 // for them: a column may then be sent while the neighbour still copies the last one out, which leaves one cluster
-// barrier per round.  96 matrices of 24 to 320 rows: 62 -> 33 ms of kernels one after the other.
+// barrier per round.  96 matrices of 24 to 320 rows: 62 -> 41 ms of kernels one after the other.
 // Shared memory: nbuf = 2q + 2 (or + 4) buffers of 2n doubles ([g | v]), then int metadata.
 __global__ void __launch_bounds__(1024) k_jacobi(const EigJob* __restrict__ jobs, const MolState* __restrict__ st,
                                                         int* __restrict__ mol_status, int force, const int* __restrict__ mask) {
