@@ -736,11 +736,14 @@ int sp2_cluster_for(std::vector<int> clu, const std::vector<int>& tiled) {
     if (count < 1 || count > 16) return 0;
     if (count <= g_clu_resident[0]) return 16;  // (0 where a device holds none)
     std::sort(clu.begin(), clu.end(), std::greater<int>());
-    auto clusters_us = [&](int C, int resident) {  // largest first, each where a place is free first
+    auto clusters_us = [&](int C, int resident, double* sum) {  // largest first, each where a place is free first
         std::vector<double> place(resident, 0.0);
+        *sum = 0.0;
         for (int n : clu) {
             const int q = (n + 31) / 32, turns = (q * (q + 1) / 2 + 2 * C - 1) / (2 * C);
-            *std::min_element(place.begin(), place.end()) += 50.0 + (C == 16 ? 15.5 : 16.5) * q * turns;
+            const double us = 50.0 + (C == 16 ? 15.5 : 16.5) * q * turns;
+            *std::min_element(place.begin(), place.end()) += us;
+            *sum += us;
         }
         return *std::max_element(place.begin(), place.end());
     };
@@ -757,12 +760,19 @@ int sp2_cluster_for(std::vector<int> clu, const std::vector<int>& tiled) {
         const double products = nmax > 1.05 * nmin ? 17.0 : 15.2;  // as many as the channel that needs most
         return tiles ? products * (12.0 + nmax * (0.105 + 0.034 * (per_sm - 1))) : 0.0;
     };
+    // beside channels that take tiles anyway, either form also takes SM time from those: the tiles theirs, the clusters some of
+    // theirs, part of which the tiles leave idle (a serving batch of 40, 12 such channels beside 8 above 448 orbitals, 98.1 ms
+    // with clusters of 16, for which the waves alone speak, 95.4 with clusters of 8)
     int best = 0;
     double least = tiles_us({&clu, &tiled});
+    if (!tiled.empty())
+        for (int n : clu) least += 17.0 * 0.034 * n * ((n + 63) / 64) * ((n + 63) / 64 + 1) / 2 / g_sms;
     for (int k = 0; k < 2; ++k) {
         const int C = k == 0 ? 16 : 8, resident = g_clu_resident[k];
         if (resident < 1) continue;
-        const double us = std::max(clusters_us(C, resident), tiles_us({&tiled}));
+        double sum;
+        const double span = clusters_us(C, resident, &sum);
+        const double us = tiled.empty() ? span : std::max(span, tiles_us({&tiled})) + 0.3 * sum * C / g_sms;
         if (us < least) {
             least = us;
             best = C;
